@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(UmmaCfg<NV>::kThreads) qlinear_umma_kernel(Umm
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   chain_release();  // the next kernel (split-K sum or the step's next operator) may be scheduled already; it waits for this one
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int tile = blockIdx.x, split = blockIdx.y;
   if (gridDim.z > 1) {  // this CTA's chunk of NV vectors: its activations, outputs and partials
     const size_t chunk = blockIdx.z;
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(UmmaCfg<NV>::kThreads) qlinear_umma_kernel(Umm
     tc_fence_before();
   } else if (warp == 4 * kGroups) {
     // ------------------------------------------------------------------ activation loader (one lane)
-    if (lane == 0) {
+    if (elect_one()) {
       chain_wait();  // the activations come from the kernel before this one; weights do not, the dequant warps run ahead
       int issued = 0;
       for (int i = 0; i < nstages; ++i) {
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(UmmaCfg<NV>::kThreads) qlinear_umma_kernel(Umm
     }
   } else {
     // ------------------------------------------------------------------ MMA issuer (one lane)
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       for (int i = 0; i < nstages && ok; ++i) {
         const int s = i % kStages;

@@ -121,6 +121,22 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// One lane of a converged warp, chosen by the hardware. tcgen05.mma must be issued under this predicate inside a branch
+// that is uniform over the warp: its operands then stay in uniform registers. Under `lane == 0` every instruction first
+// moves its descriptors across, which costs 45 to 131 cycles each whatever N is, instead of the N / 2 that the tensor
+// core needs (N = 32: 16 cycles, 128: 64, 256: 128; A in tensor memory, measured on a B200 at 1965 MHz).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t chosen;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(chosen));
+  return chosen != 0;
+}
+// The warp's index as a value the compiler knows to be uniform.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // D[tmem] (+)= A[tmem] * B[smem desc]; accumulate == 0 overwrites D.
 __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
