@@ -1,19 +1,30 @@
-// Next-token sampling on the device, one CTA per logits row: greedy, temperature softmax, top-k and top-p with the
-// splitmix64 draw of crates/runtime/src/sampling.rs:35-42, 80-206.
+// Next-token sampling on the device: temperature softmax, top-k and top-p with the splitmix64 draw of
+// crates/runtime/src/sampling.rs:35-42, 80-206 (the greedy case is argmax_kernel's).
 //
 // The reference orders candidates by (value descending, token ascending), keeps the first top_k, turns them into
 // weights exp((value - max) / temperature), keeps the smallest prefix whose weight reaches top_p x total, and walks that
 // prefix subtracting weights from draw = unit x total until it goes negative. Without top-k and top-p it walks the row in
-// token order instead. Here every candidate gets the 52-bit sort key (order-preserving bits of the f32 logit, then the
-// inverted token), so "the first n candidates", "the smallest prefix reaching a weight" and "the candidate where the walk
-// goes negative" are all the same primitive: a radix select, seven 8-bit digits from the top, over a histogram of counts
-// or of weights. No candidate list is stored and nothing is sorted; a pass re-reads the row (L2 resident) and evaluates
-// exp only for candidates that still match the digits chosen so far. The token-order walk is a block-wide prefix sum over
-// per-thread chunks.
+// token order instead.
 //
-// Sums are f64 like the reference's but associated differently (histogram bins, a tree over threads), so a comparison of
-// a running sum against the draw or the top-p threshold can come out differently only when the two are within about
-// vocab x 2^-52 of each other, relative to the total weight.
+// One row is served by a cluster of 1 to 8 CTAs; every CTA keeps its slice of the logits in shared memory, so HBM (or L2,
+// behind the head projection) is read once. Every candidate has a 52-bit sort key (order-preserving bits of the f32
+// logit, then the inverted token). "The first n candidates", "the smallest prefix reaching a weight" and "the candidate
+// where the walk goes negative" are one primitive: a histogram over 1024 bins of (max - value) / temperature, whose bins
+// are in candidate order, finds the bin in which a running sum crosses its target; that bin's few hundred candidates are
+// gathered into the first CTA, sorted by key and summed in order. A bin that holds more than the list (rows with few
+// distinct values, or everything far below the maximum) is narrowed by 10 bits of the key at a time first. When top_k
+// leaves few enough candidates the list holds all of them and decides everything, and only they are exponentiated.
+// The token-order walk is a prefix sum over the warps' slices and a second look at the one that holds the draw.
+//
+// What bounds it: at 32 rows x 128256 the logits are 16 MB (2.5 us of HBM); the rest is latency, half a dozen passes over
+// shared memory with a cluster barrier (about a microsecond) between them. A single CTA per row that re-read the row for
+// each of 7 radix digits per select, with f64 atomics on 256 bins, took 2192 us with top-k 40 and top-p 0.95; this takes 24.6.
+//
+// Sums are f64 like the reference's but associated differently (histogram bins, scans), so a comparison of a running sum
+// against the draw or the top-p threshold can come out differently only when the two are within about vocab x 2^-52 of
+// each other, relative to the total weight.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "chain.cuh"
@@ -23,7 +34,15 @@ namespace etc {
 
 namespace {
 
-constexpr int kSampleThreads = 1024;
+namespace cg = cooperative_groups;
+
+constexpr int kSampleThreads = 512;
+constexpr int kSampleWarps = kSampleThreads / 32;
+constexpr int kBins = 1024;           // also the digits of a narrowing step (10 bits of the key)
+constexpr int kList = 1024;           // candidates that can be sorted
+constexpr int kMaxSlice = 16384;      // logits a CTA keeps in shared memory (64 KB: two CTAs per SM)
+constexpr int kMaxSampleCluster = 8;  // the portable cluster size
+constexpr int kSliceTarget = 4096;    // a row is spread over more CTAs until a slice is this short
 
 struct SampleArgs {
   const float* logits;
@@ -35,6 +54,8 @@ struct SampleArgs {
   const uint64_t* counters;
   uint32_t* tokens;
   DeviceStatus* status;
+  int slice;   // logits per CTA of the row's cluster
+  int cached;  // the slice is kept in shared memory
 };
 
 __device__ __forceinline__ double random_unit(uint64_t seed, uint64_t counter) {
@@ -46,223 +67,425 @@ __device__ __forceinline__ double random_unit(uint64_t seed, uint64_t counter) {
   return (double)(value >> 11) * (1.0 / 9007199254740992.0);
 }
 
-// Larger logit -> larger key; among equal logits the lower token has the larger key. Tokens are below 2^20.
+// Larger logit -> larger key; among equal logits (0 and -0 are equal) the lower token has the larger key. Tokens are below 2^20.
 __device__ __forceinline__ uint64_t sort_key(float v, uint32_t token) {
-  const uint32_t u = __float_as_uint(v);
+  const uint32_t u = __float_as_uint(__fadd_rn(v, 0.0f));
   const uint32_t ordered = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
   return ((uint64_t)ordered << 20) | (uint64_t)(0xFFFFFu - token);
 }
 __device__ __forceinline__ uint32_t key_token(uint64_t key) { return 0xFFFFFu - (uint32_t)(key & 0xFFFFFu); }
+__device__ __forceinline__ float key_value(uint64_t key) {
+  const uint32_t ordered = (uint32_t)(key >> 20);
+  return __uint_as_float((ordered & 0x80000000u) ? (ordered ^ 0x80000000u) : ~ordered);
+}
 
 struct Shared {
-  double hist[256];
-  uint32_t count[256];
-  double warp_sum[32];
-  unsigned long long warp_key[32];
-  double acc;
-  int digit;
-  int found;
+  double weight[kBins];       // this CTA's bins; in the first CTA afterwards: inclusive sums over the row's bins
+  double sum[kBins];
+  uint32_t count[kBins];
+  uint32_t total_count[kBins];  // first CTA: inclusive counts
+  uint64_t key[kList];          // first CTA: gathered candidates, then sorted
+  double cumulative[kList];
+  double warp_sum[kSampleWarps];
+  long long warp_bad[kSampleWarps];
+  double slice_sum[kSampleWarps];  // token-order walk
+  float best;
+  long long bad;
+  uint32_t listed;
+  int crossing;  // bin or list position a search found
+  // decisions of the first CTA that the others read
+  struct Decision {
+    int bin;              // -1: the running sum never gets there
+    uint32_t in_bin, up_to;  // candidates in the bin, and up to and including it
+    double before;        // running sum ahead of the bin
+    double total;
+    uint64_t picked;
+    double at;            // running sum including `picked`
+  } decision;
 };
 
-__device__ double block_sum(Shared& sh, double v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) sh.warp_sum[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double total = 0.0;
-  for (int w = 0; w < kSampleThreads / 32; ++w) total += sh.warp_sum[w];  // the same order in every thread
-  return total;
-}
-__device__ uint64_t block_min_key(Shared& sh, uint64_t v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    const uint64_t o = __shfl_xor_sync(0xffffffffu, v, off);
-    v = o < v ? o : v;
-  }
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) sh.warp_key[threadIdx.x >> 5] = v;
-  __syncthreads();
-  uint64_t best = ~0ull;
-  for (int w = 0; w < kSampleThreads / 32; ++w) best = sh.warp_key[w] < best ? sh.warp_key[w] : best;
-  return best;
-}
-
 enum Crossing { kReaches = 0, kExceeds = 1 };  // running >= target (counts, top-p) or running > target (the draw)
+__device__ __forceinline__ bool crosses(double running, double target, Crossing c) { return c == kReaches ? running >= target : running > target; }
 
-// Among the candidates with key >= floor_key, in descending key order: the first one at which the running sum of
-// weights (including its own) reaches / exceeds `target`. Returns its key and, in *before, the sum of all candidates
-// ahead of it; found == false when the whole set stays below the target.
-template <typename Weight>
-__device__ uint64_t radix_select(Shared& sh, const float* x, int64_t vocab, uint64_t floor_key, double target, Crossing crossing,
-                                 Weight weight, double* before, bool* found) {
-  uint64_t prefix = 0, mask = 0;
-  double acc = 0.0;
-  bool ok = true;
-  for (int pass = 0; pass < 7 && ok; ++pass) {
-    const int shift = 48 - 8 * pass;
-    __syncthreads();
-    if (threadIdx.x < 256) {
-      sh.hist[threadIdx.x] = 0.0;
-      sh.count[threadIdx.x] = 0u;
+// Which candidates a pass looks at, and in which bin each falls.
+struct Scope {
+  float best, per_unit;   // first level: bins of (max - value) * per_unit
+  int bin = -1;           // >= 0: only that first-level bin, by `shift` bits of the key that match `prefix` above them
+  int shift = 0;
+  uint64_t prefix = 0, mask = 0, floor_key = 0;
+  __device__ __forceinline__ int first_level(float v) const { return (int)fminf((best - v) * per_unit, (float)(kBins - 1)); }
+  // -1: not in scope
+  __device__ __forceinline__ int digit(float v, uint64_t key) const {
+    if (key < floor_key) return -1;
+    const int b = first_level(v);
+    if (bin < 0) return b;
+    if (b != bin || (key & mask) != prefix) return -1;
+    return kBins - 1 - (int)((key >> shift) & (uint64_t)(kBins - 1));  // larger keys first
+  }
+};
+
+struct Row {
+  cg::cluster_group cluster;
+  Shared& sh;
+  Shared& first;     // the first CTA's
+  const float* x;    // this CTA's slice
+  int n;
+  uint32_t token0;
+  double mx, temperature;
+  __device__ double weight_of(float v) const { return exp(((double)v - mx) / temperature); }
+
+  // Inclusive sums of the cluster's bins, in the first CTA. WEIGHTED: of weights too.
+  template <bool WEIGHTED>
+  __device__ void histogram(const Scope& scope) {
+    for (int b = threadIdx.x; b < kBins; b += kSampleThreads) {
+      sh.count[b] = 0u;
+      if (WEIGHTED) sh.weight[b] = 0.0;
     }
     __syncthreads();
-    for (int64_t i = threadIdx.x; i < vocab; i += kSampleThreads) {
+    for (int i = threadIdx.x; i < n; i += kSampleThreads) {
       const float v = x[i];
-      const uint64_t key = sort_key(v, (uint32_t)i);
-      if (key < floor_key || (key & mask) != prefix) continue;
-      const int bin = (int)((key >> shift) & 255u);
-      atomicAdd(&sh.hist[bin], weight(v));
-      atomicAdd(&sh.count[bin], 1u);
+      const int b = scope.digit(v, sort_key(v, token0 + (uint32_t)i));
+      if (b < 0) continue;
+      atomicAdd(&sh.count[b], 1u);
+      if (WEIGHTED) atomicAdd(&sh.weight[b], weight_of(v));
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double running = acc;
-      int digit = -1;
-      for (int b = 255; b >= 0; --b) {
-        if (sh.count[b] == 0u) continue;
-        const double next = running + sh.hist[b];
-        if (crossing == kReaches ? next >= target : next > target) {
-          digit = b;
-          break;
+    cluster.sync();
+    if (cluster.block_rank() == 0) {
+      constexpr int PER = kBins / kSampleThreads;
+      const int b0 = threadIdx.x * PER, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+      uint32_t c[PER] = {};
+      double w[PER] = {};
+      for (unsigned r = 0; r < cluster.num_blocks(); ++r) {
+        const Shared* peer = cluster.map_shared_rank(&sh, r);
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+          c[j] += peer->count[b0 + j];
+          if (WEIGHTED) w[j] += peer->weight[b0 + j];
         }
-        running = next;
       }
-      sh.digit = digit;
-      sh.acc = running;
-    }
-    __syncthreads();
-    if (sh.digit < 0) {
-      ok = false;
-    } else {
-      acc = sh.acc;
-      prefix |= (uint64_t)sh.digit << shift;
-      mask |= 255ull << shift;
+      // counts are exact in f64 too, so one scan over (count, weight) pairs
+      uint32_t cs = 0;
+      double ws = 0.0;
+#pragma unroll
+      for (int j = 0; j < PER; ++j) { c[j] = cs += c[j]; w[j] = ws += w[j]; }
+      uint32_t ci = cs;
+      double wi = ws;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t oc = __shfl_up_sync(0xffffffffu, ci, off);
+        const double ow = __shfl_up_sync(0xffffffffu, wi, off);
+        if (lane >= off) { ci += oc; wi += ow; }
+      }
+      if (lane == 31) { sh.warp_sum[warp] = wi; sh.warp_bad[warp] = ci; }
+      __syncthreads();
+      uint32_t ahead_c = ci - cs;
+      double ahead_w = wi - ws;
+      for (int k = 0; k < warp; ++k) { ahead_c += (uint32_t)sh.warp_bad[k]; ahead_w += sh.warp_sum[k]; }
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        sh.total_count[b0 + j] = ahead_c + c[j];
+        sh.sum[b0 + j] = WEIGHTED ? ahead_w + w[j] : (double)(ahead_c + c[j]);
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) sh.decision.total = sh.sum[kBins - 1];
     }
   }
-  *before = acc;
-  *found = ok;
-  return prefix;
-}
+
+  // First CTA, after histogram(): the bin in which before + running sum crosses the target; the others learn it.
+  __device__ void find_bin(double before, double target, Crossing c) {
+    if (cluster.block_rank() == 0) {
+      if (threadIdx.x == 0) sh.crossing = kBins;
+      __syncthreads();
+      for (int b = threadIdx.x; b < kBins; b += kSampleThreads) {
+        const bool held = sh.total_count[b] != (b > 0 ? sh.total_count[b - 1] : 0u);
+        if (held && crosses(before + sh.sum[b], target, c)) atomicMin(&sh.crossing, b);
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        const int b = sh.crossing;
+        Shared::Decision& d = sh.decision;
+        d.bin = b < kBins ? b : -1;
+        if (b < kBins) {
+          d.up_to = sh.total_count[b];
+          d.in_bin = sh.total_count[b] - (b > 0 ? sh.total_count[b - 1] : 0u);
+          d.before = before + (b > 0 ? sh.sum[b - 1] : 0.0);
+        }
+        sh.listed = 0u;
+      }
+    }
+    cluster.sync();
+  }
+
+  // Candidates of the bins [lo, hi] of the scope, sorted by descending key, in the first CTA's list (at most kList).
+  __device__ void gather(const Scope& scope, int lo, int hi) {
+    for (int i = threadIdx.x; i < n; i += kSampleThreads) {
+      const float v = x[i];
+      const uint64_t key = sort_key(v, token0 + (uint32_t)i);
+      const int b = scope.digit(v, key);
+      if (b < lo || b > hi) continue;
+      const uint32_t at = atomicAdd(&first.listed, 1u);
+      if (at < (uint32_t)kList) first.key[at] = key;
+    }
+    cluster.sync();
+    if (cluster.block_rank() != 0) return;
+    const int m = min((int)sh.listed, kList);
+    int padded = 32;
+    while (padded < m) padded <<= 1;
+    for (int i = m + threadIdx.x; i < padded; i += kSampleThreads) sh.key[i] = 0ull;
+    for (int size = 2; size <= padded; size <<= 1)
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        __syncthreads();
+        for (int p = threadIdx.x; p < padded / 2; p += kSampleThreads) {
+          const int i = 2 * p - (p & (stride - 1)), j = i + stride;
+          const uint64_t a = sh.key[i], b = sh.key[j];
+          if (((i & size) == 0) == (a < b)) { sh.key[i] = b; sh.key[j] = a; }
+        }
+      }
+    __syncthreads();
+  }
+
+  // First CTA: inclusive sums of the first m listed candidates' weights (or of ones).
+  __device__ void accumulate(int m, bool weighted) {
+    constexpr int PER = kList / kSampleThreads;
+    const int i0 = threadIdx.x * PER, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double w[PER], s = 0.0;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      w[j] = s += i0 + j >= m ? 0.0 : (weighted ? weight_of(key_value(sh.key[i0 + j])) : 1.0);
+    }
+    double inclusive = s;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const double o = __shfl_up_sync(0xffffffffu, inclusive, off);
+      if (lane >= off) inclusive += o;
+    }
+    if (lane == 31) sh.warp_sum[warp] = inclusive;
+    __syncthreads();
+    double ahead = inclusive - s;
+    for (int k = 0; k < warp; ++k) ahead += sh.warp_sum[k];
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      if (i0 + j < kList) sh.cumulative[i0 + j] = ahead + w[j];
+    __syncthreads();
+  }
+
+  // First CTA: position of the first of m listed candidates at which before + running sum crosses the target (m: none).
+  __device__ int find_listed(int m, double before, double target, Crossing c) {
+    if (threadIdx.x == 0) sh.crossing = m;
+    __syncthreads();
+    for (int i = threadIdx.x; i < m; i += kSampleThreads)
+      if (crosses(before + sh.cumulative[i], target, c)) atomicMin(&sh.crossing, i);
+    __syncthreads();
+    const int at = sh.crossing;
+    __syncthreads();
+    return at;
+  }
+
+  // The candidate of first-level bin decision.bin at which decision.before + running sum crosses the target, into
+  // decision.picked / at. Rounding may leave the bin's own sum an ulp short of the target: then its last candidate.
+  __device__ void resolve(Scope scope, bool weighted, double target, Crossing c) {
+    int lo = first.decision.bin, hi = lo;
+    double before = first.decision.before;
+    uint32_t held = first.decision.in_bin;
+    for (int level = 0; held > (uint32_t)kList; ++level) {
+      scope.bin = level == 0 ? lo : scope.bin;
+      scope.shift = max(0, 42 - 10 * level);
+      if (weighted) histogram<true>(scope);
+      else histogram<false>(scope);
+      find_bin(before, target, c);
+      lo = first.decision.bin;
+      if (lo < 0) {  // rounding again: the scope's last digit that holds a candidate
+        cluster.sync();  // every CTA has seen that there is none
+        if (cluster.block_rank() == 0 && threadIdx.x == 0) {
+          int b = kBins - 1;
+          while (b > 0 && sh.total_count[b - 1] == sh.total_count[kBins - 1]) --b;
+          sh.decision.bin = b;
+          sh.decision.in_bin = sh.total_count[b] - (b > 0 ? sh.total_count[b - 1] : 0u);
+          sh.decision.before = before + (b > 0 ? sh.sum[b - 1] : 0.0);
+        }
+        cluster.sync();
+        lo = first.decision.bin;
+      }
+      hi = lo;
+      before = first.decision.before;
+      held = first.decision.in_bin;
+      if (held > (uint32_t)kList) {
+        scope.prefix |= (uint64_t)(kBins - 1 - lo) << scope.shift;
+        scope.mask |= (uint64_t)(kBins - 1) << scope.shift;
+      }
+      cluster.sync();  // the decision is read before the next one is written
+    }
+    gather(scope, lo, hi);
+    if (cluster.block_rank() == 0) {
+      const int m = min((int)sh.listed, kList);
+      accumulate(m, weighted);
+      const int at = min(find_listed(m, before, target, c), m - 1);
+      if (threadIdx.x == 0) {
+        sh.decision.picked = sh.key[at];
+        sh.decision.at = before + sh.cumulative[at];
+      }
+    }
+    cluster.sync();
+  }
+};
 
 __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(SampleArgs a) {
+  extern __shared__ __align__(16) float cache[];
   __shared__ Shared sh;
-  const int row = blockIdx.x;
-  const float* x = a.logits + (int64_t)row * a.vocab;
-  const int64_t V = a.vocab;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
+  const int64_t row = blockIdx.x / ranks;
+  const int64_t begin = min(a.vocab, (int64_t)rank * a.slice), end = min(a.vocab, begin + a.slice);
+  const int n = (int)(end - begin), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float* source = a.logits + row * a.vocab + begin;
   // ---- every logit must be finite; the largest one anchors the exponentials
   float best = -INFINITY;
   long long bad = 0x7fffffffffffffffll;
-  for (int64_t i = threadIdx.x; i < V; i += kSampleThreads) {
-    const float v = x[i];
-    if (!isfinite(v)) bad = min(bad, (long long)i);
+  auto see = [&](int i, float v) {
+    if (!isfinite(v)) bad = min(bad, (long long)(begin + i));
     best = fmaxf(best, v);
+  };
+  if (a.cached) {
+    int i = threadIdx.x;
+    for (; i + 3 * kSampleThreads < n; i += 4 * kSampleThreads) {  // four loads in flight
+      float v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = source[i + u * kSampleThreads];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) { cache[i + u * kSampleThreads] = v[u]; see(i + u * kSampleThreads, v[u]); }
+    }
+    for (; i < n; i += kSampleThreads) { const float v = source[i]; cache[i] = v; see(i, v); }
+  } else {
+    for (int i = threadIdx.x; i < n; i += kSampleThreads) see(i, source[i]);
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, off));
     bad = min(bad, __shfl_xor_sync(0xffffffffu, bad, off));
   }
-  if ((threadIdx.x & 31) == 0) {
-    sh.warp_sum[threadIdx.x >> 5] = (double)best;
-    sh.warp_key[threadIdx.x >> 5] = (unsigned long long)bad;
-  }
+  if (lane == 0) { sh.warp_sum[warp] = (double)best; sh.warp_bad[warp] = bad; }
   __syncthreads();
-  double mx = -INFINITY;
-  long long first_bad = 0x7fffffffffffffffll;
-  for (int w = 0; w < kSampleThreads / 32; ++w) {
-    mx = fmax(mx, sh.warp_sum[w]);
-    first_bad = min(first_bad, (long long)sh.warp_key[w]);
+  if (threadIdx.x == 0) {
+    for (int w = 0; w < kSampleWarps; ++w) { best = fmaxf(best, (float)sh.warp_sum[w]); bad = min(bad, sh.warp_bad[w]); }
+    sh.best = best;
+    sh.bad = bad;
+    sh.listed = 0u;
   }
-  if (first_bad != 0x7fffffffffffffffll) {
-    if (threadIdx.x == 0) {
+  cluster.sync();
+  best = -INFINITY;
+  bad = 0x7fffffffffffffffll;
+  for (int r = 0; r < ranks; ++r) {
+    const Shared* peer = cluster.map_shared_rank(&sh, r);
+    best = fmaxf(best, peer->best);
+    bad = min(bad, peer->bad);
+  }
+  if (bad != 0x7fffffffffffffffll) {  // the same answer in every CTA of the row
+    if (rank == 0 && threadIdx.x == 0) {
       a.tokens[row] = 0u;
       if (atomicCAS(&a.status->code, kStatusNone, kStatusNonFiniteLogit) == kStatusNone) {
-        a.status->value = first_bad;
-        a.status->bound = V;
+        a.status->value = bad;
+        a.status->bound = a.vocab;
       }
     }
+    cluster.sync();
     return;
   }
-  const double temperature = a.temperature;
-  auto weight = [mx, temperature](float v) { return exp(((double)v - mx) / temperature); };
+  Row r{cluster, sh, *cluster.map_shared_rank(&sh, 0), a.cached ? cache : source, n, (uint32_t)begin, (double)best, a.temperature};
   const double unit = random_unit(a.seeds ? a.seeds[row] : a.seed, a.counters ? a.counters[row] : a.counter);
-  const bool has_top_k = a.top_k > 0 && a.top_k < V;
+  const bool has_top_k = a.top_k > 0 && a.top_k < a.vocab;
 
   if (!has_top_k && a.top_p >= 1.0) {
-    // ---- walk in token order: per-thread chunks, exclusive prefix over the threads, then the chunk that holds the draw
-    const int64_t chunk = (V + kSampleThreads - 1) / kSampleThreads;
-    const int64_t lo = min(V, (int64_t)threadIdx.x * chunk), hi = min(V, lo + chunk);
+    // ---- walk in token order: every warp sums its part of the slice, then the one that holds the draw walks it
+    const int part = (a.slice + kSampleWarps - 1) / kSampleWarps;
+    const int lo = min(n, warp * part), hi = min(n, lo + part);
     double mine = 0.0;
-    for (int64_t i = lo; i < hi; ++i) mine += weight(x[i]);
-    // inclusive scan inside the warp, then over the warps
-    double scan = mine;
+    for (int i = lo + lane; i < hi; i += 32) mine += r.weight_of(r.x[i]);
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const double o = __shfl_up_sync(0xffffffffu, scan, off);
-      if ((threadIdx.x & 31) >= off) scan += o;
-    }
-    __syncthreads();
-    if ((threadIdx.x & 31) == 31) sh.warp_sum[threadIdx.x >> 5] = scan;
-    if (threadIdx.x == 0) sh.found = 0;
-    __syncthreads();
+    for (int off = 16; off > 0; off >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, off);
+    if (lane == 0) sh.slice_sum[warp] = mine;
+    cluster.sync();
     double ahead = 0.0, total = 0.0;
-    for (int w = 0; w < kSampleThreads / 32; ++w) {
-      if (w < (int)(threadIdx.x >> 5)) ahead += sh.warp_sum[w];
-      total += sh.warp_sum[w];
+    for (int p = 0; p < ranks * kSampleWarps; ++p) {  // the same order in every warp
+      if (p == rank * kSampleWarps + warp) ahead = total;
+      total += cluster.map_shared_rank(&sh, p / kSampleWarps)->slice_sum[p % kSampleWarps];
     }
-    const double exclusive = ahead + scan - mine;
     const double draw = unit * total;
-    if (lo < hi && exclusive <= draw && draw < exclusive + mine) {
-      double left = draw - exclusive;
-      int64_t token = hi - 1;
-      for (int64_t i = lo; i < hi; ++i) {
-        left -= weight(x[i]);
-        if (left < 0.0) {
-          token = i;
-          break;
+    const bool last = end == a.vocab && n > 0 && hi == n && lo < hi;  // the draw can reach the row's end by rounding only
+    if (lo < hi && ahead <= draw && (draw < ahead + mine || last)) {
+      double left = draw - ahead;
+      int token = hi - 1;
+      for (int i0 = lo; i0 < hi; i0 += 32) {
+        double w = i0 + lane < hi ? r.weight_of(r.x[i0 + lane]) : 0.0;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const double o = __shfl_up_sync(0xffffffffu, w, off);
+          if (lane >= off) w += o;
         }
+        const unsigned over = __ballot_sync(0xffffffffu, w > left);
+        if (over) { token = min(hi - 1, i0 + __ffs(over) - 1); break; }
+        left -= __shfl_sync(0xffffffffu, w, 31);
       }
-      a.tokens[row] = (uint32_t)token;
-      sh.found = 1;
+      if (lane == 0) a.tokens[row] = (uint32_t)(begin + token);
     }
-    __syncthreads();
-    if (threadIdx.x == 0 && !sh.found) a.tokens[row] = (uint32_t)(V - 1);
+    cluster.sync();
     return;
   }
 
   // ---- filtered: candidates in (value descending, token ascending) order
-  uint64_t floor_key = 0;  // the retained set is {key >= floor_key}
-  double before;
-  bool found;
+  Scope scope;
+  scope.best = best;
+  scope.per_unit = fminf((float)(32.0 / a.temperature), 1e30f);  // bins of 1/32 in the logarithm of the weight, the last one open
   if (has_top_k) {
-    auto one = [](float) { return 1.0; };
-    floor_key = radix_select(sh, x, V, 0, (double)a.top_k, kReaches, one, &before, &found);  // the top_k-th candidate: always found
+    r.histogram<false>(scope);
+    r.find_bin(0.0, (double)a.top_k, kReaches);
+    if (r.first.decision.up_to <= (uint32_t)kList) {
+      // ---- few enough: the list decides everything
+      r.gather(scope, 0, r.first.decision.bin);
+      if (rank != 0) return;
+      const int k = (int)a.top_k;
+      r.accumulate(k, true);
+      int kept = k;
+      double total = sh.cumulative[k - 1];
+      if (a.top_p < 1.0) {
+        const int at = r.find_listed(k, 0.0, a.top_p * total, kReaches);
+        if (at < k) { kept = at + 1; total = sh.cumulative[at]; }  // otherwise every candidate stays
+      }
+      const int at = min(r.find_listed(kept, 0.0, unit * total, kExceeds), kept - 1);
+      if (threadIdx.x == 0) a.tokens[row] = key_token(sh.key[at]);
+      return;
+    }
+    r.resolve(scope, false, (double)a.top_k, kReaches);
+    scope.floor_key = r.first.decision.picked;
+    cluster.sync();
   }
-  double mine = 0.0;
-  for (int64_t i = threadIdx.x; i < V; i += kSampleThreads)
-    if (sort_key(x[i], (uint32_t)i) >= floor_key) mine += weight(x[i]);
-  double total = block_sum(sh, mine);
+  r.histogram<true>(scope);
+  cluster.sync();  // the first CTA's total
+  double total = r.first.decision.total;
   if (a.top_p < 1.0) {
-    const uint64_t last = radix_select(sh, x, V, floor_key, a.top_p * total, kReaches, weight, &before, &found);
-    if (found) {  // the prefix ends at this candidate; otherwise every candidate stays
-      floor_key = last;
-      total = before + weight(x[key_token(last)]);
+    r.find_bin(0.0, a.top_p * total, kReaches);
+    if (r.first.decision.bin >= 0) {
+      const bool narrowed = r.first.decision.in_bin > (uint32_t)kList;
+      r.resolve(scope, true, a.top_p * total, kReaches);
+      scope.floor_key = r.first.decision.picked;
+      total = r.first.decision.at;
+      if (narrowed) r.histogram<true>(scope);  // the narrowing steps took the first-level sums' place
     }
+    cluster.sync();
   }
-  const uint64_t picked = radix_select(sh, x, V, floor_key, unit * total, kExceeds, weight, &before, &found);
-  uint32_t token;
-  if (found) {
-    token = key_token(picked);
-  } else {  // the walk never went negative: the last retained candidate
-    uint64_t lowest = ~0ull;
-    for (int64_t i = threadIdx.x; i < V; i += kSampleThreads) {
-      const uint64_t key = sort_key(x[i], (uint32_t)i);
-      if (key >= floor_key && key < lowest) lowest = key;
+  r.find_bin(0.0, unit * total, kExceeds);
+  if (r.first.decision.bin < 0) {  // the walk never went negative: the last retained candidate, in the last bin that holds one
+    cluster.sync();
+    if (rank == 0 && threadIdx.x == 0) {
+      int b = kBins - 1;
+      while (b > 0 && sh.total_count[b - 1] == sh.total_count[kBins - 1]) --b;
+      sh.decision.bin = b;
+      sh.decision.in_bin = sh.total_count[b] - (b > 0 ? sh.total_count[b - 1] : 0u);
+      sh.decision.before = b > 0 ? sh.sum[b - 1] : 0.0;
     }
-    token = key_token(block_min_key(sh, lowest));
+    cluster.sync();
   }
-  if (threadIdx.x == 0) a.tokens[row] = token;
+  r.resolve(scope, true, unit * total, kExceeds);
+  if (rank == 0 && threadIdx.x == 0) a.tokens[row] = key_token(sh.decision.picked);
 }
 
 }  // namespace
@@ -271,9 +494,24 @@ cudaError_t launch_sample_rows(const float* logits, int64_t rows, int64_t vocab,
                                uint64_t seed, uint64_t counter, const uint64_t* seeds, const uint64_t* counters, uint32_t* tokens,
                                DeviceStatus* status, cudaStream_t stream) {
   if (rows == 0) return cudaSuccess;
-  SampleArgs a{logits, vocab, temperature, top_p, top_k, seed, counter, seeds, counters, tokens, status};
-  sample_rows_kernel<<<(unsigned)rows, kSampleThreads, 0, stream>>>(a);
-  return cudaGetLastError();
+  int ranks = 1;
+  while (ranks < kMaxSampleCluster && (vocab + ranks - 1) / ranks > kSliceTarget) ranks *= 2;
+  const int slice = (int)((vocab + ranks - 1) / ranks);
+  SampleArgs a{logits, vocab, temperature, top_p, top_k, seed, counter, seeds, counters, tokens, status, slice, slice <= kMaxSlice};
+  const cudaError_t attr = opt_in_shared_memory(sample_rows_kernel, kMaxSlice * sizeof(float));
+  if (attr != cudaSuccess) return attr;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3((unsigned)(rows * ranks));
+  config.blockDim = dim3(kSampleThreads);
+  config.dynamicSmemBytes = a.cached ? (size_t)slice * sizeof(float) : 0;
+  config.stream = stream;
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeClusterDimension;
+  attribute[0].val.clusterDim.x = (unsigned)ranks;
+  attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, sample_rows_kernel, a);
 }
 
 }  // namespace etc

@@ -126,6 +126,43 @@ def test_device_sampling_agrees_with_the_reference_rule_on_many_draws(vocab):
         np.testing.assert_array_equal(got, want, err_msg=str(mode))
 
 
+@pytest.mark.parametrize("vocab", [4097, 16385, 131073, 200001])
+def test_device_sampling_at_the_edges_of_its_slices_and_lists(vocab):
+    """One more logit than a CTA's slice holds, rows whose slices stay in global memory, and candidate sets larger than the
+    sorted list: few distinct values, almost everything far below the maximum, top_k above the list's length."""
+    rt = runtime()
+    rng = np.random.default_rng(vocab)
+    rows = 6
+    logits = (rng.normal(size=(rows, vocab)) * 3.0).astype(np.float32)
+    logits[1] = np.round(logits[1] / 4.0)
+    logits[2] = -1.5
+    logits[3] = rng.normal(size=vocab) * 1e-3
+    logits[3, vocab - 1] = 60.0
+    logits[4] *= -1e30
+    d = dev(logits)
+    seeds = rng.integers(0, 2**63, size=rows, dtype=np.uint64)
+    d_seeds = dev(seeds)
+    tokens = empty(rows, dtype=torch.int32)
+    for mode in (dict(temperature=1.0), dict(temperature=0.8, top_k=40, top_p=0.95), dict(temperature=1.2, top_p=0.6), dict(temperature=1.0, top_k=2000),
+                 dict(temperature=0.7, top_k=3000, top_p=0.9), dict(temperature=1e-3, top_p=0.999999), dict(temperature=50.0, top_p=0.9999999)):
+        for counter in range(3):
+            rt.sample_rows_into(d, rows, vocab, tokens, seeds=d_seeds, counter=counter, **mode)
+            want = [orc.sample_logits(logits[r], seed=int(seeds[r]), counter=counter, **mode) for r in range(rows)]
+            np.testing.assert_array_equal(host(tokens), want, err_msg=str(mode))
+
+
+@pytest.mark.parametrize("vocab", [1, 8192, 8195, 40000, 65541])
+def test_argmax_across_the_slices_of_a_row(vocab):
+    rng = np.random.default_rng(vocab)
+    logits = rng.normal(size=(5, vocab)).astype(np.float32)
+    logits[1, -1] = 9.0
+    logits[2, vocab // 2] = logits[2, vocab - 1] = 9.0
+    logits[3] = 1.0
+    tokens = empty(5, dtype=torch.int32)
+    runtime().argmax_into(dev(logits), 5, vocab, tokens)
+    np.testing.assert_array_equal(host(tokens), [orc.argmax(r) for r in logits])
+
+
 def test_device_sampling_reports_bad_arguments_and_non_finite_logits_like_the_reference():
     rt = runtime()
     logits = np.zeros((2, 64), dtype=np.float32)
