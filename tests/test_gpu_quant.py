@@ -83,6 +83,35 @@ def test_generic_linear_matches_the_oracle(codec, vectors):
     assert helpers.rel_err(host(out), expected) <= REL_TOL
 
 
+@pytest.mark.parametrize("codec", ALL_CODECS)
+@pytest.mark.parametrize("rows,windows,vectors", [(1, 1, 1), (9, 17, 2), (33, 5, 6), (4099, 9, 4), (70, 70, 9)])
+def test_raw_kernels_at_the_edges_of_their_tiles(codec, rows, windows, vectors):
+    """Rows that do not fill a warp, columns that end inside a 256-value window, several staged chunks, a second pass over the
+    vectors; and decoding of value counts that do not fill a warp's four windows, at a 2-byte-aligned address."""
+    rng = np.random.default_rng(7 * codec + rows)
+    columns = windows * 256 if orc.block_values(codec) == 256 else windows * 256 - 96
+    packed = random_packed(codec, rows, columns, seed=rows + codec)
+    x = rng.normal(size=(vectors, columns)).astype(np.float32)
+    out = empty((vectors, rows))
+    runtime().qlinear_into(codec, dev(x), vectors, columns, dev(packed), rows, None, out)
+    expected = x.astype(np.float64) @ orc.dequantize(codec, packed, rows, columns).astype(np.float64).T
+    assert np.abs(host(out) - expected).max() <= 2e-6 * np.sqrt(columns) * np.abs(expected).max()
+    shifted = dev(np.concatenate([np.zeros(2, np.uint8), packed.reshape(-1)]))
+    decoded = empty((rows, columns))
+    runtime().dequantize_into(codec, shifted[2:], rows, columns, decoded)
+    np.testing.assert_array_equal(host(decoded).view(np.uint32), orc.dequantize(codec, packed, rows, columns).view(np.uint32))
+
+
+@pytest.mark.parametrize("codec", [gv.Q4_0, gv.Q8_0])
+@pytest.mark.parametrize("rows,columns", [(1, 32), (5, 1600), (255, 32), (257, 96)])
+def test_quantizer_tails(codec, rows, columns):
+    w = np.random.default_rng(rows).normal(0, 0.02, size=(rows, columns)).astype(np.float32)
+    w[0, 3] = -w[0, 17]  # equal magnitudes: the first decides the sign
+    packed = empty((rows, orc.encoded_row_bytes(codec, columns)), dtype=torch.uint8)
+    runtime().quantize_into(codec, dev(w), rows, columns, packed)
+    np.testing.assert_array_equal(host(packed), orc.quantize(codec, w))
+
+
 def test_linear_rejects_bad_geometry_and_observes_cancellation():
     rt = runtime()
     x, w, out = empty((1, 256)), empty((1, 144), dtype=torch.uint8), empty((1, 1))
