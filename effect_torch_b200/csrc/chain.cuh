@@ -17,19 +17,28 @@ namespace etc {
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// `cluster` CTAs along x form a thread-block cluster (1: none).
 template <typename... KernelArgs, typename... Args>
-inline cudaError_t launch_chained(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+inline cudaError_t launch_chained_cluster(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, unsigned cluster,
+                                          Args&&... args) {
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
   config.blockDim = block;
   config.dynamicSmemBytes = smem;
   config.stream = stream;
-  cudaLaunchAttribute attribute[1];
+  cudaLaunchAttribute attribute[2];
   attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute[0].val.programmaticStreamSerializationAllowed = 1;
+  attribute[1].id = cudaLaunchAttributeClusterDimension;
+  attribute[1].val.clusterDim.x = cluster;
+  attribute[1].val.clusterDim.y = attribute[1].val.clusterDim.z = 1;
   config.attrs = attribute;
-  config.numAttrs = 1;
+  config.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+}
+template <typename... KernelArgs, typename... Args>
+inline cudaError_t launch_chained(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_chained_cluster(kernel, grid, block, smem, stream, 1, std::forward<Args>(args)...);
 }
 
 // Opts a kernel in to `bytes` of dynamic shared memory once per (kernel, device): the attribute belongs to the function
