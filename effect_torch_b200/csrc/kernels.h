@@ -63,26 +63,41 @@ struct RepackParts {
 };
 cudaError_t launch_repack(const TiledWeight& w, const RepackParts& parts, cudaStream_t stream);
 
-// out_xh (optional): the result also stored as f16 in [cols/8][xh_nv][8] order for the next linear.
+// Sums split-K partials [splits][vpad][rows_padded] in split order and runs the epilogue.
 cudaError_t launch_qlinear_reduce(const float* scratch, int splits, int vpad, int vectors, int rows, int rows_padded,
-                                  const float* bias, const float* residual, int epilogue, float* out, __half* out_xh,
-                                  cudaStream_t stream, int xh_nv = 32);
+                                  const float* bias, const float* residual, int epilogue, float* out, cudaStream_t stream);
 
-// tcgen05 path (qlinear_umma.cu)
+// decode batches up to stream_max_vectors() (qlinear_stream.cu)
+struct StreamPlan {
+  int nv = 32;                  // vectors padded to the MMA N (32, 64 or 128)
+  int tiles = 1, stages = 1;    // 128-row tiles, stages of four 32-value blocks per tile
+  int splits = 1, stages_per_split = 1;  // CTAs that share a tile's K: a cluster, or with `deferred` writers of partial sums
+  bool deferred = false;
+  size_t xh_bytes = 0;          // f16 activations, at the head of the scratch (rounded to 256 bytes)
+  size_t scratch_bytes = 0;     // partial sums behind them
+};
+StreamPlan plan_stream(const TiledWeight& w, int64_t vectors, int sm_count, bool deferred);
+int stream_max_vectors();
+size_t stream_scratch_bytes(const TiledWeight& w, int64_t vectors, int sm_count);
+// x f32 [vectors, K], or xh_ready in the f16 hand-off layout with row stride xh_nv.
+cudaError_t launch_qlinear_stream(const TiledWeight& w, const float* x, const __half* xh_ready, int64_t vectors, const float* bias,
+                                  const float* residual, int epilogue, float* out, __half* out_xh, void* scratch, DeviceStatus* status,
+                                  int sm_count, cudaStream_t stream, int* launches, int xh_nv = 32, DeferredSum* defer = nullptr);
+
+// prefill and large batches (qlinear_umma.cu)
 struct UmmaPlan {
-  int nv = 32;               // vectors per chunk padded to the MMA N (32, 64, 128 or 256)
-  int chunks = 1;            // chunks of nv vectors the call is cut into (grid.z); more than one only at nv = 256
+  int nv = 256;              // vectors per chunk (the MMA N)
+  int chunks = 1;            // chunks the call is cut into (grid.z)
   int tiles = 1, splits = 1, blocks_per_split = 0;
   size_t xh_bytes = 0;       // f16 activations in [chunk][K/8][nv][8] order, all chunks
   size_t scratch_bytes = 0;  // split-K partials [chunk][split][nv][rows_padded], all chunks
 };
 UmmaPlan plan_umma(const TiledWeight& w, int64_t vectors, int sm_count);
 cudaError_t launch_repack_umma(const TiledWeight& w, const RepackParts& parts, cudaStream_t stream);
-// x: f32 [vectors, K], converted to xh8 into `xh` first — unless xh_ready (already [K/8][32][8] f16, vectors <= 32) is given.
-cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, const __half* xh_ready, int64_t vectors, const float* bias,
-                                const float* residual, int epilogue, float* out, __half* out_xh, __half* xh, float* scratch,
-                                DeviceStatus* status, int sm_count, cudaStream_t stream, int* launches, int xh_nv = 32,
-                                DeferredSum* defer = nullptr);
+// x: f32 [vectors, K], converted to f16 in xh first.
+cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, int64_t vectors, const float* bias, const float* residual, int epilogue,
+                                float* out, __half* xh, float* scratch, DeviceStatus* status, int sm_count, cudaStream_t stream,
+                                int* launches);
 
 // small-batch matvec on the 128-row layout (qlinear_mv.cu): up to 32 vectors per pass, mma.sync fed by a bulk-copy ring
 struct MvPlan {

@@ -1,0 +1,478 @@
+// Dequant linear for decode batches (up to 128 vectors) on the 5th-generation tensor cores, streaming weights at HBM rate.
+//
+//   out[v, r] = sum_k x[v, k] * deq(W[r, k])        (quantized_linear, crates/runtime-cpu/src/quantized.rs:419-499)
+//
+// The 128 rows of a layout tile are the A operand of tcgen05.mma.kind::f16 (M = 128, N = NV, K = 16) in tensor memory; the
+// NV input vectors are the B operand in shared memory, in the canonical K-major layout the producer already stored
+// ([K/8][NV][8] f16). A CTA does one tile, or a range of its K, with eleven warps:
+//   * weight loader: bulk copies (cp.async.bulk, completion counted in bytes on an mbarrier) of the packed weights and block
+//     scales of a stage (128 rows x 128 columns) into a deep shared-memory ring. Weights depend on no earlier kernel, so
+//     under programmatic dependent launch the whole ring is requested while the previous kernel still runs.
+//   * activation loader: the stage's B operand, one bulk copy, after the grid dependency wait.
+//   * two groups of four dequant warps (stages alternate): a thread owns one TMEM lane = one weight row, reads 16 payload
+//     bytes per 32-value block from the ring, expands to f16, scales and stores 16 TMEM columns per block.
+//   * MMA warp: one elected lane issues 8 MMAs per stage (N / 2 cycles each); tcgen05.commit frees the stage's buffers.
+// Two CTAs share an SM (half the shared memory, 256 TMEM columns each), so that one expands while the other starts, waits
+// or stores; a CTA of the next launch can take the place of one that has ended and fill its ring under this launch's tail.
+//
+// Split over K. Deferred sums: grid (splits, tiles), partial sums to memory, added up by the kernel that consumes them.
+// Otherwise the CTAs of a tile form a cluster: each puts its accumulator into its shared memory, and after a cluster
+// barrier every CTA adds up, in rank order, its share of the vectors from all of them and runs the epilogue. (Equal runs
+// of (tile, stage) units with the pieces of cut tiles exchanged through memory and a ticket per tile took 10 to 17 us for
+// the exchange on [28672 x 4096] and [4096 x 4096]: a fence, an atomic and a chain of L2 round trips.)
+//
+// Roofline: HBM, rows*K/32*{18,34} bytes. Expanding a weight takes about 1.7 instructions, so at 39.5 Q4_0 weights per cycle
+// per SM (the HBM rate) the SM issues 2 of its 4 instructions per cycle. Measured alone at 32 vectors with the conversion of
+// f32 activations, before (register-fed dequant warps, MMAs issued at 131 cycles each) and now: [28672 x 4096] 38.8 -> 23.5
+// us, [4096 x 14336] 21.9 -> 17, [4096 x 4096] 12.4 -> 9.4, [128256 x 4096] 118 -> 73.5 (0.61 of the copy bandwidth; Q8_0
+// 123 -> 101, 0.85). In the steady state an SM with two CTAs does a stage in 440 cycles (HBM: 415); what is left is the
+// start of a launch (3 us to the first MMA), the uneven last tiles and the epilogue.
+//
+// Every mbarrier wait is bounded: on expiry the abort flag and the status word (3) are raised, all roles run dry, copies
+// in flight are awaited, TMEM is freed.
+#include <cooperative_groups.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <type_traits>
+
+#include "chain.cuh"
+#include "dequant.cuh"
+#include "kernels.h"
+
+namespace etc {
+
+namespace {
+
+namespace cg = cooperative_groups;
+using namespace tc05;
+
+constexpr int kRows = 128;       // of a layout tile
+constexpr int kStageBlocks = 4;  // 32-value blocks per stage
+constexpr int kDequantGroups = 2;
+constexpr int kWeightWarp = 4 * kDequantGroups, kMmaWarp = kWeightWarp + 1, kActivationWarp = kMmaWarp + 1;
+constexpr int kMaxStreamCluster = 8;  // the portable size
+constexpr int kStreamThreads = (kActivationWarp + 1) * 32;
+
+template <int CODEC, int NV>
+struct StreamCfg {
+  static constexpr bool kNibbles = CODEC == 2 || CODEC == 12;
+  static constexpr bool kPair = CODEC >= 12;  // two f16 per (row, block): (scale, min) or the two half-block scales
+  static constexpr uint32_t kBlockQ = kNibbles ? 2048 : 4096;
+  static constexpr uint32_t kBlockS = kPair ? 512 : 256;
+  static constexpr uint32_t kStageQ = kStageBlocks * kBlockQ;
+  static constexpr uint32_t kStageW = kStageBlocks * (kBlockQ + kBlockS);
+  static constexpr uint32_t kStageB = NV * kStageBlocks * 64;
+  static constexpr int kSlots = NV <= 32 ? 3 : 2;  // expanded stages in TMEM
+  static constexpr int kStagesB = NV <= 32 ? (kNibbles ? 6 : 4) : (NV <= 64 && kNibbles ? 3 : 2);
+  // a whole number of stages per dequant group: a ring buffer then belongs to one group, whose own previous round is what
+  // tells two phases of the buffer's barrier apart (copies of neighbouring stages may land in either order)
+  static constexpr int kStagesW = (int)((104u * 1024 - kStagesB * kStageB) / kStageW) / kDequantGroups * kDequantGroups;
+  static constexpr uint32_t kTmemCols = 256;
+  static constexpr int kDone = kStagesB > kSlots ? kStagesB : kSlots;  // barriers on which the MMAs of a stage report
+  static constexpr int kBars = 2 * kStagesW + kStagesB + kSlots + kDone + 1;
+  static constexpr size_t kSmemBytes = (size_t)kStagesB * kStageB + (size_t)kStagesW * kStageW + kBars * sizeof(uint64_t) + 32;
+  static_assert(NV + kSlots * kStageBlocks * 16 <= (int)kTmemCols, "tensor memory of half an SM");
+  static_assert(kStagesW >= kDequantGroups, "ring");
+  static_assert(kSmemBytes <= 112 * 1024, "two CTAs per SM");
+  static_assert((size_t)NV * kRows * sizeof(float) <= (size_t)kStagesB * kStageB + (size_t)kStagesW * kStageW, "the accumulator fits the rings");
+};
+
+struct StreamArgs {
+  const unsigned char* quants;  // [tile][kblock][128 rows][16 B] or 8-bit codes [tile][kblock][128 rows][32 B]
+  const unsigned char* scales;  // [tile][kblock][128] f16 or f16 pairs
+  const __half* xh;             // [K/8][NV][8] f16
+  const float* bias;
+  const float* residual;
+  float* out;
+  float* scratch;               // deferred sums: [splits][NV][rows_padded]
+  unsigned long long* status;
+  __half* out_xh;               // optional: the result also as f16 [cols/8][out_xh_nv][8] for the next linear
+  int out_xh_nv;
+  int vectors, rows, rows_padded, kblocks, epilogue;
+  int tile0;                    // first tile of this launch in the output (a segment of a weight fused from several codecs)
+  int stages, stages_per_split; // of a tile; of a CTA
+  int deferred;                 // partial sums only
+  Splice splice;
+};
+
+__device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+__device__ __forceinline__ float sat16(float v) { return fminf(fmaxf(v, -65504.f), 65504.f); }
+__device__ __forceinline__ uint2 pack4(const float4& v) {
+  return make_uint2(h2u(__floats2half2_rn(sat16(v.x), sat16(v.y))), h2u(__floats2half2_rn(sat16(v.z), sat16(v.w))));
+}
+
+// Four consecutive values of an output row: columns c .. c + 3 of vector v, the first `n` of them inside the row.
+__device__ __forceinline__ void store4(const StreamArgs& a, int v, int c, int n, int out_cols, const float4& val) {
+  if (a.out) {
+    float* dst = a.out + (size_t)v * out_cols + c;
+    if (n == 4 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+      *reinterpret_cast<float4*>(dst) = val;
+    } else {
+      dst[0] = val.x;
+      if (n > 1) dst[1] = val.y;
+      if (n > 2) dst[2] = val.z;
+      if (n > 3) dst[3] = val.w;
+    }
+  }
+  if (a.out_xh) *reinterpret_cast<uint2*>(a.out_xh + ((size_t)(c >> 3) * a.out_xh_nv + v) * 8 + (c & 7)) = pack4(val);
+}
+
+template <int CODEC, int NV>
+__global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(StreamArgs a) {
+  using Cfg = StreamCfg<CODEC, NV>;
+  constexpr int WS = Cfg::kStagesW, BS = Cfg::kStagesB, AS = Cfg::kSlots, DONE = Cfg::kDone;
+  constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(NV >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);  // f16 x f16 -> f32
+  extern __shared__ __align__(128) unsigned char smem[];
+  unsigned char* b_ring = smem;
+  unsigned char* w_ring = smem + BS * Cfg::kStageB;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(w_ring + WS * Cfg::kStageW);
+  // `done[i % DONE]` completes when the MMAs of stage i have read its operands: one commit frees both the TMEM slot and the
+  // activation buffer, whose owners wait for the stage that used them last (at most DONE stages back)
+  uint64_t *w_full = bars, *w_empty = w_full + WS, *b_full = w_empty + WS, *a_full = b_full + BS;
+  uint64_t *done = a_full + AS, *d_full = done + DONE;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(d_full + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
+
+  chain_release();  // the next kernel of the stream may be scheduled already; it waits for this one
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
+  const int split = blockIdx.x, tile = blockIdx.y;
+  const int s0 = split * a.stages_per_split, n = min(a.stages, s0 + a.stages_per_split) - s0;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < WS; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], 4); }
+    for (int i = 0; i < BS; ++i) mbar_init(&b_full[i], 1);
+    for (int i = 0; i < AS; ++i) mbar_init(&a_full[i], 4);
+    for (int i = 0; i < DONE; ++i) mbar_init(&done[i], 1);
+    mbar_init(d_full, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kMmaWarp) tmem_alloc(tmem_holder, Cfg::kTmemCols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_holder;         // the accumulator at columns [0, NV), then the expanded stages
+  const uint32_t a_tmem = tmem + NV;
+
+  if (warp < kWeightWarp) {
+    // ------------------------------------------------------------------ dequant warps
+    const int group = warp >> 2, row = (warp & 3) * 32 + lane;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    Ring<WS> w;
+    Ring<AS> slot;
+    Ring<DONE> freed;  // the stage AS before this one
+    w.skip(group);
+    slot.skip(group);
+    int behind = group - AS;
+    const unsigned char* payload = w_ring + row * (Cfg::kBlockQ / kRows);
+    const unsigned char* scales = w_ring + Cfg::kStageQ + row * (Cfg::kBlockS / kRows);
+    const Splice splice = a.splice;
+    bool ok = true;
+    for (int i = group; i < n && ok; i += kDequantGroups) {
+      ok = wait_warp(&w_full[w.at], w.parity, abort_flag) && (behind < 0 || wait_warp(&done[freed.at], freed.parity, abort_flag));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t stage = (uint32_t)w.at * Cfg::kStageW;
+#pragma unroll
+      for (int b = 0; b < kStageBlocks; ++b) {  // blocks beyond the tile's K hold stale bytes that no MMA reads
+        uint32_t regs[16];
+        expand_block<CODEC>(payload + stage + b * Cfg::kBlockQ, scales + stage + b * Cfg::kBlockS, splice, regs);
+        tmem_st16(a_tmem + lane_base + (uint32_t)(slot.at * kStageBlocks * 16 + b * 16), regs);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&w_empty[w.at]);
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&a_full[slot.at]);
+      w.skip(kDequantGroups);
+      slot.skip(kDequantGroups);
+      if (behind >= 0) freed.skip(kDequantGroups);
+      else if (behind + kDequantGroups > 0) freed.skip(behind + kDequantGroups);
+      behind += kDequantGroups;
+    }
+    // ------------------------------------------------------------------ accumulator out of TMEM (half of it per group)
+    chain_wait();  // outputs, residual and scratch may still be in use by the kernel before this one
+    if (wait_warp(d_full, 0, abort_flag)) {
+      tc_fence_after();
+      const int r = (a.tile0 + tile) * kRows + row;
+      // to the consumer's partial sums, or to this CTA's shared memory (the rings are free: every stage has been read)
+      float* dst = a.deferred ? a.scratch + (size_t)split * NV * a.rows_padded + r : reinterpret_cast<float*>(smem) + row;
+      const size_t stride = a.deferred ? a.rows_padded : kRows;
+#pragma unroll 1
+      for (int v0 = group * 16; v0 < NV && v0 < a.vectors; v0 += 16 * kDequantGroups) {
+        uint32_t acc[16];
+        tmem_ld16(tmem + lane_base + (uint32_t)v0, acc);
+        tmem_wait_ld();
+#pragma unroll
+        for (int v = 0; v < 16; ++v) dst[(size_t)(v0 + v) * stride] = __uint_as_float(acc[v]);
+      }
+    }
+  } else if (warp == kWeightWarp) {
+    // ------------------------------------------------------------------ weight loader (one lane)
+    if (elect_one()) {
+      Ring<WS> w;
+      int issued = 0;
+      for (int i = 0; i < n; ++i) {
+        if (!mbar_wait(&w_empty[w.at], w.parity ^ 1u, abort_flag)) break;
+        const int kb = (s0 + i) * kStageBlocks;
+        const uint32_t valid = (uint32_t)min(kStageBlocks, a.kblocks - kb);
+        const size_t block = (size_t)tile * a.kblocks + kb;
+        unsigned char* dst = w_ring + (size_t)w.at * Cfg::kStageW;
+        mbar_arrive_expect_tx(&w_full[w.at], valid * (Cfg::kBlockQ + Cfg::kBlockS));
+        bulk_copy_g2s(dst, a.quants + block * Cfg::kBlockQ, valid * Cfg::kBlockQ, &w_full[w.at]);
+        bulk_copy_g2s(dst + Cfg::kStageQ, a.scales + block * Cfg::kBlockS, valid * Cfg::kBlockS, &w_full[w.at]);
+        issued = i + 1;
+        w.next();
+      }
+      if (*abort_flag)  // give up: this warp's own copies land (bounded) before shared memory is released
+        for (int i = max(0, issued - WS); i < issued; ++i)
+          for (unsigned spin = 0; spin < (1u << 20) && !mbar_try_wait(&w_full[i % WS], (uint32_t)(i / WS) & 1u); ++spin) __nanosleep(64);
+    }
+  } else if (warp == kActivationWarp) {
+    // ------------------------------------------------------------------ activation loader (one lane)
+    if (elect_one()) {
+      chain_wait();  // the activations come from the kernel before this one
+      Ring<BS> b;
+      Ring<DONE> freed;  // the stage BS before this one
+      int issued = 0;
+      for (int i = 0; i < n; ++i) {
+        if (i >= BS) {
+          if (!mbar_wait(&done[freed.at], freed.parity, abort_flag)) break;
+          freed.next();
+        }
+        const int kb = (s0 + i) * kStageBlocks;
+        const uint32_t bytes = (uint32_t)min(kStageBlocks, a.kblocks - kb) * 4u * NV * 16u;
+        mbar_arrive_expect_tx(&b_full[b.at], bytes);
+        bulk_copy_g2s(b_ring + (size_t)b.at * Cfg::kStageB, a.xh + (size_t)kb * 4 * NV * 8, bytes, &b_full[b.at]);
+        issued = i + 1;
+        b.next();
+      }
+      if (*abort_flag)
+        for (int i = max(0, issued - BS); i < issued; ++i)
+          for (unsigned spin = 0; spin < (1u << 20) && !mbar_try_wait(&b_full[i % BS], (uint32_t)(i / BS) & 1u); ++spin) __nanosleep(64);
+    }
+  } else {
+    // ------------------------------------------------------------------ MMA issuer (one lane)
+    if (elect_one()) {
+      Ring<BS> b;
+      Ring<AS> slot;
+      Ring<DONE> report;
+      bool ok = true;
+      const uint64_t desc0 = make_b_desc(smem_u32(b_ring), NV * 16u, 128u);
+      for (int i = 0; i < n && ok; ++i) {
+        ok = mbar_wait(&b_full[b.at], b.parity, abort_flag) && mbar_wait(&a_full[slot.at], slot.parity, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        const int valid = min(kStageBlocks, a.kblocks - (s0 + i) * kStageBlocks);
+        // two K = 16 instructions per block: two column groups of B, 8 TMEM columns of A each. Whole stages are unrolled:
+        // with constant steps the operands stay in uniform registers (58 cycles per instruction in a loop, 16 unrolled)
+        const uint64_t desc = desc0 + (uint64_t)(b.at * (int)(Cfg::kStageB / 16));
+        const uint32_t a_cols = a_tmem + (uint32_t)(slot.at * kStageBlocks * 16);
+        umma_ts(tmem, a_cols, desc, kIdesc, i > 0 ? 1u : 0u);
+        if (valid == kStageBlocks) {
+#pragma unroll
+          for (int j = 1; j < 2 * kStageBlocks; ++j) umma_ts(tmem, a_cols + 8u * j, desc + 2u * NV * j, kIdesc, 1u);
+        } else {
+          for (int j = 1; j < 2 * valid; ++j) umma_ts(tmem, a_cols + 8u * j, desc + 2u * NV * j, kIdesc, 1u);
+        }
+        tc_commit(&done[report.at]);
+        b.next();
+        slot.next();
+        report.next();
+      }
+      if (ok) tc_commit(d_full);
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  if (!a.deferred) {
+    // ------------------------------------------------------------------ the tile's CTAs add up and finish
+    cg::cluster_group cluster = cg::this_cluster();
+    if (gridDim.x > 1) cluster.sync();
+    else __syncthreads();
+    if (!*abort_flag) {
+      chain_wait();
+      const int ranks = gridDim.x, per = (a.vectors + ranks - 1) / ranks;  // this CTA's share of the vectors
+      const int v_lo = split * per, v_hi = min(a.vectors, v_lo + per);
+      const int row0 = (a.tile0 + tile) * kRows;
+      auto sum4 = [&](int v, int quad) {
+        const float* mine = reinterpret_cast<const float*>(smem) + v * kRows + 4 * quad;
+        float4 sum = *reinterpret_cast<const float4*>(ranks == 1 ? mine : cluster.map_shared_rank(mine, 0));
+        for (int p = 1; p < ranks; ++p) sum = add4(sum, *reinterpret_cast<const float4*>(cluster.map_shared_rank(mine, p)));
+        if (a.bias) {
+          const int r = row0 + 4 * quad;
+          sum = add4(sum, make_float4(r < a.rows ? a.bias[r] : 0.f, r + 1 < a.rows ? a.bias[r + 1] : 0.f, r + 2 < a.rows ? a.bias[r + 2] : 0.f,
+                                      r + 3 < a.rows ? a.bias[r + 3] : 0.f));
+        }
+        return sum;
+      };
+      if (a.epilogue == ETC_EPILOGUE_SWIGLU) {
+        // rows are interleaved in groups of 8: quads 0, 1 of every four are gate rows, 2, 3 their up rows
+        for (int i = threadIdx.x; i < (v_hi - v_lo) * 16; i += kStreamThreads) {
+          const int v = v_lo + (i >> 4), q = (i & 15), gate = (q >> 1) * 4 + (q & 1);
+          const float4 g = sum4(v, gate), u = sum4(v, gate + 2);
+          const int c = row0 / 2 + 4 * q;
+          if (c < a.rows / 2)
+            store4(a, v, c, 4, a.rows / 2,
+                   make_float4(silu_tanh(g.x) * u.x, silu_tanh(g.y) * u.y, silu_tanh(g.z) * u.z, silu_tanh(g.w) * u.w));
+        }
+      } else {
+        for (int i = threadIdx.x; i < (v_hi - v_lo) * 32; i += kStreamThreads) {
+          const int v = v_lo + (i >> 5), q = i & 31, r = row0 + 4 * q, inside = min(4, a.rows - r);
+          if (inside <= 0) continue;
+          float4 val = sum4(v, q);
+          if (a.epilogue == ETC_EPILOGUE_RESIDUAL) {
+            const float* res = a.residual + (size_t)v * a.rows + r;
+            val = add4(make_float4(res[0], inside > 1 ? res[1] : 0.f, inside > 2 ? res[2] : 0.f, inside > 3 ? res[3] : 0.f), val);
+          }
+          store4(a, v, r, inside, a.rows, val);
+        }
+      }
+    }
+    if (gridDim.x > 1) cluster.sync();  // the other CTAs may still be reading this one's shared memory
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag) atomicCAS(a.status, 0ull, 3ull);  // a bounded wait expired
+  if (warp == kMmaWarp) {
+    tc_fence_after();
+    tmem_dealloc(tmem, Cfg::kTmemCols);
+  }
+}
+
+// f32 [vectors, K] -> [K/8][NV][8] f16 (rows >= vectors are zero), saturating at the f16 range.
+__global__ void convert_hand_off_kernel(const float* __restrict__ x, int vectors, int K, int nv_shift, __half* __restrict__ xh) {
+  chain_release();
+  chain_wait();
+  const int total = (K / 8) << nv_shift;
+  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    const int kg = idx >> nv_shift, n = idx & ((1 << nv_shift) - 1);
+    uint2 lo = make_uint2(0u, 0u), hi = lo;
+    if (n < vectors) {
+      lo = pack4(*reinterpret_cast<const float4*>(x + (size_t)n * K + kg * 8));
+      hi = pack4(*reinterpret_cast<const float4*>(x + (size_t)n * K + kg * 8 + 4));
+    }
+    reinterpret_cast<uint4*>(xh)[idx] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+  }
+}
+
+template <int CODEC, int NV>
+cudaError_t launch_stream_pass(const StreamArgs& args, int tiles, int splits, cudaStream_t stream) {
+  constexpr size_t smem = StreamCfg<CODEC, NV>::kSmemBytes;
+  auto kernel = qlinear_stream_kernel<CODEC, NV>;
+  const cudaError_t attr = opt_in_shared_memory(kernel, smem);
+  if (attr != cudaSuccess) return attr;
+  return launch_chained_cluster(kernel, dim3((unsigned)splits, (unsigned)tiles), dim3(kStreamThreads), smem, stream, args.deferred ? 1u : (unsigned)splits, args);
+}
+
+}  // namespace
+
+int stream_max_vectors() { return 128; }
+
+StreamPlan plan_stream(const TiledWeight& w, int64_t vectors, int sm_count, bool deferred) {
+  StreamPlan p;
+  const int sms = std::max(1, sm_count);
+  p.nv = vectors <= 32 ? 32 : (vectors <= 64 ? 64 : 128);
+  p.tiles = (int)(w.rows_padded / kRows);
+  p.stages = (int)((w.columns / 32 + kStageBlocks - 1) / kStageBlocks);
+  p.xh_bytes = ((size_t)(w.columns / 8) * p.nv * 16 + 255) & ~(size_t)255;
+  if (deferred) {
+    // as many splits as fit at two CTAs per SM (one at 128 vectors), of at least two stages: the consumer's sum costs little
+    // per split, and a shape's sums keep their order whoever computes them
+    const int splits = std::min(std::max(1, sms * (p.nv <= 64 ? 2 : 1) / p.tiles), std::max(1, p.stages / 2));
+    p.stages_per_split = (p.stages + splits - 1) / splits;
+  } else {
+    // The stages of the fullest SM, a third more when it has one CTA (nothing overlaps its waits), plus two per CTA of a
+    // cluster for its exchange (measured on 32 to 112 tiles). Clusters are powers of two (three or six CTAs pack a GPC badly)
+    // and are used while all of them are resident at once: [128256 x 4096] takes 73 us with one CTA per tile, 96 with two.
+    double best = 1e30;
+    for (int s = 1; s <= std::min(kMaxStreamCluster, std::max(1, p.stages / 2)) && (s == 1 || p.tiles * s <= 2 * sms); s *= 2) {
+      const int per = (p.stages + s - 1) / s, ctas = (p.tiles * s + sms - 1) / sms;
+      const double cost = ctas * per * (ctas > 1 ? 1.0 : 1.33) + 2.0 * s;
+      if (cost < best) { best = cost; p.stages_per_split = per; }
+    }
+  }
+  p.splits = (p.stages + p.stages_per_split - 1) / p.stages_per_split;
+  p.deferred = deferred && p.splits > 1;
+  p.scratch_bytes = p.deferred ? (size_t)p.splits * p.nv * w.rows_padded * sizeof(float) : 0;
+  return p;
+}
+
+size_t stream_scratch_bytes(const TiledWeight& w, int64_t vectors, int sm_count) {
+  const StreamPlan p = plan_stream(w, vectors, sm_count, true);
+  return p.xh_bytes + p.scratch_bytes;
+}
+
+cudaError_t launch_qlinear_stream(const TiledWeight& w, const float* x, const __half* xh_ready, int64_t vectors, const float* bias,
+                                  const float* residual, int epilogue, float* out, __half* out_xh, void* scratch, DeviceStatus* status,
+                                  int sm_count, cudaStream_t stream, int* launches, int xh_nv, DeferredSum* defer) {
+  if (defer) *defer = DeferredSum();
+  const StreamPlan plan = plan_stream(w, vectors, sm_count, defer && !bias && !out_xh && epilogue != ETC_EPILOGUE_SWIGLU);
+  const int K = (int)w.columns;
+  __half* xh = reinterpret_cast<__half*>(scratch);
+  float* partials = reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + plan.xh_bytes);
+  const bool ready = xh_ready != nullptr && plan.nv == xh_nv;  // the producer stored the f16 layout with this row stride
+  cudaError_t e;
+  if (!ready) {
+    if (!x) return cudaErrorInvalidValue;
+    const int total = (K / 8) * plan.nv, shift = plan.nv == 32 ? 5 : (plan.nv == 64 ? 6 : 7);
+    e = launch_chained(convert_hand_off_kernel, dim3((unsigned)std::min((total + 255) / 256, 148 * 4)), dim3(256), 0, stream, x, (int)vectors, K, shift, xh);
+    if (e != cudaSuccess) return e;
+    if (launches) ++*launches;
+  }
+  StreamArgs args;
+  args.xh = ready ? xh_ready : xh;
+  args.bias = bias;
+  args.residual = residual;
+  args.out = out;
+  args.scratch = partials;
+  args.status = &status->code;
+  args.out_xh = vectors <= xh_nv ? out_xh : nullptr;
+  args.out_xh_nv = xh_nv;
+  args.vectors = (int)vectors;
+  args.rows = (int)w.rows;
+  args.rows_padded = (int)w.rows_padded;
+  args.kblocks = K / 32;
+  args.epilogue = epilogue;
+  args.stages = plan.stages;
+  args.stages_per_split = plan.stages_per_split;
+  args.deferred = plan.deferred;
+  // one launch per run of equal codecs; all of them share the plan of the whole weight
+  for (int sgm = 0; sgm < std::max(1, w.n_segments); ++sgm) {
+    int codec = w.codec, tiles = plan.tiles;
+    args.quants = w.quants;
+    args.scales = reinterpret_cast<const unsigned char*>(w.scales);
+    args.tile0 = 0;
+    if (w.n_segments > 0) {
+      const TiledSegment& seg = w.segments[sgm];
+      codec = seg.codec;
+      tiles = seg.tiles;
+      args.tile0 = seg.tile0;
+      args.quants += seg.quant_offset;
+      args.scales += seg.scale_offset;
+    }
+    auto pass = [&](auto nv_tag) {
+      constexpr int NV = decltype(nv_tag)::value;
+      switch (codec) {
+        case 2: return launch_stream_pass<2, NV>(args, tiles, plan.splits, stream);
+        case 8: return launch_stream_pass<8, NV>(args, tiles, plan.splits, stream);
+        case 12: return launch_stream_pass<12, NV>(args, tiles, plan.splits, stream);
+        case 13: return launch_stream_pass<13, NV>(args, tiles, plan.splits, stream);
+        default: return launch_stream_pass<14, NV>(args, tiles, plan.splits, stream);  // 14, and 11 whose re-cut form is the same
+      }
+    };
+    e = plan.nv == 32 ? pass(std::integral_constant<int, 32>()) : plan.nv == 64 ? pass(std::integral_constant<int, 64>()) : pass(std::integral_constant<int, 128>());
+    if (e != cudaSuccess) return e;
+    if (launches) ++*launches;
+  }
+  if (plan.deferred) {
+    // the consumer sums the partials itself (and adds the residual stream where the epilogue asks for it)
+    defer->partials = partials;
+    defer->splits = plan.splits;
+    defer->vpad = plan.nv;
+    defer->rows_padded = (int)w.rows_padded;
+  }
+  return cudaSuccess;
+}
+
+}  // namespace etc

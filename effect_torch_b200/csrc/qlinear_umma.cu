@@ -43,11 +43,11 @@ constexpr int kUmmaRows = 128;
 constexpr int kDequantThreads = 128;  // one TMEM lane (weight row) per thread of a dequant group
 
 // Pipeline shape: stages of four 32-value blocks in a ring of three (TMEM for the expanded weights, shared memory for
-// the activations); for NV <= 64 two CTAs share an SM (256 TMEM columns each) and overlap each other's phases.
+// the activations).
+constexpr int kStageBlocks = 4;  // 32-value blocks per stage (K = 16 per MMA: 2 MMAs per block)
 template <int NV>
 struct UmmaCfg {
-  static constexpr int kGroups = NV == 256 ? 2 : 1;  // at 256 vectors the MMAs of a stage take as long as one group needs to expand it
-  static constexpr int kStageBlocks = 4;   // 32-value blocks per stage (K = 16 per MMA: 2 MMAs per block)
+  static constexpr int kGroups = 2;        // the MMAs of a stage take as long as one group needs to expand it
   static constexpr int kStages = 3;
   static constexpr int kAColsPerStage = kStageBlocks * 16;  // 32-bit TMEM columns holding the stage's f16 per lane
   static constexpr int kThreads = (4 * kGroups + 2) * 32;  // dequant warps + bulk-copy warp + MMA warp
@@ -55,7 +55,6 @@ struct UmmaCfg {
   static constexpr uint32_t kTmemCols = NV + kStages * kAColsPerStage <= 256 ? 256 : 512;
   static constexpr size_t kSmemBytes = (size_t)kStages * kStageBBytes + (3 * kStages + 1) * sizeof(uint64_t) + 16;
 };
-constexpr int stage_blocks_for(int) { return 4; }
 using namespace tc05;
 
 struct UmmaArgs {
@@ -67,8 +66,6 @@ struct UmmaArgs {
   float* out;
   float* scratch;         // [splits][NV][rows_padded]
   unsigned long long* status;
-  __half* out_xh;         // optional: result additionally stored as xh8 f16 [cols/8][out_xh_nv][8] for the next linear
-  int out_xh_nv;
   int vectors, rows, rows_padded, kblocks, blocks_per_split, epilogue;
   int tile0;              // first row tile of this launch in the output (a segment of a weight fused from several codecs)
 };
@@ -76,7 +73,7 @@ struct UmmaArgs {
 template <int CODEC, int NV>
 __global__ void __launch_bounds__(UmmaCfg<NV>::kThreads) qlinear_umma_kernel(UmmaArgs a) {
   using Cfg = UmmaCfg<NV>;
-  constexpr int kGroups = Cfg::kGroups, kStageBlocks = Cfg::kStageBlocks, kStages = Cfg::kStages;
+  constexpr int kGroups = Cfg::kGroups, kStages = Cfg::kStages;
   constexpr int kAColsPerStage = Cfg::kAColsPerStage;
   constexpr bool kNibbles = CODEC == 2 || CODEC == 12;      // 4-bit codes (Q4_0, re-cut Q4_K) or 8-bit (Q8_0, re-cut Q3_K / Q5_K / Q6_K)
   constexpr bool kPair = CODEC >= 12;                       // two f16 per (row, block): (scale, min) or the two half-block scales
@@ -101,7 +98,7 @@ __global__ void __launch_bounds__(UmmaCfg<NV>::kThreads) qlinear_umma_kernel(Umm
     const size_t chunk = blockIdx.z;
     const size_t out_cols = a.epilogue == ETC_EPILOGUE_SWIGLU ? a.rows / 2 : a.rows;
     a.xh += chunk * ((size_t)a.kblocks * 4 * NV * 8);
-    if (a.out) a.out += chunk * NV * out_cols;
+    a.out += chunk * NV * out_cols;
     if (a.residual) a.residual += chunk * NV * out_cols;
     a.scratch += chunk * ((size_t)gridDim.y * NV * a.rows_padded);
     a.vectors = max(0, min(NV, a.vectors - (int)chunk * NV));
@@ -254,10 +251,7 @@ __global__ void __launch_bounds__(UmmaCfg<NV>::kThreads) qlinear_umma_kernel(Umm
             const float partner = __shfl_xor_sync(0xffffffffu, mine, 8);
             if ((r & 8) == 0 && r + 8 < a.rows && c0 + v < a.vectors) {
               const float act = silu_tanh(mine) * partner;
-              if (a.out) a.out[(size_t)(c0 + v) * (a.rows / 2) + oc] = act;
-              if (a.out_xh)
-                a.out_xh[((size_t)(oc >> 3) * a.out_xh_nv + (c0 + v)) * 8 + (oc & 7)] =
-                    __float2half_rn(fminf(fmaxf(act, -65504.f), 65504.f));
+              a.out[(size_t)(c0 + v) * (a.rows / 2) + oc] = act;
             }
           }
         } else if (r < a.rows) {
@@ -516,19 +510,13 @@ cudaError_t launch_repack_umma(const TiledWeight& w, const RepackParts& parts, c
   return cudaGetLastError();
 }
 
-int umma_vector_pad(int64_t vectors) { return vectors <= 32 ? 32 : (vectors <= 64 ? 64 : (vectors <= 128 ? 128 : 256)); }
-
 UmmaPlan plan_umma(const TiledWeight& w, int64_t vectors, int sm_count) {
   UmmaPlan p;
-  p.nv = umma_vector_pad(std::min<int64_t>(vectors, 256));
   p.chunks = (int)std::max<int64_t>(1, (vectors + p.nv - 1) / p.nv);
   p.tiles = (int)(w.rows_padded / kUmmaRows);
   const int kblocks = (int)(w.columns / 32);
-  const int kStageBlocks = stage_blocks_for(p.nv);
   const int stages = (kblocks + kStageBlocks - 1) / kStageBlocks;
-  const int ctas_per_sm = p.nv <= 64 ? 2 : 1;
-  const int target = std::max(1, sm_count) * ctas_per_sm;
-  int splits = std::max(1, target / std::max(1, p.tiles * p.chunks));
+  int splits = std::max(1, std::max(1, sm_count) / std::max(1, p.tiles * p.chunks));
   splits = std::min(splits, std::max(1, stages / 2));  // at least two stages per split
   const int stages_per_split = (stages + splits - 1) / splits;
   p.blocks_per_split = stages_per_split * kStageBlocks;
@@ -539,32 +527,22 @@ UmmaPlan plan_umma(const TiledWeight& w, int64_t vectors, int sm_count) {
 }
 
 // qlinear_reduce_kernel lives in quant_kernels.cu
-cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, const __half* xh_ready, int64_t vectors, const float* bias,
-                                const float* residual, int epilogue, float* out, __half* out_xh, __half* xh, float* scratch,
-                                DeviceStatus* status, int sm_count, cudaStream_t stream, int* launches, int xh_nv, DeferredSum* defer) {
-  if (defer) *defer = DeferredSum();
+cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, int64_t vectors, const float* bias, const float* residual, int epilogue,
+                                float* out, __half* xh, float* scratch, DeviceStatus* status, int sm_count, cudaStream_t stream,
+                                int* launches) {
   if (vectors <= 0) return cudaSuccess;
   const int out_cols = (int)(epilogue == ETC_EPILOGUE_SWIGLU ? w.rows / 2 : w.rows);
   const UmmaPlan plan = plan_umma(w, vectors, sm_count);
   const int K = (int)w.columns;
   const int64_t total = (int64_t)(K / 8) * plan.nv * plan.chunks;
-  const unsigned cgrid = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 8);
-  const bool ready = xh_ready != nullptr && vectors <= 128 && plan.nv == xh_nv;  // the producer stored the f16 layout with this row stride
-  if (!ready) switch (plan.nv) {
-    case 32: convert_xh8_kernel<32><<<cgrid, 256, 0, stream>>>(x, (int)vectors, K, xh); break;
-    case 64: convert_xh8_kernel<64><<<cgrid, 256, 0, stream>>>(x, (int)vectors, K, xh); break;
-    case 128: convert_xh8_kernel<128><<<cgrid, 256, 0, stream>>>(x, (int)vectors, K, xh); break;
-    default: convert_xh8_kernel<256><<<cgrid, 256, 0, stream>>>(x, (int)vectors, K, xh); break;
-  }
+  convert_xh8_kernel<256><<<(unsigned)std::min<int64_t>((total + 255) / 256, 148 * 8), 256, 0, stream>>>(x, (int)vectors, K, xh);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  if (launches && !ready) ++*launches;
+  if (launches) ++*launches;
   UmmaArgs args;
   args.quants = reinterpret_cast<const uint4*>(w.quants);
   args.scales = w.scales;
-  args.xh = ready ? xh_ready : xh;
-  args.out_xh = vectors <= xh_nv ? out_xh : nullptr;
-  args.out_xh_nv = xh_nv;
+  args.xh = xh;
   args.bias = bias;
   args.residual = residual;
   args.out = out;
@@ -577,21 +555,9 @@ cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, const __ha
   args.blocks_per_split = plan.blocks_per_split;
   args.epilogue = epilogue;
   args.tile0 = 0;
-  int codec = w.codec, tiles = plan.tiles;
-  auto pass = [&](auto nv_tag) {
-    constexpr int NV = decltype(nv_tag)::value;
-    switch (codec) {
-      case 2: return launch_umma_pass<2, NV>(args, tiles, plan.splits, plan.chunks, stream);
-      case 8: return launch_umma_pass<8, NV>(args, tiles, plan.splits, plan.chunks, stream);
-      case 12: return launch_umma_pass<12, NV>(args, tiles, plan.splits, plan.chunks, stream);
-      case 13: return launch_umma_pass<13, NV>(args, tiles, plan.splits, plan.chunks, stream);
-      default:  // 14, and 11 whose re-cut form is the same
-        return launch_umma_pass<14, NV>(args, tiles, plan.splits, plan.chunks, stream);
-    }
-  };
   // one launch per run of equal codecs; all of them share the plan (split count, partial layout) of the whole weight
-  const int n_segments = std::max(1, w.n_segments);
-  for (int sgm = 0; sgm < n_segments; ++sgm) {
+  for (int sgm = 0; sgm < std::max(1, w.n_segments); ++sgm) {
+    int codec = w.codec, tiles = plan.tiles;
     if (w.n_segments > 0) {
       const TiledSegment& seg = w.segments[sgm];
       codec = seg.codec;
@@ -600,31 +566,22 @@ cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, const __ha
       args.quants = reinterpret_cast<const uint4*>(w.quants + seg.quant_offset);
       args.scales = reinterpret_cast<const __half*>(reinterpret_cast<const uint8_t*>(w.scales) + seg.scale_offset);
     }
-    switch (plan.nv) {
-      case 32: e = pass(std::integral_constant<int, 32>()); break;
-      case 64: e = pass(std::integral_constant<int, 64>()); break;
-      case 128: e = pass(std::integral_constant<int, 128>()); break;
-      default: e = pass(std::integral_constant<int, 256>()); break;
+    switch (codec) {
+      case 2: e = launch_umma_pass<2, 256>(args, tiles, plan.splits, plan.chunks, stream); break;
+      case 8: e = launch_umma_pass<8, 256>(args, tiles, plan.splits, plan.chunks, stream); break;
+      case 12: e = launch_umma_pass<12, 256>(args, tiles, plan.splits, plan.chunks, stream); break;
+      case 13: e = launch_umma_pass<13, 256>(args, tiles, plan.splits, plan.chunks, stream); break;
+      default: e = launch_umma_pass<14, 256>(args, tiles, plan.splits, plan.chunks, stream);  // 14, and 11 whose re-cut form is the same
     }
     if (e != cudaSuccess) return e;
     if (launches) ++*launches;
   }
-  if (plan.splits > 1 && defer && plan.chunks == 1 && !bias && !out_xh && epilogue != ETC_EPILOGUE_SWIGLU) {
-    // the consumer sums the partials itself (and adds the residual stream where the epilogue asks for it)
-    defer->partials = scratch;
-    defer->splits = plan.splits;
-    defer->vpad = plan.nv;
-    defer->rows_padded = (int)w.rows_padded;
-  } else if (plan.splits > 1) {
-    for (int c = 0; c < plan.chunks; ++c) {  // one sum launch per chunk of vectors
-      const int64_t v0 = (int64_t)c * plan.nv;
-      const float* partials = scratch + (size_t)c * plan.splits * plan.nv * w.rows_padded;
-      e = launch_qlinear_reduce(partials, plan.splits, plan.nv, (int)std::min<int64_t>(plan.nv, vectors - v0), (int)w.rows, (int)w.rows_padded,
-                                bias, residual ? residual + v0 * out_cols : nullptr, epilogue, out + v0 * out_cols, c == 0 ? args.out_xh : nullptr,
-                                stream, xh_nv);
-      if (e != cudaSuccess) return e;
-      if (launches) ++*launches;
-    }
+  for (int c = 0; plan.splits > 1 && c < plan.chunks; ++c) {  // one sum launch per chunk of vectors
+    const int64_t v0 = (int64_t)c * plan.nv;
+    e = launch_qlinear_reduce(scratch + (size_t)c * plan.splits * plan.nv * w.rows_padded, plan.splits, plan.nv, (int)std::min<int64_t>(plan.nv, vectors - v0),
+                              (int)w.rows, (int)w.rows_padded, bias, residual ? residual + v0 * out_cols : nullptr, epilogue, out + v0 * out_cols, stream);
+    if (e != cudaSuccess) return e;
+    if (launches) ++*launches;
   }
   return cudaSuccess;
 }

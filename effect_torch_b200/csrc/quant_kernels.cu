@@ -1,7 +1,7 @@
 // Block-quantized weight kernels for sm_100a: dequantise, quantise, the generic (any codec, raw
 // GGUF layout) linear, the row-gather embedding, the split-K sum of the tcgen05 linear and the
 // front end that routes a tiled linear to the matvec kernel (qlinear_mv.cu, up to 16 vectors) or
-// to the tcgen05 kernel (qlinear_umma.cu).
+// to the streaming tcgen05 kernel (qlinear_stream.cu, up to 128) or to the large-batch one (qlinear_umma.cu).
 //
 // Replaces crates/runtime-cpu/src/quantized.rs (decode_block :90, linear_into :419,
 // embedding_into :546) of the reference for the CUDA backend.
@@ -409,7 +409,7 @@ __device__ __forceinline__ float silu_tanh_form(float x) { return x * (tanhf(x *
 // neither carries a no-alias promise.
 __global__ void qlinear_reduce_kernel(const float* __restrict__ scratch, int splits, int vpad, int vectors, int rows,
                                       int rows_padded, const float* __restrict__ bias, const float* residual,
-                                      int epilogue, float* out, __half* __restrict__ out_xh, int xh_nv) {
+                                      int epilogue, float* out) {
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   chain_wait();
   const int out_cols = epilogue == ETC_EPILOGUE_SWIGLU ? rows / 2 : rows;
@@ -426,29 +426,25 @@ __global__ void qlinear_reduce_kernel(const float* __restrict__ scratch, int spl
       }
       if (bias) { gsum += bias[r_gate]; usum += bias[r_up]; }
       const float act = silu_tanh_form(gsum) * usum;
-      if (out) out[idx] = act;
-      if (out_xh)  // f16 copy in [cols/8][xh_nv][8] order: the next linear's B operand
-        out_xh[((size_t)(c >> 3) * xh_nv + v) * 8 + (c & 7)] = __float2half_rn(fminf(fmaxf(act, -65504.f), 65504.f));
+      out[idx] = act;
     } else {
       float sum = 0.f;
       for (int s = 0; s < splits; ++s) sum += scratch[((size_t)s * vpad + v) * rows_padded + c];
       if (bias) sum += bias[c];
       const float val = epilogue == ETC_EPILOGUE_RESIDUAL ? residual[idx] + sum : sum;
-      if (out) out[idx] = val;
-      if (out_xh) out_xh[((size_t)(c >> 3) * xh_nv + v) * 8 + (c & 7)] = __float2half_rn(fminf(fmaxf(val, -65504.f), 65504.f));
+      out[idx] = val;
     }
   }
 }
 
 cudaError_t launch_qlinear_reduce(const float* scratch, int splits, int vpad, int vectors, int rows, int rows_padded,
-                                  const float* bias, const float* residual, int epilogue, float* out, __half* out_xh,
-                                  cudaStream_t stream, int xh_nv) {
+                                  const float* bias, const float* residual, int epilogue, float* out, cudaStream_t stream) {
   const int out_cols = epilogue == ETC_EPILOGUE_SWIGLU ? rows / 2 : rows;
   const int64_t total = (int64_t)vectors * out_cols;
   if (total == 0) return cudaSuccess;
   const unsigned grid = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 8);
   return launch_chained(qlinear_reduce_kernel, dim3(grid), dim3(256), 0, stream, scratch, splits, vpad, vectors, rows, rows_padded, bias, residual,
-                        epilogue, out, vectors <= xh_nv ? out_xh : (__half*)nullptr, xh_nv);
+                        epilogue, out);
 }
 
 // Scratch layout of the tcgen05 path: [xh8 activations, rounded to 256 B][split-K partials].
@@ -459,6 +455,7 @@ size_t tiled_scratch_bytes(const TiledWeight& w, int64_t vectors, int sm_count) 
     const MvPlan p = plan_mv(w, vectors, sm_count);
     return p.xh_bytes + p.partial_bytes;
   }
+  if (vectors <= stream_max_vectors()) return stream_scratch_bytes(w, vectors, sm_count);
   const UmmaPlan p = plan_umma(w, vectors, sm_count);
   return umma_xh_region(p) + p.scratch_bytes;
 }
@@ -471,10 +468,11 @@ cudaError_t launch_qlinear_tiled(const TiledWeight& w, const float* x, int64_t v
   if (w.counters && vectors <= mv_max_vectors())
     return launch_qlinear_mv(w, x, xh_ready, vectors, bias, residual, epilogue, out, out_xh, scratch, status, sm_count, stream,
                              launches, xh_nv);
+  if (vectors <= stream_max_vectors())
+    return launch_qlinear_stream(w, x, xh_ready, vectors, bias, residual, epilogue, out, out_xh, scratch, status, sm_count, stream, launches, xh_nv, defer);
   const size_t xh_region = umma_xh_region(plan_umma(w, vectors, sm_count));  // f16 activations of every chunk, then the partials
-  return launch_qlinear_umma(w, x, xh_ready, vectors, bias, residual, epilogue, out, out_xh, reinterpret_cast<__half*>(scratch),
-                             reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + xh_region), status, sm_count, stream,
-                             launches, xh_nv, defer);
+  return launch_qlinear_umma(w, x, vectors, bias, residual, epilogue, out, reinterpret_cast<__half*>(scratch),
+                             reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + xh_region), status, sm_count, stream, launches);
 }
 
 }  // namespace etc

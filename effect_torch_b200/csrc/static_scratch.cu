@@ -74,12 +74,20 @@ etc_status etc_qlinear_tiled_static_into(etc_runtime* rt, const etc_qweight* w, 
     return fail(ETC_INVALID_ARGUMENT, "quantized_linear: the residual epilogue needs a residual input");
   if (vectors <= 0) return ETC_OK;
   // the whole call in one pass when its scratch fits; otherwise 256 vectors at a time (a slice needs an eighth or so of
-  // what the one-pass plan of a long call needs), and only a slice that does not fit is refused
-  const int64_t slice = tiled_scratch_bytes(w->tiled, vectors, rt->sm_count) <= kStaticScratchBytes ? vectors : 256;
-  for (int64_t v0 = 0; v0 < vectors; v0 += slice) {
-    const size_t need = tiled_scratch_bytes(w->tiled, std::min(slice, vectors - v0), rt->sm_count);
-    if (need > kStaticScratchBytes)
-      return fail(ETC_INVALID_ARGUMENT, "quantized_linear: this call needs " + std::to_string(need) +
+  // what the one-pass plan of a long call needs), a rest below that in the longest slices that fit; only a 256-vector slice
+  // that does not fit is refused
+  auto bytes = [&](int64_t n) { return tiled_scratch_bytes(w->tiled, n, rt->sm_count); };
+  auto slice_of = [&](int64_t left) {
+    if (bytes(left) <= kStaticScratchBytes) return left;
+    if (left > 256) return (int64_t)256;
+    for (int64_t n : {128, 64, 32})
+      if (left < 256 && left > n && bytes(n) <= kStaticScratchBytes) return n;
+    return left;
+  };
+  for (int64_t v0 = 0, n; v0 < vectors; v0 += n) {
+    n = slice_of(vectors - v0);
+    if (bytes(n) > kStaticScratchBytes)
+      return fail(ETC_INVALID_ARGUMENT, "quantized_linear: this call needs " + std::to_string(bytes(n)) +
                                             " bytes of scratch, the static scratch holds " + std::to_string(kStaticScratchBytes) +
                                             "; use etc_qlinear_tiled_into with caller scratch");
   }
@@ -87,10 +95,11 @@ etc_status etc_qlinear_tiled_static_into(etc_runtime* rt, const etc_qweight* w, 
   ETC_CUDA(static_scratch_for_device(rt->device, &scratch));
   int launches = 0;
   const int64_t out_cols = epilogue == ETC_EPILOGUE_SWIGLU ? w->tiled.rows / 2 : w->tiled.rows;
-  for (int64_t v0 = 0; v0 < vectors; v0 += slice)
-    ETC_CUDA(launch_qlinear_tiled(w->tiled, d_x + v0 * w->tiled.columns, std::min(slice, vectors - v0), d_bias,
-                                  d_residual ? d_residual + v0 * out_cols : nullptr, epilogue, d_out + v0 * out_cols, scratch, rt->d_status,
-                                  rt->sm_count, rt->stream, &launches));
+  for (int64_t v0 = 0, n; v0 < vectors; v0 += n) {
+    n = slice_of(vectors - v0);
+    ETC_CUDA(launch_qlinear_tiled(w->tiled, d_x + v0 * w->tiled.columns, n, d_bias, d_residual ? d_residual + v0 * out_cols : nullptr, epilogue,
+                                  d_out + v0 * out_cols, scratch, rt->d_status, rt->sm_count, rt->stream, &launches));
+  }
   rt->launches += (uint64_t)launches;
   return ETC_OK;
 }
