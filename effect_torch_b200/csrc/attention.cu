@@ -127,19 +127,40 @@ cudaError_t launch_kv_append(const PoolView& pool, const float* k, const float* 
 // the output over positions in order with separate multiply and add, exactly like the
 // reference's loop, and divides by the denominator it accumulated the same way.
 // Only exp() can differ from the host libm, by an ulp of f64.
+//
+// Latency-bound: two dependent f64 chains, head_dim long (scores) and context long (output). What is not part of them is
+// kept off them: block-table look-ups and their divisions are done once per position, K rows and V elements are fetched
+// four and eight at a time ahead of the adds, weights of contexts up to kExactKept stay in shared memory.
 // --------------------------------------------------------------------------------------------
+constexpr int kExactKept = 2048;
+
+template <int DTYPE>
+__device__ __forceinline__ float exact_load(const void* slab, size_t elem, float scale) {
+  if (DTYPE == kKvF32) return reinterpret_cast<const float*>(slab)[elem];
+  if (DTYPE == kKvF16) return __half2float(reinterpret_cast<const __half*>(slab)[elem]);
+  if (DTYPE == kKvBF16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(slab)[elem]);
+  return __fmul_rn(__fsub_rn((float)reinterpret_cast<const uint8_t*>(slab)[elem], 128.0f), scale);
+}
+
+// `tokens_first`: q and out are [B, tokens, Hq, D] (the fused projection's order) instead of [B, Hq, tokens, D].
+template <int DTYPE>
 __global__ void __launch_bounds__(128) attention_exact_kernel(PoolView pool, const float* __restrict__ q,
                                                               const LaneInfo* __restrict__ lanes,
                                                               const int* __restrict__ tables, int q_heads, int tokens,
                                                               double scale, long long op_window, float* __restrict__ out,
-                                                              double* __restrict__ scratch, int max_ctx) {
+                                                              double* __restrict__ scratch, int max_ctx, int tokens_first) {
+  extern __shared__ float q_s[];  // the query row
+  __shared__ double kept[kExactKept];
+  __shared__ int row_of[kExactKept];  // (page * kv_heads + head) * block_size + slot of each position
   __shared__ double red[4];
-  __shared__ double max_s;
+  chain_release();
+  chain_wait();
   const int head = blockIdx.x, query = blockIdx.y, lane_id = blockIdx.z;
   const LaneInfo info = lanes[lane_id];
   const int D = pool.head_dim;
   const size_t row_index = ((size_t)lane_id * q_heads + head) * tokens + query;
-  float* orow = out + row_index * D;
+  const size_t io = (tokens_first ? ((size_t)lane_id * tokens + query) * q_heads + head : row_index) * D;
+  float* orow = out + io;
   if (info.advance == 0) {  // padded lane: output stays zero (napi/mod.rs:3371-3372)
     for (int d = threadIdx.x; d < D; d += blockDim.x) orow[d] = 0.0f;
     return;
@@ -150,18 +171,35 @@ __global__ void __launch_bounds__(128) attention_exact_kernel(PoolView pool, con
   int begin = info.start;
   if (op_window >= 0) begin = max((int)max((long long)end - op_window, 0ll), info.start);
   const int span = max(end - begin, 0);
-  const float* qrow = q + row_index * D;
-  double* wrow = scratch + row_index * (size_t)max_ctx;
+  for (int d = threadIdx.x; d < D; d += blockDim.x) q_s[d] = q[io + d];
+  const bool keep = span <= kExactKept;
+  double* wrow = keep ? kept : scratch + row_index * (size_t)max_ctx;
   const int* table = tables + info.table_offset;
+  auto find_row = [&](int i) {
+    const int pos = begin + i, block = pos / pool.block_size;
+    return (table[block] * pool.kv_heads + kv_head) * pool.block_size + (pos - block * pool.block_size);
+  };
+  auto row_at = [&](int i) { return keep ? row_of[i] : find_row(i); };
+  auto k_scale = [&](int row) { return DTYPE == kKvU8 ? pool.k_scale[row] : 0.0f; };
+  auto v_scale = [&](int row) { return DTYPE == kKvU8 ? pool.v_scale[row] : 0.0f; };
+  __syncthreads();
 
   double local_max = -INFINITY;
   for (int i = threadIdx.x; i < span; i += blockDim.x) {
-    const int pos = begin + i;
-    const int page = table[pos / pool.block_size], slot = pos % pool.block_size;
-    const size_t base = pool_elem(pool, page, kv_head, slot);
-    const size_t si = pool_scale_index(pool, page, kv_head, slot);
+    const int row = find_row(i);
+    if (keep) row_of[i] = row;
+    const size_t base = (size_t)row * D;
+    const float ks = k_scale(row);
     double score = 0.0;
-    for (int c = 0; c < D; ++c) score += (double)qrow[c] * (double)pool_load(pool, pool.k, pool.k_scale, base + c, si);
+    int c = 0;
+    for (; c + 4 <= D; c += 4) {
+      float kv[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) kv[u] = exact_load<DTYPE>(pool.k, base + c + u, ks);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) score += (double)q_s[c + u] * (double)kv[u];
+    }
+    for (; c < D; ++c) score += (double)q_s[c] * (double)exact_load<DTYPE>(pool.k, base + c, ks);
     const double scaled = __dmul_rn(score, scale);
     wrow[i] = scaled;
     local_max = fmax(local_max, scaled);
@@ -170,24 +208,30 @@ __global__ void __launch_bounds__(128) attention_exact_kernel(PoolView pool, con
   for (int off = 16; off > 0; off >>= 1) local_max = fmax(local_max, __shfl_xor_sync(0xffffffffu, local_max, off));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = local_max;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double m = red[0];
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
-    max_s = m;
-  }
-  __syncthreads();
-  const double maximum = max_s;
+  const double maximum = fmax(fmax(red[0], red[1]), fmax(red[2], red[3]));
   for (int i = threadIdx.x; i < span; i += blockDim.x) wrow[i] = exp(__dsub_rn(wrow[i], maximum));
   __syncthreads();
   for (int c = threadIdx.x; c < D; c += blockDim.x) {
     double result = 0.0, denominator = 0.0;
-    for (int i = 0; i < span; ++i) {
-      const int pos = begin + i;
-      const int page = table[pos / pool.block_size], slot = pos % pool.block_size;
+    int i = 0;
+    for (; i + 8 <= span; i += 8) {
+      float value[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int row = row_at(i + u);
+        value[u] = exact_load<DTYPE>(pool.v, (size_t)row * D + c, v_scale(row));
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const double w = wrow[i + u];
+        result = __dadd_rn(result, __dmul_rn(w, (double)value[u]));
+        denominator = __dadd_rn(denominator, w);
+      }
+    }
+    for (; i < span; ++i) {
+      const int row = row_at(i);
       const double w = wrow[i];
-      const float value = pool_load(pool, pool.v, pool.v_scale, pool_elem(pool, page, kv_head, slot) + c,
-                                    pool_scale_index(pool, page, kv_head, slot));
-      result = __dadd_rn(result, __dmul_rn(w, (double)value));
+      result = __dadd_rn(result, __dmul_rn(w, (double)exact_load<DTYPE>(pool.v, (size_t)row * D + c, v_scale(row))));
       denominator = __dadd_rn(denominator, w);
     }
     orow[c] = (float)__ddiv_rn(result, denominator);
@@ -196,12 +240,18 @@ __global__ void __launch_bounds__(128) attention_exact_kernel(PoolView pool, con
 
 cudaError_t launch_attention_exact(const PoolView& pool, const float* q, const LaneInfo* lanes, const int* tables,
                                    int batch, int q_heads, int tokens, double scale, long long op_window, float* out,
-                                   double* scratch, int max_ctx, cudaStream_t stream) {
+                                   double* scratch, int max_ctx, cudaStream_t stream, bool tokens_first) {
   if (batch == 0 || tokens == 0) return cudaSuccess;
-  dim3 grid((unsigned)q_heads, (unsigned)tokens, (unsigned)batch);
-  attention_exact_kernel<<<grid, 128, 0, stream>>>(pool, q, lanes, tables, q_heads, tokens, scale, op_window, out,
-                                                   scratch, max_ctx);
-  return cudaGetLastError();
+  auto launch = [&](auto kernel) {
+    return launch_chained(kernel, dim3((unsigned)q_heads, (unsigned)tokens, (unsigned)batch), dim3(128), (size_t)pool.head_dim * sizeof(float), stream, pool,
+                          q, lanes, tables, q_heads, tokens, scale, op_window, out, scratch, max_ctx, (int)tokens_first);
+  };
+  switch (pool.dtype) {
+    case kKvF32: return launch(attention_exact_kernel<kKvF32>);
+    case kKvF16: return launch(attention_exact_kernel<kKvF16>);
+    case kKvBF16: return launch(attention_exact_kernel<kKvBF16>);
+    default: return launch(attention_exact_kernel<kKvU8>);
+  }
 }
 
 // --------------------------------------------------------------------------------------------
@@ -725,8 +775,8 @@ __global__ void rope_append_kernel(PoolView pool, const float* __restrict__ qkv,
   const int head = blockIdx.x, lane_id = blockIdx.y, tok = blockIdx.z, tokens = gridDim.z;
   const LaneInfo info = lanes[lane_id];
   const int D = pool.head_dim, half = D / 2;
-  const int j = threadIdx.x;
-  if (j >= half) return;
+  const bool live = (int)threadIdx.x < half;  // head dims below 64 leave threads of the warp without a pair
+  const int j = live ? threadIdx.x : 0;
   const size_t row_width = (size_t)(q_heads + 2 * pool.kv_heads) * D;
   const size_t row = (size_t)lane_id * tokens + tok;
   const float* src = qkv + row * row_width + (size_t)head * D;
@@ -763,6 +813,7 @@ __global__ void rope_append_kernel(PoolView pool, const float* __restrict__ qkv,
     r0 = src[i0];
     r1 = src[i1];
   }
+  if (!live) r0 = r1 = 0.f;
   if (is_q || is_k) {
     const double angle = (double)(info.cursor + tok) * inv_freq[j];
     double s, c;
@@ -773,8 +824,10 @@ __global__ void rope_append_kernel(PoolView pool, const float* __restrict__ qkv,
   }
   if (is_q) {
     float* dst = q_out + (row * q_heads + head) * D;
-    dst[i0] = r0;
-    dst[i1] = r1;
+    if (live) {
+      dst[i0] = r0;
+      dst[i1] = r1;
+    }
     return;
   }
   if (info.advance == 0) return;  // padded lane: nothing is cached
@@ -797,10 +850,13 @@ __global__ void rope_append_kernel(PoolView pool, const float* __restrict__ qkv,
     if (threadIdx.x == 0) (is_k ? pool.k_scale : pool.v_scale)[pool_scale_index(pool, page, kv_head, slot)] = scale;
     const float c0 = fminf(fmaxf(roundf(__fdiv_rn(r0, scale)), -127.0f), 127.0f) + 128.0f;
     const float c1 = fminf(fmaxf(roundf(__fdiv_rn(r1, scale)), -127.0f), 127.0f) + 128.0f;
-    reinterpret_cast<uint8_t*>(slab)[dst + i0] = (uint8_t)c0;
-    reinterpret_cast<uint8_t*>(slab)[dst + i1] = (uint8_t)c1;
+    if (live) {
+      reinterpret_cast<uint8_t*>(slab)[dst + i0] = (uint8_t)c0;
+      reinterpret_cast<uint8_t*>(slab)[dst + i1] = (uint8_t)c1;
+    }
     return;
   }
+  if (!live) return;
   pool_store(pool, slab, dst + i0, r0);
   pool_store(pool, slab, dst + i1, r1);
 }
@@ -810,7 +866,7 @@ cudaError_t launch_rope_append(const PoolView& pool, const float* qkv, const Lan
                                cudaStream_t stream, const DeferredSum* sum, int tokens) {
   if (batch == 0) return cudaSuccess;
   dim3 grid((unsigned)(q_heads + 2 * pool.kv_heads), (unsigned)batch, (unsigned)tokens);
-  return launch_chained(rope_append_kernel, grid, dim3((unsigned)std::max(32, pool.head_dim / 2)), 0, stream, pool, qkv, lanes, tables, inv_freq, layout, q_heads,
+  return launch_chained(rope_append_kernel, grid, dim3((unsigned)std::max(32, (pool.head_dim / 2 + 31) / 32 * 32)), 0, stream, pool, qkv, lanes, tables, inv_freq, layout, q_heads,
                         q_out, sum ? *sum : DeferredSum());
 }
 

@@ -49,8 +49,7 @@ struct etc_decoder {
   double* d_inv_freq = nullptr;
 
   // device workspaces
-  float *hidden = nullptr, *normed = nullptr, *qkv = nullptr, *qh = nullptr, *kh = nullptr, *vh = nullptr, *qr = nullptr,
-        *kr = nullptr, *att = nullptr, *attl = nullptr, *proj = nullptr, *g = nullptr, *u = nullptr, *act = nullptr,
+  float *hidden = nullptr, *normed = nullptr, *qkv = nullptr, *qr = nullptr, *attl = nullptr, *proj = nullptr, *g = nullptr, *u = nullptr, *act = nullptr,
         *last = nullptr, *logits = nullptr;
   // f16 activation hand-off between kernels of the one-token fast path ([K/8][32][8] order, rows >= batch stay zero)
   __half *xh_norm = nullptr, *xh_att = nullptr, *xh_act = nullptr;
@@ -211,6 +210,52 @@ struct StepContext {
   int launches = 0;
 };
 
+// A dense weight of the decoder as (the first) weight of a dense launch.
+DenseArgs dense_args(const float* x, int64_t rows, const BoundWeight& w) {
+  DenseArgs a;
+  a.x = x;
+  a.m = rows;
+  a.k = w.columns;
+  a.w[0] = (const float*)w.d_raw;
+  a.n[0] = w.rows;
+  a.constant_weights = 1;
+  return a;
+}
+
+// q, k and v of raw weights side by side in d->qkv, the layout of the fused projection.
+etc_status project_qkv_raw(StepContext& s, size_t layer, const float* x, int64_t rows, int64_t stride) {
+  etc_decoder* d = s.dec;
+  cudaStream_t stream = d->rt->stream;
+  const BoundWeight* w[3] = {&d->wq[layer], &d->wk[layer], &d->wv[layer]};
+  float* out[3] = {d->qkv, d->qkv + w[0]->rows, d->qkv + w[0]->rows + w[1]->rows};
+  if (w[0]->codec == ETC_CODEC_F32 && w[1]->codec == ETC_CODEC_F32 && w[2]->codec == ETC_CODEC_F32) {
+    DenseArgs a = dense_args(x, rows, *w[0]);
+    a.parts = 3;
+    a.out_stride = stride;
+    for (int p = 0; p < 3; ++p) {
+      a.w[p] = (const float*)w[p]->d_raw;
+      a.n[p] = w[p]->rows;
+      a.out[p] = out[p];
+    }
+    ETC_CUDA(launch_dense_linear(a, stream));
+    s.launches += dense_linear_supported(a) ? 1 : 3;
+    return ETC_OK;
+  }
+  for (int p = 0; p < 3; ++p) {
+    if (w[p]->codec == ETC_CODEC_F32) {
+      DenseArgs a = dense_args(x, rows, *w[p]);
+      a.out[0] = out[p];
+      a.out_stride = stride;
+      ETC_CUDA(launch_dense_linear(a, stream));
+      ++s.launches;
+    } else {
+      ETC_CUDA(launch_qlinear_generic(w[p]->codec, x, rows, w[p]->columns, (const uint8_t*)w[p]->d_raw, w[p]->rows, nullptr, out[p], stream, &s.launches,
+                                      stride));
+    }
+  }
+  return ETC_OK;
+}
+
 // out = x W^T (+ epilogue) for one projection, choosing the tensor-core tiling when it exists.
 etc_status run_linear(StepContext& s, const BoundWeight& raw, etc_qweight* tiled_w, const float* x, int64_t vectors, float* out,
                       int epilogue, const float* residual, const __half* xh_ready = nullptr, __half* out_xh = nullptr,
@@ -223,14 +268,17 @@ etc_status run_linear(StepContext& s, const BoundWeight& raw, etc_qweight* tiled
                                   d->rt->d_status, d->rt->sm_count, stream, &s.launches, xh_ready, out_xh, d->xh_nv, defer));
     return ETC_OK;
   }
-  float* target = epilogue == ETC_EPILOGUE_RESIDUAL ? d->proj : out;
   if (raw.codec == ETC_CODEC_F32) {
-    ETC_CUDA(launch_linear_f32(x, vectors, raw.columns, (const float*)raw.d_raw, raw.rows, nullptr, target, stream));
+    DenseArgs dense = dense_args(x, vectors, raw);
+    dense.out[0] = out;
+    dense.out_stride = raw.rows;
+    dense.residual = epilogue == ETC_EPILOGUE_RESIDUAL ? residual : nullptr;
+    ETC_CUDA(launch_dense_linear(dense, stream));
     ++s.launches;
-  } else {
-    ETC_CUDA(launch_qlinear_generic(raw.codec, x, vectors, raw.columns, (const uint8_t*)raw.d_raw, raw.rows, nullptr, target,
-                                    stream, &s.launches));
+    return ETC_OK;
   }
+  float* target = epilogue == ETC_EPILOGUE_RESIDUAL ? d->proj : out;
+  ETC_CUDA(launch_qlinear_generic(raw.codec, x, vectors, raw.columns, (const uint8_t*)raw.d_raw, raw.rows, nullptr, target, stream, &s.launches));
   if (epilogue == ETC_EPILOGUE_RESIDUAL) {
     ETC_CUDA(launch_add(residual, target, vectors * raw.rows, out, stream));
     ++s.launches;
@@ -317,28 +365,15 @@ etc_status enqueue_step(StepContext& s) {
       ETC_CUDA(launch_rmsnorm(d->hidden, (const float*)d->attn_norm[li].d_raw, c.rms_eps, rows, c.d_model, d->normed, stream));
       ++s.launches;
     }
-    const float *qp, *kp, *vp;
-    int64_t stride_q, stride_kv;
     const bool fast_attention = d->tiled && !c.exact && attention_mma_supported(view, Hq, T);
     DeferredSum qkv_sum;  // the RoPE / append kernel can sum the fused projection's partials itself
-    if (d->tiled) {
-      ETC_TRY(run_linear(s, d->wq[li], d->t_qkv[li], d->normed, rows, d->qkv, ETC_EPILOGUE_NONE, nullptr, xh ? d->xh_norm : nullptr,
-                         nullptr, fast_attention ? &qkv_sum : nullptr));
-      qp = d->qkv; kp = d->qkv + qw; vp = d->qkv + qw + kvw;
-      stride_q = stride_kv = qkvw;
-    } else {
-      float* qb = d->qkv;
-      float* kb = qb + rows * qw;
-      float* vb = kb + rows * kvw;
-      ETC_TRY(run_linear(s, d->wq[li], nullptr, d->normed, rows, qb, ETC_EPILOGUE_NONE, nullptr));
-      ETC_TRY(run_linear(s, d->wk[li], nullptr, d->normed, rows, kb, ETC_EPILOGUE_NONE, nullptr));
-      ETC_TRY(run_linear(s, d->wv[li], nullptr, d->normed, rows, vb, ETC_EPILOGUE_NONE, nullptr));
-      qp = qb; kp = kb; vp = vb;
-      stride_q = qw; stride_kv = kvw;
-    }
+    if (d->tiled)
+      ETC_TRY(run_linear(s, d->wq[li], d->t_qkv[li], d->normed, rows, d->qkv, ETC_EPILOGUE_NONE, nullptr, xh ? d->xh_norm : nullptr, nullptr, &qkv_sum));
+    else
+      ETC_TRY(project_qkv_raw(s, li, d->normed, rows, qkvw));
+    ETC_CUDA(launch_rope_append(view, d->qkv, d->d_lanes, d->d_tables, d->d_inv_freq, c.rope_layout, B, Hq, d->qr, stream, &qkv_sum, T));
+    ++s.launches;
     if (fast_attention) {
-      ETC_CUDA(launch_rope_append(view, d->qkv, d->d_lanes, d->d_tables, d->d_inv_freq, c.rope_layout, B, Hq, d->qr, stream, &qkv_sum, T));
-      ++s.launches;
       const AttnPlan plan = plan_attention(B, Hq, Hkv, D, std::max(1, s.max_pages), d->rt->sm_count);
       if (plan.scratch_bytes > d->attn_scratch_bytes)
         return fail(ETC_EXECUTION, "kv attention: split plan for " + std::to_string(s.max_pages) + " pages needs " +
@@ -347,16 +382,8 @@ etc_status enqueue_step(StepContext& s) {
       ETC_CUDA(launch_attention_mma(view, d->qr, d->d_lanes, d->d_tables, B, Hq, scale, c.window, d->attl, plan,
                                     d->attn_scratch, stream, &s.launches, xh ? d->xh_att : nullptr, d->xh_nv, T));
     } else {
-      ETC_CUDA(launch_heads_first(qp, d->qh, B, T, Hq, D, stride_q, stream));
-      ETC_CUDA(launch_heads_first(kp, d->kh, B, T, Hkv, D, stride_kv, stream));
-      ETC_CUDA(launch_heads_first(vp, d->vh, B, T, Hkv, D, stride_kv, stream));
-      ETC_CUDA(launch_rope(d->qh, d->d_cursors, B, d->d_inv_freq, c.rope_layout, B, Hq, T, D, d->qr, stream));
-      ETC_CUDA(launch_rope(d->kh, d->d_cursors, B, d->d_inv_freq, c.rope_layout, B, Hkv, T, D, d->kr, stream));
-      ETC_CUDA(launch_kv_append(view, d->kr, d->vh, d->d_lanes, d->d_tables, B, T, (int64_t)Hkv * T * D, (int64_t)T * D, D, stream));
-      ETC_CUDA(launch_attention_exact(view, d->qr, d->d_lanes, d->d_tables, B, Hq, T, scale, c.window, d->att, d->exact_scratch,
-                                      s.max_ctx, stream));
-      ETC_CUDA(launch_heads_last(d->att, d->attl, B, T, Hq, D, stream));
-      s.launches += 8;
+      ETC_CUDA(launch_attention_exact(view, d->qr, d->d_lanes, d->d_tables, B, Hq, T, scale, c.window, d->attl, d->exact_scratch, s.max_ctx, stream, true));
+      ++s.launches;
     }
     const bool xh_o = xh && fast_attention;
     ETC_TRY(project_into_hidden(s, d->wo[li], d->tiled ? d->t_o[li] : nullptr, d->attl, rows, xh_o ? d->xh_att : nullptr, 0,
@@ -370,6 +397,15 @@ etc_status enqueue_step(StepContext& s) {
     if (d->tiled) {
       ETC_TRY(run_linear(s, d->gate[li], d->t_gu[li], d->normed, rows, xh ? nullptr : d->act, ETC_EPILOGUE_SWIGLU, nullptr,
                          xh ? d->xh_norm : nullptr, xh ? d->xh_act : nullptr));
+    } else if (DenseArgs ffn = dense_args(d->normed, rows, d->gate[li]);
+               d->gate[li].codec == ETC_CODEC_F32 && d->up[li].codec == ETC_CODEC_F32 && dense_linear_supported(ffn)) {
+      ffn.w[1] = (const float*)d->up[li].d_raw;
+      ffn.out[0] = d->act;
+      ffn.out_stride = c.ffn;
+      ffn.swiglu = 1;
+      ffn.exact = c.exact;
+      ETC_CUDA(launch_dense_linear(ffn, stream));
+      ++s.launches;
     } else {
       ETC_TRY(run_linear(s, d->gate[li], nullptr, d->normed, rows, d->g, ETC_EPILOGUE_NONE, nullptr));
       ETC_TRY(run_linear(s, d->up[li], nullptr, d->normed, rows, d->u, ETC_EPILOGUE_NONE, nullptr));
@@ -918,12 +954,7 @@ etc_status etc_decoder_finalize(etc_decoder* dec) {
   ETC_TRY(dalloc(dec, &dec->hidden, R * c.d_model));
   ETC_TRY(dalloc(dec, &dec->normed, R * c.d_model));
   ETC_TRY(dalloc(dec, &dec->qkv, R * (qw + 2 * kvw)));
-  ETC_TRY(dalloc(dec, &dec->qh, R * qw));
-  ETC_TRY(dalloc(dec, &dec->kh, R * kvw));
-  ETC_TRY(dalloc(dec, &dec->vh, R * kvw));
   ETC_TRY(dalloc(dec, &dec->qr, R * qw));
-  ETC_TRY(dalloc(dec, &dec->kr, R * kvw));
-  ETC_TRY(dalloc(dec, &dec->att, R * qw));
   ETC_TRY(dalloc(dec, &dec->attl, R * qw));
   ETC_TRY(dalloc(dec, &dec->proj, R * std::max<size_t>(c.d_model, 1)));
   ETC_TRY(dalloc(dec, &dec->g, R * c.ffn));
@@ -998,8 +1029,8 @@ etc_status etc_decoder_destroy(etc_decoder* dec) {
   for (auto* list : {&dec->t_qkv, &dec->t_o, &dec->t_gu, &dec->t_down})
     for (etc_qweight* w : *list) destroy_qweight(w);
   destroy_qweight(dec->t_head);
-  for (void* p : {(void*)dec->d_inv_freq, (void*)dec->hidden, (void*)dec->normed, (void*)dec->qkv, (void*)dec->qh, (void*)dec->kh,
-                  (void*)dec->vh, (void*)dec->qr, (void*)dec->kr, (void*)dec->att, (void*)dec->attl, (void*)dec->proj, (void*)dec->g,
+  for (void* p : {(void*)dec->d_inv_freq, (void*)dec->hidden, (void*)dec->normed, (void*)dec->qkv,
+                  (void*)dec->qr, (void*)dec->attl, (void*)dec->proj, (void*)dec->g,
                   (void*)dec->u, (void*)dec->act, (void*)dec->last, (void*)dec->logits, (void*)dec->lin_scratch, (void*)dec->xh_norm,
                   (void*)dec->xh_att, (void*)dec->xh_act,
                   (void*)dec->attn_scratch, (void*)dec->exact_scratch, (void*)dec->d_ids, (void*)dec->d_cursors, (void*)dec->d_tokens,

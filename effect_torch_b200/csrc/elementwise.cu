@@ -17,14 +17,105 @@
 
 namespace etc {
 
+// silu(gate) * up as the reference's expression interpreter evaluates it, see swiglu_kernel.
+__device__ __forceinline__ float swiglu_value(float g, float up, int exact) {
+  const float half_g = __fdiv_rn(g, 2.0f);
+  const float th = exact ? (float)tanh((double)half_g) : tanhf(half_g);
+  const float sig = __fadd_rn(__fdiv_rn(th, 2.0f), 0.5f);
+  return __fmul_rn(__fmul_rn(g, sig), up);
+}
+
 // --------------------------------------------------------------------------------------------
-// Dense linear, bit-exact with the reference: every output element is one sequential fmaf chain
-// over k (out = fma(x[m,k], W[n,k], out)). A CTA computes 32 outputs x 8 input rows; W is staged
-// 32 columns at a time through shared memory so global reads stay coalesced.
+// Dense linear, bit-exact with the reference: every output element is one sequential fmaf chain over k
+// (out = fma(x[m,k], W[n,k], out)), four cycles per k whatever is done, so for the small models that run in f32 what counts is
+// that nothing else adds to the chain: a ring of four 64-column stages filled by cp.async (one exposed load latency per
+// launch instead of one per 32 columns), 16-byte shared-memory reads (rows padded to 272 bytes: conflict free), launches
+// chained, and up to three weights per launch (q, k and v side by side in one output; gate and up with the SwiGLU between
+// them; the residual added on the way out). A CTA computes 32 outputs x 8 * MT input rows; MT = 4 reuses a weight read for
+// four rows' chains where there are that many.
 // --------------------------------------------------------------------------------------------
+constexpr int kDenseK = 64, kDenseStages = 4, kDensePad = kDenseK + 4;
+
+template <int MT, bool SWIGLU>
+struct DenseCfg {
+  static constexpr int kRowsW = 32 * (SWIGLU ? 2 : 1), kRowsX = 8 * MT;
+  static constexpr int kStageFloats = (kRowsW + kRowsX) * kDensePad;
+  static constexpr size_t kSmemBytes = (size_t)kDenseStages * kStageFloats * sizeof(float);
+};
+
+template <int MT, bool SWIGLU>
+__global__ void __launch_bounds__(256) dense_linear_kernel(DenseArgs a) {
+  using Cfg = DenseCfg<MT, SWIGLU>;
+  chain_release();
+  extern __shared__ __align__(16) float ring[];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // output within the tile, input row within the tile
+  int tile = blockIdx.x, part = 0;
+  if (!SWIGLU)
+    while (part + 1 < a.parts && tile >= (int)((a.n[part] + 31) / 32)) tile -= (int)((a.n[part++] + 31) / 32);
+  const int64_t n = a.n[part], n0 = (int64_t)tile * 32, m0 = (int64_t)blockIdx.y * Cfg::kRowsX;
+  const int k = (int)a.k, chunks = (k + kDenseK - 1) / kDenseK;
+  // rows beyond the matrix repeat its last one: their results are not stored
+  auto fill = [&](int chunk, bool weights, bool inputs) {
+    float* stage = ring + (chunk % kDenseStages) * Cfg::kStageFloats;
+    for (int i = threadIdx.x; i < (Cfg::kRowsW + Cfg::kRowsX) * (kDenseK / 4); i += 256) {
+      const int row = i / (kDenseK / 4), c = chunk * kDenseK + 4 * (i % (kDenseK / 4));
+      const bool is_w = row < Cfg::kRowsW;
+      if (c >= k || !(is_w ? weights : inputs)) continue;
+      const float* src = is_w ? a.w[SWIGLU ? row / 32 : part] + min(n0 + row % 32, n - 1) * k + c : a.x + min(m0 + row - Cfg::kRowsW, a.m - 1) * k + c;
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(stage + row * kDensePad + 4 * (i % (kDenseK / 4)));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    }
+  };
+  auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+  // the first stages' weights depend on no earlier kernel of the decoder's step (a.constant_weights)
+  if (a.constant_weights)
+    for (int c = 0; c < kDenseStages - 1; ++c) fill(c, c < chunks, false);
+  chain_wait();
+  for (int c = 0; c < kDenseStages - 1; ++c) {
+    fill(c, c < chunks && !a.constant_weights, c < chunks);
+    commit();
+  }
+  float acc[MT] = {}, up[MT] = {};
+  for (int c = 0; c < chunks; ++c) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kDenseStages - 2) : "memory");
+    __syncthreads();
+    if (c + kDenseStages - 1 < chunks) fill(c + kDenseStages - 1, true, true);
+    commit();
+    const float* stage = ring + (c % kDenseStages) * Cfg::kStageFloats;
+    const int len = min(kDenseK, k - c * kDenseK);
+#pragma unroll 4
+    for (int kk = 0; kk < len; kk += 4) {
+      const float4 w = *reinterpret_cast<const float4*>(stage + tx * kDensePad + kk);
+      float4 w2;
+      if (SWIGLU) w2 = *reinterpret_cast<const float4*>(stage + (32 + tx) * kDensePad + kk);
+#pragma unroll
+      for (int t = 0; t < MT; ++t) {
+        const float4 x = *reinterpret_cast<const float4*>(stage + (Cfg::kRowsW + ty + 8 * t) * kDensePad + kk);
+        acc[t] = fmaf(x.w, w.w, fmaf(x.z, w.z, fmaf(x.y, w.y, fmaf(x.x, w.x, acc[t]))));
+        if (SWIGLU) up[t] = fmaf(x.w, w2.w, fmaf(x.z, w2.z, fmaf(x.y, w2.y, fmaf(x.x, w2.x, up[t]))));
+      }
+    }
+  }
+  const int64_t col = n0 + tx;
+  if (col >= n) return;
+#pragma unroll
+  for (int t = 0; t < MT; ++t) {
+    const int64_t row = m0 + ty + 8 * t;
+    if (row >= a.m) break;
+    const int64_t at = row * a.out_stride + col;
+    if (SWIGLU) {
+      a.out[0][at] = swiglu_value(acc[t], up[t], a.exact);
+    } else {
+      const float v = a.bias ? acc[t] + a.bias[col] : acc[t];
+      a.out[part][at] = a.residual ? __fadd_rn(a.residual[at], v) : v;
+    }
+  }
+}
+
+// The same chain for operands that 16-byte copies cannot fetch (k not a multiple of 4, unaligned pointers).
 __global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict__ x, int64_t m, int64_t k,
                                                          const float* __restrict__ w, int64_t n,
-                                                         const float* __restrict__ bias, float* __restrict__ out) {
+                                                         const float* __restrict__ bias, const float* residual, float* out, int64_t out_stride) {
   __shared__ float ws[32][33];
   __shared__ float xs[8][32];
   const int tx = threadIdx.x, ty = threadIdx.y;  // tx: output column within tile, ty: input row within tile
@@ -46,15 +137,49 @@ __global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict
     __syncthreads();
   }
   const int64_t mm = m0 + ty, nn = n0 + tx;
-  if (mm < m && nn < n) out[mm * n + nn] = bias ? acc + bias[nn] : acc;
+  if (mm < m && nn < n) {
+    const float v = bias ? acc + bias[nn] : acc;
+    out[mm * out_stride + nn] = residual ? __fadd_rn(residual[mm * out_stride + nn], v) : v;
+  }
+}
+
+bool dense_linear_supported(const DenseArgs& a) {
+  if (a.k <= 0 || a.k % 4 != 0 || a.k > INT32_MAX || ((uintptr_t)a.x % 16) != 0) return false;
+  for (const float* w : a.w)
+    if (((uintptr_t)w % 16) != 0) return false;
+  return true;
+}
+
+template <int MT, bool SWIGLU>
+static cudaError_t launch_dense_t(const DenseArgs& a, cudaStream_t stream) {
+  constexpr size_t smem = DenseCfg<MT, SWIGLU>::kSmemBytes;
+  auto kernel = dense_linear_kernel<MT, SWIGLU>;
+  const cudaError_t attr = opt_in_shared_memory(kernel, smem);
+  if (attr != cudaSuccess) return attr;
+  unsigned tiles = 0;
+  for (int p = 0; p < (SWIGLU ? 1 : a.parts); ++p) tiles += (unsigned)((a.n[p] + 31) / 32);
+  return launch_chained(kernel, dim3(tiles, (unsigned)((a.m + 8 * MT - 1) / (8 * MT))), dim3(256), smem, stream, a);
+}
+
+cudaError_t launch_dense_linear(const DenseArgs& a, cudaStream_t stream) {
+  if (a.m == 0 || a.n[0] == 0) return cudaSuccess;
+  if (!dense_linear_supported(a)) {
+    if (a.swiglu) return cudaErrorInvalidValue;
+    for (int p = 0; p < a.parts; ++p) {
+      const dim3 grid((unsigned)((a.n[p] + 31) / 32), (unsigned)((a.m + 7) / 8));
+      linear_f32_kernel<<<grid, dim3(32, 8), 0, stream>>>(a.x, a.m, a.k, a.w[p], a.n[p], a.bias, a.residual, a.out[p], a.out_stride);
+    }
+    return cudaGetLastError();
+  }
+  if (a.m > 16) return a.swiglu ? launch_dense_t<4, true>(a, stream) : launch_dense_t<4, false>(a, stream);
+  return a.swiglu ? launch_dense_t<1, true>(a, stream) : launch_dense_t<1, false>(a, stream);
 }
 
 cudaError_t launch_linear_f32(const float* x, int64_t m, int64_t k, const float* w, int64_t n, const float* bias,
                               float* out, cudaStream_t stream) {
-  if (m == 0 || n == 0) return cudaSuccess;
-  dim3 block(32, 8), grid((unsigned)((n + 31) / 32), (unsigned)((m + 7) / 8));
-  linear_f32_kernel<<<grid, block, 0, stream>>>(x, m, k, w, n, bias, out);
-  return cudaGetLastError();
+  DenseArgs a;
+  a.x = x; a.m = m; a.k = k; a.w[0] = w; a.n[0] = n; a.out[0] = out; a.out_stride = n; a.bias = bias;
+  return launch_dense_linear(a, stream);
 }
 
 // --------------------------------------------------------------------------------------------
@@ -247,11 +372,7 @@ cudaError_t launch_rope(const float* x, const int64_t* offsets, int64_t n_offset
 __global__ void swiglu_kernel(const float* __restrict__ gate, const float* __restrict__ up, int64_t n,
                               float* __restrict__ out, int exact) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float g = gate[i];
-    const float half_g = __fdiv_rn(g, 2.0f);
-    const float th = exact ? (float)tanh((double)half_g) : tanhf(half_g);
-    const float sig = __fadd_rn(__fdiv_rn(th, 2.0f), 0.5f);
-    out[i] = __fmul_rn(__fmul_rn(g, sig), up[i]);
+    out[i] = swiglu_value(gate[i], up[i], exact);
   }
 }
 cudaError_t launch_swiglu(const float* gate, const float* up, int64_t n, float* out, int exact, cudaStream_t stream) {
@@ -394,38 +515,6 @@ cudaError_t launch_embedding_f32(const void* indexes, int index_is_i64, int64_t 
     return launch_chained(embedding_f32_kernel<long long>, grid, dim3(256), 0, stream, (const long long*)indexes, count, table, rows, columns, out, status);
   else
     return launch_chained(embedding_f32_kernel<unsigned int>, grid, dim3(256), 0, stream, (const unsigned int*)indexes, count, table, rows, columns, out, status);
-  return cudaGetLastError();
-}
-
-// [B,T,H*D] (row stride src_row_stride floats) -> [B,H,T,D]
-__global__ void heads_first_kernel(const float* __restrict__ src, float* __restrict__ dst, int64_t B, int64_t T, int64_t H,
-                                   int64_t D, int64_t src_row_stride) {
-  const int64_t total = B * H * T * D;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t d = idx % D, t = (idx / D) % T, h = (idx / (D * T)) % H, b = idx / (D * T * H);
-    dst[idx] = src[(b * T + t) * src_row_stride + h * D + d];
-  }
-}
-cudaError_t launch_heads_first(const float* src, float* dst, int64_t B, int64_t T, int64_t H, int64_t D,
-                               int64_t src_row_stride, cudaStream_t stream) {
-  const int64_t total = B * H * T * D;
-  if (total == 0) return cudaSuccess;
-  heads_first_kernel<<<(unsigned)std::min<int64_t>((total + 255) / 256, 148 * 8), 256, 0, stream>>>(src, dst, B, T, H, D, src_row_stride);
-  return cudaGetLastError();
-}
-// [B,H,T,D] -> [B,T,H*D]
-__global__ void heads_last_kernel(const float* __restrict__ src, float* __restrict__ dst, int64_t B, int64_t T, int64_t H,
-                                  int64_t D) {
-  const int64_t total = B * H * T * D;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t d = idx % D, h = (idx / D) % H, t = (idx / (D * H)) % T, b = idx / (D * H * T);
-    dst[idx] = src[((b * H + h) * T + t) * D + d];
-  }
-}
-cudaError_t launch_heads_last(const float* src, float* dst, int64_t B, int64_t T, int64_t H, int64_t D, cudaStream_t stream) {
-  const int64_t total = B * H * T * D;
-  if (total == 0) return cudaSuccess;
-  heads_last_kernel<<<(unsigned)std::min<int64_t>((total + 255) / 256, 148 * 8), 256, 0, stream>>>(src, dst, B, T, H, D);
   return cudaGetLastError();
 }
 

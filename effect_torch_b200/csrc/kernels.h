@@ -16,7 +16,7 @@ cudaError_t launch_dequantize(int codec, const uint8_t* packed, int64_t rows, in
 cudaError_t launch_quantize(int codec, const float* x, int64_t rows, int64_t columns, uint8_t* packed,
                             cudaStream_t stream);
 cudaError_t launch_qlinear_generic(int codec, const float* x, int64_t vectors, int64_t columns, const uint8_t* weight,
-                                   int64_t rows, const float* bias, float* out, cudaStream_t stream, int* launches);
+                                   int64_t rows, const float* bias, float* out, cudaStream_t stream, int* launches, int64_t out_stride = 0);
 cudaError_t launch_qembedding(int codec, const void* indexes, int index_is_i64, int64_t count, const uint8_t* weight,
                               int64_t rows, int64_t columns, float* out, DeviceStatus* status, cudaStream_t stream);
 
@@ -172,6 +172,23 @@ cudaError_t launch_tp_pick(const PeerView& view, int batch, uint32_t* tokens, ui
                            DeviceStatus* status, cudaStream_t stream);
 
 // ---- dense / elementwise (elementwise.cu) --------------------------------------------------
+// Dense f32 linear(s) over one input: out[p][row, col] = x W[p]^T for up to three weights of one launch, all with row stride
+// out_stride. `residual` (same layout as the one output) is added; `swiglu`: two weights of n[0] rows, silu(gate) * up.
+struct DenseArgs {
+  const float* x = nullptr;
+  int64_t m = 0, k = 0;
+  const float* w[3] = {};
+  int64_t n[3] = {};
+  float* out[3] = {};
+  int64_t out_stride = 0;
+  int parts = 1;
+  const float* bias = nullptr;      // parts == 1 only
+  const float* residual = nullptr;  // parts == 1 only
+  int swiglu = 0, exact = 0;
+  int constant_weights = 0;         // no earlier kernel of the stream writes the weights: they are fetched ahead of it
+};
+bool dense_linear_supported(const DenseArgs& a);  // k a multiple of 4, 16-byte aligned operands
+cudaError_t launch_dense_linear(const DenseArgs& a, cudaStream_t stream);
 cudaError_t launch_linear_f32(const float* x, int64_t m, int64_t k, const float* w, int64_t n, const float* bias,
                               float* out, cudaStream_t stream);
 cudaError_t launch_rmsnorm(const float* x, const float* weight, double eps, int64_t rows, int64_t n, float* out,
@@ -190,11 +207,6 @@ cudaError_t launch_sample_rows(const float* logits, int64_t rows, int64_t vocab,
                                DeviceStatus* status, cudaStream_t stream);
 cudaError_t launch_embedding_f32(const void* indexes, int index_is_i64, int64_t count, const float* table, int64_t rows,
                                  int64_t columns, float* out, DeviceStatus* status, cudaStream_t stream);
-// [B,T,H*D] <-> [B,H,T,D] (the reshape/transpose pairs around attention)
-cudaError_t launch_heads_first(const float* src, float* dst, int64_t B, int64_t T, int64_t H, int64_t D, int64_t src_row_stride,
-                               cudaStream_t stream);
-cudaError_t launch_heads_last(const float* src, float* dst, int64_t B, int64_t T, int64_t H, int64_t D,
-                              cudaStream_t stream);
 // Copy row (advance-1) of each lane's [T, width] block into [lanes, width] (LastTokenRow).
 cudaError_t launch_last_token_rows(const float* src, int64_t lanes, int64_t steps, int64_t width, int64_t advance,
                                    float* out, cudaStream_t stream);
@@ -219,11 +231,11 @@ struct LaneInfo {
 cudaError_t launch_kv_append(const PoolView& pool, const float* k, const float* v, const LaneInfo* lanes,
                              const int* tables, int batch, int tokens, int64_t lane_stride, int64_t head_stride,
                              int64_t token_stride, cudaStream_t stream);
-// Reference-order attention in f64 (any tier, any block size, window). q/out [B,Hq,T,D] f32.
+// Reference-order attention in f64 (any tier, any block size, window). q/out [B,Hq,T,D] f32, or [B,T,Hq,D].
 // scratch: f64 [B*Hq*T][max_ctx]. op_window < 0: none.
 cudaError_t launch_attention_exact(const PoolView& pool, const float* q, const LaneInfo* lanes, const int* tables,
                                    int batch, int q_heads, int tokens, double scale, long long op_window, float* out,
-                                   double* scratch, int max_ctx, cudaStream_t stream);
+                                   double* scratch, int max_ctx, cudaStream_t stream, bool tokens_first = false);
 // Tensor-core flash-decoding over the block table (f16/bf16 tiers, block_size 16, head_dim 64/128,
 // one query token per lane). q [B,Hq,D] f32; out [B,Hq,D] f32. partial scratch for splits > 1.
 struct AttnPlan {

@@ -265,7 +265,7 @@ template <int CODEC, int VC, int RG, bool WIDE>
 __global__ void __launch_bounds__(kRawWarps * 32, 2) qlinear_raw_kernel(const float* __restrict__ x, int vectors, int64_t columns,
                                                                         const uint8_t* __restrict__ weight, int64_t rows,
                                                                         const float* __restrict__ bias, float* __restrict__ out,
-                                                                        int chunk_windows) {
+                                                                        int64_t out_stride, int chunk_windows) {
   extern __shared__ __align__(16) float4 staged[];  // [four windows][vector][8 quads][4 windows x 8 threads]
   constexpr int kValues = CodecTraits<CODEC>::kValues, kBytes = CodecTraits<CODEC>::kBytes;
   constexpr int kWindowBytes = 256 / kValues * kBytes;
@@ -346,14 +346,14 @@ __global__ void __launch_bounds__(kRawWarps * 32, 2) qlinear_raw_kernel(const fl
         float t = __uint_as_float((uint32_t)acc[g][v]) + __uint_as_float((uint32_t)(acc[g][v] >> 32));
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
-        if (lane == (g * VC + v) % 32 && row0 + g < rows && v0 + v < vectors) out[(int64_t)(v0 + v) * rows + row0 + g] = t + (bias ? bias[row0 + g] : 0.0f);
+        if (lane == (g * VC + v) % 32 && row0 + g < rows && v0 + v < vectors) out[(int64_t)(v0 + v) * out_stride + row0 + g] = t + (bias ? bias[row0 + g] : 0.0f);
       }
   }
 }
 
 template <int CODEC, int VC, int RG>
 cudaError_t launch_qlinear_raw(const float* x, int64_t vectors, int64_t columns, const uint8_t* weight, int64_t rows, const float* bias,
-                               float* out, cudaStream_t stream) {
+                               float* out, int64_t out_stride, cudaStream_t stream) {
   const int windows = (int)((columns + 255) / 256);
   const int chunk = std::min((windows + 3) / 4 * 4, kRawStageBytes / (VC * 4096) * 4);
   const bool wide = kWideBlocks<CODEC> && (reinterpret_cast<uintptr_t>(weight) & 15) == 0;
@@ -363,35 +363,36 @@ cudaError_t launch_qlinear_raw(const float* x, int64_t vectors, int64_t columns,
   const int64_t groups = (rows + RG - 1) / RG;
   const unsigned grid = (unsigned)std::min<int64_t>((groups + kRawWarps - 1) / kRawWarps, 148 * 2);
   kernel<<<dim3(grid, (unsigned)((vectors + VC - 1) / VC)), kRawWarps * 32, (size_t)chunk * VC * 1024, stream>>>(x, (int)vectors, columns, weight, rows, bias,
-                                                                                                                 out, chunk);
+                                                                                                                 out, out_stride, chunk);
   return cudaGetLastError();
 }
 // Rows of a warp: four, unless that leaves warps without any (below 148 SMs x 16 warps x 2).
 template <int CODEC, int VC>
 cudaError_t launch_qlinear_raw(const float* x, int64_t vectors, int64_t columns, const uint8_t* weight, int64_t rows, const float* bias,
-                               float* out, cudaStream_t stream) {
-  if (rows > 148 * 32) return launch_qlinear_raw<CODEC, VC, 4>(x, vectors, columns, weight, rows, bias, out, stream);
-  return launch_qlinear_raw<CODEC, VC, 1>(x, vectors, columns, weight, rows, bias, out, stream);
+                               float* out, int64_t out_stride, cudaStream_t stream) {
+  if (rows > 148 * 32) return launch_qlinear_raw<CODEC, VC, 4>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
+  return launch_qlinear_raw<CODEC, VC, 1>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
 }
 
 struct GenericLaunch {
-  const float* x; int64_t vectors, columns; const uint8_t* weight; int64_t rows; const float* bias; float* out;
+  const float* x; int64_t vectors, columns; const uint8_t* weight; int64_t rows; const float* bias; float* out; int64_t out_stride;
   cudaStream_t stream; cudaError_t err; int launches;
   template <int CODEC> void operator()() {
     err = cudaSuccess;
     if (rows == 0 || vectors == 0) return;
     ++launches;
     // a pass over the weights serves up to 8 vectors; passes of one launch share their rows' bytes in L2
-    if (vectors <= 1) err = launch_qlinear_raw<CODEC, 1>(x, vectors, columns, weight, rows, bias, out, stream);
-    else if (vectors <= 2) err = launch_qlinear_raw<CODEC, 2>(x, vectors, columns, weight, rows, bias, out, stream);
-    else if (vectors <= 4) err = launch_qlinear_raw<CODEC, 4>(x, vectors, columns, weight, rows, bias, out, stream);
-    else if (vectors <= 6) err = launch_qlinear_raw<CODEC, 6>(x, vectors, columns, weight, rows, bias, out, stream);
-    else err = launch_qlinear_raw<CODEC, 8>(x, vectors, columns, weight, rows, bias, out, stream);
+    if (vectors <= 1) err = launch_qlinear_raw<CODEC, 1>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
+    else if (vectors <= 2) err = launch_qlinear_raw<CODEC, 2>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
+    else if (vectors <= 4) err = launch_qlinear_raw<CODEC, 4>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
+    else if (vectors <= 6) err = launch_qlinear_raw<CODEC, 6>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
+    else err = launch_qlinear_raw<CODEC, 8>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
   }
 };
 cudaError_t launch_qlinear_generic(int codec, const float* x, int64_t vectors, int64_t columns, const uint8_t* weight,
-                                   int64_t rows, const float* bias, float* out, cudaStream_t stream, int* launches) {
-  GenericLaunch l{x, vectors, columns, weight, rows, bias, out, stream, cudaSuccess, 0};
+                                   int64_t rows, const float* bias, float* out, cudaStream_t stream, int* launches,
+                                   int64_t out_stride) {
+  GenericLaunch l{x, vectors, columns, weight, rows, bias, out, out_stride ? out_stride : rows, stream, cudaSuccess, 0};
   if (!dispatch_codec(codec, l)) return cudaErrorInvalidValue;
   if (launches) *launches += l.launches;
   return l.err;

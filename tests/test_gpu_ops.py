@@ -87,6 +87,17 @@ def test_argmax_large_rows_and_non_finite_logits():
         rt.synchronize()
 
 
+@pytest.mark.parametrize("m,k,n", [(1, 4, 1), (16, 64, 33), (17, 68, 31), (33, 260, 65), (5, 192, 640), (3, 66, 40)])
+def test_dense_linear_at_the_edges_of_its_tiles(m, k, n):
+    """Stages that are not full, rows and columns that do not fill a tile, both row counts per CTA, and a k that 16-byte copies
+    cannot fetch: every element one fused multiply-add chain over k, bit for bit."""
+    rng = np.random.default_rng(m + k + n)
+    x, w = rng.normal(size=(m, k)).astype(np.float32), rng.normal(size=(n, k)).astype(np.float32)
+    out = empty((m, n))
+    runtime().linear_f32_into(dev(x), m, k, dev(w), n, None, out)
+    np.testing.assert_array_equal(host(out), orc.linear_rows(x, w, threads=4))
+
+
 def test_sample_row_replays_the_reference_stream():
     rng = np.random.default_rng(6)
     logits = rng.normal(size=512).astype(np.float32)
