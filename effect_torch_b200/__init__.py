@@ -10,6 +10,9 @@ without the built library, or calling them without a CUDA device, raises.
 from __future__ import annotations
 
 import ctypes as C
+import sys
+import threading
+import weakref
 
 import numpy as np
 
@@ -50,6 +53,33 @@ def _ptr(t):
     if isinstance(t, np.ndarray):
         return C.c_void_p(t.ctypes.data)
     return C.c_void_p(t.data_ptr())
+
+
+# Results of up to this many bytes at a time sit in page-locked memory, which the device writes without a detour through a
+# staging buffer. It comes from torch's caching host allocator, so that it costs neither a registration nor fresh pages once
+# an earlier result has been released; Runtime.close() gives the cache back.
+_PAGE_LOCKED_MOST = 256 << 20
+_page_locked_lock = threading.RLock()  # a finalizer may run while its thread holds it
+_page_locked_bytes = 0
+
+
+def _page_locked_add(nbytes: int) -> bool:
+    global _page_locked_bytes
+    with _page_locked_lock:
+        if nbytes > 0 and _page_locked_bytes + nbytes > _PAGE_LOCKED_MOST:
+            return False
+        _page_locked_bytes += nbytes
+        return True
+
+
+def _result_buffer(shape) -> np.ndarray:
+    nbytes = 4 * int(np.prod(shape))
+    if nbytes == 0 or not _page_locked_add(nbytes):
+        return np.empty(shape, dtype=np.float32)
+    import torch
+    array = torch.empty(shape, dtype=torch.float32, pin_memory=True).numpy()
+    weakref.finalize(array, _page_locked_add, -nbytes).atexit = False
+    return array
 
 
 def device_count() -> int:
@@ -107,6 +137,9 @@ class Runtime:
         if getattr(self, "h", None):
             self.L.etc_runtime_destroy(self.h)
             self.h = None
+            torch = sys.modules.get("torch")
+            if torch is not None and hasattr(torch._C, "_host_emptyCache"):
+                torch._C._host_emptyCache()
 
     def __del__(self):
         try:
@@ -467,7 +500,7 @@ class Executable:
     def execute(self, pool, seqs, tokens, cancelled: bool = False) -> np.ndarray:
         tokens = np.ascontiguousarray(tokens, dtype=np.uint32)
         active, advance = tokens.shape
-        logits = np.empty((active, self.vocab), dtype=np.float32)
+        logits = _result_buffer((active, self.vocab))
         flag = C.c_int(int(cancelled))
         _check(self.rt.L.etc_decoder_execute(self.h, pool.h, self._seq_array(seqs), active, _ptr(tokens), advance, _ptr(logits),
                                              C.cast(C.byref(flag), C.c_void_p)))

@@ -871,8 +871,8 @@ cudaError_t launch_rope_append(const PoolView& pool, const float* qkv, const Lan
 }
 
 __global__ void record_step_kernel(const uint32_t* __restrict__ tokens, uint32_t* __restrict__ ids,
-                                   uint32_t* __restrict__ history, int* step_counter, LaneInfo* lanes, int64_t* cursors,
-                                   int batch, long long window) {
+                                   uint32_t* __restrict__ history, int* step_counter, LaneInfo* lanes, int batch,
+                                   long long window) {
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   chain_wait();
   const int step = *step_counter;
@@ -882,7 +882,6 @@ __global__ void record_step_kernel(const uint32_t* __restrict__ tokens, uint32_t
     history[(size_t)step * batch + i] = tok;
     if (lanes[i].advance > 0) {
       lanes[i].cursor += 1;
-      cursors[i] += 1;
       if (window >= 0) lanes[i].start = (int)max((long long)lanes[i].cursor + 1 - window, 0ll);
     }
   }
@@ -890,8 +889,8 @@ __global__ void record_step_kernel(const uint32_t* __restrict__ tokens, uint32_t
   if (threadIdx.x == 0) *step_counter = step + 1;
 }
 cudaError_t launch_record_step(const uint32_t* tokens, uint32_t* ids, uint32_t* history, int* step_counter, LaneInfo* lanes,
-                               int64_t* cursors, int batch, long long window, cudaStream_t stream) {
-  return launch_chained(record_step_kernel, dim3(1), dim3(128), 0, stream, tokens, ids, history, step_counter, lanes, cursors, batch, window);
+                               int batch, long long window, cudaStream_t stream) {
+  return launch_chained(record_step_kernel, dim3(1), dim3(128), 0, stream, tokens, ids, history, step_counter, lanes, batch, window);
 }
 
 // Debug/test read-back of logical token rows (row = block*block_size + offset) as f32

@@ -60,7 +60,7 @@ struct etc_runtime {
   int sm_count = 0;
   cudaStream_t stream = nullptr;
   etc::DeviceStatus* d_status = nullptr;
-  etc::DeviceStatus* h_status = nullptr;  // pinned
+  etc::DeviceStatus* h_status = nullptr;  // the same word, in mapped pinned memory
   uint32_t* d_sampled = nullptr;          // one token: etc_sample_row's device output and its pinned copy
   uint32_t* h_sampled = nullptr;
   void* d_workspace = nullptr;

@@ -61,8 +61,12 @@ struct etc_decoder {
   size_t attn_scratch_bytes = 0;
   double* exact_scratch = nullptr;
   size_t exact_scratch_bytes = 0;
-  uint32_t* d_ids = nullptr;       // [batch * max_advance] token ids
-  int64_t* d_cursors = nullptr;    // [batch] i64 cursors for RoPE
+  // what the host refreshes before a step is one block in pinned memory and one in device memory, so that it travels as one
+  // copy of what the step needs: lanes [batch], token ids [batch * max_advance], then the live block tables packed
+  unsigned char *h_inputs = nullptr, *d_inputs = nullptr;
+  size_t inputs_bytes = 0, tables_offset = 0;
+  size_t staged_tables = 0;        // ints of tables staged for the next step
+  uint32_t* d_ids = nullptr;
   uint32_t* d_tokens = nullptr;    // [batch] sampled tokens
   uint32_t* d_history = nullptr;   // generate_greedy: [steps][batch]
   size_t history_capacity = 0;
@@ -72,7 +76,6 @@ struct etc_decoder {
   int max_blocks = 0;
   // pinned staging
   uint32_t* h_ids = nullptr;
-  int64_t* h_cursors = nullptr;
   LaneInfo* h_lanes = nullptr;
   int* h_tables = nullptr;
   uint32_t* h_tokens = nullptr;
@@ -442,7 +445,7 @@ etc_status enqueue_step(StepContext& s) {
                             d->rt->d_status, stream));
     s.launches += 2;
   } else {
-    ETC_CUDA(launch_argmax(d->logits, B, c.vocab, d->d_tokens, d->rt->d_status, stream));
+    ETC_CUDA(launch_argmax(d->logits, B, c.vocab, d->d_tokens, d->rt->d_status, stream, nullptr, 0, d->h_tokens));
     ++s.launches;
   }
   return ETC_OK;
@@ -501,7 +504,7 @@ etc_status begin(etc_decoder* dec, etc_pool* pool, etc_seq* const* seqs, int act
   ctx.max_ctx = 1;
   ctx.max_pages = 1;
   std::memset(dec->h_lanes, 0, sizeof(LaneInfo) * (size_t)c.batch);
-  std::memset(dec->h_cursors, 0, sizeof(int64_t) * (size_t)c.batch);
+  dec->staged_tables = 0;
   std::memset(dec->h_ids, 0, sizeof(uint32_t) * (size_t)c.batch * (size_t)advance);  // pad lanes feed token 0
   for (int i = 0; i < active; ++i) {
     etc_seq* s = seqs[i];
@@ -526,9 +529,9 @@ etc_status begin(etc_decoder* dec, etc_pool* pool, etc_seq* const* seqs, int act
       tx.rollback();
       return fail(ETC_EXECUTION, "execute: block table exceeds the compiled capacity");
     }
-    info.table_offset = i * dec->max_blocks - (int)s->head;
-    for (size_t b = 0; b < live; ++b) dec->h_tables[(size_t)i * dec->max_blocks + b] = (int)s->blocks[s->head + b];
-    dec->h_cursors[i] = (int64_t)cursor;
+    info.table_offset = (int)dec->staged_tables - (int)s->head;
+    if (live > 0) std::memcpy(dec->h_tables + dec->staged_tables, s->blocks.data() + s->head, live * sizeof(uint32_t));
+    dec->staged_tables += live;
     ctx.max_ctx = std::max(ctx.max_ctx, (int)(needed - start));
     const int first_page = info.start / c.block_size;
     ctx.max_pages = std::max(ctx.max_pages, (int)((needed + c.block_size - 1) / c.block_size) - first_page);
@@ -537,13 +540,9 @@ etc_status begin(etc_decoder* dec, etc_pool* pool, etc_seq* const* seqs, int act
   return ETC_OK;
 }
 
-etc_status upload_step_inputs(etc_decoder* dec, int advance) {
-  const etc_decoder_config& c = dec->cfg;
-  cudaStream_t stream = dec->rt->stream;
-  ETC_CUDA(cudaMemcpyAsync(dec->d_lanes, dec->h_lanes, sizeof(LaneInfo) * (size_t)c.batch, cudaMemcpyHostToDevice, stream));
-  ETC_CUDA(cudaMemcpyAsync(dec->d_tables, dec->h_tables, sizeof(int) * (size_t)c.batch * dec->max_blocks, cudaMemcpyHostToDevice, stream));
-  ETC_CUDA(cudaMemcpyAsync(dec->d_cursors, dec->h_cursors, sizeof(int64_t) * (size_t)c.batch, cudaMemcpyHostToDevice, stream));
-  ETC_CUDA(cudaMemcpyAsync(dec->d_ids, dec->h_ids, sizeof(uint32_t) * (size_t)c.batch * advance, cudaMemcpyHostToDevice, stream));
+etc_status upload_step_inputs(etc_decoder* dec) {
+  const size_t bytes = dec->tables_offset + std::max<size_t>(dec->staged_tables, 1) * sizeof(int);
+  ETC_CUDA(cudaMemcpyAsync(dec->d_inputs, dec->h_inputs, bytes, cudaMemcpyHostToDevice, dec->rt->stream));
   return ETC_OK;
 }
 
@@ -560,6 +559,15 @@ etc_status ensure_exact_scratch(etc_decoder* dec, const StepContext& ctx) {
   dec->exact_scratch = (double*)p;
   dec->exact_scratch_bytes = need * 2;
   return ETC_OK;
+}
+
+bool page_locked(const void* p) {
+  cudaPointerAttributes attributes;
+  if (cudaPointerGetAttributes(&attributes, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return attributes.type == cudaMemoryTypeHost;
 }
 
 bool uses_exact_attention(const etc_decoder* dec, const etc_pool* pool, int T) {
@@ -586,7 +594,7 @@ etc_status execute_impl(etc_decoder* dec, etc_pool* pool, etc_seq* const* seqs, 
     etc_status st = ensure_exact_scratch(dec, ctx);
     if (st != ETC_OK) return abort_with(st);
   }
-  etc_status st = upload_step_inputs(dec, advance);
+  etc_status st = upload_step_inputs(dec);
   if (st != ETC_OK) return abort_with(st);
   if (advance == 1 && dec->ran_eagerly && !uses_exact_attention(dec, pool, 1)) {
     const int bucket = (ctx.max_pages + 7) / 8 * 8;
@@ -632,9 +640,13 @@ etc_status execute_impl(etc_decoder* dec, etc_pool* pool, etc_seq* const* seqs, 
   rt->launches += (uint64_t)ctx.launches;
   const etc_decoder_config& c = dec->cfg;
   cudaError_t e = cudaSuccess;
-  if (h_out_tokens) e = cudaMemcpyAsync(dec->h_tokens, dec->d_tokens, sizeof(uint32_t) * (size_t)c.batch, cudaMemcpyDeviceToHost, rt->stream);
+  // the argmax kernel stores its tokens into pinned memory itself; those of a sharded head are settled between the ranks
+  if (h_out_tokens && dec->vocab_global > 0 && dec->tp_world > 1)
+    e = cudaMemcpyAsync(dec->h_tokens, dec->d_tokens, sizeof(uint32_t) * (size_t)c.batch, cudaMemcpyDeviceToHost, rt->stream);
+  // logits go straight into the caller's buffer when that is page-locked, else through the decoder's own
+  float* const logits_to = h_logits && page_locked(h_logits) ? h_logits : dec->h_logits;
   if (e == cudaSuccess && h_logits)
-    e = cudaMemcpyAsync(dec->h_logits, dec->logits, sizeof(float) * (size_t)active * c.vocab, cudaMemcpyDeviceToHost, rt->stream);
+    e = cudaMemcpyAsync(logits_to, dec->logits, sizeof(float) * (size_t)active * c.vocab, cudaMemcpyDeviceToHost, rt->stream);
   if (e != cudaSuccess) {
     fail(ETC_TRANSFER, std::string("readback failed: ") + cudaGetErrorString(e));
     return abort_with(ETC_TRANSFER);
@@ -652,7 +664,7 @@ etc_status execute_impl(etc_decoder* dec, etc_pool* pool, etc_seq* const* seqs, 
     return abort_with(ETC_CANCELLED);
   }
   if (h_out_tokens) std::memcpy(h_out_tokens, dec->h_tokens, sizeof(uint32_t) * (size_t)active);
-  if (h_logits) std::memcpy(h_logits, dec->h_logits, sizeof(float) * (size_t)active * c.vocab);
+  if (h_logits && logits_to != h_logits) std::memcpy(h_logits, dec->h_logits, sizeof(float) * (size_t)active * c.vocab);
   for (int i = 0; i < active; ++i) {
     etc_seq* s = seqs[i];
     const int start = dec->h_lanes[i].start;
@@ -962,13 +974,9 @@ etc_status etc_decoder_finalize(etc_decoder* dec) {
   ETC_TRY(dalloc(dec, &dec->act, R * c.ffn));
   ETC_TRY(dalloc(dec, &dec->last, (size_t)c.batch * c.d_model));
   ETC_TRY(dalloc(dec, &dec->logits, (size_t)c.batch * c.vocab));
-  ETC_TRY(dalloc(dec, &dec->d_ids, R));
-  ETC_TRY(dalloc(dec, &dec->d_cursors, (size_t)c.batch));
   ETC_TRY(dalloc(dec, &dec->d_tokens, (size_t)c.batch));
   ETC_TRY(dalloc(dec, &dec->d_step_counter, 1));
-  ETC_TRY(dalloc(dec, &dec->d_lanes, (size_t)c.batch));
   dec->max_blocks = decoder_max_blocks(c, dec->max_advance);
-  ETC_TRY(dalloc(dec, &dec->d_tables, (size_t)c.batch * dec->max_blocks));
   if (tiled) {
     size_t need = 0;
     // the plan (vector padding, split count) changes at these vector counts; cover every one up to R rows
@@ -998,15 +1006,22 @@ etc_status etc_decoder_finalize(etc_decoder* dec) {
     dec->attn_scratch_bytes = attn_need;
     ETC_TRY(dalloc(dec, &dec->attn_scratch, attn_need / sizeof(float) + 1));
   }
-  cudaError_t e = cudaMallocHost((void**)&dec->h_ids, sizeof(uint32_t) * std::max<size_t>(R, 1));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&dec->h_cursors, sizeof(int64_t) * (size_t)c.batch);
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&dec->h_lanes, sizeof(LaneInfo) * (size_t)c.batch);
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&dec->h_tables, sizeof(int) * (size_t)c.batch * dec->max_blocks);
+  const size_t ids_offset = sizeof(LaneInfo) * (size_t)c.batch;
+  dec->tables_offset = (ids_offset + sizeof(uint32_t) * std::max<size_t>(R, 1) + 15) & ~(size_t)15;
+  dec->inputs_bytes = dec->tables_offset + sizeof(int) * (size_t)c.batch * dec->max_blocks;
+  ETC_TRY(dalloc(dec, &dec->d_inputs, dec->inputs_bytes));
+  dec->d_lanes = (LaneInfo*)dec->d_inputs;
+  dec->d_ids = (uint32_t*)(dec->d_inputs + ids_offset);
+  dec->d_tables = (int*)(dec->d_inputs + dec->tables_offset);
+  cudaError_t e = cudaMallocHost((void**)&dec->h_inputs, dec->inputs_bytes);
+  dec->h_lanes = (LaneInfo*)dec->h_inputs;
+  dec->h_ids = (uint32_t*)(dec->h_inputs + ids_offset);
+  dec->h_tables = (int*)(dec->h_inputs + dec->tables_offset);
   if (e == cudaSuccess) e = cudaMallocHost((void**)&dec->h_tokens, sizeof(uint32_t) * (size_t)c.batch);
   dec->h_logits_bytes = sizeof(float) * (size_t)c.batch * c.vocab;
   if (e == cudaSuccess) e = cudaMallocHost((void**)&dec->h_logits, dec->h_logits_bytes);
   if (e != cudaSuccess) return fail(ETC_COMPILATION, std::string("compile: pinned staging allocation failed: ") + cudaGetErrorString(e));
-  std::memset(dec->h_tables, 0, sizeof(int) * (size_t)c.batch * dec->max_blocks);
+  std::memset(dec->h_inputs, 0, dec->inputs_bytes);
   dec->finalized = true;
   return ETC_OK;
 }
@@ -1033,10 +1048,10 @@ etc_status etc_decoder_destroy(etc_decoder* dec) {
                   (void*)dec->qr, (void*)dec->attl, (void*)dec->proj, (void*)dec->g,
                   (void*)dec->u, (void*)dec->act, (void*)dec->last, (void*)dec->logits, (void*)dec->lin_scratch, (void*)dec->xh_norm,
                   (void*)dec->xh_att, (void*)dec->xh_act,
-                  (void*)dec->attn_scratch, (void*)dec->exact_scratch, (void*)dec->d_ids, (void*)dec->d_cursors, (void*)dec->d_tokens,
-                  (void*)dec->d_history, (void*)dec->d_step_counter, (void*)dec->d_lanes, (void*)dec->d_tables})
+                  (void*)dec->attn_scratch, (void*)dec->exact_scratch, (void*)dec->d_inputs, (void*)dec->d_tokens,
+                  (void*)dec->d_history, (void*)dec->d_step_counter})
     if (p) rt->device_free(p);
-  for (void* p : {(void*)dec->h_ids, (void*)dec->h_cursors, (void*)dec->h_lanes, (void*)dec->h_tables, (void*)dec->h_tokens, (void*)dec->h_logits})
+  for (void* p : {(void*)dec->h_inputs, (void*)dec->h_tokens, (void*)dec->h_logits})
     if (p) cudaFreeHost(p);
   dec->magic = 0;
   delete dec;
@@ -1085,7 +1100,7 @@ etc_status etc_decoder_generate_greedy(etc_decoder* dec, etc_pool* pool, etc_seq
     dec->d_history = (uint32_t*)p;
     dec->history_capacity = (size_t)steps * c.batch;
   }
-  etc_status st = upload_step_inputs(dec, 1);
+  etc_status st = upload_step_inputs(dec);
   if (st != ETC_OK) return abort_with(st);
   cudaError_t e = cudaMemsetAsync(dec->d_step_counter, 0, sizeof(int), rt->stream);
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -1106,7 +1121,7 @@ etc_status etc_decoder_generate_greedy(etc_decoder* dec, etc_pool* pool, etc_seq
     sc.launches = 0;
     sc.max_pages = final_pages;
     ETC_TRY(enqueue_step(sc));
-    ETC_CUDA(launch_record_step(dec->d_tokens, dec->d_ids, dec->d_history, dec->d_step_counter, dec->d_lanes, dec->d_cursors,
+    ETC_CUDA(launch_record_step(dec->d_tokens, dec->d_ids, dec->d_history, dec->d_step_counter, dec->d_lanes,
                                 c.batch, c.window, rt->stream));
     dec->launches_last_step = sc.launches + 1;
     return ETC_OK;

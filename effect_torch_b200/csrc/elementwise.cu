@@ -403,10 +403,10 @@ constexpr int kArgmaxThreads = 512;
 constexpr int kArgmaxSlice = 8192;  // a row is spread over more CTAs until a slice is this short
 
 // `picks` (optional): the row's (best logit bits, index_base + index) pair, for the exchange between the ranks of a
-// vocabulary-parallel head.
+// vocabulary-parallel head. `mirror` (optional): a second copy of the tokens, in page-locked host memory.
 __global__ void __launch_bounds__(kArgmaxThreads) argmax_kernel(const float* __restrict__ logits, int64_t vocab, int64_t slice,
                                                                 uint32_t* __restrict__ tokens, DeviceStatus* status, uint2* picks,
-                                                                uint32_t index_base) {
+                                                                uint32_t index_base, uint32_t* mirror) {
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   chain_wait();
   namespace cg = cooperative_groups;
@@ -471,6 +471,7 @@ __global__ void __launch_bounds__(kArgmaxThreads) argmax_kernel(const float* __r
     // a row of only -inf keeps index 0 like the reference's loop would before it errors
     const uint32_t token = index_base + (best.index == kNone ? 0u : (uint32_t)best.index);
     tokens[row_index] = token;
+    if (mirror) mirror[row_index] = token;
     if (picks) picks[row_index] = make_uint2(__float_as_uint(best.value), token);
     if (best.bad != kNone && atomicCAS(&status->code, kStatusNone, kStatusNonFiniteLogit) == kStatusNone) {
       status->value = best.bad;
@@ -480,13 +481,13 @@ __global__ void __launch_bounds__(kArgmaxThreads) argmax_kernel(const float* __r
   cluster.sync();  // the other CTAs' shared memory lives until it has been read
 }
 cudaError_t launch_argmax(const float* logits, int64_t rows, int64_t vocab, uint32_t* tokens, DeviceStatus* status,
-                          cudaStream_t stream, uint2* picks, uint32_t index_base) {
+                          cudaStream_t stream, uint2* picks, uint32_t index_base, uint32_t* mirror) {
   if (rows == 0) return cudaSuccess;
   unsigned ranks = 1;
   while (ranks < 8 && (vocab + ranks - 1) / ranks > kArgmaxSlice) ranks *= 2;
   const int64_t slice = ((vocab + ranks - 1) / ranks + 3) & ~(int64_t)3;
   return launch_chained_cluster(argmax_kernel, dim3((unsigned)rows * ranks), dim3(kArgmaxThreads), 0, stream, ranks, logits, vocab, slice, tokens, status,
-                                picks, index_base);
+                                picks, index_base, mirror);
 }
 
 // Dense f32 embedding gather with the same bounds rule as the quantized embedding.

@@ -199,7 +199,7 @@ cudaError_t launch_swiglu(const float* gate, const float* up, int64_t n, float* 
 cudaError_t launch_add(const float* a, const float* b, int64_t n, float* out, cudaStream_t stream);
 cudaError_t launch_argmax(const float* logits, int64_t rows, int64_t vocab, uint32_t* tokens, DeviceStatus* status,
                           cudaStream_t stream,
-                          uint2* picks = nullptr, uint32_t index_base = 0);
+                          uint2* picks = nullptr, uint32_t index_base = 0, uint32_t* mirror = nullptr);
 // One token per logits row by temperature / top-k / top-p sampling with the splitmix64 draw (sampling.cu); temperature
 // must be positive here (zero is the argmax kernel's case). seeds / counters: optional per-row device arrays.
 cudaError_t launch_sample_rows(const float* logits, int64_t rows, int64_t vocab, double temperature, int64_t top_k, double top_p,
@@ -259,7 +259,7 @@ cudaError_t launch_rope_append(const PoolView& pool, const float* qkv, const Lan
 // Tail of a device-resident greedy step: feeds the sampled tokens back as the next ids, appends
 // them to the history, and advances every live lane's cursor (and window start) by one.
 cudaError_t launch_record_step(const uint32_t* tokens, uint32_t* ids, uint32_t* history, int* step_counter, LaneInfo* lanes,
-                               int64_t* cursors, int batch, long long window, cudaStream_t stream);
+                               int batch, long long window, cudaStream_t stream);
 cudaError_t launch_pool_read_rows(const PoolView& pool, const uint32_t* rows, int64_t n, float* out, int which,
                                   cudaStream_t stream);
 

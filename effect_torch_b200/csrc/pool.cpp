@@ -10,13 +10,76 @@
 namespace etc {
 
 uint64_t chain_hash(uint64_t previous, const uint32_t* tokens, size_t count) {  // napi/mod.rs:2381-2390
+  // FNV-1a over the tokens' little-endian bytes. A zero byte only multiplies, so the top byte of a token below 2^24 shares
+  // the multiplication of the byte before it: three steps of the serial chain per token instead of four.
+  constexpr uint64_t kPrimeSquared = kHashPrime * kHashPrime;
   uint64_t hash = previous;
-  for (size_t i = 0; i < count; ++i)
-    for (int byte = 0; byte < 4; ++byte) {
-      hash ^= (uint64_t)((tokens[i] >> (8 * byte)) & 0xff);
-      hash *= kHashPrime;
-    }
+  for (size_t i = 0; i < count; ++i) {
+    const uint32_t t = tokens[i];
+    hash = (hash ^ (t & 0xff)) * kHashPrime;
+    hash = (hash ^ ((t >> 8) & 0xff)) * kHashPrime;
+    hash ^= (t >> 16) & 0xff;
+    if (t >> 24) hash = ((hash * kHashPrime) ^ (t >> 24)) * kHashPrime;
+    else hash *= kPrimeSquared;
+  }
   return hash;
+}
+
+void HashIndex::init(size_t blocks) {
+  size_t size = 16;
+  while (size < 2 * blocks) size *= 2;  // at most one slot per block: never more than half full
+  mask = size - 1;
+  slots.assign(size, Slot{0, -1, -1});
+  next.assign(blocks, -1);
+  previous.assign(blocks, -1);
+  listed.assign(blocks, 0);
+}
+size_t HashIndex::find(uint64_t hash) const {
+  size_t at = home(hash);
+  while (slots[at].first >= 0 && slots[at].hash != hash) at = (at + 1) & mask;
+  return at;
+}
+int32_t HashIndex::first(uint64_t hash) const { return slots[find(hash)].first; }
+void HashIndex::append(uint32_t block, uint64_t hash) {
+  Slot& slot = slots[find(hash)];
+  const int32_t b = (int32_t)block;
+  next[block] = -1;
+  previous[block] = slot.first < 0 ? -1 : slot.last;
+  if (slot.first < 0) {
+    slot = Slot{hash, b, b};
+  } else {
+    next[(size_t)slot.last] = b;
+    slot.last = b;
+  }
+  listed[block] = 1;
+}
+void HashIndex::remove(uint32_t block, uint64_t hash) {
+  if (!listed[block]) return;
+  const size_t at = find(hash);
+  Slot& slot = slots[at];
+  const int32_t b = (int32_t)block, moved = slot.last;
+  // take the last block out, then let it stand in for the removed one
+  slot.last = previous[(size_t)moved];
+  if (slot.last >= 0) next[(size_t)slot.last] = -1;
+  if (moved != b) {
+    const int32_t before = previous[block], after = next[block];
+    previous[(size_t)moved] = before;
+    next[(size_t)moved] = after;
+    if (before >= 0) next[(size_t)before] = moved;
+    else slot.first = moved;
+    if (after >= 0) previous[(size_t)after] = moved;
+    else slot.last = moved;
+  }
+  listed[block] = 0;
+  if (slot.last >= 0) return;
+  // the list is empty: close the gap in the probe sequence
+  slot.first = -1;
+  for (size_t hole = at, i = (at + 1) & mask; slots[i].first >= 0; i = (i + 1) & mask) {
+    if (((i - home(slots[i].hash)) & mask) < ((i - hole) & mask)) continue;  // its home lies behind the hole
+    slots[hole] = slots[i];
+    slots[i].first = slots[i].last = -1;
+    hole = i;
+  }
 }
 
 void BlockStore::init(size_t blocks) {
@@ -25,27 +88,13 @@ void BlockStore::init(size_t blocks) {
   refcounts.assign(blocks, 0);
   has_hash.assign(blocks, 0);
   hashes.assign(blocks, 0);
+  by_hash.init(blocks);
 }
-bool BlockStore::is_cached(uint32_t block) const {
-  if (refcounts[block] != 0 || !has_hash[block]) return false;
-  auto it = by_hash.find(hashes[block]);
-  return it != by_hash.end() && std::find(it->second.begin(), it->second.end(), block) != it->second.end();
-}
-void BlockStore::uncache(uint32_t block, uint64_t hash) {
-  auto it = by_hash.find(hash);
-  if (it == by_hash.end()) return;
-  auto& list = it->second;
-  auto pos = std::find(list.begin(), list.end(), block);
-  if (pos != list.end()) {
-    *pos = list.back();
-    list.pop_back();
-  }
-  if (list.empty()) by_hash.erase(it);
-}
+bool BlockStore::is_cached(uint32_t block) const { return refcounts[block] == 0 && has_hash[block] && by_hash.listed[block]; }
+void BlockStore::uncache(uint32_t block, uint64_t hash) { by_hash.remove(block, hash); }
 size_t BlockStore::cached() const {
   size_t n = 0;
-  for (const auto& kv : by_hash)
-    for (uint32_t b : kv.second) n += refcounts[b] == 0;
+  for (size_t b = 0; b < refcounts.size(); ++b) n += by_hash.listed[b] && refcounts[b] == 0;
   return n;
 }
 long long BlockStore::alloc_block() {  // :2516-2534 — free list first, then the LRU of cached blocks
@@ -68,10 +117,9 @@ long long BlockStore::alloc_block() {  // :2516-2534 — free list first, then t
   return -1;
 }
 long long BlockStore::take_block(uint64_t hash) {  // :2536-2541
-  auto it = by_hash.find(hash);
-  if (it == by_hash.end() || it->second.empty()) return -1;
-  const uint32_t b = it->second.front();
-  refcounts[b] += 1;
+  const int32_t b = by_hash.first(hash);
+  if (b < 0) return -1;
+  refcounts[(size_t)b] += 1;
   return b;
 }
 void BlockStore::unref_block(uint32_t block) {  // :2543-2554
@@ -83,9 +131,10 @@ void BlockStore::unref_block(uint32_t block) {  // :2543-2554
   }
 }
 void BlockStore::set_hash(uint32_t block, uint64_t hash) {  // :2556-2561
+  by_hash.remove(block, hashes[block]);  // nothing is listed twice
   has_hash[block] = 1;
   hashes[block] = hash;
-  by_hash[hash].push_back(block);
+  by_hash.append(block, hash);
 }
 
 etc_status kv_prepare(etc_pool* pool, etc_seq* seq, int layer, int64_t pool_window, int heads, int width, int tokens,

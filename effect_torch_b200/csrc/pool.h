@@ -8,7 +8,6 @@
 #include <deque>
 #include <mutex>
 #include <string>
-#include <unordered_map>
 #include <vector>
 
 #include "common.h"
@@ -20,12 +19,33 @@ constexpr uint64_t kHashSeed = 0xcbf29ce484222325ull;
 constexpr uint64_t kHashPrime = 0x00000100000001b3ull;
 uint64_t chain_hash(uint64_t previous, const uint32_t* tokens, size_t count);
 
+// Blocks by content hash, in the order of a vector per hash that is appended to and removed from by moving its last element
+// into the gap. A prefix match looks every block of a prompt up (18 thousand for a batch of 64 long prompts), which in a
+// node-based map of vectors is a chain of cache misses each; here it is a probe of one flat table that is sized for the
+// pool's blocks once, with the lists threaded through arrays indexed by block.
+struct HashIndex {
+  struct Slot { uint64_t hash; int32_t first, last; };  // first < 0: empty
+  std::vector<Slot> slots;
+  std::vector<int32_t> next, previous;  // neighbours in the block's list
+  std::vector<uint8_t> listed;
+  size_t mask = 0;
+
+  void init(size_t blocks);
+  int32_t first(uint64_t hash) const;  // -1: none
+  void append(uint32_t block, uint64_t hash);
+  void remove(uint32_t block, uint64_t hash);
+
+ private:
+  size_t home(uint64_t hash) const { return (size_t)(hash ^ (hash >> 32)) & mask; }
+  size_t find(uint64_t hash) const;  // its slot, or the empty slot where it belongs
+};
+
 struct BlockStore {
   std::vector<uint32_t> free_list;
   std::vector<uint32_t> refcounts;
   std::vector<uint8_t> has_hash;
   std::vector<uint64_t> hashes;
-  std::unordered_map<uint64_t, std::vector<uint32_t>> by_hash;
+  HashIndex by_hash;
   std::deque<uint32_t> lru;
 
   void init(size_t blocks);

@@ -126,12 +126,12 @@ etc_status etc_runtime::workspace(size_t bytes, void** out) {
 }
 
 etc_status etc_runtime::check_status() {
-  ETC_CUDA(cudaMemcpyAsync(h_status, d_status, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, stream));
+  // the word lives in mapped host memory: kernels touch it only to report a problem, and reading it costs no copy
   ETC_CUDA(cudaStreamSynchronize(stream));
-  if (h_status->code == kStatusNone) return ETC_OK;
+  volatile DeviceStatus* word = h_status;
+  if (word->code == kStatusNone) return ETC_OK;
   const DeviceStatus seen = *h_status;
-  ETC_CUDA(cudaMemsetAsync(d_status, 0, sizeof(DeviceStatus), stream));
-  ETC_CUDA(cudaStreamSynchronize(stream));
+  std::memset(h_status, 0, sizeof(DeviceStatus));
   if (seen.code == kStatusIndexOutOfRange)
     return fail(ETC_EXECUTION, "quantized_embedding: index " + std::to_string(seen.value) + " is outside 0.." + std::to_string(seen.bound));
   if (seen.code == kStatusNonFiniteLogit)
@@ -181,9 +181,8 @@ etc_status etc_runtime_create(int device_ordinal, etc_runtime** out) {
   rt->device = device_ordinal;
   rt->sm_count = prop.multiProcessorCount;
   e = cudaStreamCreateWithFlags(&rt->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&rt->d_status, sizeof(DeviceStatus));
-  if (e == cudaSuccess) e = cudaMemset(rt->d_status, 0, sizeof(DeviceStatus));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&rt->h_status, sizeof(DeviceStatus));
+  if (e == cudaSuccess) e = cudaHostAlloc((void**)&rt->h_status, sizeof(DeviceStatus), cudaHostAllocMapped);
+  if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&rt->d_status, rt->h_status, 0);
   if (e == cudaSuccess) e = cudaMalloc((void**)&rt->d_sampled, sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMallocHost((void**)&rt->h_sampled, sizeof(uint32_t));
   // reserve the fixed scratch array of the allocation-free linear now, not inside its first call
@@ -222,7 +221,6 @@ etc_status etc_runtime_destroy(etc_runtime* rt) {
   cudaStreamSynchronize(rt->stream);
   for (auto& kv : rt->allocations) cudaFree(kv.first);
   rt->allocations.clear();
-  cudaFree(rt->d_status);
   cudaFreeHost(rt->h_status);
   cudaFree(rt->d_sampled);
   cudaFreeHost(rt->h_sampled);
