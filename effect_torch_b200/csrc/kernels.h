@@ -63,7 +63,7 @@ struct RepackParts {
 };
 cudaError_t launch_repack(const TiledWeight& w, const RepackParts& parts, cudaStream_t stream);
 
-// Sums split-K partials [splits][vpad][rows_padded] in split order and runs the epilogue.
+// Sums split-K partials [chunk of vpad vectors][splits][vpad][rows_padded] in split order and runs the epilogue.
 cudaError_t launch_qlinear_reduce(const float* scratch, int splits, int vpad, int vectors, int rows, int rows_padded,
                                   const float* bias, const float* residual, int epilogue, float* out, cudaStream_t stream);
 
@@ -86,9 +86,9 @@ cudaError_t launch_qlinear_stream(const TiledWeight& w, const float* x, const __
 
 // prefill and large batches (qlinear_umma.cu)
 struct UmmaPlan {
-  int nv = 256;              // vectors per chunk (the MMA N)
-  int chunks = 1;            // chunks the call is cut into (grid.z)
-  int tiles = 1, splits = 1, blocks_per_split = 0;
+  int nv = 128;              // vectors per chunk (the MMA N)
+  int chunks = 1, tiles = 1, stages = 1;  // 128-row tiles, stages of four 32-value blocks per tile
+  int splits = 1, stages_per_split = 1;
   size_t xh_bytes = 0;       // f16 activations in [chunk][K/8][nv][8] order, all chunks
   size_t scratch_bytes = 0;  // split-K partials [chunk][split][nv][rows_padded], all chunks
 };

@@ -1,330 +1,289 @@
-// Dequant linear on the 5th-generation tensor cores (tcgen05) for Q4_0 / Q8_0 weights.
+// Dequant linear for prefill chunks and large batches (more than 128 vectors) on the 5th-generation tensor cores.
 //
 //   out[v, r] = sum_k x[v, k] * deq(W[r, k])        (quantized_linear, crates/runtime-cpu/src/quantized.rs:419-499)
 //
-// Mapping onto tcgen05.mma.cta_group::1.kind::f16 (M = 128, N = NV, K = 16 per instruction):
-//   * A operand = 128 weight rows, read from TENSOR MEMORY. Four "dequant" warps own one TMEM lane
-//     (= one weight row) per thread: a thread streams its row's packed blocks from HBM (16-byte coalesced
-//     loads, prefetched in registers), expands nibbles/bytes to f16 in registers, multiplies by the block
-//     scale and writes 16 columns per 32-value block with tcgen05.st. Weights never touch shared memory.
-//   * B operand = the NV input vectors (activations), f16 in shared memory in the canonical K-major
-//     no-swizzle layout: 8-column groups of [NV rows][8 halves] (16 bytes per row), which is exactly how
-//     the producer stores activations in global memory ("xh8": [K/8][NV][8] f16), so a stage of 128
-//     columns is ONE contiguous cp.async.bulk copy completing on an mbarrier.
-//   * D = f32 accumulator [128 x NV] in TMEM, read back once per CTA with tcgen05.ld.
-// A CTA is 6 warps: 4 dequant/epilogue warps, 1 bulk-copy warp, 1 MMA-issue warp (one elected lane each).
-// Stages of 4 blocks (128 columns) cycle through a ring of kStages TMEM A buffers + smem B buffers guarded
-// by full_a / full_b / empty mbarriers; tcgen05.commit releases a stage when its MMAs have retired.
-// Split-K over grid.y writes f32 partials that qlinear_reduce_kernel sums; with one split the epilogue
-// (bias, residual add, SwiGLU over interleaved gate/up rows) runs straight from TMEM.
+// A CTA computes 256 weight rows x 128 vectors: two layout tiles of 128 rows, each the A operand of tcgen05.mma.kind::f16
+// (M = 128, N = 128, K = 16) in TENSOR MEMORY, against one B operand of 128 vectors in shared memory ([K/8][128][8] f16, the
+// canonical K-major layout, so that a stage of 128 columns is one contiguous bulk copy). Nineteen warps:
+//   * weight loader / activation loader: bulk copies into rings of 3 to 6 and 3 stages, completion counted in bytes;
+//   * sixteen dequant warps: a thread owns one TMEM lane = one weight row of one tile and half of a stage's blocks; it reads
+//     16 or 32 payload bytes per block from shared memory, expands them to f16, scales and stores 16 TMEM columns;
+//   * MMA warp: one elected lane issues 16 MMAs per stage (64 cycles each), tcgen05.commit frees TMEM slot and buffers.
+// Tensor memory holds the two 128-column accumulators and two stages of the two expanded tiles.
 //
-// Every mbarrier wait is bounded: on expiry the thread raises the abort flag and the status word, all
-// roles fall through to the teardown, TMEM is freed and the kernel returns.
+// Why two row tiles x 128 vectors: a stage then moves 32 KB of activations and 18 KB of packed Q4_0 weights (from L2) for
+// 1024 cycles of tensor work. One row tile x 256 vectors moved 64 KB + 9 KB, 69 bytes per cycle and SM, which is what L2 gave:
+// 890 TFLOP/s on [14336 x 4096] x 512. Expansion takes half of the SM's issue slots and ends inside the MMAs of the stage
+// before.
 //
-// Roofline: algorithmic bytes = rows*K/32*{18,34} + 2*NV*K + 4*V*rows. At NV <= 128 the kernel is bound by the rate at
-// which an SM retires tcgen05.mma instructions: measured 131 cycles each at 1965 MHz for every N <= 128 (M = 64 or 128,
-// A in tensor or shared memory, one to four accumulators), i.e. 2048 weights per 131 cycles = 0.39 of what HBM could
-// feed for Q4_0; at NV = 256 (138 cycles) it is tensor-throughput bound.
+// Split-K over grid.z writes f32 partials that qlinear_reduce_kernel sums; with one split the epilogue (bias, residual add,
+// SwiGLU over interleaved gate/up rows) runs straight from TMEM.
+// Every mbarrier wait is bounded: on expiry the thread raises the abort flag and the status word, all roles fall through to
+// the teardown, copies in flight are awaited, TMEM is freed and the kernel returns.
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <type_traits>
 
 #include "chain.cuh"
 #include "codecs.cuh"
+#include "dequant.cuh"
 #include "kernels.h"
-#include "tc05.cuh"
 
 namespace etc {
 
 namespace {
 
-constexpr int kUmmaRows = 128;
-constexpr int kDequantThreads = 128;  // one TMEM lane (weight row) per thread of a dequant group
-
-// Pipeline shape: stages of four 32-value blocks in a ring of three (TMEM for the expanded weights, shared memory for
-// the activations).
-constexpr int kStageBlocks = 4;  // 32-value blocks per stage (K = 16 per MMA: 2 MMAs per block)
-template <int NV>
-struct UmmaCfg {
-  static constexpr int kGroups = 2;        // the MMAs of a stage take as long as one group needs to expand it
-  static constexpr int kStages = 3;
-  static constexpr int kAColsPerStage = kStageBlocks * 16;  // 32-bit TMEM columns holding the stage's f16 per lane
-  static constexpr int kThreads = (4 * kGroups + 2) * 32;  // dequant warps + bulk-copy warp + MMA warp
-  static constexpr uint32_t kStageBBytes = NV * kStageBlocks * 32 * 2;
-  static constexpr uint32_t kTmemCols = NV + kStages * kAColsPerStage <= 256 ? 256 : 512;
-  static constexpr size_t kSmemBytes = (size_t)kStages * kStageBBytes + (3 * kStages + 1) * sizeof(uint64_t) + 16;
-};
 using namespace tc05;
 
-struct UmmaArgs {
-  const uint4* quants;    // Q4_0: [tile][kblock][128] uint4 ; Q8_0: [tile][kblock][128][2] uint4
-  const __half* scales;   // [tile][kblock][128]
-  const __half* xh;       // [K/8][NV][8] f16
+constexpr int kUmmaRows = 128;    // of a layout tile
+constexpr int kGemmTiles = 2;     // per CTA
+constexpr int kGemmVectors = 128;
+constexpr int kStageBlocks = 4;   // 32-value blocks per stage (K = 16 per MMA: 2 MMAs per block)
+constexpr int kGemmDequantWarps = 16;
+constexpr int kGemmWeightWarp = kGemmDequantWarps, kGemmMmaWarp = kGemmWeightWarp + 1, kGemmActivationWarp = kGemmMmaWarp + 1;
+constexpr int kGemmThreads = (kGemmActivationWarp + 1) * 32;
+
+template <int CODEC>
+struct GemmCfg {
+  static constexpr bool kNibbles = CODEC == 2 || CODEC == 12;
+  static constexpr bool kPair = CODEC >= 12;  // two f16 per (row, block): (scale, min) or the two half-block scales
+  static constexpr uint32_t kBlockQ = kNibbles ? 2048 : 4096;
+  static constexpr uint32_t kBlockS = kPair ? 512 : 256;
+  static constexpr uint32_t kTileQ = kStageBlocks * kBlockQ;
+  static constexpr uint32_t kTileW = kStageBlocks * (kBlockQ + kBlockS);
+  static constexpr uint32_t kStageW = kGemmTiles * kTileW;
+  static constexpr uint32_t kStageB = kGemmVectors * kStageBlocks * 64;
+  static constexpr int kSlots = 2;    // expanded stages in TMEM
+  static constexpr int kStagesB = 3;
+  static constexpr int kStagesW = kNibbles ? 6 : 3;
+  static constexpr int kBars = 2 * kStagesW + 2 * kStagesB + kSlots + 1;
+  static constexpr size_t kSmemBytes = (size_t)kStagesB * kStageB + (size_t)kStagesW * kStageW + kBars * sizeof(uint64_t) + 32;
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory of an SM");
+};
+
+struct GemmArgs {
+  const unsigned char* quants;  // [tile][kblock][128 rows][16 B] or 8-bit codes [tile][kblock][128 rows][32 B]
+  const unsigned char* scales;  // [tile][kblock][128] f16 or f16 pairs
+  const __half* xh;             // [chunk][K/8][128][8] f16
   const float* bias;
   const float* residual;
   float* out;
-  float* scratch;         // [splits][NV][rows_padded]
+  float* scratch;               // [chunk][split][128][rows_padded]
   unsigned long long* status;
-  int vectors, rows, rows_padded, kblocks, blocks_per_split, epilogue;
-  int tile0;              // first row tile of this launch in the output (a segment of a weight fused from several codecs)
+  int vectors, rows, rows_padded, kblocks, epilogue;
+  int tiles, tile0;             // of this launch (a segment of a weight fused from several codecs), and its first in the output
+  int stages, stages_per_split;
+  Splice splice;
 };
 
-template <int CODEC, int NV>
-__global__ void __launch_bounds__(UmmaCfg<NV>::kThreads) qlinear_umma_kernel(UmmaArgs a) {
-  using Cfg = UmmaCfg<NV>;
-  constexpr int kGroups = Cfg::kGroups, kStages = Cfg::kStages;
-  constexpr int kAColsPerStage = Cfg::kAColsPerStage;
-  constexpr bool kNibbles = CODEC == 2 || CODEC == 12;      // 4-bit codes (Q4_0, re-cut Q4_K) or 8-bit (Q8_0, re-cut Q3_K / Q5_K / Q6_K)
-  constexpr bool kPair = CODEC >= 12;                       // two f16 per (row, block): (scale, min) or the two half-block scales
-  constexpr int QW = kNibbles ? 1 : 2;                      // uint4 words per (row, block)
-  constexpr uint32_t kStageBBytes = Cfg::kStageBBytes;      // one stage of activations
-  constexpr uint32_t kTmemCols = Cfg::kTmemCols;
+template <int CODEC>
+__global__ void __launch_bounds__(kGemmThreads, 1) qlinear_gemm_kernel(GemmArgs a) {
+  using Cfg = GemmCfg<CODEC>;
+  constexpr int WS = Cfg::kStagesW, BS = Cfg::kStagesB, AS = Cfg::kSlots, NV = kGemmVectors;
   constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(NV >> 3) << 17) | ((uint32_t)(kUmmaRows >> 4) << 24);  // f16 x f16 -> f32
   extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char* b_ring = smem;                                            // kStages * kStageBBytes
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * kStageBBytes);
-  uint64_t* full_a = bars;                // [kStages] 128 arrivals
-  uint64_t* full_b = bars + kStages;      // [kStages] 1 arrival + tx bytes
-  uint64_t* empty = bars + 2 * kStages;   // [kStages] 1 arrival (tcgen05.commit)
-  uint64_t* done = bars + 3 * kStages;    // accumulator complete
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 1);
+  unsigned char* b_ring = smem;
+  unsigned char* w_ring = smem + BS * Cfg::kStageB;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(w_ring + WS * Cfg::kStageW);
+  // done[i % BS] completes when the MMAs of stage i have read its operands: it frees the activation buffer and the TMEM slot
+  uint64_t *w_full = bars, *w_empty = w_full + WS, *b_full = w_empty + WS, *done = b_full + BS, *a_full = done + BS, *d_full = a_full + AS;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(d_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  chain_release();  // the next kernel (split-K sum or the step's next operator) may be scheduled already; it waits for this one
+  chain_release();  // the next kernel of the stream may be scheduled already; it waits for this one
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
-  const int tile = blockIdx.x, split = blockIdx.y;
-  if (gridDim.z > 1) {  // this CTA's chunk of NV vectors: its activations, outputs and partials
-    const size_t chunk = blockIdx.z;
-    const size_t out_cols = a.epilogue == ETC_EPILOGUE_SWIGLU ? a.rows / 2 : a.rows;
-    a.xh += chunk * ((size_t)a.kblocks * 4 * NV * 8);
-    a.out += chunk * NV * out_cols;
-    if (a.residual) a.residual += chunk * NV * out_cols;
-    a.scratch += chunk * ((size_t)gridDim.y * NV * a.rows_padded);
-    a.vectors = max(0, min(NV, a.vectors - (int)chunk * NV));
-  }
-  const int kb0 = split * a.blocks_per_split;
-  const int kb1 = min(a.kblocks, kb0 + a.blocks_per_split);
-  const int nstages = (kb1 - kb0 + kStageBlocks - 1) / kStageBlocks;
-
-  // ---- dequant warps: group g = warp / 4 expands stages g, g + kGroups, ...; inside a group warp w owns TMEM lanes 32*(w%4)...
-  const int group = warp >> 2;
-  const int row = (warp & 3) * 32 + lane;  // TMEM lane == row inside the tile
-  const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-  const uint4* qrow = a.quants + ((size_t)tile * a.kblocks) * (kUmmaRows * QW) + (size_t)row * QW;
-  constexpr int SW = kPair ? 2 : 1;  // halves per (row, block) in the scale array
-  const __half* srow = a.scales + (((size_t)tile * a.kblocks) * kUmmaRows + row) * SW;
-  constexpr int PF = 2;  // of this group's stages, held packed in registers ahead of use
-  uint4 qbuf[PF][kStageBlocks][QW];
-  uint32_t sbuf[PF][kStageBlocks];  // one f16 (low half) or a pair
-  auto load_stage = [&](int stage_index, int slot) {
-#pragma unroll
-    for (int b = 0; b < kStageBlocks; ++b) {
-      const int kb = min(kb0 + stage_index * kStageBlocks + b, kb1 - 1);  // clamped: masked at use
-#pragma unroll
-      for (int w = 0; w < QW; ++w) qbuf[slot][b][w] = __ldg(qrow + (size_t)kb * (kUmmaRows * QW) + w);
-      if (kPair) sbuf[slot][b] = __ldg(reinterpret_cast<const uint32_t*>(srow + (size_t)kb * kUmmaRows * 2));
-      else sbuf[slot][b] = (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(srow + (size_t)kb * kUmmaRows));
-    }
-  };
-  const int my_stages = nstages > group ? (nstages - group + kGroups - 1) / kGroups : 0;
-  // the first packed stages are requested before tensor memory and the barriers are set up: weights depend on nothing
-  if (warp < 4 * kGroups) {
-#pragma unroll
-    for (int p = 0; p < PF; ++p)
-      if (p < my_stages) load_stage(group + p * kGroups, p);
-  }
-
+  const int chunk = blockIdx.x, tile = blockIdx.y * kGemmTiles, split = blockIdx.z;
+  const int live_tiles = min(kGemmTiles, a.tiles - tile);
+  const int s0 = split * a.stages_per_split, n = min(a.stages, s0 + a.stages_per_split) - s0;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(&full_a[s], kDequantThreads);
-      mbar_init(&full_b[s], 1);
-      mbar_init(&empty[s], 1);
-    }
-    mbar_init(done, 1);
+    for (int i = 0; i < WS; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], kGemmDequantWarps); }
+    for (int i = 0; i < BS; ++i) { mbar_init(&b_full[i], 1); mbar_init(&done[i], 1); }
+    for (int i = 0; i < AS; ++i) mbar_init(&a_full[i], kGemmDequantWarps);
+    mbar_init(d_full, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) tmem_alloc(tmem_holder, kTmemCols);
+  if (warp == kGemmMmaWarp) tmem_alloc(tmem_holder, 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_holder;
-  const uint32_t d_tmem = tmem_base;             // columns [0, NV)
-  const uint32_t a_tmem0 = tmem_base + NV;       // stage s at columns NV + s*kAColsPerStage
+  const uint32_t tmem = *tmem_holder;  // accumulator of tile t at columns [t * NV, (t + 1) * NV), then the expanded stages
+  const uint32_t a_tmem = tmem + kGemmTiles * NV;
 
-  if (warp < 4 * kGroups) {
+  if (warp < kGemmDequantWarps) {
     // ------------------------------------------------------------------ dequant warps
-    bool ok = true;
-    // Software pipeline: stage j is expanded in registers while the TMEM stores of stage j-1 are still in
-    // flight; only then are those stores awaited and published, so the store latency hides behind ALU work.
-    int pending_slot = -1;
-    for (int j0 = 0; j0 < my_stages && ok; j0 += PF) {
+    const int mine = (warp >> 2) & 1, half = warp >> 3, row = (warp & 3) * 32 + lane;  // tile, half of the stage's blocks, row
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const unsigned char* payload = w_ring + mine * Cfg::kTileW + row * (Cfg::kBlockQ / kUmmaRows);
+    const unsigned char* scales = w_ring + mine * Cfg::kTileW + Cfg::kTileQ + row * (Cfg::kBlockS / kUmmaRows);
+    const Splice splice = a.splice;
+    {
+      Ring<WS> w;
+      Ring<AS> slot;
+      Ring<BS> freed;  // the stage AS before this one
+      bool ok = true;
+      for (int i = 0; i < n && ok; ++i) {
+        ok = wait_warp(&w_full[w.at], w.parity, abort_flag) && (i < AS || wait_warp(&done[freed.at], freed.parity, abort_flag));
+        if (!ok) break;
+        if (i >= AS) freed.next();
+        tc_fence_after();
+        if (mine < live_tiles) {
+          const uint32_t stage = (uint32_t)w.at * Cfg::kStageW;
 #pragma unroll
-      for (int p = 0; p < PF; ++p) {
-        const int j = j0 + p;
-        if (j >= my_stages || !ok) break;
-        const int i = group + j * kGroups;  // global stage index
-        const int s = i % kStages;
-        const uint32_t round = (uint32_t)(i / kStages);
-        const int valid = min(kStageBlocks, kb1 - (kb0 + i * kStageBlocks));
-        uint32_t regs[kStageBlocks][16];
-#pragma unroll
-        for (int b = 0; b < kStageBlocks; ++b) {
-          const uint32_t sraw = b < valid ? sbuf[p][b] : 0u;
-          const __half2 pair = u2h(sraw);
-          // first f16 of the entry: the block scale (codec 14: of values 0-15); second: the min (12, 13) or the scale of values 16-31 (14)
-          const __half2 sc = __half2half2(__low2half(pair));
-          const __half2 second = __half2half2(__high2half(pair));
-          if (CODEC == 2) {
-            const uint4 q = qbuf[p][b][0];
-            expand_q4(q.x, sc, regs[b] + 0);
-            expand_q4(q.y, sc, regs[b] + 4);
-            expand_q4(q.z, sc, regs[b] + 8);
-            expand_q4(q.w, sc, regs[b] + 12);
-          } else if (CODEC == 12) {
-            const uint4 q = qbuf[p][b][0];
-            const __half2 neg_min = __hneg2(second);
-            expand_q4k(q.x, sc, neg_min, regs[b] + 0);
-            expand_q4k(q.y, sc, neg_min, regs[b] + 4);
-            expand_q4k(q.z, sc, neg_min, regs[b] + 8);
-            expand_q4k(q.w, sc, neg_min, regs[b] + 12);
-          } else if (CODEC == 13) {
-            const __half2 neg_min = __hneg2(second);
-            const uint4 q0 = qbuf[p][b][0], q1 = qbuf[p][b][QW - 1];
-            expand_q8k(q0.x, sc, neg_min, regs[b] + 0); expand_q8k(q0.y, sc, neg_min, regs[b] + 2);
-            expand_q8k(q0.z, sc, neg_min, regs[b] + 4); expand_q8k(q0.w, sc, neg_min, regs[b] + 6);
-            expand_q8k(q1.x, sc, neg_min, regs[b] + 8); expand_q8k(q1.y, sc, neg_min, regs[b] + 10);
-            expand_q8k(q1.z, sc, neg_min, regs[b] + 12); expand_q8k(q1.w, sc, neg_min, regs[b] + 14);
-          } else {
-            const __half2 sc_hi = CODEC == 14 ? second : sc;
-            const uint4 q0 = qbuf[p][b][0], q1 = qbuf[p][b][QW - 1];
-            expand_q8(q0.x, sc, regs[b] + 0); expand_q8(q0.y, sc, regs[b] + 2); expand_q8(q0.z, sc, regs[b] + 4); expand_q8(q0.w, sc, regs[b] + 6);
-            expand_q8(q1.x, sc_hi, regs[b] + 8); expand_q8(q1.y, sc_hi, regs[b] + 10); expand_q8(q1.z, sc_hi, regs[b] + 12); expand_q8(q1.w, sc_hi, regs[b] + 14);
+          for (int j = 0; j < kStageBlocks / 2; ++j) {  // blocks beyond the weight's K hold stale bytes that no MMA reads
+            const int b = half * (kStageBlocks / 2) + j;
+            uint32_t regs[16];
+            expand_block<CODEC>(payload + stage + b * Cfg::kBlockQ, scales + stage + b * Cfg::kBlockS, splice, regs);
+            tmem_st16(a_tmem + lane_base + (uint32_t)((slot.at * kGemmTiles + mine) * kStageBlocks * 16 + b * 16), regs);
           }
         }
-        if (j + PF < my_stages) load_stage(group + (j + PF) * kGroups, p);  // refill this register slot
-        if (pending_slot >= 0) {  // publish the previous stage of this group
-          tmem_wait_st();
-          tc_fence_before();
-          mbar_arrive(&full_a[pending_slot]);
-        }
-        // the MMAs that read this TMEM stage in the previous round must have retired
-        ok = mbar_wait_warp(&empty[s], (round & 1) ^ 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-#pragma unroll
-        for (int b = 0; b < kStageBlocks; ++b)
-          tmem_st16(a_tmem0 + lane_base + (uint32_t)(s * kAColsPerStage + b * 16), regs[b]);
-        pending_slot = s;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&w_empty[w.at]);
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&a_full[slot.at]);
+        w.next();
+        slot.next();
       }
     }
-    if (ok && pending_slot >= 0) {
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(&full_a[pending_slot]);
-    }
-    // ------------------------------------------------------------------ epilogue (first group)
-    if (group != 0) ok = false;
-    if (ok) ok = mbar_wait(done, 0, abort_flag);
+    // ------------------------------------------------------------------ epilogue: half of a tile's vectors per warp
     chain_wait();  // outputs, residual and scratch may still be in use by the kernel before this one
-    ok = __all_sync(0xffffffffu, ok);  // warp-uniform: the epilogue below shuffles across the warp
-    if (ok) {
+    if (wait_warp(d_full, 0, abort_flag) && mine < live_tiles) {
       tc_fence_after();
-      const int r = (a.tile0 + tile) * kUmmaRows + row;
+      const int r = (a.tile0 + tile + mine) * kUmmaRows + row;
+      const int v_base = chunk * NV;
+      const float bias_v = a.bias && r < a.rows ? a.bias[r] : 0.0f;
+      const bool partial = gridDim.z > 1;
 #pragma unroll 1
-      for (int c0 = 0; c0 < NV; c0 += 32) {
-        uint32_t acc[32];
-        tmem_ld32(d_tmem + lane_base + (uint32_t)c0, acc);
+      for (int v0 = half * (NV / 2); v0 < (half + 1) * (NV / 2) && v_base + v0 < a.vectors; v0 += 16) {
+        uint32_t bits[16];
+        tmem_ld16(tmem + lane_base + (uint32_t)(mine * NV + v0), bits);
         tmem_wait_ld();
-        if (gridDim.y > 1) {
-          float* dst = a.scratch + ((size_t)split * NV + c0) * a.rows_padded + r;
+        const int left = a.vectors - v_base - v0;
+        if (partial) {
+          float* dst = a.scratch + (((size_t)chunk * gridDim.z + split) * NV + v0) * a.rows_padded + r;
 #pragma unroll
-          for (int v = 0; v < 32; ++v) dst[(size_t)v * a.rows_padded] = __uint_as_float(acc[v]);
+          for (int v = 0; v < 16; ++v) dst[(size_t)v * a.rows_padded] = __uint_as_float(bits[v]);
         } else if (a.epilogue == ETC_EPILOGUE_SWIGLU) {
-          // rows are interleaved in groups of 8: lanes 0-7 of each 16 hold gate rows, lanes 8-15 their up rows
+          // rows are interleaved in groups of 8: lanes 0-7 of each 16 hold gate rows, lanes 8-15 their up rows; of two
+          // vectors the gate lane finishes the first and the up lane the second
+          const bool is_up = r & 8;
           const int oc = (r >> 4) * 8 + (r & 7);
-          const float bias_v = a.bias && r < a.rows ? a.bias[r] : 0.0f;
 #pragma unroll
-          for (int v = 0; v < 32; ++v) {
-            const float mine = __uint_as_float(acc[v]) + bias_v;
-            const float partner = __shfl_xor_sync(0xffffffffu, mine, 8);
-            if ((r & 8) == 0 && r + 8 < a.rows && c0 + v < a.vectors) {
-              const float act = silu_tanh(mine) * partner;
-              a.out[(size_t)(c0 + v) * (a.rows / 2) + oc] = act;
-            }
+          for (int v = 0; v < 16; v += 2) {
+            const float first = __uint_as_float(bits[v]) + bias_v, second = __uint_as_float(bits[v + 1]) + bias_v;
+            const float other = __shfl_xor_sync(0xffffffffu, is_up ? first : second, 8);
+            const float act = silu_tanh(is_up ? other : first) * (is_up ? second : other);
+            if (oc < a.rows / 2 && v + is_up < left) a.out[(size_t)(v_base + v0 + v + is_up) * (a.rows / 2) + oc] = act;
           }
         } else if (r < a.rows) {
-          const float bias_v = a.bias ? a.bias[r] : 0.0f;
+          const size_t at = (size_t)(v_base + v0) * a.rows + r;
+          float extra[16];
 #pragma unroll
-          for (int v = 0; v < 32; ++v) {
-            if (c0 + v >= a.vectors) break;
-            const size_t o = (size_t)(c0 + v) * a.rows + r;
-            const float val = __uint_as_float(acc[v]) + bias_v;
-            a.out[o] = a.epilogue == ETC_EPILOGUE_RESIDUAL ? a.residual[o] + val : val;
-          }
+          for (int v = 0; v < 16; ++v) extra[v] = a.epilogue == ETC_EPILOGUE_RESIDUAL && v < left ? a.residual[at + (size_t)v * a.rows] : 0.0f;
+#pragma unroll
+          for (int v = 0; v < 16; ++v)
+            if (v < left) a.out[at + (size_t)v * a.rows] = extra[v] + (__uint_as_float(bits[v]) + bias_v);
         }
       }
     }
-    tc_fence_before();
-  } else if (warp == 4 * kGroups) {
+  } else if (warp == kGemmWeightWarp) {
+    // ------------------------------------------------------------------ weight loader (one lane)
+    if (elect_one()) {
+      Ring<WS> w;
+      int issued = 0;
+      for (int i = 0; i < n; ++i) {
+        if (!mbar_wait(&w_empty[w.at], w.parity ^ 1u, abort_flag)) break;
+        const int kb = (s0 + i) * kStageBlocks;
+        const uint32_t valid = (uint32_t)min(kStageBlocks, a.kblocks - kb);
+        unsigned char* dst = w_ring + (size_t)w.at * Cfg::kStageW;
+        mbar_arrive_expect_tx(&w_full[w.at], (uint32_t)live_tiles * valid * (Cfg::kBlockQ + Cfg::kBlockS));
+        for (int t = 0; t < live_tiles; ++t) {
+          const size_t block = (size_t)(tile + t) * a.kblocks + kb;
+          bulk_copy_g2s(dst + t * Cfg::kTileW, a.quants + block * Cfg::kBlockQ, valid * Cfg::kBlockQ, &w_full[w.at]);
+          bulk_copy_g2s(dst + t * Cfg::kTileW + Cfg::kTileQ, a.scales + block * Cfg::kBlockS, valid * Cfg::kBlockS, &w_full[w.at]);
+        }
+        issued = i + 1;
+        w.next();
+      }
+      if (*abort_flag)  // give up: this warp's own copies land (bounded) before shared memory is released
+        for (int i = max(0, issued - WS); i < issued; ++i)
+          for (unsigned spin = 0; spin < (1u << 20) && !mbar_try_wait(&w_full[i % WS], (uint32_t)(i / WS) & 1u); ++spin) __nanosleep(64);
+    }
+  } else if (warp == kGemmActivationWarp) {
     // ------------------------------------------------------------------ activation loader (one lane)
     if (elect_one()) {
-      chain_wait();  // the activations come from the kernel before this one; weights do not, the dequant warps run ahead
+      chain_wait();  // the activations come from the kernel before this one
+      const __half* xh = a.xh + (size_t)chunk * a.kblocks * 4 * NV * 8;
+      Ring<BS> b;
       int issued = 0;
-      for (int i = 0; i < nstages; ++i) {
-        const int s = i % kStages;
-        const uint32_t round = (uint32_t)(i / kStages);
-        if (!mbar_wait(&empty[s], (round & 1) ^ 1, abort_flag)) break;
-        const int kb = kb0 + i * kStageBlocks;
-        const int valid = min(kStageBlocks, kb1 - kb);
-        const uint32_t bytes = (uint32_t)valid * 4u * NV * 16u;  // 4 column groups of 8 per block
-        mbar_arrive_expect_tx(&full_b[s], bytes);
-        bulk_copy_g2s(b_ring + (size_t)s * kStageBBytes, a.xh + (size_t)kb * 4 * NV * 8, bytes, &full_b[s]);
+      for (int i = 0; i < n; ++i) {
+        if (i >= BS && !mbar_wait(&done[b.at], b.parity ^ 1u, abort_flag)) break;  // stage i - BS used this buffer and barrier
+        const int kb = (s0 + i) * kStageBlocks;
+        const uint32_t bytes = (uint32_t)min(kStageBlocks, a.kblocks - kb) * 4u * NV * 16u;
+        mbar_arrive_expect_tx(&b_full[b.at], bytes);
+        bulk_copy_g2s(b_ring + (size_t)b.at * Cfg::kStageB, xh + (size_t)kb * 4 * NV * 8, bytes, &b_full[b.at]);
         issued = i + 1;
+        b.next();
       }
-      if (*abort_flag) {
-        // give up path: let this warp's own bulk copies land (bounded) before shared memory is released
-        for (int i = max(0, issued - kStages); i < issued; ++i) {
-          const uint32_t parity = (uint32_t)(i / kStages) & 1;
-          for (unsigned spin = 0; spin < (1u << 20) && !mbar_try_wait(&full_b[i % kStages], parity); ++spin) __nanosleep(64);
-        }
-      }
+      if (*abort_flag)
+        for (int i = max(0, issued - BS); i < issued; ++i)
+          for (unsigned spin = 0; spin < (1u << 20) && !mbar_try_wait(&b_full[i % BS], (uint32_t)(i / BS) & 1u); ++spin) __nanosleep(64);
     }
   } else {
     // ------------------------------------------------------------------ MMA issuer (one lane)
     if (elect_one()) {
+      Ring<BS> b;
+      Ring<AS> slot;
       bool ok = true;
-      for (int i = 0; i < nstages && ok; ++i) {
-        const int s = i % kStages;
-        const uint32_t parity = (uint32_t)(i / kStages) & 1;
-        ok = mbar_wait(&full_b[s], parity, abort_flag) && mbar_wait(&full_a[s], parity, abort_flag);
+      const uint64_t desc0 = make_b_desc(smem_u32(b_ring), NV * 16u, 128u);
+      for (int i = 0; i < n && ok; ++i) {
+        ok = mbar_wait(&b_full[b.at], b.parity, abort_flag) && mbar_wait(&a_full[slot.at], slot.parity, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        const int valid = min(kStageBlocks, kb1 - (kb0 + i * kStageBlocks));
-        const uint32_t b_base = smem_u32(b_ring + (size_t)s * kStageBBytes);
-        for (int j = 0; j < 2 * valid; ++j) {  // K = 16 per MMA: two column groups of B, 8 TMEM columns of A
-          const uint64_t b_desc = make_b_desc(b_base + (uint32_t)j * 2u * NV * 16u, NV * 16u, 128u);
-          umma_ts(d_tmem, a_tmem0 + (uint32_t)(s * kAColsPerStage + j * 8), b_desc, kIdesc, (i > 0 || j > 0) ? 1u : 0u);
+        const int valid = min(kStageBlocks, a.kblocks - (s0 + i) * kStageBlocks);
+        // two K = 16 instructions per block and tile: two column groups of B, 8 TMEM columns of A each; whole stages unrolled
+        // with constant steps, so that the operands stay in uniform registers
+        const uint64_t desc = desc0 + (uint64_t)(b.at * (int)(Cfg::kStageB / 16));
+        const uint32_t a0 = a_tmem + (uint32_t)(slot.at * kGemmTiles * kStageBlocks * 16), a1 = a0 + kStageBlocks * 16;
+        umma_ts(tmem, a0, desc, kIdesc, i > 0 ? 1u : 0u);
+        umma_ts(tmem + NV, a1, desc, kIdesc, i > 0 ? 1u : 0u);
+        if (valid == kStageBlocks) {
+#pragma unroll
+          for (int j = 1; j < 2 * kStageBlocks; ++j) {
+            umma_ts(tmem, a0 + 8u * j, desc + 2u * NV * j, kIdesc, 1u);
+            umma_ts(tmem + NV, a1 + 8u * j, desc + 2u * NV * j, kIdesc, 1u);
+          }
+        } else {
+          for (int j = 1; j < 2 * valid; ++j) {
+            umma_ts(tmem, a0 + 8u * j, desc + 2u * NV * j, kIdesc, 1u);
+            umma_ts(tmem + NV, a1 + 8u * j, desc + 2u * NV * j, kIdesc, 1u);
+          }
         }
-        tc_commit(&empty[s]);  // arrives when the MMAs above have finished reading this stage
+        tc_commit(&done[b.at]);
+        b.next();
+        slot.next();
       }
-      if (ok) tc_commit(done);
-      tc_fence_before();
+      if (ok) tc_commit(d_full);
     }
   }
+  __syncwarp();
+  tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0 && *abort_flag) atomicCAS(a.status, 0ull, 3ull);  // bounded wait expired
-  if (warp == 0) {
+  if (warp == kGemmMmaWarp) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTmemCols);
+    tmem_dealloc(tmem, 512);
   }
 }
 
 // f32 [vectors, K] -> xh8 [K/8][NV][8] f16 (rows >= vectors are zero), saturating like the mma.sync path.
 // More than NV vectors: chunk c holds vectors c*NV ... in its own [K/8][NV][8] block.
-template <int NV>
 __global__ void convert_xh8_kernel(const float* __restrict__ x, int vectors, int K, __half* __restrict__ xh) {
+  constexpr int NV = kGemmVectors;
+  chain_release();
+  chain_wait();
   const int per_chunk = (K / 8) * NV;
   const int64_t total = (int64_t)per_chunk * ((vectors + NV - 1) / NV);
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
@@ -489,14 +448,14 @@ __global__ void repack_umma_kernel(RepackParts parts, int codec, int64_t rows, i
   }
 }
 
-template <int CODEC, int NV>
-cudaError_t launch_umma_pass(const UmmaArgs& args, int tiles, int splits, int chunks, cudaStream_t stream) {
-  constexpr size_t smem = UmmaCfg<NV>::kSmemBytes;
-  auto kernel = qlinear_umma_kernel<CODEC, NV>;
+template <int CODEC>
+cudaError_t launch_gemm_pass(const GemmArgs& args, int chunks, int splits, cudaStream_t stream) {
+  constexpr size_t smem = GemmCfg<CODEC>::kSmemBytes;
+  auto kernel = qlinear_gemm_kernel<CODEC>;
   const cudaError_t attr = opt_in_shared_memory(kernel, smem);
   if (attr != cudaSuccess) return attr;
-  // chained: set-up, weight loads and their expansion do not depend on the previous kernel and start under its tail
-  return launch_chained(kernel, dim3((unsigned)tiles, (unsigned)splits, (unsigned)chunks), dim3((unsigned)UmmaCfg<NV>::kThreads), smem, stream, args);
+  // chained: set-up and the first weight stages do not depend on the previous kernel and start under its tail
+  return launch_chained(kernel, dim3((unsigned)chunks, (unsigned)((args.tiles + kGemmTiles - 1) / kGemmTiles), (unsigned)splits), dim3(kGemmThreads), smem, stream, args);
 }
 
 }  // namespace
@@ -514,13 +473,12 @@ UmmaPlan plan_umma(const TiledWeight& w, int64_t vectors, int sm_count) {
   UmmaPlan p;
   p.chunks = (int)std::max<int64_t>(1, (vectors + p.nv - 1) / p.nv);
   p.tiles = (int)(w.rows_padded / kUmmaRows);
-  const int kblocks = (int)(w.columns / 32);
-  const int stages = (kblocks + kStageBlocks - 1) / kStageBlocks;
-  int splits = std::max(1, std::max(1, sm_count) / std::max(1, p.tiles * p.chunks));
-  splits = std::min(splits, std::max(1, stages / 2));  // at least two stages per split
-  const int stages_per_split = (stages + splits - 1) / splits;
-  p.blocks_per_split = stages_per_split * kStageBlocks;
-  p.splits = (kblocks + p.blocks_per_split - 1) / p.blocks_per_split;
+  p.stages = (int)((w.columns / 32 + kStageBlocks - 1) / kStageBlocks);
+  // as many splits as there are SMs for (one CTA each), of at least two stages
+  const int ctas = (p.tiles + kGemmTiles - 1) / kGemmTiles * p.chunks;
+  const int splits = std::min(std::max(1, std::max(1, sm_count) / ctas), std::max(1, p.stages / 2));
+  p.stages_per_split = (p.stages + splits - 1) / splits;
+  p.splits = (p.stages + p.stages_per_split - 1) / p.stages_per_split;
   p.xh_bytes = (size_t)p.chunks * (w.columns / 8) * p.nv * 16;
   p.scratch_bytes = p.splits > 1 ? (size_t)p.chunks * p.splits * p.nv * w.rows_padded * sizeof(float) : 0;
   return p;
@@ -531,17 +489,13 @@ cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, int64_t ve
                                 float* out, __half* xh, float* scratch, DeviceStatus* status, int sm_count, cudaStream_t stream,
                                 int* launches) {
   if (vectors <= 0) return cudaSuccess;
-  const int out_cols = (int)(epilogue == ETC_EPILOGUE_SWIGLU ? w.rows / 2 : w.rows);
   const UmmaPlan plan = plan_umma(w, vectors, sm_count);
   const int K = (int)w.columns;
   const int64_t total = (int64_t)(K / 8) * plan.nv * plan.chunks;
-  convert_xh8_kernel<256><<<(unsigned)std::min<int64_t>((total + 255) / 256, 148 * 8), 256, 0, stream>>>(x, (int)vectors, K, xh);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_chained(convert_xh8_kernel, dim3((unsigned)std::min<int64_t>((total + 255) / 256, 148 * 8)), dim3(256), 0, stream, x, (int)vectors, K, xh);
   if (e != cudaSuccess) return e;
   if (launches) ++*launches;
-  UmmaArgs args;
-  args.quants = reinterpret_cast<const uint4*>(w.quants);
-  args.scales = w.scales;
+  GemmArgs args;
   args.xh = xh;
   args.bias = bias;
   args.residual = residual;
@@ -552,38 +506,37 @@ cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, int64_t ve
   args.rows = (int)w.rows;
   args.rows_padded = (int)w.rows_padded;
   args.kblocks = K / 32;
-  args.blocks_per_split = plan.blocks_per_split;
   args.epilogue = epilogue;
-  args.tile0 = 0;
+  args.stages = plan.stages;
+  args.stages_per_split = plan.stages_per_split;
   // one launch per run of equal codecs; all of them share the plan (split count, partial layout) of the whole weight
   for (int sgm = 0; sgm < std::max(1, w.n_segments); ++sgm) {
-    int codec = w.codec, tiles = plan.tiles;
+    int codec = w.codec;
+    args.quants = w.quants;
+    args.scales = reinterpret_cast<const unsigned char*>(w.scales);
+    args.tiles = plan.tiles;
+    args.tile0 = 0;
     if (w.n_segments > 0) {
       const TiledSegment& seg = w.segments[sgm];
       codec = seg.codec;
-      tiles = seg.tiles;
+      args.tiles = seg.tiles;
       args.tile0 = seg.tile0;
-      args.quants = reinterpret_cast<const uint4*>(w.quants + seg.quant_offset);
-      args.scales = reinterpret_cast<const __half*>(reinterpret_cast<const uint8_t*>(w.scales) + seg.scale_offset);
+      args.quants += seg.quant_offset;
+      args.scales += seg.scale_offset;
     }
     switch (codec) {
-      case 2: e = launch_umma_pass<2, 256>(args, tiles, plan.splits, plan.chunks, stream); break;
-      case 8: e = launch_umma_pass<8, 256>(args, tiles, plan.splits, plan.chunks, stream); break;
-      case 12: e = launch_umma_pass<12, 256>(args, tiles, plan.splits, plan.chunks, stream); break;
-      case 13: e = launch_umma_pass<13, 256>(args, tiles, plan.splits, plan.chunks, stream); break;
-      default: e = launch_umma_pass<14, 256>(args, tiles, plan.splits, plan.chunks, stream);  // 14, and 11 whose re-cut form is the same
+      case 2: e = launch_gemm_pass<2>(args, plan.chunks, plan.splits, stream); break;
+      case 8: e = launch_gemm_pass<8>(args, plan.chunks, plan.splits, stream); break;
+      case 12: e = launch_gemm_pass<12>(args, plan.chunks, plan.splits, stream); break;
+      case 13: e = launch_gemm_pass<13>(args, plan.chunks, plan.splits, stream); break;
+      default: e = launch_gemm_pass<14>(args, plan.chunks, plan.splits, stream);  // 14, and 11 whose re-cut form is the same
     }
     if (e != cudaSuccess) return e;
     if (launches) ++*launches;
   }
-  for (int c = 0; plan.splits > 1 && c < plan.chunks; ++c) {  // one sum launch per chunk of vectors
-    const int64_t v0 = (int64_t)c * plan.nv;
-    e = launch_qlinear_reduce(scratch + (size_t)c * plan.splits * plan.nv * w.rows_padded, plan.splits, plan.nv, (int)std::min<int64_t>(plan.nv, vectors - v0),
-                              (int)w.rows, (int)w.rows_padded, bias, residual ? residual + v0 * out_cols : nullptr, epilogue, out + v0 * out_cols, stream);
-    if (e != cudaSuccess) return e;
-    if (launches) ++*launches;
-  }
-  return cudaSuccess;
+  if (plan.splits == 1) return cudaSuccess;
+  if (launches) ++*launches;
+  return launch_qlinear_reduce(scratch, plan.splits, plan.nv, (int)vectors, (int)w.rows, (int)w.rows_padded, bias, residual, epilogue, out, stream);
 }
 
 }  // namespace etc

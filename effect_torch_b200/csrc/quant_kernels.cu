@@ -405,7 +405,7 @@ cudaError_t launch_repack(const TiledWeight& w, const RepackParts& parts, cudaSt
 
 __device__ __forceinline__ float silu_tanh_form(float x) { return x * (tanhf(x * 0.5f) * 0.5f + 0.5f); }
 
-// Sums the split-K partials in split order (deterministic) and applies bias / epilogue.
+// Sums the split-K partials [chunk of vpad vectors][split][vpad][rows_padded] in split order and applies bias / epilogue.
 // `residual` and `out` may be the same buffer (the decoder adds projections onto its hidden state in place), so
 // neither carries a no-alias promise.
 __global__ void qlinear_reduce_kernel(const float* __restrict__ scratch, int splits, int vpad, int vectors, int rows,
@@ -421,7 +421,7 @@ __global__ void qlinear_reduce_kernel(const float* __restrict__ scratch, int spl
       const int r_gate = (c >> 3) * 16 + (c & 7), r_up = r_gate + 8;
       float gsum = 0.f, usum = 0.f;
       for (int s = 0; s < splits; ++s) {
-        const float* p = scratch + ((size_t)s * vpad + v) * rows_padded;
+        const float* p = scratch + ((size_t)(v / vpad * splits + s) * vpad + v % vpad) * rows_padded;
         gsum += p[r_gate];
         usum += p[r_up];
       }
@@ -430,7 +430,7 @@ __global__ void qlinear_reduce_kernel(const float* __restrict__ scratch, int spl
       out[idx] = act;
     } else {
       float sum = 0.f;
-      for (int s = 0; s < splits; ++s) sum += scratch[((size_t)s * vpad + v) * rows_padded + c];
+      for (int s = 0; s < splits; ++s) sum += scratch[((size_t)(v / vpad * splits + s) * vpad + v % vpad) * rows_padded + c];
       if (bias) sum += bias[c];
       const float val = epilogue == ETC_EPILOGUE_RESIDUAL ? residual[idx] + sum : sum;
       out[idx] = val;

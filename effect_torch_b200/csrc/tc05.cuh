@@ -1,6 +1,5 @@
 // Inline-PTX helpers for the tcgen05 kernels: mbarriers with bounded waits, bulk copies, tensor-memory
-// allocation / loads / stores, MMA issue and commit, shared-memory matrix descriptors, and the f16 expansion of
-// packed Q4_0 / Q8_0 words. Everything here is sm_100a only.
+// allocation / loads / stores, MMA issue and commit, shared-memory matrix descriptors. Everything here is sm_100a only.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -102,16 +101,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
         "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,"
-      "%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-        "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-        "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-        "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr) : "memory");
-}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -160,60 +149,7 @@ __device__ __forceinline__ uint64_t make_b_desc(uint32_t smem_addr, uint32_t lbo
 __device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ __half2 u2h(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 
-// One packed u32 = 8 nibbles, logical column j of the word at bit {0,16,8,24,4,20,12,28}[j] -> four half2
-// in column order (c0,c1)(c2,c3)(c4,c5)(c6,c7), times the block scale.
-__device__ __forceinline__ void expand_q4(uint32_t q, __half2 scale, uint32_t* out4) {
-  const uint32_t magic = 0x64006400u;
-  const uint32_t qs = q >> 8;
-  const __half2 bias_lo = __floats2half2_rn(1032.0f, 1032.0f);
-  const __half2 sixteenth = __floats2half2_rn(0.0625f, 0.0625f);
-  const __half2 bias_hi = __floats2half2_rn(-72.0f, -72.0f);
-  out4[0] = h2u(__hmul2(__hsub2(u2h((q & 0x000F000Fu) | magic), bias_lo), scale));
-  out4[1] = h2u(__hmul2(__hsub2(u2h((qs & 0x000F000Fu) | magic), bias_lo), scale));
-  out4[2] = h2u(__hmul2(__hfma2(u2h((q & 0x00F000F0u) | magic), sixteenth, bias_hi), scale));
-  out4[3] = h2u(__hmul2(__hfma2(u2h((qs & 0x00F000F0u) | magic), sixteenth, bias_hi), scale));
-}
-// Four int8 -> (b0,b1)(b2,b3) times scale.
-__device__ __forceinline__ void expand_q8(uint32_t w, __half2 scale, uint32_t* out2) {
-  const uint32_t x = w ^ 0x80808080u;
-  const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);
-  out2[0] = h2u(__hmul2(__hsub2(u2h(__byte_perm(x, 0x64646464u, 0x4140)), bias), scale));
-  out2[1] = h2u(__hmul2(__hsub2(u2h(__byte_perm(x, 0x64646464u, 0x4342)), bias), scale));
-}
-
-// Q4_K block re-cut to 32 values: code * scale - min (scale = d * sc, min = dmin * m, both rounded to f16 at load).
-__device__ __forceinline__ void expand_q4k(uint32_t q, __half2 scale, __half2 neg_min, uint32_t* out4) {
-  const uint32_t magic = 0x64006400u;
-  const uint32_t qs = q >> 8;
-  const __half2 bias_lo = __floats2half2_rn(1024.0f, 1024.0f);
-  const __half2 sixteenth = __floats2half2_rn(0.0625f, 0.0625f);
-  const __half2 bias_hi = __floats2half2_rn(-64.0f, -64.0f);
-  out4[0] = h2u(__hfma2(__hsub2(u2h((q & 0x000F000Fu) | magic), bias_lo), scale, neg_min));
-  out4[1] = h2u(__hfma2(__hsub2(u2h((qs & 0x000F000Fu) | magic), bias_lo), scale, neg_min));
-  out4[2] = h2u(__hfma2(__hfma2(u2h((q & 0x00F000F0u) | magic), sixteenth, bias_hi), scale, neg_min));
-  out4[3] = h2u(__hfma2(__hfma2(u2h((qs & 0x00F000F0u) | magic), sixteenth, bias_hi), scale, neg_min));
-}
-
-// Q5_K block re-cut to 32 int8 codes: code * scale - min.
-__device__ __forceinline__ void expand_q8k(uint32_t w, __half2 scale, __half2 neg_min, uint32_t* out2) {
-  const uint32_t x = w ^ 0x80808080u;
-  const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);
-  out2[0] = h2u(__hfma2(__hsub2(u2h(__byte_perm(x, 0x64646464u, 0x4140)), bias), scale, neg_min));
-  out2[1] = h2u(__hfma2(__hsub2(u2h(__byte_perm(x, 0x64646464u, 0x4342)), bias), scale, neg_min));
-}
-
 __device__ __forceinline__ float silu_tanh(float x) { return x * (tanhf(x * 0.5f) * 0.5f + 0.5f); }
-
-// D[tmem] (+)= A[smem desc] * B[smem desc].
-__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
-}
-// Makes this thread's earlier generic-proxy writes to shared memory visible to the async proxy (tensor core reads).
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 }  // namespace tc05
 }  // namespace etc
