@@ -323,7 +323,7 @@ struct AttnArgs {
   const LaneInfo* lanes;
   const int* tables;
   float* out;              // [B, Hq, D] f32 (splits == 1)
-  __half* out_xh;          // optional f16 copy of out in [Hq*D/8][out_xh_nv][8] order: the o-projection's B operand
+  __half* out_xh;          // optional f16 copy of out in the hand-off layout: the o-projection's B operand
   int out_xh_nv;
   float* partial;          // [B, Hq, splits, D + 2] f32: O unnormalised, then m (log2 domain), l
   int q_heads, kv_heads;
@@ -340,14 +340,19 @@ __device__ __forceinline__ int swizzled_offset(int row, int chunk) {  // in byte
   return row * (D * 2) + ((chunk & ~7) | ((chunk ^ row) & 7)) * 16;
 }
 
-// CHUNK = false: one query token per lane; the 16 MMA rows are the query heads of one KV head and grid.x splits the pages.
-// CHUNK = true: a chunk of a.tokens query tokens per lane (chunked prefill, napi/mod.rs:3420-3477 semantics: token t of
-// the chunk attends positions up to cursor + t); the 16 MMA rows are (token, query head) pairs, 16 / G tokens per CTA,
-// grid.x counts row tiles and every row carries its own causal bound.
+// Four bytes b0..b3 -> halves 1024 + b, minus 1152 = b - 128 (exact).
+__device__ __forceinline__ void bytes_to_half2(uint32_t w, uint32_t& lo, uint32_t& hi) {
+  const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);
+  uint32_t lo_bits = __byte_perm(w, 0x64646464u, 0x4140), hi_bits = __byte_perm(w, 0x64646464u, 0x4342);
+  const __half2 l = __hsub2(*reinterpret_cast<__half2*>(&lo_bits), bias), h = __hsub2(*reinterpret_cast<__half2*>(&hi_bits), bias);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+}
+
 // U8: the int8 tier (code - 128) * scale with one scale per cached row (napi/mod.rs:3474-3476): pages travel as bytes, a warp
 // widens the page it is about to use to f16 integers in a staging page of its own, and the row scales multiply the score
 // columns (K) and the probabilities before P V (V), so the tensor core only ever sees exact small integers.
-template <int D, bool BF16, bool CHUNK, bool U8>
+template <int D, bool BF16, bool U8>
 __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int PAGE_BYTES = kPageTokens * D * 2;               // one page as MMA operands (f16 / bf16)
@@ -362,36 +367,19 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs
   const int g = lane >> 2, t = lane & 3;
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   chain_wait();
-  const int split = CHUNK ? 0 : blockIdx.x, kv_head = blockIdx.y, lane_id = blockIdx.z;
+  const int split = blockIdx.x, kv_head = blockIdx.y, lane_id = blockIdx.z;
   const LaneInfo info = a.lanes[lane_id];
   const int G = a.q_heads / a.kv_heads;
-  const int nsplits = CHUNK ? 1 : gridDim.x;
-  // rows g and g + 8 of the MMA tile: which query token and head they are, and the positions [begin, end) they attend
-  const int T = CHUNK ? a.tokens : 1;
-  const int tokens_per_tile = CHUNK ? max(1, 16 / G) : 1;
-  const int tile_token0 = CHUNK ? blockIdx.x * tokens_per_tile : 0;
-  auto row_token = [&](int row) { return CHUNK ? tile_token0 + row / G : 0; };
-  auto row_head = [&](int row) { return CHUNK ? row % G : row; };
-  auto row_valid = [&](int row) { return CHUNK ? (row / G < tokens_per_tile && row_token(row) < T) : row < G; };
-  auto row_end = [&](int row) { return CHUNK ? (row_valid(row) && info.advance > 0 ? info.cursor + row_token(row) + 1 : 0) : info.cursor + info.advance; };
-  auto row_begin = [&](int row, int row_end_) {
-    int b = info.start;
-    if (a.op_window >= 0) b = max((int)max((long long)row_end_ - a.op_window, 0ll), info.start);
-    return b;
-  };
-  const int end_lo = row_end(g), end_hi = row_end(g + 8);
-  const int begin_lo = row_begin(g, end_lo), begin_hi = row_begin(g + 8, end_hi);
-  // the tile as a whole: pages from the earliest begin to the latest end of its rows
-  const int last_token = CHUNK ? min(T, tile_token0 + tokens_per_tile) - 1 : 0;
-  const int end = CHUNK ? (info.advance > 0 && last_token >= tile_token0 ? info.cursor + last_token + 1 : 0) : info.cursor + info.advance;
+  const int nsplits = gridDim.x;
+  const int end = info.cursor + info.advance;
   int begin = info.start;
-  if (a.op_window >= 0) begin = max((int)max((long long)(CHUNK ? info.cursor + tile_token0 + 1 : end) - a.op_window, 0ll), info.start);
+  if (a.op_window >= 0) begin = max((int)max((long long)end - a.op_window, 0ll), info.start);
   const bool idle_lane = info.advance == 0 || end <= begin;
   // page range of this split (pages are indexed from the table start, i.e. position 0)
   const int first_page = begin / kPageTokens;
   const int last_page = idle_lane ? first_page : (end - 1) / kPageTokens + 1;  // exclusive
   const int p0 = first_page + split * a.pages_per_split;
-  const int p1 = CHUNK ? last_page : min(last_page, p0 + a.pages_per_split);
+  const int p1 = min(last_page, p0 + a.pages_per_split);
 
   unsigned char* my_smem = smem + (size_t)warp * WARP_BYTES;
   unsigned char* wide = my_smem + kAttnStages * STAGE_BYTES;  // U8: this warp's widened K page, then V page
@@ -441,15 +429,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs
       const uint32_t w[4] = {codes.x, codes.y, codes.z, codes.w};
       uint32_t h[8];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        // bytes b0..b3 -> halves 1024 + b, minus 1152 = b - 128 (exact)
-        const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);
-        uint32_t lo_bits = __byte_perm(w[j], 0x64646464u, 0x4140), hi_bits = __byte_perm(w[j], 0x64646464u, 0x4342);
-        const __half2 lo = __hsub2(*reinterpret_cast<__half2*>(&lo_bits), bias);
-        const __half2 hi = __hsub2(*reinterpret_cast<__half2*>(&hi_bits), bias);
-        h[2 * j] = *reinterpret_cast<const uint32_t*>(&lo);
-        h[2 * j + 1] = *reinterpret_cast<const uint32_t*>(&hi);
-      }
+      for (int j = 0; j < 4; ++j) bytes_to_half2(w[j], h[2 * j], h[2 * j + 1]);
       *reinterpret_cast<uint4*>(dst + swizzled_offset<D>(row, chunk)) = make_uint4(h[0], h[1], h[2], h[3]);
       *reinterpret_cast<uint4*>(dst + swizzled_offset<D>(row, chunk + 1)) = make_uint4(h[4], h[5], h[6], h[7]);
     }
@@ -466,9 +446,9 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs
   // Q fragments: rows 0..G-1 = query heads of this KV head, scaled into the exp2 domain
   uint32_t qf[KSTEPS][4];
   {
-    const bool lo_ok = row_valid(g), hi_ok = row_valid(g + 8);
-    const float* qrow_lo = a.q + (((size_t)lane_id * T + (lo_ok ? row_token(g) : 0)) * a.q_heads + kv_head * G + (lo_ok ? row_head(g) : 0)) * D;
-    const float* qrow_hi = a.q + (((size_t)lane_id * T + (hi_ok ? row_token(g + 8) : 0)) * a.q_heads + kv_head * G + (hi_ok ? row_head(g + 8) : 0)) * D;
+    const bool lo_ok = g < G, hi_ok = g + 8 < G;
+    const float* qrow_lo = a.q + ((size_t)lane_id * a.q_heads + kv_head * G + (lo_ok ? g : 0)) * D;
+    const float* qrow_hi = a.q + ((size_t)lane_id * a.q_heads + kv_head * G + (hi_ok ? g + 8 : 0)) * D;
 #pragma unroll
     for (int ks = 0; ks < KSTEPS; ++ks) {
       const int c0 = ks * 16 + 2 * t;
@@ -528,10 +508,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const int pa = base_pos + 2 * t + j, pb = pa + 8;
-      if (pa < begin_lo || pa >= end_lo) s0[j] = -INFINITY;
-      if (pa < begin_hi || pa >= end_hi) s0[2 + j] = -INFINITY;
-      if (pb < begin_lo || pb >= end_lo) s1[j] = -INFINITY;
-      if (pb < begin_hi || pb >= end_hi) s1[2 + j] = -INFINITY;
+      if (pa < begin || pa >= end) s0[j] = s0[2 + j] = -INFINITY;
+      if (pb < begin || pb >= end) s1[j] = s1[2 + j] = -INFINITY;
     }
     // online softmax for rows g (index 0,1) and g+8 (index 2,3)
     float mx_lo = fmaxf(fmaxf(s0[0], s0[1]), fmaxf(s1[0], s1[1]));
@@ -605,9 +583,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs
     ml[warp * 16 + g] = l_lo; ml[warp * 16 + g + 8] = l_hi;
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < (CHUNK ? 16 : G) * D; idx += blockDim.x) {
+  for (int idx = threadIdx.x; idx < G * D; idx += blockDim.x) {
     const int row = idx / D, d = idx - row * D;
-    if (CHUNK && !row_valid(row)) continue;
     float m = -INFINITY;
 #pragma unroll
     for (int w = 0; w < kAttnWarps; ++w) m = fmaxf(m, mm[w * 16 + row]);
@@ -619,13 +596,13 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs
       acc += f * mo[((size_t)w * 16 + row) * D + d];
       l += f * ml[w * 16 + row];
     }
-    const int head = kv_head * G + row_head(row);
+    const int head = kv_head * G + row;
     if (nsplits == 1) {
       const float val = l > 0.0f ? acc / l : 0.0f;
-      a.out[(((size_t)lane_id * T + row_token(row)) * a.q_heads + head) * D + d] = val;
-      if (!CHUNK && a.out_xh) {
+      if (a.out) a.out[((size_t)lane_id * a.q_heads + head) * D + d] = val;
+      if (a.out_xh) {
         const int k = head * D + d;
-        a.out_xh[((size_t)(k >> 3) * a.out_xh_nv + lane_id) * 8 + (k & 7)] = __float2half_rn(fminf(fmaxf(val, -65504.f), 65504.f));
+        a.out_xh[hand_off_cell(k >> 3, lane_id, a.out_xh_nv, a.q_heads * (D / 8)) + (k & 7)] = __float2half_rn(fminf(fmaxf(val, -65504.f), 65504.f));
       }
     } else {
       float* dst = a.partial + (((size_t)lane_id * a.q_heads + head) * nsplits + split) * (D + 2);
@@ -642,23 +619,281 @@ __global__ void attention_merge_kernel(const float* __restrict__ partial, int q_
   chain_wait();
   const int head = blockIdx.x, lane_id = blockIdx.y;
   const float* base = partial + ((size_t)lane_id * q_heads + head) * splits * (D + 2);
+  // every thread needs every split's (m, l): fetched once per CTA, eight output loads in flight, added in split order
+  extern __shared__ float factor[];  // [splits] 2^(m_s - m), then [splits] l_s
   float m = -INFINITY;
-  for (int s = 0; s < splits; ++s) m = fmaxf(m, base[(size_t)s * (D + 2) + D]);
+  for (int s = threadIdx.x & 31; s < splits; s += 32) m = fmaxf(m, base[(size_t)s * (D + 2) + D]);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+  for (int s = threadIdx.x; s < splits; s += blockDim.x) {
+    const float ms = base[(size_t)s * (D + 2) + D];
+    factor[s] = ms == -INFINITY ? 0.0f : exp2f(ms - m);
+    factor[splits + s] = base[(size_t)s * (D + 2) + D + 1];
+  }
+  __syncthreads();
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
     float acc = 0.0f, l = 0.0f;
-    for (int s = 0; s < splits; ++s) {
-      const float* p = base + (size_t)s * (D + 2);
-      const float f = p[D] == -INFINITY ? 0.0f : exp2f(p[D] - m);
-      acc += f * p[d];
-      l += f * p[D + 1];
+    for (int s0 = 0; s0 < splits; s0 += 8) {
+      float p[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) p[u] = s0 + u < splits ? base[(size_t)(s0 + u) * (D + 2) + d] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (s0 + u >= splits) break;
+        acc += factor[s0 + u] * p[u];
+        l += factor[s0 + u] * factor[splits + s0 + u];
+      }
     }
     const float val = l > 0.0f ? acc / l : 0.0f;
-    out[((size_t)lane_id * q_heads + head) * D + d] = val;
+    if (out) out[((size_t)lane_id * q_heads + head) * D + d] = val;
     if (out_xh) {
       const int k = head * D + d;
-      out_xh[((size_t)(k >> 3) * xh_nv + lane_id) * 8 + (k & 7)] = __float2half_rn(fminf(fmaxf(val, -65504.f), 65504.f));
+      out_xh[hand_off_cell(k >> 3, lane_id, xh_nv, q_heads * (D / 8)) + (k & 7)] = __float2half_rn(fminf(fmaxf(val, -65504.f), 65504.f));
     }
   }
+}
+
+// --------------------------------------------------------------------------------------------
+// Chunked prefill: T query tokens per lane on top of the cached ones (napi/mod.rs:3420-3477 semantics: token t of the chunk
+// attends positions up to cursor + t). Grid (token tiles, kv_heads, batch), longest tiles first. A CTA of 4 warps serves 64
+// MMA rows = (token, query head) pairs of 64 / G tokens, 16 rows per warp; the warps walk the lane's pages together, four
+// pages (64 positions) at a time, which arrive by cp.async one step ahead in a ring of two stages. Per step a warp does
+// S = Q K^T (16 x 64), the online softmax in registers and O += P V with mma.sync.
+//
+// Bound by the legacy tensor path (a step is 512 mma.sync per CTA at head dim 128, three CTAs per SM). One 16-row tile per
+// CTA whose warps took alternate pages and merged at the end read every page four times as often and computed a score in
+// twice the instructions.
+// --------------------------------------------------------------------------------------------
+constexpr int kChunkRows = 64;       // MMA rows per CTA
+constexpr int kChunkTokens = 64;     // cached positions per step
+constexpr int kChunkPages = kChunkTokens / kPageTokens;
+
+template <int D, bool U8>
+struct ChunkCfg {
+  static constexpr int kSide = kChunkTokens * D * 2;                 // K or V of a step as MMA operands
+  static constexpr int kRawSide = U8 ? kChunkTokens * D : kSide;     // as cached
+  static constexpr int kScales = U8 ? 2 * kChunkTokens * 4 : 0;      // row scales of K, then of V
+  static constexpr int kStage = 2 * kRawSide + kScales;
+  static constexpr size_t kSmemBytes = 2 * (size_t)kStage + (U8 ? 2 * kSide : 0);
+};
+
+__device__ __forceinline__ void cp_async16_or_zero(void* smem_dst, const void* gmem_src, bool live) {
+  const unsigned dst = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(gmem_src), "r"(live ? 16 : 0));
+}
+
+template <int D, bool BF16, bool U8>
+__global__ void __launch_bounds__(128, U8 ? 2 : 3) attention_chunk_kernel(AttnArgs a) {
+  using Cfg = ChunkCfg<D, U8>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  constexpr int CHUNKS = D / 8, KSTEPS = D / 16, DTILES = D / 8, NT = kChunkTokens / 8;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
+  chain_wait();
+  const int kv_head = blockIdx.y, lane_id = blockIdx.z, T = a.tokens;
+  const LaneInfo info = a.lanes[lane_id];
+  const int G = a.q_heads / a.kv_heads, tile_tokens = kChunkRows / G;
+  const int token0 = (int)(gridDim.x - 1 - blockIdx.x) * tile_tokens, tokens_here = min(tile_tokens, T - token0);
+  const int row_lo = warp * 16 + g, row_hi = row_lo + 8;  // this thread's rows; row r is query token r / G, head r % G
+  const bool live_lo = row_lo < tokens_here * G, live_hi = row_hi < tokens_here * G;
+  const int token_lo = token0 + row_lo / G, token_hi = token0 + row_hi / G;
+  auto begin_of = [&](int end) { return a.op_window >= 0 ? max((int)max((long long)end - a.op_window, 0ll), info.start) : info.start; };
+  const bool idle = info.advance == 0;
+  const int end_lo = live_lo && !idle ? info.cursor + token_lo + 1 : 0, end_hi = live_hi && !idle ? info.cursor + token_hi + 1 : 0;
+  const int begin_lo = begin_of(end_lo), begin_hi = begin_of(end_hi);
+  // the tile as a whole, and the positions that every row of this warp attends
+  const int end = idle ? 0 : info.cursor + token0 + tokens_here, begin = begin_of(idle ? 0 : info.cursor + token0 + 1);
+  const int full_begin = begin_of(info.cursor + token0 + min(warp * 16 + 15, tokens_here * G - 1) / G + 1);
+  const int full_end = warp * 16 + 15 < tokens_here * G && !idle ? info.cursor + token0 + warp * 16 / G + 1 : 0;
+  const int first_page = begin / kPageTokens, last_page = end > begin ? (end - 1) / kPageTokens + 1 : first_page;
+  const int steps = (last_page - first_page + kChunkPages - 1) / kChunkPages;
+
+  const int* table = a.tables + info.table_offset;
+  constexpr int RAW_PAGE = Cfg::kRawSide / kChunkPages;
+  const size_t page_stride = (size_t)a.kv_heads * RAW_PAGE;
+  const unsigned char* kbase = reinterpret_cast<const unsigned char*>(a.k) + (size_t)kv_head * RAW_PAGE;
+  const unsigned char* vbase = reinterpret_cast<const unsigned char*>(a.v) + (size_t)kv_head * RAW_PAGE;
+  auto load = [&](int step) {
+    unsigned char* ks = smem + (step & 1) * Cfg::kStage;
+    unsigned char* vs = ks + Cfg::kRawSide;
+    const int page0 = first_page + step * kChunkPages;
+    size_t page[kChunkPages];
+#pragma unroll
+    for (int p = 0; p < kChunkPages; ++p) page[p] = (size_t)table[min(page0 + p, last_page - 1)];
+    constexpr int PER_PAGE = RAW_PAGE / 16;  // 16-byte chunks; pages beyond the last are zeros (0 x NaN is not 0)
+#pragma unroll
+    for (int p = 0; p < kChunkPages; ++p) {
+      const bool live = page0 + p < last_page;
+#pragma unroll
+      for (int c = threadIdx.x; c < PER_PAGE; c += 128) {
+        const size_t src = page[p] * page_stride + (size_t)c * 16;
+        const int at = U8 ? (p * PER_PAGE + c) * 16 : swizzled_offset<D>(p * kPageTokens + c / CHUNKS, c % CHUNKS);
+        cp_async16_or_zero(ks + at, kbase + src, live);
+        cp_async16_or_zero(vs + at, vbase + src, live);
+      }
+    }
+    if (U8 && threadIdx.x < 8 * kChunkPages) {  // 16 f32 scales per page and side: 4 chunks each
+      const int p = threadIdx.x >> 3, c = threadIdx.x & 7;
+      const size_t si = ((size_t)table[min(page0 + p, last_page - 1)] * a.kv_heads + kv_head) * kPageTokens + (c & 3) * 4;
+      cp_async16_or_zero(ks + 2 * Cfg::kRawSide + (c >> 2) * kChunkTokens * 4 + p * kPageTokens * 4 + (c & 3) * 16, (c < 4 ? a.k_scale : a.v_scale) + si,
+                         page0 + p < last_page);
+    }
+    cp_async_commit();
+  };
+  if (steps > 0) load(0);
+
+  uint32_t qf[KSTEPS][4];
+  {
+    const float* q_lo = a.q + (((size_t)lane_id * T + (live_lo ? token_lo : 0)) * a.q_heads + kv_head * G + (live_lo ? row_lo % G : 0)) * D;
+    const float* q_hi = a.q + (((size_t)lane_id * T + (live_hi ? token_hi : 0)) * a.q_heads + kv_head * G + (live_hi ? row_hi % G : 0)) * D;
+#pragma unroll
+    for (int ks = 0; ks < KSTEPS; ++ks) {
+      const int c0 = ks * 16 + 2 * t;
+      const float2 x0 = *reinterpret_cast<const float2*>(q_lo + c0), x1 = *reinterpret_cast<const float2*>(q_hi + c0);
+      const float2 x2 = *reinterpret_cast<const float2*>(q_lo + c0 + 8), x3 = *reinterpret_cast<const float2*>(q_hi + c0 + 8);
+      qf[ks][0] = pack2<BF16>(x0.x * a.scale_log2, x0.y * a.scale_log2);
+      qf[ks][1] = pack2<BF16>(x1.x * a.scale_log2, x1.y * a.scale_log2);
+      qf[ks][2] = pack2<BF16>(x2.x * a.scale_log2, x2.y * a.scale_log2);
+      qf[ks][3] = pack2<BF16>(x3.x * a.scale_log2, x3.y * a.scale_log2);
+    }
+  }
+  float o[DTILES][4];
+#pragma unroll
+  for (int i = 0; i < DTILES; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[i][j] = 0.0f;
+  float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.0f, l_hi = 0.0f;
+
+  for (int step = 0; step < steps; ++step) {
+    cp_async_wait<0>();
+    __syncthreads();  // this step's pages are in, and every warp is done with the stage that the next load overwrites
+    if (step + 1 < steps) load(step + 1);
+    const unsigned char* raw = smem + (step & 1) * Cfg::kStage;
+    const unsigned char* ks_page = raw;
+    const unsigned char* vs_page = raw + Cfg::kRawSide;
+    const float* scales = reinterpret_cast<const float*>(raw + 2 * Cfg::kRawSide);
+    if (U8) {  // bytes -> f16 integers (code - 128) in the swizzled operand layout; the row scales come in below
+      unsigned char* wide = smem + 2 * Cfg::kStage;
+      for (int c = threadIdx.x; c < 2 * Cfg::kRawSide / 16; c += 128) {
+        const int side = c / (Cfg::kRawSide / 16), cc = c % (Cfg::kRawSide / 16), row = cc / (D / 16), chunk = 2 * (cc % (D / 16));
+        const uint4 codes = *reinterpret_cast<const uint4*>(raw + (size_t)c * 16);
+        const uint32_t w[4] = {codes.x, codes.y, codes.z, codes.w};
+        uint32_t h[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bytes_to_half2(w[j], h[2 * j], h[2 * j + 1]);
+        unsigned char* dst = wide + side * Cfg::kSide;
+        *reinterpret_cast<uint4*>(dst + swizzled_offset<D>(row, chunk)) = make_uint4(h[0], h[1], h[2], h[3]);
+        *reinterpret_cast<uint4*>(dst + swizzled_offset<D>(row, chunk + 1)) = make_uint4(h[4], h[5], h[6], h[7]);
+      }
+      __syncthreads();
+      ks_page = wide;
+      vs_page = wide + Cfg::kSide;
+    }
+    // S = Q K^T: eight n-tiles of 8 positions
+    float s[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.0f;
+#pragma unroll
+    for (int ks = 0; ks < KSTEPS; ++ks)
+#pragma unroll
+      for (int n = 0; n < NT; n += 2) {
+        uint32_t kf[4];
+        ldmatrix_x4(kf, ks_page + swizzled_offset<D>(n * 8 + (lane & 7) + ((lane >> 4) << 3), 2 * ks + ((lane >> 3) & 1)));
+        mma_16816<BF16>(s[n], qf[ks], kf[0], kf[1]);
+        mma_16816<BF16>(s[n + 1], qf[ks], kf[2], kf[3]);
+      }
+    const int base = (first_page + step * kChunkPages) * kPageTokens;
+    if (U8) {
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        const float2 sc = *reinterpret_cast<const float2*>(scales + n * 8 + 2 * t);
+        s[n][0] *= sc.x; s[n][1] *= sc.y; s[n][2] *= sc.x; s[n][3] *= sc.y;
+      }
+    }
+    if (base < full_begin || base + kChunkTokens > full_end) {
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int pos = base + n * 8 + 2 * t + j;
+          if (pos < begin_lo || pos >= end_lo) s[n][j] = -INFINITY;
+          if (pos < begin_hi || pos >= end_hi) s[n][2 + j] = -INFINITY;
+        }
+    }
+    float mx_lo = m_lo, mx_hi = m_hi;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      mx_lo = fmaxf(mx_lo, fmaxf(s[n][0], s[n][1]));
+      mx_hi = fmaxf(mx_hi, fmaxf(s[n][2], s[n][3]));
+    }
+    mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1));
+    mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
+    mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
+    mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
+    // a row with every position masked so far keeps its maximum at -inf: keep factors finite
+    const float sub_lo = mx_lo == -INFINITY ? 0.0f : mx_lo, sub_hi = mx_hi == -INFINITY ? 0.0f : mx_hi;
+    const float alpha_lo = exp2f(m_lo - sub_lo), alpha_hi = exp2f(m_hi - sub_hi);
+    m_lo = mx_lo; m_hi = mx_hi;
+    l_lo *= alpha_lo; l_hi *= alpha_hi;
+#pragma unroll
+    for (int i = 0; i < DTILES; ++i) { o[i][0] *= alpha_lo; o[i][1] *= alpha_lo; o[i][2] *= alpha_hi; o[i][3] *= alpha_hi; }
+    // O += P V, 16 positions at a time
+#pragma unroll
+    for (int n = 0; n < NT; n += 2) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float (&p)[4] = s[n + h];
+        p[0] = exp2f(p[0] - sub_lo); p[1] = exp2f(p[1] - sub_lo); p[2] = exp2f(p[2] - sub_hi); p[3] = exp2f(p[3] - sub_hi);
+        l_lo += p[0] + p[1];
+        l_hi += p[2] + p[3];
+        if (U8) {  // V row scales ride on the probabilities; the denominators stay unscaled
+          const float2 sc = *reinterpret_cast<const float2*>(scales + kChunkTokens + (n + h) * 8 + 2 * t);
+          p[0] *= sc.x; p[1] *= sc.y; p[2] *= sc.x; p[3] *= sc.y;
+        }
+      }
+      const uint32_t pf[4] = {pack2<BF16>(s[n][0], s[n][1]), pack2<BF16>(s[n][2], s[n][3]), pack2<BF16>(s[n + 1][0], s[n + 1][1]),
+                              pack2<BF16>(s[n + 1][2], s[n + 1][3])};
+#pragma unroll
+      for (int dp = 0; dp < DTILES / 2; ++dp) {
+        uint32_t vf[4];
+        ldmatrix_x4_trans(vf, vs_page + swizzled_offset<D>(n * 8 + (lane & 7) + (((lane >> 3) & 1) << 3), 2 * dp + (lane >> 4)));
+        mma_16816<BF16>(o[2 * dp], pf, vf[0], vf[1]);
+        mma_16816<BF16>(o[2 * dp + 1], pf, vf[2], vf[3]);
+      }
+    }
+  }
+  // quad-reduce the denominators (each lane summed its own columns)
+  l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
+  l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
+  l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
+  l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (!(h ? live_hi : live_lo)) continue;
+    const float l = h ? l_hi : l_lo, inv = l > 0.0f ? 1.0f / l : 0.0f;
+    const size_t row = (size_t)lane_id * T + (h ? token_hi : token_lo);
+    const int head = kv_head * G + (h ? row_hi : row_lo) % G;
+#pragma unroll
+    for (int i = 0; i < DTILES; ++i) {
+      const float x = o[i][2 * h] * inv, y = o[i][2 * h + 1] * inv;
+      if (a.out) *reinterpret_cast<float2*>(a.out + (row * a.q_heads + head) * D + i * 8 + 2 * t) = make_float2(x, y);
+      if (a.out_xh) {
+        const __half2 v = __floats2half2_rn(fminf(fmaxf(x, -65504.f), 65504.f), fminf(fmaxf(y, -65504.f), 65504.f));
+        *reinterpret_cast<__half2*>(a.out_xh + hand_off_cell(head * (D / 8) + i, row, a.out_xh_nv, a.q_heads * (D / 8)) + 2 * t) = v;
+      }
+    }
+  }
+}
+
+template <int D, bool BF16, bool U8>
+static cudaError_t launch_attention_chunk_t(const AttnArgs& args, int batch, cudaStream_t stream) {
+  constexpr size_t smem = ChunkCfg<D, U8>::kSmemBytes;
+  auto kernel = attention_chunk_kernel<D, BF16, U8>;
+  const cudaError_t attr = opt_in_shared_memory(kernel, smem);
+  if (attr != cudaSuccess) return attr;
+  const int tile_tokens = kChunkRows / (args.q_heads / args.kv_heads);
+  return launch_chained(kernel, dim3((unsigned)((args.tokens + tile_tokens - 1) / tile_tokens), (unsigned)args.kv_heads, (unsigned)batch), dim3(128), smem, stream,
+                        args);
 }
 
 bool attention_mma_supported(const PoolView& pool, int q_heads, int tokens) {
@@ -687,7 +922,7 @@ size_t plan_attention_max_scratch(int batch, int q_heads, int kv_heads, int head
   return need;
 }
 
-template <int D, bool BF16, bool CHUNK, bool U8>
+template <int D, bool BF16, bool U8>
 static cudaError_t launch_attention_mma_t(const PoolView& pool, const AttnArgs& args, int batch, int grid_x,
                                           cudaStream_t stream) {
   constexpr size_t page = (size_t)kPageTokens * D * 2;
@@ -695,7 +930,7 @@ static cudaError_t launch_attention_mma_t(const PoolView& pool, const AttnArgs& 
                              : (size_t)kAttnWarps * kAttnStages * 2 * page;
   constexpr size_t merge = (size_t)kAttnWarps * 16 * (D + 2) * sizeof(float);
   constexpr size_t smem = ring > merge ? ring : merge;
-  auto kernel = attention_mma_kernel<D, BF16, CHUNK, U8>;
+  auto kernel = attention_mma_kernel<D, BF16, U8>;
   const cudaError_t attr = opt_in_shared_memory(kernel, smem);
   if (attr != cudaSuccess) return attr;
   dim3 grid((unsigned)grid_x, (unsigned)pool.kv_heads, (unsigned)batch);
@@ -707,7 +942,6 @@ cudaError_t launch_attention_mma(const PoolView& pool, const float* q, const Lan
                                  const AttnPlan& plan, float* scratch, cudaStream_t stream, int* launches, __half* out_xh, int xh_nv,
                                  int tokens) {
   if (batch == 0) return cudaSuccess;
-  if (batch > xh_nv || tokens > 1) out_xh = nullptr;
   AttnArgs args;
   args.out_xh = out_xh;
   args.out_xh_nv = xh_nv;
@@ -720,34 +954,24 @@ cudaError_t launch_attention_mma(const PoolView& pool, const float* q, const Lan
   args.k_scale = pool.k_scale;
   args.v_scale = pool.v_scale;
   cudaError_t e;
-  // the tier and the head width pick the instantiation; `chunk` the row mapping
-  auto dispatch = [&](auto chunk_tag, int grid_x) {
-    constexpr bool CHUNK = decltype(chunk_tag)::value;
-    const bool wide = pool.head_dim == 128;
-    if (pool.dtype == kKvU8)
-      return wide ? launch_attention_mma_t<128, false, CHUNK, true>(pool, args, batch, grid_x, stream)
-                  : launch_attention_mma_t<64, false, CHUNK, true>(pool, args, batch, grid_x, stream);
-    if (pool.dtype == kKvBF16)
-      return wide ? launch_attention_mma_t<128, true, CHUNK, false>(pool, args, batch, grid_x, stream)
-                  : launch_attention_mma_t<64, true, CHUNK, false>(pool, args, batch, grid_x, stream);
-    return wide ? launch_attention_mma_t<128, false, CHUNK, false>(pool, args, batch, grid_x, stream)
-                : launch_attention_mma_t<64, false, CHUNK, false>(pool, args, batch, grid_x, stream);
+  // the tier and the head width pick the instantiation
+  auto launch = [&](auto wide, auto bf16, auto u8) {
+    constexpr int D = decltype(wide)::value ? 128 : 64;
+    constexpr bool BF16 = decltype(bf16)::value, U8 = decltype(u8)::value;
+    return tokens > 1 ? launch_attention_chunk_t<D, BF16, U8>(args, batch, stream) : launch_attention_mma_t<D, BF16, U8>(pool, args, batch, plan.splits, stream);
   };
-  if (tokens > 1) {
-    // a prefill chunk: one CTA per tile of 16 / G tokens, no split over the pages
-    const int G = q_heads / pool.kv_heads;
-    const int per_tile = std::max(1, 16 / G);
-    e = dispatch(std::true_type(), (tokens + per_tile - 1) / per_tile);
-    if (e != cudaSuccess) return e;
-    if (launches) ++*launches;
-    return cudaSuccess;
-  }
-  e = dispatch(std::false_type(), plan.splits);
+  auto dispatch = [&](auto wide) {
+    if (pool.dtype == kKvU8) return launch(wide, std::false_type(), std::true_type());
+    if (pool.dtype == kKvBF16) return launch(wide, std::true_type(), std::false_type());
+    return launch(wide, std::false_type(), std::false_type());
+  };
+  e = pool.head_dim == 128 ? dispatch(std::true_type()) : dispatch(std::false_type());
   if (e != cudaSuccess) return e;
   if (launches) ++*launches;
+  if (tokens > 1) return cudaSuccess;
   if (plan.splits > 1) {
     dim3 grid((unsigned)q_heads, (unsigned)batch);
-    e = launch_chained(attention_merge_kernel, grid, dim3((unsigned)std::min(128, pool.head_dim)), 0, stream, (const float*)scratch, q_heads, plan.splits,
+    e = launch_chained(attention_merge_kernel, grid, dim3((unsigned)std::min(128, pool.head_dim)), 2 * (size_t)plan.splits * sizeof(float), stream, (const float*)scratch, q_heads, plan.splits,
                        pool.head_dim, out, out_xh, xh_nv);
     if (e != cudaSuccess) return e;
     if (launches) ++*launches;
@@ -756,7 +980,7 @@ cudaError_t launch_attention_mma(const PoolView& pool, const float* q, const Lan
 }
 
 // --------------------------------------------------------------------------------------------
-// Fused RoPE + KV append. grid (q_heads + 2*kv_heads, batch, tokens), D/2 threads: token t of lane b is row b*tokens + t
+// Fused RoPE + KV append. grid (groups of heads, batch, tokens), D/2 threads: token t of lane b is row b*tokens + t
 // of qkv, sits at position cursor + t, and its rotated query goes to q_out[b, t, head, :].
 // qkv row layout: [q heads | k heads | v heads] x D. Query heads are rotated into q_out, key heads
 // are rotated and stored into the pool, value heads are stored. Angles in f64 like rope_kernel.
@@ -767,106 +991,112 @@ __device__ __forceinline__ void pool_store(const PoolView& p, void* slab, size_t
   else reinterpret_cast<__nv_bfloat16*>(slab)[elem] = __float2bfloat16_rn(value);
 }
 
+// A CTA serves heads_per_cta consecutive heads of one row. One for decode steps, whose few rows need every SM and whose chain
+// is short; eight for chunks, where the f64 sine and cosine, the same for all heads of a row, would otherwise dominate (104 us
+// for 2048 rows x 48 heads).
 __global__ void rope_append_kernel(PoolView pool, const float* __restrict__ qkv, const LaneInfo* __restrict__ lanes,
                                    const int* __restrict__ tables, const double* __restrict__ inv_freq, int layout,
-                                   int q_heads, float* __restrict__ q_out, DeferredSum sum) {
+                                   int q_heads, int heads_per_cta, float* __restrict__ q_out, DeferredSum sum) {
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   chain_wait();
-  const int head = blockIdx.x, lane_id = blockIdx.y, tok = blockIdx.z, tokens = gridDim.z;
+  const int lane_id = blockIdx.y, tok = blockIdx.z, tokens = gridDim.z;
   const LaneInfo info = lanes[lane_id];
-  const int D = pool.head_dim, half = D / 2;
+  const int D = pool.head_dim, half = D / 2, heads = q_heads + 2 * pool.kv_heads;
   const bool live = (int)threadIdx.x < half;  // head dims below 64 leave threads of the warp without a pair
   const int j = live ? threadIdx.x : 0;
-  const size_t row_width = (size_t)(q_heads + 2 * pool.kv_heads) * D;
+  const size_t row_width = (size_t)heads * D;
   const size_t row = (size_t)lane_id * tokens + tok;
-  const float* src = qkv + row * row_width + (size_t)head * D;
   const int i0 = layout == 0 ? j : 2 * j, i1 = layout == 0 ? half + j : 2 * j + 1;
-  const bool is_q = head < q_heads, is_k = !is_q && head < q_heads + pool.kv_heads;
-  float r0, r1;
-  if (sum.splits > 0) {  // the projection left its split-K partials unsummed: add them up here, in split order
-    // (a narrow shard of a tensor-parallel group has up to 32 splits: eight loads are in flight at a time)
-    r0 = r1 = 0.f;
-    const float* p = sum.partials + row * sum.rows_padded + (size_t)head * D;
-    const size_t split_stride = (size_t)sum.vpad * sum.rows_padded;
-    if (sum.splits <= 8) {
-      for (int s = 0; s < sum.splits; ++s) {
-        r0 += p[(size_t)s * split_stride + i0];
-        r1 += p[(size_t)s * split_stride + i1];
-      }
-    } else for (int s0 = 0; s0 < sum.splits; s0 += 8) {
-      float first[8], second[8];
+  const int head0 = blockIdx.x * heads_per_cta, head1 = min(heads, head0 + heads_per_cta);
+  const int pos = info.cursor + tok;
+  int page = 0, slot = 0;
+  if (info.advance > 0 && head1 > q_heads) {
+    const int block = pos / pool.block_size;
+    page = tables[info.table_offset + block];
+    slot = pos - block * pool.block_size;
+  }
+  double s = 0.0, c = 1.0;
+  if (head0 < q_heads + pool.kv_heads) sincos((double)pos * inv_freq[j], &s, &c);
+  for (int head = head0; head < head1; ++head) {
+    const bool is_q = head < q_heads, is_k = !is_q && head < q_heads + pool.kv_heads;
+    float r0 = 0.f, r1 = 0.f;
+    if (sum.splits > 0) {  // the projection left its split-K partials unsummed: add them up here, in split order
+      // (a narrow shard of a tensor-parallel group has up to 32 splits: eight loads are in flight at a time)
+      const float* p = sum.partials + row * sum.rows_padded + (size_t)head * D;
+      const size_t split_stride = (size_t)sum.vpad * sum.rows_padded;
+      for (int s0 = 0; s0 < sum.splits; s0 += 8) {
+        float first[8], second[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const bool live = s0 + u < sum.splits;
-        first[u] = live ? p[(size_t)(s0 + u) * split_stride + i0] : 0.f;
-        second[u] = live ? p[(size_t)(s0 + u) * split_stride + i1] : 0.f;
-      }
+        for (int u = 0; u < 8; ++u) {
+          const bool there = s0 + u < sum.splits;
+          first[u] = there ? p[(size_t)(s0 + u) * split_stride + i0] : 0.f;
+          second[u] = there ? p[(size_t)(s0 + u) * split_stride + i1] : 0.f;
+        }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (s0 + u < sum.splits) {
-          r0 += first[u];
-          r1 += second[u];
+        for (int u = 0; u < 8; ++u) {
+          if (s0 + u < sum.splits) {
+            r0 += first[u];
+            r1 += second[u];
+          }
         }
       }
+    } else {
+      const float* src = qkv + row * row_width + (size_t)head * D;
+      r0 = src[i0];
+      r1 = src[i1];
     }
-  } else {
-    r0 = src[i0];
-    r1 = src[i1];
-  }
-  if (!live) r0 = r1 = 0.f;
-  if (is_q || is_k) {
-    const double angle = (double)(info.cursor + tok) * inv_freq[j];
-    double s, c;
-    sincos(angle, &s, &c);
-    const double first = (double)r0, second = (double)r1;
-    r0 = (float)__dsub_rn(__dmul_rn(first, c), __dmul_rn(second, s));
-    r1 = (float)__dadd_rn(__dmul_rn(second, c), __dmul_rn(first, s));
-  }
-  if (is_q) {
-    float* dst = q_out + (row * q_heads + head) * D;
-    if (live) {
-      dst[i0] = r0;
-      dst[i1] = r1;
+    if (!live) r0 = r1 = 0.f;
+    if (is_q || is_k) {
+      const double first = (double)r0, second = (double)r1;
+      r0 = (float)__dsub_rn(__dmul_rn(first, c), __dmul_rn(second, s));
+      r1 = (float)__dadd_rn(__dmul_rn(second, c), __dmul_rn(first, s));
     }
-    return;
-  }
-  if (info.advance == 0) return;  // padded lane: nothing is cached
-  const int kv_head = is_k ? head - q_heads : head - q_heads - pool.kv_heads;
-  const int pos = info.cursor + tok;
-  const int page = tables[info.table_offset + pos / pool.block_size], slot = pos % pool.block_size;
-  const size_t dst = pool_elem(pool, page, kv_head, slot);
-  void* slab = is_k ? pool.k : pool.v;
-  if (pool.dtype == kKvU8) {
-    // the int8 tier: one scale per cached row, as kv_append_kernel (pool.rs:224-240)
-    __shared__ float red[32];
-    float amax = fmaxf(fabsf(r0), fabsf(r1));
+    if (is_q) {
+      float* dst = q_out + (row * q_heads + head) * D;
+      if (live) {
+        dst[i0] = r0;
+        dst[i1] = r1;
+      }
+      continue;
+    }
+    if (info.advance == 0) continue;  // padded lane: nothing is cached
+    const int kv_head = is_k ? head - q_heads : head - q_heads - pool.kv_heads;
+    const size_t dst = pool_elem(pool, page, kv_head, slot);
+    void* slab = is_k ? pool.k : pool.v;
+    if (pool.dtype == kKvU8) {
+      // the int8 tier: one scale per cached row, as kv_append_kernel (pool.rs:224-240)
+      __shared__ float red[32];
+      float amax = fmaxf(fabsf(r0), fabsf(r1));
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
-    __syncthreads();
-    amax = 0.0f;
-    for (int w = 0; w < (int)((blockDim.x + 31) >> 5); ++w) amax = fmaxf(amax, red[w]);
-    const float scale = __fadd_rn(__fdiv_rn(amax, 127.0f), 1e-12f);
-    if (threadIdx.x == 0) (is_k ? pool.k_scale : pool.v_scale)[pool_scale_index(pool, page, kv_head, slot)] = scale;
-    const float c0 = fminf(fmaxf(roundf(__fdiv_rn(r0, scale)), -127.0f), 127.0f) + 128.0f;
-    const float c1 = fminf(fmaxf(roundf(__fdiv_rn(r1, scale)), -127.0f), 127.0f) + 128.0f;
-    if (live) {
-      reinterpret_cast<uint8_t*>(slab)[dst + i0] = (uint8_t)c0;
-      reinterpret_cast<uint8_t*>(slab)[dst + i1] = (uint8_t)c1;
+      for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+      __syncthreads();  // the previous head's maxima have been read
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+      __syncthreads();
+      amax = 0.0f;
+      for (int w = 0; w < (int)((blockDim.x + 31) >> 5); ++w) amax = fmaxf(amax, red[w]);
+      const float scale = __fadd_rn(__fdiv_rn(amax, 127.0f), 1e-12f);
+      if (threadIdx.x == 0) (is_k ? pool.k_scale : pool.v_scale)[pool_scale_index(pool, page, kv_head, slot)] = scale;
+      const float c0 = fminf(fmaxf(roundf(__fdiv_rn(r0, scale)), -127.0f), 127.0f) + 128.0f;
+      const float c1 = fminf(fmaxf(roundf(__fdiv_rn(r1, scale)), -127.0f), 127.0f) + 128.0f;
+      if (live) {
+        reinterpret_cast<uint8_t*>(slab)[dst + i0] = (uint8_t)c0;
+        reinterpret_cast<uint8_t*>(slab)[dst + i1] = (uint8_t)c1;
+      }
+      continue;
     }
-    return;
+    if (!live) continue;
+    pool_store(pool, slab, dst + i0, r0);
+    pool_store(pool, slab, dst + i1, r1);
   }
-  if (!live) return;
-  pool_store(pool, slab, dst + i0, r0);
-  pool_store(pool, slab, dst + i1, r1);
 }
 
 cudaError_t launch_rope_append(const PoolView& pool, const float* qkv, const LaneInfo* lanes, const int* tables,
                                const double* inv_freq, int layout, int batch, int q_heads, float* q_out,
                                cudaStream_t stream, const DeferredSum* sum, int tokens) {
   if (batch == 0) return cudaSuccess;
-  dim3 grid((unsigned)(q_heads + 2 * pool.kv_heads), (unsigned)batch, (unsigned)tokens);
-  return launch_chained(rope_append_kernel, grid, dim3((unsigned)std::max(32, (pool.head_dim / 2 + 31) / 32 * 32)), 0, stream, pool, qkv, lanes, tables, inv_freq, layout, q_heads,
+  const int heads = q_heads + 2 * pool.kv_heads, per = (int64_t)batch * tokens >= 512 ? 8 : 1;
+  dim3 grid((unsigned)((heads + per - 1) / per), (unsigned)batch, (unsigned)tokens);
+  return launch_chained(rope_append_kernel, grid, dim3((unsigned)std::max(32, (pool.head_dim / 2 + 31) / 32 * 32)), 0, stream, pool, qkv, lanes, tables, inv_freq, layout, q_heads, per,
                         q_out, sum ? *sum : DeferredSum());
 }
 

@@ -51,10 +51,9 @@ struct etc_decoder {
   // device workspaces
   float *hidden = nullptr, *normed = nullptr, *qkv = nullptr, *qr = nullptr, *attl = nullptr, *proj = nullptr, *g = nullptr, *u = nullptr, *act = nullptr,
         *last = nullptr, *logits = nullptr;
-  // f16 activation hand-off between kernels of the one-token fast path ([K/8][32][8] order, rows >= batch stay zero)
+  // f16 activation hand-off between the kernels of a tiled model
   __half *xh_norm = nullptr, *xh_att = nullptr, *xh_act = nullptr;
   bool xh_path = false;
-  int xh_nv = 32;  // row stride of the hand-off layout: the batch padded to 32, 64 or 128
   float* lin_scratch = nullptr;
   size_t lin_scratch_bytes = 0;
   float* attn_scratch = nullptr;
@@ -268,7 +267,7 @@ etc_status run_linear(StepContext& s, const BoundWeight& raw, etc_qweight* tiled
   if (defer) *defer = DeferredSum();
   if (tiled_w) {
     ETC_CUDA(launch_qlinear_tiled(tiled_w->tiled, x, vectors, nullptr, residual, epilogue, out, d->lin_scratch,
-                                  d->rt->d_status, d->rt->sm_count, stream, &s.launches, xh_ready, out_xh, d->xh_nv, defer));
+                                  d->rt->d_status, d->rt->sm_count, stream, &s.launches, xh_ready, out_xh, hand_off_stride(vectors), defer));
     return ETC_OK;
   }
   if (raw.codec == ETC_CODEC_F32) {
@@ -322,15 +321,16 @@ etc_status project_into_hidden(StepContext& s, const BoundWeight& raw, etc_qweig
   return ETC_OK;
 }
 
-// RMSNorm of the residual stream into the f16 hand-off layout; `pending` holds the split-K partials of the projection
+// RMSNorm of `x` (the residual stream) into the f16 hand-off layout; `pending` holds the split-K partials of the projection
 // before it when that projection left them unsummed.
-etc_status norm_hand_off(StepContext& s, const BoundWeight& weight, int64_t rows, DeferredSum& pending) {
+etc_status norm_hand_off(StepContext& s, float* x, const BoundWeight& weight, int64_t rows, DeferredSum& pending) {
   etc_decoder* d = s.dec;
   const etc_decoder_config& c = d->cfg;
+  const int nv = hand_off_stride(rows);
   if (pending.splits > 0)
-    ETC_CUDA(launch_sum_rmsnorm_xh8(d->hidden, pending, (const float*)weight.d_raw, c.rms_eps, rows, c.d_model, d->xh_norm, d->rt->stream, d->xh_nv));
+    ETC_CUDA(launch_sum_rmsnorm_xh8(x, pending, (const float*)weight.d_raw, c.rms_eps, rows, c.d_model, d->xh_norm, d->rt->stream, nv));
   else
-    ETC_CUDA(launch_rmsnorm_xh8(d->hidden, (const float*)weight.d_raw, c.rms_eps, rows, c.d_model, d->xh_norm, d->rt->stream, d->xh_nv));
+    ETC_CUDA(launch_rmsnorm_xh8(x, (const float*)weight.d_raw, c.rms_eps, rows, c.d_model, d->xh_norm, d->rt->stream, nv));
   pending = DeferredSum();
   ++s.launches;
   return ETC_OK;
@@ -356,14 +356,13 @@ etc_status enqueue_step(StepContext& s) {
   }
   ++s.launches;
 
+  const bool xh = d->xh_path;  // activations go from kernel to kernel as f16 in the tensor-core operand order
   DeferredSum pending;  // partials of the last projection onto the residual stream, summed by the next RMSNorm
   for (int l = 0; l < c.layers; ++l) {
     const size_t li = (size_t)l;
     const PoolView view = s.pool->view(l);
-    // one-token steps of a tiled model hand activations from kernel to kernel as f16 in the tensor-core operand order
-    const bool xh = d->xh_path && T == 1;
     if (xh) {
-      ETC_TRY(norm_hand_off(s, d->attn_norm[li], rows, pending));
+      ETC_TRY(norm_hand_off(s, d->hidden, d->attn_norm[li], rows, pending));
     } else {
       ETC_CUDA(launch_rmsnorm(d->hidden, (const float*)d->attn_norm[li].d_raw, c.rms_eps, rows, c.d_model, d->normed, stream));
       ++s.launches;
@@ -382,8 +381,8 @@ etc_status enqueue_step(StepContext& s) {
         return fail(ETC_EXECUTION, "kv attention: split plan for " + std::to_string(s.max_pages) + " pages needs " +
                                        std::to_string(plan.scratch_bytes) + " bytes of partials, the decoder holds " +
                                        std::to_string(d->attn_scratch_bytes));
-      ETC_CUDA(launch_attention_mma(view, d->qr, d->d_lanes, d->d_tables, B, Hq, scale, c.window, d->attl, plan,
-                                    d->attn_scratch, stream, &s.launches, xh ? d->xh_att : nullptr, d->xh_nv, T));
+      ETC_CUDA(launch_attention_mma(view, d->qr, d->d_lanes, d->d_tables, B, Hq, scale, c.window, xh ? nullptr : d->attl, plan,
+                                    d->attn_scratch, stream, &s.launches, xh ? d->xh_att : nullptr, hand_off_stride(rows), T));
     } else {
       ETC_CUDA(launch_attention_exact(view, d->qr, d->d_lanes, d->d_tables, B, Hq, T, scale, c.window, d->attl, d->exact_scratch, s.max_ctx, stream, true));
       ++s.launches;
@@ -392,7 +391,7 @@ etc_status enqueue_step(StepContext& s) {
     ETC_TRY(project_into_hidden(s, d->wo[li], d->tiled ? d->t_o[li] : nullptr, d->attl, rows, xh_o ? d->xh_att : nullptr, 0,
                                 xh ? &pending : nullptr));
     if (xh) {
-      ETC_TRY(norm_hand_off(s, d->ffn_norm[li], rows, pending));
+      ETC_TRY(norm_hand_off(s, d->hidden, d->ffn_norm[li], rows, pending));
     } else {
       ETC_CUDA(launch_rmsnorm(d->hidden, (const float*)d->ffn_norm[li].d_raw, c.rms_eps, rows, c.d_model, d->normed, stream));
       ++s.launches;
@@ -415,26 +414,26 @@ etc_status enqueue_step(StepContext& s) {
       ETC_CUDA(launch_swiglu(d->g, d->u, rows * c.ffn, d->act, c.exact, stream));
       ++s.launches;
     }
+    // the last rows of a chunk are gathered from the finished residual stream
+    const bool finish = T > 1 && l + 1 == c.layers;
     ETC_TRY(project_into_hidden(s, d->down[li], d->tiled ? d->t_down[li] : nullptr, d->act, rows, xh ? d->xh_act : nullptr, 1,
-                                xh ? &pending : nullptr));
+                                xh && !finish ? &pending : nullptr));
   }
-  const bool xh_head = d->xh_path && T == 1;
-  if (xh_head) {
-    ETC_TRY(norm_hand_off(s, d->out_norm, rows, pending));
-  } else {
-    ETC_CUDA(launch_rmsnorm(d->hidden, (const float*)d->out_norm.d_raw, c.rms_eps, rows, c.d_model, d->normed, stream));
-    ++s.launches;
-  }
-  // LastTokenRow then the head: only the selected row of each lane reaches the head projection
-  // (each head output is an independent dot product, so the result equals projecting all rows first).
-  const float* head_in = d->normed;
+  // LastTokenRow, the final norm and the head: each row's norm and each head output stand alone, so only the selected row of
+  // each lane goes through them
+  float* head_in = d->hidden;
   if (T > 1) {
-    ETC_CUDA(launch_last_token_rows(d->normed, B, T, c.d_model, T, d->last, stream));
+    ETC_CUDA(launch_last_token_rows(d->hidden, B, T, c.d_model, T, d->last, stream));
     ++s.launches;
     head_in = d->last;
   }
-  ETC_TRY(run_linear(s, d->head, d->tiled ? d->t_head : nullptr, head_in, B, d->logits, ETC_EPILOGUE_NONE, nullptr,
-                     xh_head ? d->xh_norm : nullptr));
+  if (xh) {
+    ETC_TRY(norm_hand_off(s, head_in, d->out_norm, B, pending));
+  } else {
+    ETC_CUDA(launch_rmsnorm(head_in, (const float*)d->out_norm.d_raw, c.rms_eps, B, c.d_model, d->normed, stream));
+    ++s.launches;
+  }
+  ETC_TRY(run_linear(s, d->head, d->tiled ? d->t_head : nullptr, d->normed, B, d->logits, ETC_EPILOGUE_NONE, nullptr, xh ? d->xh_norm : nullptr));
   if (d->vocab_global > 0 && d->tp_world > 1) {
     // vocabulary-parallel head: every rank picks its best row, the ranks exchange (logit, token) pairs over peer memory
     if (!d->tp_peer) return fail(ETC_EXECUTION, "tensor parallel: a vocabulary-parallel head needs the peer exchange regions (etc_decoder_tp_peer_import)");
@@ -987,17 +986,13 @@ etc_status etc_decoder_finalize(etc_decoder* dec) {
           need = std::max(need, tiled_scratch_bytes(w->tiled, std::min<int64_t>(v, (int64_t)R), rt->sm_count));
     for (int64_t v : probes)
       need = std::max(need, tiled_scratch_bytes(dec->t_head->tiled, std::min<int64_t>(v, c.batch), rt->sm_count));
-    dec->xh_nv = hand_off_stride(c.batch) ? hand_off_stride(c.batch) : 32;
-    dec->xh_path = hand_off_stride(c.batch) != 0 && c.d_model % 8 == 0 && c.ffn % 8 == 0 && (c.q_heads * c.head_dim) % 8 == 0 &&
-                   c.d_model <= 8192;
+    dec->xh_path = c.d_model % 8 == 0 && c.ffn % 8 == 0 && (c.q_heads * c.head_dim) % 8 == 0 && c.d_model <= 8192;
     if (dec->xh_path) {
-      const size_t nv = (size_t)dec->xh_nv;
-      ETC_TRY(dalloc(dec, &dec->xh_norm, (size_t)c.d_model * nv));
-      ETC_TRY(dalloc(dec, &dec->xh_att, qw * nv));
-      ETC_TRY(dalloc(dec, &dec->xh_act, (size_t)c.ffn * nv));
-      ETC_CUDA(cudaMemsetAsync(dec->xh_norm, 0, (size_t)c.d_model * nv * sizeof(__half), rt->stream));
-      ETC_CUDA(cudaMemsetAsync(dec->xh_att, 0, qw * nv * sizeof(__half), rt->stream));
-      ETC_CUDA(cudaMemsetAsync(dec->xh_act, 0, (size_t)c.ffn * nv * sizeof(__half), rt->stream));
+      const size_t padded = (size_t)hand_off_rows((int64_t)R);
+      for (auto [buffer, width] : {std::pair{&dec->xh_norm, (size_t)c.d_model}, std::pair{&dec->xh_att, qw}, std::pair{&dec->xh_act, (size_t)c.ffn}}) {
+        ETC_TRY(dalloc(dec, buffer, width * padded));
+        ETC_CUDA(cudaMemsetAsync(*buffer, 0, width * padded * sizeof(__half), rt->stream));
+      }
       ETC_CUDA(cudaStreamSynchronize(rt->stream));
     }
     dec->lin_scratch_bytes = need;

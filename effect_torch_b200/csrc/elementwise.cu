@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_rows_kernel(const float* x, c
       __half2 h01 = __floats2half2_rn(sat(r0), sat(r1)), h23 = __floats2half2_rn(sat(r2), sat(r3));
       const int k = 4 * c;
       uint2 packed = make_uint2(*reinterpret_cast<uint32_t*>(&h01), *reinterpret_cast<uint32_t*>(&h23));
-      *reinterpret_cast<uint2*>(out_xh + ((size_t)(k >> 3) * xh_nv + row) * 8 + (k & 7)) = packed;
+      *reinterpret_cast<uint2*>(out_xh + hand_off_cell(k >> 3, row, xh_nv, n / 8) + (k & 7)) = packed;
     } else {
       reinterpret_cast<float4*>(out + (size_t)row * n)[c] = make_float4(r0, r1, r2, r3);
     }
@@ -313,7 +313,7 @@ cudaError_t launch_rmsnorm(const float* x, const float* weight, double eps, int6
 cudaError_t launch_rmsnorm_xh8(const float* x, const float* weight, double eps, int64_t rows, int64_t n, __half* out_xh,
                                cudaStream_t stream, int xh_nv) {
   if (rows == 0) return cudaSuccess;
-  if (rows > xh_nv || n % 8 != 0 || !rmsnorm_fast_ok(x, weight, n)) return cudaErrorInvalidValue;
+  if ((rows > xh_nv && xh_nv != 128) || n % 8 != 0 || !rmsnorm_fast_ok(x, weight, n)) return cudaErrorInvalidValue;
   return launch_chained(rmsnorm_rows_kernel<true, false, 256>, dim3((unsigned)rows), dim3(256), 0, stream, x, weight, eps, (int)n, (float*)nullptr, out_xh, xh_nv,
                         DeferredSum(), (float*)nullptr);
 }
@@ -505,13 +505,19 @@ __global__ void embedding_f32_kernel(const Index* __restrict__ indexes, int64_t 
     }
     return;
   }
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < columns; c += (int64_t)gridDim.x * blockDim.x)
-    out[i * columns + c] = table[row * columns + c];
+  const float* src = table + row * columns;
+  float* dst = out + i * columns;
+  if ((columns & 3) == 0 && ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < columns / 4; c += (int64_t)gridDim.x * blockDim.x)
+      reinterpret_cast<float4*>(dst)[c] = reinterpret_cast<const float4*>(src)[c];
+    return;
+  }
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < columns; c += (int64_t)gridDim.x * blockDim.x) dst[c] = src[c];
 }
 cudaError_t launch_embedding_f32(const void* indexes, int index_is_i64, int64_t count, const float* table, int64_t rows,
                                  int64_t columns, float* out, DeviceStatus* status, cudaStream_t stream) {
   if (count == 0) return cudaSuccess;
-  dim3 grid((unsigned)std::min<int64_t>((columns + 255) / 256, 32), (unsigned)count);
+  dim3 grid((unsigned)std::min<int64_t>((columns + 1023) / 1024, 8), (unsigned)count);
   if (index_is_i64)
     return launch_chained(embedding_f32_kernel<long long>, grid, dim3(256), 0, stream, (const long long*)indexes, count, table, rows, columns, out, status);
   else

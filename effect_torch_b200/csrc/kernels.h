@@ -10,6 +10,17 @@
 
 namespace etc {
 
+// ---- f16 activation hand-off ------------------------------------------------------------------
+// Activations travel between the kernels of an invocation as f16 in the tensor cores' operand order: [chunk of nv rows]
+// [K/8][nv][8] with nv = hand_off_stride(rows) = 32, 64 or 128; only 128 has more than one chunk.
+inline int hand_off_stride(int64_t rows) { return rows <= 32 ? 32 : (rows <= 64 ? 64 : 128); }
+// Rows padded to whole chunks: the size of a buffer that any number of rows up to `rows` fits.
+inline int64_t hand_off_rows(int64_t rows) { return rows <= 64 ? hand_off_stride(rows) : (rows + 127) / 128 * 128; }
+// Offset (in halves) of columns 8 * k8 .. 8 * k8 + 7 of a row of k8_total * 8 columns.
+__host__ __device__ inline size_t hand_off_cell(int k8, size_t row, int nv, int k8_total) {
+  return (((row / nv) * k8_total + k8) * nv + row % nv) * 8;
+}
+
 // ---- block-quantized weights (quant_kernels.cu) ------------------------------------------
 cudaError_t launch_dequantize(int codec, const uint8_t* packed, int64_t rows, int64_t columns, float* out,
                               cudaStream_t stream);
@@ -65,7 +76,7 @@ cudaError_t launch_repack(const TiledWeight& w, const RepackParts& parts, cudaSt
 
 // Sums split-K partials [chunk of vpad vectors][splits][vpad][rows_padded] in split order and runs the epilogue.
 cudaError_t launch_qlinear_reduce(const float* scratch, int splits, int vpad, int vectors, int rows, int rows_padded,
-                                  const float* bias, const float* residual, int epilogue, float* out, cudaStream_t stream);
+                                  const float* bias, const float* residual, int epilogue, float* out, __half* out_xh, int xh_nv, cudaStream_t stream);
 
 // decode batches up to stream_max_vectors() (qlinear_stream.cu)
 struct StreamPlan {
@@ -94,9 +105,9 @@ struct UmmaPlan {
 };
 UmmaPlan plan_umma(const TiledWeight& w, int64_t vectors, int sm_count);
 cudaError_t launch_repack_umma(const TiledWeight& w, const RepackParts& parts, cudaStream_t stream);
-// x: f32 [vectors, K], converted to f16 in xh first.
-cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, int64_t vectors, const float* bias, const float* residual, int epilogue,
-                                float* out, __half* xh, float* scratch, DeviceStatus* status, int sm_count, cudaStream_t stream,
+// x: f32 [vectors, K], converted to f16 in xh first, or xh_ready in the hand-off layout.
+cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, const __half* xh_ready, int64_t vectors, const float* bias,
+                                const float* residual, int epilogue, float* out, __half* out_xh, __half* xh, float* scratch, DeviceStatus* status, int sm_count, cudaStream_t stream,
                                 int* launches);
 
 // small-batch matvec on the 128-row layout (qlinear_mv.cu): up to 32 vectors per pass, mma.sync fed by a bulk-copy ring
@@ -117,15 +128,12 @@ cudaError_t launch_qlinear_mv(const TiledWeight& w, const float* x, const __half
 
 // Front end of the tiled linear. `scratch` must hold tiled_scratch_bytes(w, vectors, sm_count).
 size_t tiled_scratch_bytes(const TiledWeight& w, int64_t vectors, int sm_count);
-// xh_ready / out_xh: optional f16 activation hand-off between kernels, [K/8][xh_nv][8] with xh_nv = hand_off_stride(batch)
-// (up to 128 vectors).
+// xh_ready / out_xh: optional f16 activation hand-off between kernels with xh_nv = hand_off_stride(vectors).
 cudaError_t launch_qlinear_tiled(const TiledWeight& w, const float* x, int64_t vectors, const float* bias,
                                  const float* residual, int epilogue, float* out, void* scratch, DeviceStatus* status,
                                  int sm_count, cudaStream_t stream, int* launches, const __half* xh_ready = nullptr,
                                  __half* out_xh = nullptr, int xh_nv = 32, DeferredSum* defer = nullptr);
-// Row stride of the f16 hand-off layout for `vectors` rows: 32, 64 or 128 (0: no hand-off above 128 vectors).
-inline int hand_off_stride(int64_t vectors) { return vectors <= 32 ? 32 : (vectors <= 64 ? 64 : (vectors <= 128 ? 128 : 0)); }
-// RMSNorm whose output is stored as f16 [n/8][xh_nv][8] (rows <= xh_nv).
+// RMSNorm whose output is stored in the hand-off layout.
 cudaError_t launch_rmsnorm_xh8(const float* x, const float* weight, double eps, int64_t rows, int64_t n, __half* out_xh,
                                cudaStream_t stream, int xh_nv = 32);
 // The same after x += sum of a projection's split-K partials (x is updated in place: the residual stream).

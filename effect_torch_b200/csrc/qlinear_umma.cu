@@ -68,6 +68,7 @@ struct GemmArgs {
   const float* bias;
   const float* residual;
   float* out;
+  __half* out_xh;               // SwiGLU only: the result (also) as f16 for the next linear
   float* scratch;               // [chunk][split][128][rows_padded]
   unsigned long long* status;
   int vectors, rows, rows_padded, kblocks, epilogue;
@@ -175,7 +176,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qlinear_gemm_kernel(GemmArgs 
             const float first = __uint_as_float(bits[v]) + bias_v, second = __uint_as_float(bits[v + 1]) + bias_v;
             const float other = __shfl_xor_sync(0xffffffffu, is_up ? first : second, 8);
             const float act = silu_tanh(is_up ? other : first) * (is_up ? second : other);
-            if (oc < a.rows / 2 && v + is_up < left) a.out[(size_t)(v_base + v0 + v + is_up) * (a.rows / 2) + oc] = act;
+            const int at = v_base + v0 + v + is_up;
+            if (oc >= a.rows / 2 || v + is_up >= left) continue;
+            if (a.out) a.out[(size_t)at * (a.rows / 2) + oc] = act;
+            if (a.out_xh) a.out_xh[hand_off_cell(oc >> 3, at, NV, a.rows / 16) + (oc & 7)] = __float2half_rn(fminf(fmaxf(act, -65504.f), 65504.f));
           }
         } else if (r < a.rows) {
           const size_t at = (size_t)(v_base + v0) * a.rows + r;
@@ -485,18 +489,22 @@ UmmaPlan plan_umma(const TiledWeight& w, int64_t vectors, int sm_count) {
 }
 
 // qlinear_reduce_kernel lives in quant_kernels.cu
-cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, int64_t vectors, const float* bias, const float* residual, int epilogue,
-                                float* out, __half* xh, float* scratch, DeviceStatus* status, int sm_count, cudaStream_t stream,
+cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, const __half* xh_ready, int64_t vectors, const float* bias,
+                                const float* residual, int epilogue, float* out, __half* out_xh, __half* xh, float* scratch, DeviceStatus* status, int sm_count, cudaStream_t stream,
                                 int* launches) {
   if (vectors <= 0) return cudaSuccess;
   const UmmaPlan plan = plan_umma(w, vectors, sm_count);
   const int K = (int)w.columns;
-  const int64_t total = (int64_t)(K / 8) * plan.nv * plan.chunks;
-  cudaError_t e = launch_chained(convert_xh8_kernel, dim3((unsigned)std::min<int64_t>((total + 255) / 256, 148 * 8)), dim3(256), 0, stream, x, (int)vectors, K, xh);
-  if (e != cudaSuccess) return e;
-  if (launches) ++*launches;
+  cudaError_t e = cudaSuccess;
+  if (!xh_ready) {
+    const int64_t total = (int64_t)(K / 8) * plan.nv * plan.chunks;
+    e = launch_chained(convert_xh8_kernel, dim3((unsigned)std::min<int64_t>((total + 255) / 256, 148 * 8)), dim3(256), 0, stream, x, (int)vectors, K, xh);
+    if (e != cudaSuccess) return e;
+    if (launches) ++*launches;
+  }
   GemmArgs args;
-  args.xh = xh;
+  args.xh = xh_ready ? xh_ready : xh;
+  args.out_xh = epilogue == ETC_EPILOGUE_SWIGLU ? out_xh : nullptr;
   args.bias = bias;
   args.residual = residual;
   args.out = out;
@@ -536,7 +544,7 @@ cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, int64_t ve
   }
   if (plan.splits == 1) return cudaSuccess;
   if (launches) ++*launches;
-  return launch_qlinear_reduce(scratch, plan.splits, plan.nv, (int)vectors, (int)w.rows, (int)w.rows_padded, bias, residual, epilogue, out, stream);
+  return launch_qlinear_reduce(scratch, plan.splits, plan.nv, (int)vectors, (int)w.rows, (int)w.rows_padded, bias, residual, epilogue, out, args.out_xh, plan.nv, stream);
 }
 
 }  // namespace etc

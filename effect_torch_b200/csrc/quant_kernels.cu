@@ -410,7 +410,7 @@ __device__ __forceinline__ float silu_tanh_form(float x) { return x * (tanhf(x *
 // neither carries a no-alias promise.
 __global__ void qlinear_reduce_kernel(const float* __restrict__ scratch, int splits, int vpad, int vectors, int rows,
                                       int rows_padded, const float* __restrict__ bias, const float* residual,
-                                      int epilogue, float* out) {
+                                      int epilogue, float* out, __half* __restrict__ out_xh, int xh_nv) {
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   chain_wait();
   const int out_cols = epilogue == ETC_EPILOGUE_SWIGLU ? rows / 2 : rows;
@@ -427,7 +427,8 @@ __global__ void qlinear_reduce_kernel(const float* __restrict__ scratch, int spl
       }
       if (bias) { gsum += bias[r_gate]; usum += bias[r_up]; }
       const float act = silu_tanh_form(gsum) * usum;
-      out[idx] = act;
+      if (out) out[idx] = act;
+      if (out_xh) out_xh[hand_off_cell(c >> 3, v, xh_nv, out_cols / 8) + (c & 7)] = __float2half_rn(fminf(fmaxf(act, -65504.f), 65504.f));
     } else {
       float sum = 0.f;
       for (int s = 0; s < splits; ++s) sum += scratch[((size_t)(v / vpad * splits + s) * vpad + v % vpad) * rows_padded + c];
@@ -439,13 +440,14 @@ __global__ void qlinear_reduce_kernel(const float* __restrict__ scratch, int spl
 }
 
 cudaError_t launch_qlinear_reduce(const float* scratch, int splits, int vpad, int vectors, int rows, int rows_padded,
-                                  const float* bias, const float* residual, int epilogue, float* out, cudaStream_t stream) {
+                                  const float* bias, const float* residual, int epilogue, float* out, __half* out_xh, int xh_nv,
+                                  cudaStream_t stream) {
   const int out_cols = epilogue == ETC_EPILOGUE_SWIGLU ? rows / 2 : rows;
   const int64_t total = (int64_t)vectors * out_cols;
   if (total == 0) return cudaSuccess;
   const unsigned grid = (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 8);
   return launch_chained(qlinear_reduce_kernel, dim3(grid), dim3(256), 0, stream, scratch, splits, vpad, vectors, rows, rows_padded, bias, residual,
-                        epilogue, out);
+                        epilogue, out, out_xh, xh_nv);
 }
 
 // Scratch layout of the tcgen05 path: [xh8 activations, rounded to 256 B][split-K partials].
@@ -472,7 +474,7 @@ cudaError_t launch_qlinear_tiled(const TiledWeight& w, const float* x, int64_t v
   if (vectors <= stream_max_vectors())
     return launch_qlinear_stream(w, x, xh_ready, vectors, bias, residual, epilogue, out, out_xh, scratch, status, sm_count, stream, launches, xh_nv, defer);
   const size_t xh_region = umma_xh_region(plan_umma(w, vectors, sm_count));  // f16 activations of every chunk, then the partials
-  return launch_qlinear_umma(w, x, vectors, bias, residual, epilogue, out, reinterpret_cast<__half*>(scratch),
+  return launch_qlinear_umma(w, x, xh_ready, vectors, bias, residual, epilogue, out, out_xh, reinterpret_cast<__half*>(scratch),
                              reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + xh_region), status, sm_count, stream, launches);
 }
 

@@ -396,3 +396,24 @@ def test_the_operator_by_operator_route_agrees_with_the_fused_decoder():
         assert helpers.rel_err(by_ops, by_decoder) <= LOGIT_TOL, f"operators vs decoder, advance {advance}"
         np.testing.assert_array_equal(picked, by_ops.argmax(axis=1))
         assert [s.cursor for s in seqs_ops] == [s.cursor for s in seqs_fused]
+
+
+@pytest.mark.parametrize("q_heads,kv_heads,head_dim,kv_dtype,okv,tol,window", [
+    (6, 2, 64, et.KV_F16, orc.F16, LOGIT_TOL, None), (8, 1, 128, et.KV_BF16, orc.BF16, 2e-2, None),
+    (16, 1, 64, et.KV_F16, orc.F16, LOGIT_TOL, 40), (2, 2, 128, et.KV_U8, orc.U8, 1e-2, None)])
+def test_chunks_at_the_edges_of_the_attention_tiles(q_heads, kv_heads, head_dim, kv_dtype, okv, tol, window):
+    """Query heads that do not divide the 64 rows of a tile, chunks of one row more or less than tiles and pages hold, odd
+    cursors, a window that starts inside a step, a padded lane, and row counts on both sides of each hand-off stride."""
+    cfg = dict(helpers.TINY_Q, layers=2, q_heads=q_heads, kv_heads=kv_heads, head_dim=head_dim)
+    weights = helpers.make_weights(cfg, seed=5, codec=orc.Q4_0)
+    odec = helpers.oracle_decoder(cfg, weights, batch=3, window=window)
+    gdec = gpu_decoder(cfg, weights, batch=3, max_tokens=1536, kv_dtype=kv_dtype, exact=False, max_advance=70, window=window)
+    opool = orc.Pool(cfg["layers"], kv_heads, head_dim, 1536, 16, okv)
+    gpool = et.NativeKvPool(runtime(), cfg["layers"], kv_heads, head_dim, 1536, 16, kv_dtype)
+    oseqs, gseqs = [opool.make_sequence() for _ in range(2)], [gpool.makeSequence() for _ in range(2)]
+    rng = np.random.default_rng(q_heads)
+    for advance in (1, 21, 65, 2, 10, 43, 64, 1):
+        toks = rng.integers(0, cfg["vocab"], size=(2, advance)).astype(np.uint32)
+        ol, _ = odec.execute(opool, oseqs, toks)
+        gl = gdec.execute(gpool, gseqs, toks)
+        assert helpers.rel_err(gl, ol) <= 2 * tol, f"advance {advance}"
