@@ -144,11 +144,11 @@ __device__ __forceinline__ float exact_load(const void* slab, size_t elem, float
 
 // `tokens_first`: q and out are [B, tokens, Hq, D] (the fused projection's order) instead of [B, Hq, tokens, D].
 template <int DTYPE>
-__global__ void __launch_bounds__(128) attention_exact_kernel(PoolView pool, const float* __restrict__ q,
-                                                              const LaneInfo* __restrict__ lanes,
-                                                              const int* __restrict__ tables, int q_heads, int tokens,
-                                                              double scale, long long op_window, float* __restrict__ out,
-                                                              double* __restrict__ scratch, int max_ctx, int tokens_first) {
+__global__ void __launch_bounds__(128) attention_exact_kernel(PoolView pool, const float* q,
+                                                              const LaneInfo* lanes,
+                                                              const int* tables, int q_heads, int tokens,
+                                                              double scale, long long op_window, float* out,
+                                                              double* scratch, int max_ctx, int tokens_first) {
   extern __shared__ float q_s[];  // the query row
   __shared__ double kept[kExactKept];
   __shared__ int row_of[kExactKept];  // (page * kv_heads + head) * block_size + slot of each position
@@ -613,8 +613,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs
 }
 
 // Combines split partials: out = sum_s 2^(m_s - m) O_s / sum_s 2^(m_s - m) l_s. grid (Hq, B).
-__global__ void attention_merge_kernel(const float* __restrict__ partial, int q_heads, int splits, int D,
-                                       float* __restrict__ out, __half* __restrict__ out_xh, int xh_nv) {
+__global__ void attention_merge_kernel(const float* partial, int q_heads, int splits, int D,
+                                       float* out, __half* out_xh, int xh_nv) {
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   chain_wait();
   const int head = blockIdx.x, lane_id = blockIdx.y;
@@ -991,37 +991,36 @@ __device__ __forceinline__ void pool_store(const PoolView& p, void* slab, size_t
   else reinterpret_cast<__nv_bfloat16*>(slab)[elem] = __float2bfloat16_rn(value);
 }
 
-// A CTA serves heads_per_cta consecutive heads of one row. One for decode steps, whose few rows need every SM and whose chain
-// is short; eight for chunks, where the f64 sine and cosine, the same for all heads of a row, would otherwise dominate (104 us
-// for 2048 rows x 48 heads).
-__global__ void rope_append_kernel(PoolView pool, const float* __restrict__ qkv, const LaneInfo* __restrict__ lanes,
-                                   const int* __restrict__ tables, const double* __restrict__ inv_freq, int layout,
-                                   int q_heads, int heads_per_cta, float* __restrict__ q_out, DeferredSum sum) {
+// A CTA is GROUPS groups of half threads (the pairs of a head), each of which serves HEADS heads. One head per CTA for decode
+// steps, whose few rows need every SM and whose chain is short; sixteen for chunks, where the f64 sine and cosine, the same for
+// all heads of a row, otherwise dominate (2048 rows x 48 heads: 104 us with one head per CTA).
+template <int HEADS, int GROUPS>
+__global__ void rope_append_kernel(PoolView pool, const float* qkv, const LaneInfo* lanes,
+                                   const int* tables, const double* __restrict__ inv_freq, int layout,
+                                   int q_heads, float* q_out, DeferredSum sum) {
+  __shared__ double2 angle[GROUPS > 1 ? 64 : 1];  // (sine, cosine) per pair
+  __shared__ float red[32];
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   chain_wait();
   const int lane_id = blockIdx.y, tok = blockIdx.z, tokens = gridDim.z;
   const LaneInfo info = lanes[lane_id];
   const int D = pool.head_dim, half = D / 2, heads = q_heads + 2 * pool.kv_heads;
-  const bool live = (int)threadIdx.x < half;  // head dims below 64 leave threads of the warp without a pair
-  const int j = live ? threadIdx.x : 0;
+  const int width = GROUPS > 1 ? (int)blockDim.x / GROUPS : (int)blockDim.x;  // whole warps
+  const int group = GROUPS > 1 ? (int)threadIdx.x / width : 0, pair = (int)threadIdx.x - group * width;
+  const bool live = pair < half;  // head dims below 64 leave threads of the warp without a pair
+  const int j = live ? pair : 0;
   const size_t row_width = (size_t)heads * D;
   const size_t row = (size_t)lane_id * tokens + tok;
   const int i0 = layout == 0 ? j : 2 * j, i1 = layout == 0 ? half + j : 2 * j + 1;
-  const int head0 = blockIdx.x * heads_per_cta, head1 = min(heads, head0 + heads_per_cta);
+  const int head0 = blockIdx.x * HEADS * GROUPS + group;  // this group's heads: head0, head0 + GROUPS, ...
   const int pos = info.cursor + tok;
-  int page = 0, slot = 0;
-  if (info.advance > 0 && head1 > q_heads) {
-    const int block = pos / pool.block_size;
-    page = tables[info.table_offset + block];
-    slot = pos - block * pool.block_size;
-  }
-  double s = 0.0, c = 1.0;
-  if (head0 < q_heads + pool.kv_heads) sincos((double)pos * inv_freq[j], &s, &c);
-  for (int head = head0; head < head1; ++head) {
-    const bool is_q = head < q_heads, is_k = !is_q && head < q_heads + pool.kv_heads;
+  float in0[HEADS], in1[HEADS];
+#pragma unroll
+  for (int h = 0; h < HEADS; ++h) {
+    const int head = head0 + h * GROUPS;
     float r0 = 0.f, r1 = 0.f;
-    if (sum.splits > 0) {  // the projection left its split-K partials unsummed: add them up here, in split order
-      // (a narrow shard of a tensor-parallel group has up to 32 splits: eight loads are in flight at a time)
+    if (HEADS * GROUPS == 1 && sum.splits > 0) {  // the projection left its split-K partials unsummed: added up here, in split
+      // order (a narrow shard of a tensor-parallel group has up to 32 splits: eight loads are in flight at a time)
       const float* p = sum.partials + row * sum.rows_padded + (size_t)head * D;
       const size_t split_stride = (size_t)sum.vpad * sum.rows_padded;
       for (int s0 = 0; s0 < sum.splits; s0 += 8) {
@@ -1040,12 +1039,33 @@ __global__ void rope_append_kernel(PoolView pool, const float* __restrict__ qkv,
           }
         }
       }
-    } else {
+    } else if (head < heads) {
       const float* src = qkv + row * row_width + (size_t)head * D;
       r0 = src[i0];
       r1 = src[i1];
     }
-    if (!live) r0 = r1 = 0.f;
+    in0[h] = live ? r0 : 0.f;
+    in1[h] = live ? r1 : 0.f;
+  }
+  int page = 0, slot = 0;
+  if (info.advance > 0 && head0 + (HEADS - 1) * GROUPS >= q_heads) {
+    const int block = pos / pool.block_size;
+    page = tables[info.table_offset + block];
+    slot = pos - block * pool.block_size;
+  }
+  double s = 0.0, c = 1.0;
+  if (group == 0 && (int)blockIdx.x * HEADS * GROUPS < q_heads + pool.kv_heads) sincos((double)pos * inv_freq[j], &s, &c);
+  if (GROUPS > 1) {
+    if (group == 0 && live) angle[j] = make_double2(s, c);
+    __syncthreads();
+    s = angle[j].x;
+    c = angle[j].y;
+  }
+#pragma unroll
+  for (int h = 0; h < HEADS; ++h) {
+    const int head = head0 + h * GROUPS;
+    const bool is_q = head < q_heads, is_k = !is_q && head < q_heads + pool.kv_heads;
+    float r0 = in0[h], r1 = in1[h];
     if (is_q || is_k) {
       const double first = (double)r0, second = (double)r1;
       r0 = (float)__dsub_rn(__dmul_rn(first, c), __dmul_rn(second, s));
@@ -1057,25 +1077,25 @@ __global__ void rope_append_kernel(PoolView pool, const float* __restrict__ qkv,
         dst[i0] = r0;
         dst[i1] = r1;
       }
-      continue;
     }
-    if (info.advance == 0) continue;  // padded lane: nothing is cached
+    const bool cached = !is_q && head < heads && info.advance > 0;  // a padded lane caches nothing
     const int kv_head = is_k ? head - q_heads : head - q_heads - pool.kv_heads;
-    const size_t dst = pool_elem(pool, page, kv_head, slot);
+    const size_t dst = cached ? pool_elem(pool, page, kv_head, slot) : 0;
     void* slab = is_k ? pool.k : pool.v;
     if (pool.dtype == kKvU8) {
       // the int8 tier: one scale per cached row, as kv_append_kernel (pool.rs:224-240)
-      __shared__ float red[32];
+      if (HEADS * GROUPS == 1 && !cached) return;  // the same for the whole CTA; with more heads all threads meet at the barriers
       float amax = fmaxf(fabsf(r0), fabsf(r1));
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-      __syncthreads();  // the previous head's maxima have been read
+      if (h > 0) __syncthreads();  // the previous head's maxima have been read
       if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
       __syncthreads();
+      if (!cached) continue;
       amax = 0.0f;
-      for (int w = 0; w < (int)((blockDim.x + 31) >> 5); ++w) amax = fmaxf(amax, red[w]);
+      for (int w = group * (width >> 5); w < (group + 1) * (width >> 5); ++w) amax = fmaxf(amax, red[w]);
       const float scale = __fadd_rn(__fdiv_rn(amax, 127.0f), 1e-12f);
-      if (threadIdx.x == 0) (is_k ? pool.k_scale : pool.v_scale)[pool_scale_index(pool, page, kv_head, slot)] = scale;
+      if (pair == 0) (is_k ? pool.k_scale : pool.v_scale)[pool_scale_index(pool, page, kv_head, slot)] = scale;
       const float c0 = fminf(fmaxf(roundf(__fdiv_rn(r0, scale)), -127.0f), 127.0f) + 128.0f;
       const float c1 = fminf(fmaxf(roundf(__fdiv_rn(r1, scale)), -127.0f), 127.0f) + 128.0f;
       if (live) {
@@ -1084,7 +1104,7 @@ __global__ void rope_append_kernel(PoolView pool, const float* __restrict__ qkv,
       }
       continue;
     }
-    if (!live) continue;
+    if (!live || !cached) continue;
     pool_store(pool, slab, dst + i0, r0);
     pool_store(pool, slab, dst + i1, r1);
   }
@@ -1094,14 +1114,17 @@ cudaError_t launch_rope_append(const PoolView& pool, const float* qkv, const Lan
                                const double* inv_freq, int layout, int batch, int q_heads, float* q_out,
                                cudaStream_t stream, const DeferredSum* sum, int tokens) {
   if (batch == 0) return cudaSuccess;
-  const int heads = q_heads + 2 * pool.kv_heads, per = (int64_t)batch * tokens >= 512 ? 8 : 1;
-  dim3 grid((unsigned)((heads + per - 1) / per), (unsigned)batch, (unsigned)tokens);
-  return launch_chained(rope_append_kernel, grid, dim3((unsigned)std::max(32, (pool.head_dim / 2 + 31) / 32 * 32)), 0, stream, pool, qkv, lanes, tables, inv_freq, layout, q_heads, per,
-                        q_out, sum ? *sum : DeferredSum());
+  const int heads = q_heads + 2 * pool.kv_heads, width = std::max(32, (pool.head_dim / 2 + 31) / 32 * 32);
+  // several heads per CTA once the rows alone fill the SMs; the sums of split projections are only taken head by head
+  const bool many = (int64_t)batch * tokens >= 128 && !(sum && sum->splits > 0) && width <= 64;
+  const int per = many ? 16 : 1;
+  const dim3 grid((unsigned)((heads + per - 1) / per), (unsigned)batch, (unsigned)tokens);
+  return launch_chained(many ? rope_append_kernel<4, 4> : rope_append_kernel<1, 1>, grid, dim3((unsigned)(many ? 4 * width : width)), 0, stream, pool, qkv, lanes,
+                        tables, inv_freq, layout, q_heads, q_out, sum ? *sum : DeferredSum());
 }
 
-__global__ void record_step_kernel(const uint32_t* __restrict__ tokens, uint32_t* __restrict__ ids,
-                                   uint32_t* __restrict__ history, int* step_counter, LaneInfo* lanes, int batch,
+__global__ void record_step_kernel(const uint32_t* tokens, uint32_t* ids,
+                                   uint32_t* history, int* step_counter, LaneInfo* lanes, int batch,
                                    long long window) {
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   chain_wait();

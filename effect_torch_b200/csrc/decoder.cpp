@@ -327,10 +327,7 @@ etc_status norm_hand_off(StepContext& s, float* x, const BoundWeight& weight, in
   etc_decoder* d = s.dec;
   const etc_decoder_config& c = d->cfg;
   const int nv = hand_off_stride(rows);
-  if (pending.splits > 0)
-    ETC_CUDA(launch_sum_rmsnorm_xh8(x, pending, (const float*)weight.d_raw, c.rms_eps, rows, c.d_model, d->xh_norm, d->rt->stream, nv));
-  else
-    ETC_CUDA(launch_rmsnorm_xh8(x, (const float*)weight.d_raw, c.rms_eps, rows, c.d_model, d->xh_norm, d->rt->stream, nv));
+  ETC_CUDA(launch_sum_rmsnorm_xh8(x, pending, (const float*)weight.d_raw, c.rms_eps, rows, c.d_model, d->xh_norm, d->rt->stream, nv));
   pending = DeferredSum();
   ++s.launches;
   return ETC_OK;
@@ -978,8 +975,9 @@ etc_status etc_decoder_finalize(etc_decoder* dec) {
   dec->max_blocks = decoder_max_blocks(c, dec->max_advance);
   if (tiled) {
     size_t need = 0;
-    // the plan (vector padding, split count) changes at these vector counts; cover every one up to R rows
-    const int64_t probes[] = {1, 9, 17, 32, 64, 128, 256, (int64_t)R};
+    // the plan (vector padding, split count) changes at these vector counts and, above 128, with every chunk of 128
+    std::vector<int64_t> probes = {1, 9, 17, 32, 64, 128};
+    for (int64_t v = 256; v < (int64_t)R + 128; v += 128) probes.push_back(v);
     for (size_t l = 0; l < L; ++l)
       for (etc_qweight* w : {dec->t_qkv[l], dec->t_o[l], dec->t_gu[l], dec->t_down[l]})
         for (int64_t v : probes)

@@ -215,83 +215,181 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
   }
 }
 
-// Single-pass variant for n <= 8192, n % 4 == 0: the row stays in registers between the reduction and the
-// scaling (same f64 arithmetic). XH = true stores the result as f16 in [n/8][32][8] order (row < 32), the
-// B-operand layout of the tcgen05 linear, instead of f32 row-major.
-// SUM = true first adds a projection's split-K partials (summed in split order) onto the row and stores it back: the
-// residual update the projection's own sum kernel would have done.
-template <bool XH, bool SUM, int THREADS>
-__global__ void __launch_bounds__(THREADS) rmsnorm_rows_kernel(const float* x, const float* __restrict__ weight,
-                                                               double eps, int n, float* __restrict__ out, __half* __restrict__ out_xh,
-                                                               int xh_nv, DeferredSum sum_in, float* x_out) {
-  chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
-  constexpr int ITEMS = 2048 / THREADS;  // float4 chunks per thread: rows of up to 8192 values
-  const int chunks = n / 4;
-  float4 w[ITEMS];
-  auto load_weight = [&]() {
+__device__ __forceinline__ double square4(const float4& v) {
+  return (double)v.x * (double)v.x + (double)v.y * (double)v.y + (double)v.z * (double)v.z + (double)v.w * (double)v.w;
+}
+__device__ __forceinline__ float4 scale4(const float4& v, double scale, const float4& w) {
+  return make_float4((float)__dmul_rn(__dmul_rn((double)v.x, scale), (double)w.x), (float)__dmul_rn(__dmul_rn((double)v.y, scale), (double)w.y),
+                     (float)__dmul_rn(__dmul_rn((double)v.z, scale), (double)w.z), (float)__dmul_rn(__dmul_rn((double)v.w, scale), (double)w.w));
+}
+__device__ __forceinline__ uint2 pack_sat4(const float4& v) {
+  auto sat = [](float f) { return fminf(fmaxf(f, -65504.f), 65504.f); };
+  const __half2 lo = __floats2half2_rn(sat(v.x), sat(v.y)), hi = __floats2half2_rn(sat(v.z), sat(v.w));
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+__device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-      const int c = threadIdx.x + THREADS * j;
-      w[j] = weight && c < chunks ? reinterpret_cast<const float4*>(weight)[c] : make_float4(1.f, 1.f, 1.f, 1.f);
-    }
-  };
-  // The f16 hand-off forms are launched by the decoder alone, whose norm weights no kernel writes after the load: they
-  // are fetched while the kernel before this one is still running. The plain form may be given a weight that the
-  // previous kernel of the stream produced, and reads it after the wait.
-  if (XH) load_weight();
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+
+// Single-pass variants for n <= 8192, n % 4 == 0: the row stays in registers between the reduction and the scaling (same
+// f64 arithmetic). f32 row-major:
+constexpr int kNormThreads = 256, kNormItems = 8192 / 4 / kNormThreads;
+__global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const float* x, const float* weight, double eps, int n,
+                                                                   float* out) {
+  __shared__ double partial[kNormThreads / 32];
+  chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   chain_wait();
-  if (!XH) load_weight();
-  __shared__ double partial[THREADS / 32];
-  const int row = blockIdx.x;
-  const float4* src = reinterpret_cast<const float4*>(x + (size_t)row * n);
+  const int chunks = n / 4;
+  const float4* src = reinterpret_cast<const float4*>(x + (size_t)blockIdx.x * n);
+  float4 v[kNormItems];
+  double sum = 0.0;
+#pragma unroll
+  for (int j = 0; j < kNormItems; ++j) {
+    const int c = threadIdx.x + kNormThreads * j;
+    v[j] = c < chunks ? src[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+    sum += square4(v[j]);
+  }
+  sum = warp_sum(sum);
+  if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  double total = 0.0;
+#pragma unroll
+  for (int i = 0; i < kNormThreads / 32; ++i) total += partial[i];
+  const double scale = 1.0 / sqrt(total / (double)n + eps);
+#pragma unroll
+  for (int j = 0; j < kNormItems; ++j) {
+    const int c = threadIdx.x + kNormThreads * j;
+    if (c >= chunks) continue;
+    const float4 w = weight ? reinterpret_cast<const float4*>(weight)[c] : make_float4(1.f, 1.f, 1.f, 1.f);
+    reinterpret_cast<float4*>(out + (size_t)blockIdx.x * n)[c] = scale4(v[j], scale, w);
+  }
+}
+
+// The same for a few rows into the f16 hand-off layout, first adding a projection's split-K partials (in split order) onto
+// the row and storing it back: the residual update that the projection's own sum kernel would have done. sum_in.splits may
+// be 0: the row as it is.
+//
+// Bound by latency: a row and its partials (up to 10 x 32 KB) come from L2, and every kernel of a decode step waits for this
+// one. A cluster of four CTAs shares a row, so that the partials come through four SMs; each thread has its loads of ten
+// splits in flight at once, and the warps' sums of squares are exchanged through distributed shared memory. One CTA per row
+// with four loads in flight took 7.5 us for 32 rows of 4096 with 9 splits.
+constexpr int kNormCluster = 4;
+__global__ void __launch_bounds__(kNormThreads) sum_rmsnorm_xh_kernel(float* x, const float* __restrict__ weight, double eps, int n, __half* out_xh,
+                                                                     int xh_nv, DeferredSum sum_in) {
+  namespace cg = cooperative_groups;
+  constexpr int ITEMS = kNormItems / kNormCluster, WARPS = kNormThreads / 32;
+  static_assert(kNormCluster * WARPS == 32, "one sum per lane");
+  __shared__ double partial[32];
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();  // waited for below: the peers' shared memory exists
+  chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
+  const int chunks = n / 4, first = blockIdx.x * kNormThreads + threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // launched by the decoder alone, whose norm weights no kernel writes after the load: they are fetched while the kernel
+  // before this one is still running
+  float4 w[ITEMS];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const int c = first + kNormCluster * kNormThreads * j;
+    w[j] = weight && c < chunks ? reinterpret_cast<const float4*>(weight)[c] : make_float4(1.f, 1.f, 1.f, 1.f);
+  }
+  chain_wait();
+  const int row = blockIdx.y;
+  float4* src = reinterpret_cast<float4*>(x + (size_t)row * n);
   float4 v[ITEMS];
   double sum = 0.0;
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
-    const int c = threadIdx.x + THREADS * j;
-    v[j] = c < chunks ? src[c] : make_float4(0.f, 0.f, 0.f, 0.f);
-    if (SUM && c < chunks) {
-      // all splits' loads are independent: issued together, added in split order
+    const int c = first + kNormCluster * kNormThreads * j;
+    v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c >= chunks) continue;
+    v[j] = src[c];
+    if (sum_in.splits > 0) {
+      constexpr int IN_FLIGHT = 10;
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
       const float* base = sum_in.partials + (size_t)row * sum_in.rows_padded + 4 * c;
       const size_t split_stride = (size_t)sum_in.vpad * sum_in.rows_padded;
-#pragma unroll 4
-      for (int s = 0; s < sum_in.splits; ++s) {
-        const float4 p = *reinterpret_cast<const float4*>(base + (size_t)s * split_stride);
-        acc.x += p.x; acc.y += p.y; acc.z += p.z; acc.w += p.w;
+      for (int s0 = 0; s0 < sum_in.splits; s0 += IN_FLIGHT) {
+        float4 p[IN_FLIGHT];
+#pragma unroll
+        for (int u = 0; u < IN_FLIGHT; ++u)
+          if (s0 + u < sum_in.splits) p[u] = *reinterpret_cast<const float4*>(base + (size_t)(s0 + u) * split_stride);
+#pragma unroll
+        for (int u = 0; u < IN_FLIGHT; ++u)
+          if (s0 + u < sum_in.splits) { acc.x += p[u].x; acc.y += p[u].y; acc.z += p[u].z; acc.w += p[u].w; }
       }
       v[j].x += acc.x; v[j].y += acc.y; v[j].z += acc.z; v[j].w += acc.w;
-      reinterpret_cast<float4*>(x_out + (size_t)row * n)[c] = v[j];
     }
-    sum += (double)v[j].x * (double)v[j].x + (double)v[j].y * (double)v[j].y + (double)v[j].z * (double)v[j].z +
-           (double)v[j].w * (double)v[j].w;
+    sum += square4(v[j]);
   }
+  if (sum_in.splits > 0) {
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-  if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = sum;
-  __syncthreads();
-  // every thread adds the warps' sums in the same order and takes the reciprocal root itself: one barrier, no hand-over
-  double total = 0.0;
-#pragma unroll
-  for (int i = 0; i < THREADS / 32; ++i) total += partial[i];
-  const double scale = 1.0 / sqrt(total / (double)n + eps);
+    for (int j = 0; j < ITEMS; ++j)
+      if (first + kNormCluster * kNormThreads * j < chunks) src[first + kNormCluster * kNormThreads * j] = v[j];
+  }
+  sum = warp_sum(sum);
+  cluster.barrier_wait();
+  if (lane < kNormCluster) cluster.map_shared_rank(partial, lane)[blockIdx.x * WARPS + warp] = sum;
+  cluster.sync();
+  const double scale = 1.0 / sqrt(warp_sum(partial[lane]) / (double)n + eps);
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
-    const int c = threadIdx.x + THREADS * j;
-    if (c >= chunks) continue;
-    const float r0 = (float)__dmul_rn(__dmul_rn((double)v[j].x, scale), (double)w[j].x);
-    const float r1 = (float)__dmul_rn(__dmul_rn((double)v[j].y, scale), (double)w[j].y);
-    const float r2 = (float)__dmul_rn(__dmul_rn((double)v[j].z, scale), (double)w[j].z);
-    const float r3 = (float)__dmul_rn(__dmul_rn((double)v[j].w, scale), (double)w[j].w);
-    if (XH) {
-      auto sat = [](float f) { return fminf(fmaxf(f, -65504.f), 65504.f); };
-      __half2 h01 = __floats2half2_rn(sat(r0), sat(r1)), h23 = __floats2half2_rn(sat(r2), sat(r3));
-      const int k = 4 * c;
-      uint2 packed = make_uint2(*reinterpret_cast<uint32_t*>(&h01), *reinterpret_cast<uint32_t*>(&h23));
-      *reinterpret_cast<uint2*>(out_xh + hand_off_cell(k >> 3, row, xh_nv, n / 8) + (k & 7)) = packed;
-    } else {
-      reinterpret_cast<float4*>(out + (size_t)row * n)[c] = make_float4(r0, r1, r2, r3);
-    }
+    const int c = first + kNormCluster * kNormThreads * j;
+    if (c < chunks) *reinterpret_cast<uint2*>(out_xh + hand_off_cell(c >> 1, row, xh_nv, n / 8) + 4 * (c & 1)) = pack_sat4(scale4(v[j], scale, w[j]));
+  }
+}
+
+// The same for many rows (hand-off chunks of 128), without partials. A CTA takes two neighbouring rows: two lanes exchange
+// halves, so that each stores 16 bytes and the pair fills a sector of the hand-off layout. With one row per CTA and stores of
+// 8 bytes that each touch a sector of their own, 2048 rows of 4096 took 32 us.
+template <int ITEMS>
+__global__ void __launch_bounds__(kNormThreads) rmsnorm_chunk_xh_kernel(const float* x, const float* __restrict__ weight, double eps, int rows, int n,
+                                                                       __half* out_xh) {
+  __shared__ double partial[2][kNormThreads / 32];
+  chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
+  chain_wait();
+  const int chunks = n / 4, row0 = 2 * blockIdx.x;
+  const bool both = row0 + 1 < rows;
+  const float4* src0 = reinterpret_cast<const float4*>(x + (size_t)row0 * n);
+  const float4* src1 = both ? src0 + chunks : src0;
+  float4 v0[ITEMS], v1[ITEMS];
+  double sum0 = 0.0, sum1 = 0.0;
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const int c = threadIdx.x + kNormThreads * j;
+    v0[j] = c < chunks ? src0[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+    v1[j] = c < chunks ? src1[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    sum0 += square4(v0[j]);
+    sum1 += square4(v1[j]);
+  }
+  sum0 = warp_sum(sum0);
+  sum1 = warp_sum(sum1);
+  if ((threadIdx.x & 31) == 0) {
+    partial[0][threadIdx.x >> 5] = sum0;
+    partial[1][threadIdx.x >> 5] = sum1;
+  }
+  __syncthreads();
+  sum0 = sum1 = 0.0;
+#pragma unroll
+  for (int i = 0; i < kNormThreads / 32; ++i) {
+    sum0 += partial[0][i];
+    sum1 += partial[1][i];
+  }
+  const double scale0 = 1.0 / sqrt(sum0 / (double)n + eps), scale1 = 1.0 / sqrt(sum1 / (double)n + eps);
+  const bool odd = threadIdx.x & 1;
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const int c = threadIdx.x + kNormThreads * j;
+    const float4 w = weight && c < chunks ? reinterpret_cast<const float4*>(weight)[c] : make_float4(1.f, 1.f, 1.f, 1.f);
+    const uint2 a = pack_sat4(scale4(v0[j], scale0, w)), b = pack_sat4(scale4(v1[j], scale1, w)), give = odd ? a : b;
+    const uint2 got = make_uint2(__shfl_xor_sync(0xffffffffu, give.x, 1), __shfl_xor_sync(0xffffffffu, give.y, 1));
+    if (c < chunks && (!odd || both))  // n % 8 == 0: both lanes of a pair are inside the row
+      *reinterpret_cast<uint4*>(out_xh + hand_off_cell(c >> 1, row0 + odd, 128, n / 8)) =
+          odd ? make_uint4(got.x, got.y, b.x, b.y) : make_uint4(a.x, a.y, got.x, got.y);
   }
 }
 
@@ -303,28 +401,24 @@ cudaError_t launch_rmsnorm(const float* x, const float* weight, double eps, int6
                            cudaStream_t stream) {
   if (rows == 0) return cudaSuccess;
   if (rmsnorm_fast_ok(x, weight, n) && ((uintptr_t)out % 16) == 0)
-    return launch_chained(rmsnorm_rows_kernel<false, false, 256>, dim3((unsigned)rows), dim3(256), 0, stream, x, weight, eps, (int)n, out, (__half*)nullptr, 32,
-                          DeferredSum(), (float*)nullptr);
+    return launch_chained(rmsnorm_rows_kernel, dim3((unsigned)rows), dim3(kNormThreads), 0, stream, x, weight, eps, (int)n, out);
   else
     rmsnorm_kernel<<<(unsigned)rows, 256, 0, stream>>>(x, weight, eps, n, out);
   return cudaGetLastError();
 }
 
-cudaError_t launch_rmsnorm_xh8(const float* x, const float* weight, double eps, int64_t rows, int64_t n, __half* out_xh,
-                               cudaStream_t stream, int xh_nv) {
-  if (rows == 0) return cudaSuccess;
-  if ((rows > xh_nv && xh_nv != 128) || n % 8 != 0 || !rmsnorm_fast_ok(x, weight, n)) return cudaErrorInvalidValue;
-  return launch_chained(rmsnorm_rows_kernel<true, false, 256>, dim3((unsigned)rows), dim3(256), 0, stream, x, weight, eps, (int)n, (float*)nullptr, out_xh, xh_nv,
-                        DeferredSum(), (float*)nullptr);
-}
-
 cudaError_t launch_sum_rmsnorm_xh8(float* x, const DeferredSum& sum, const float* weight, double eps, int64_t rows, int64_t n,
                                    __half* out_xh, cudaStream_t stream, int xh_nv) {
   if (rows == 0) return cudaSuccess;
-  if (rows > xh_nv || n % 8 != 0 || !rmsnorm_fast_ok(x, weight, n) || sum.splits <= 0 || sum.rows_padded % 4 != 0 || rows > sum.vpad)
-    return cudaErrorInvalidValue;
-  return launch_chained(rmsnorm_rows_kernel<true, true, 1024>, dim3((unsigned)rows), dim3(1024), 0, stream, (const float*)x, weight, eps, (int)n,
-                        (float*)nullptr, out_xh, xh_nv, sum, x);
+  if (rows > xh_nv && xh_nv != 128) return cudaErrorInvalidValue;
+  if (n % 8 != 0 || !rmsnorm_fast_ok(x, weight, n)) return cudaErrorInvalidValue;
+  if (sum.splits > 0 && (sum.rows_padded % 4 != 0 || rows > sum.vpad)) return cudaErrorInvalidValue;
+  if (rows > 128 && sum.splits == 0) {  // two rows per CTA fill half the SMs, and the sums of a cluster cost more than they save
+    const auto kernel = n <= 4096 ? rmsnorm_chunk_xh_kernel<kNormItems / 2> : rmsnorm_chunk_xh_kernel<kNormItems>;
+    return launch_chained(kernel, dim3((unsigned)((rows + 1) / 2)), dim3(kNormThreads), 0, stream, (const float*)x, weight, eps, (int)rows, (int)n, out_xh);
+  }
+  return launch_chained_cluster(sum_rmsnorm_xh_kernel, dim3(kNormCluster, (unsigned)rows), dim3(kNormThreads), 0, stream, (unsigned)kNormCluster, x, weight, eps,
+                                (int)n, out_xh, xh_nv, sum);
 }
 
 // --------------------------------------------------------------------------------------------
@@ -404,8 +498,8 @@ constexpr int kArgmaxSlice = 8192;  // a row is spread over more CTAs until a sl
 
 // `picks` (optional): the row's (best logit bits, index_base + index) pair, for the exchange between the ranks of a
 // vocabulary-parallel head. `mirror` (optional): a second copy of the tokens, in page-locked host memory.
-__global__ void __launch_bounds__(kArgmaxThreads) argmax_kernel(const float* __restrict__ logits, int64_t vocab, int64_t slice,
-                                                                uint32_t* __restrict__ tokens, DeviceStatus* status, uint2* picks,
+__global__ void __launch_bounds__(kArgmaxThreads) argmax_kernel(const float* logits, int64_t vocab, int64_t slice,
+                                                                uint32_t* tokens, DeviceStatus* status, uint2* picks,
                                                                 uint32_t index_base, uint32_t* mirror) {
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   chain_wait();
@@ -492,8 +586,8 @@ cudaError_t launch_argmax(const float* logits, int64_t rows, int64_t vocab, uint
 
 // Dense f32 embedding gather with the same bounds rule as the quantized embedding.
 template <typename Index>
-__global__ void embedding_f32_kernel(const Index* __restrict__ indexes, int64_t count, const float* __restrict__ table,
-                                     int64_t rows, int64_t columns, float* __restrict__ out, DeviceStatus* status) {
+__global__ void embedding_f32_kernel(const Index* indexes, int64_t count, const float* __restrict__ table,
+                                     int64_t rows, int64_t columns, float* out, DeviceStatus* status) {
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   chain_wait();
   const int64_t i = blockIdx.y;

@@ -18,7 +18,8 @@ inline int hand_off_stride(int64_t rows) { return rows <= 32 ? 32 : (rows <= 64 
 inline int64_t hand_off_rows(int64_t rows) { return rows <= 64 ? hand_off_stride(rows) : (rows + 127) / 128 * 128; }
 // Offset (in halves) of columns 8 * k8 .. 8 * k8 + 7 of a row of k8_total * 8 columns.
 __host__ __device__ inline size_t hand_off_cell(int k8, size_t row, int nv, int k8_total) {
-  return (((row / nv) * k8_total + k8) * nv + row % nv) * 8;
+  const int shift = nv == 32 ? 5 : (nv == 64 ? 6 : 7);
+  return ((((row >> shift) * k8_total + k8) << shift) + (row & (nv - 1))) * 8;
 }
 
 // ---- block-quantized weights (quant_kernels.cu) ------------------------------------------
@@ -133,12 +134,10 @@ cudaError_t launch_qlinear_tiled(const TiledWeight& w, const float* x, int64_t v
                                  const float* residual, int epilogue, float* out, void* scratch, DeviceStatus* status,
                                  int sm_count, cudaStream_t stream, int* launches, const __half* xh_ready = nullptr,
                                  __half* out_xh = nullptr, int xh_nv = 32, DeferredSum* defer = nullptr);
-// RMSNorm whose output is stored in the hand-off layout.
-cudaError_t launch_rmsnorm_xh8(const float* x, const float* weight, double eps, int64_t rows, int64_t n, __half* out_xh,
-                               cudaStream_t stream, int xh_nv = 32);
-// The same after x += sum of a projection's split-K partials (x is updated in place: the residual stream).
+// RMSNorm whose output is stored in the hand-off layout, after x += the sum of a projection's split-K partials where
+// sum.splits > 0 (x, the residual stream, is updated in place).
 cudaError_t launch_sum_rmsnorm_xh8(float* x, const DeferredSum& sum, const float* weight, double eps, int64_t rows, int64_t n,
-                                   __half* out_xh, cudaStream_t stream, int xh_nv = 32);
+                                   __half* out_xh, cudaStream_t stream, int xh_nv);
 
 // ---- tensor-parallel all-reduce over peer memory (tp_kernels.cu) -----------------------------
 constexpr int kMaxTpRanks = 8;

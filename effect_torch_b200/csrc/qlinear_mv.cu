@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(kMvThreads, (MvCfg<CODEC, NT>::kCtasPerSm)) ql
 
 // f32 [vectors, K] -> f16 [K/8][NV][8] (rows >= vectors are zero), saturating at the f16 range.
 template <int NV>
-__global__ void mv_convert_kernel(const float* __restrict__ x, int vectors, int K, __half* __restrict__ xh) {
+__global__ void mv_convert_kernel(const float* x, int vectors, int K, __half* xh) {
   chain_release();
   chain_wait();
   const int total = (K / 8) * NV;

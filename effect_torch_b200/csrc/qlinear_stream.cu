@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
 }
 
 // f32 [vectors, K] -> [K/8][NV][8] f16 (rows >= vectors are zero), saturating at the f16 range.
-__global__ void convert_hand_off_kernel(const float* __restrict__ x, int vectors, int K, int nv_shift, __half* __restrict__ xh) {
+__global__ void convert_hand_off_kernel(const float* x, int vectors, int K, int nv_shift, __half* xh) {
   chain_release();
   chain_wait();
   const int total = (K / 8) << nv_shift;

@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qlinear_gemm_kernel(GemmArgs 
 
 // f32 [vectors, K] -> xh8 [K/8][NV][8] f16 (rows >= vectors are zero), saturating like the mma.sync path.
 // More than NV vectors: chunk c holds vectors c*NV ... in its own [K/8][NV][8] block.
-__global__ void convert_xh8_kernel(const float* __restrict__ x, int vectors, int K, __half* __restrict__ xh) {
+__global__ void convert_xh8_kernel(const float* x, int vectors, int K, __half* xh) {
   constexpr int NV = kGemmVectors;
   chain_release();
   chain_wait();

@@ -408,9 +408,9 @@ __device__ __forceinline__ float silu_tanh_form(float x) { return x * (tanhf(x *
 // Sums the split-K partials [chunk of vpad vectors][split][vpad][rows_padded] in split order and applies bias / epilogue.
 // `residual` and `out` may be the same buffer (the decoder adds projections onto its hidden state in place), so
 // neither carries a no-alias promise.
-__global__ void qlinear_reduce_kernel(const float* __restrict__ scratch, int splits, int vpad, int vectors, int rows,
-                                      int rows_padded, const float* __restrict__ bias, const float* residual,
-                                      int epilogue, float* out, __half* __restrict__ out_xh, int xh_nv) {
+__global__ void qlinear_reduce_kernel(const float* scratch, int splits, int vpad, int vectors, int rows,
+                                      int rows_padded, const float* bias, const float* residual,
+                                      int epilogue, float* out, __half* out_xh, int xh_nv) {
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   chain_wait();
   const int out_cols = epilogue == ETC_EPILOGUE_SWIGLU ? rows / 2 : rows;

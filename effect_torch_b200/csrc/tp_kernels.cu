@@ -100,8 +100,8 @@ __device__ void arrive_and_publish(const PeerView& pv, uint32_t* bar, int which,
 
 // ctr: [0] epoch of the last completed all-reduce, [1] CTAs done, [2] / [3] phase arrivals, [4] epoch of the last pick exchange
 template <bool TWO_SHOT>
-__global__ void __launch_bounds__(256) tp_allreduce_kernel(PeerView pv, int buffer, float* __restrict__ hidden, size_t count4,
-                                                           DeferredSum sum, int columns, const float* __restrict__ partial,
+__global__ void __launch_bounds__(256) tp_allreduce_kernel(PeerView pv, int buffer, float* hidden, size_t count4,
+                                                           DeferredSum sum, int columns, const float* partial,
                                                            uint32_t* ctr, long long wait_cycles, unsigned long long* status,
                                                            int chain) {
   __shared__ uint32_t epoch_s;

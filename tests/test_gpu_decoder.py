@@ -417,3 +417,22 @@ def test_chunks_at_the_edges_of_the_attention_tiles(q_heads, kv_heads, head_dim,
         ol, _ = odec.execute(opool, oseqs, toks)
         gl = gdec.execute(gpool, gseqs, toks)
         assert helpers.rel_err(gl, ol) <= 2 * tol, f"advance {advance}"
+
+
+@pytest.mark.parametrize("d_model", [1088, 4160, 8192])
+def test_norms_at_the_edges_of_their_row_widths(d_model):
+    """Residual widths that end inside a cluster's share, just above the width of the narrower form and at the limit, for
+    few rows (with split projections to add up), for an odd number of many rows, and for whole chunks."""
+    cfg = dict(helpers.TINY_Q, layers=2, d_model=d_model, ffn=512)
+    weights = helpers.make_weights(cfg, seed=7, codec=orc.Q4_0)
+    odec = helpers.oracle_decoder(cfg, weights, batch=3)
+    gdec = gpu_decoder(cfg, weights, batch=3, max_tokens=1024, kv_dtype=et.KV_F16, exact=False, max_advance=86)
+    opool = orc.Pool(cfg["layers"], cfg["kv_heads"], cfg["head_dim"], 1024, 16, orc.F16)
+    gpool = et.NativeKvPool(runtime(), cfg["layers"], cfg["kv_heads"], cfg["head_dim"], 1024, 16, et.KV_F16)
+    oseqs, gseqs = [opool.make_sequence() for _ in range(3)], [gpool.makeSequence() for _ in range(3)]
+    rng = np.random.default_rng(d_model)
+    for advance in (1, 43, 86, 1):  # 3, 129, 258 and 3 rows
+        toks = rng.integers(0, cfg["vocab"], size=(3, advance)).astype(np.uint32)
+        ol, _ = odec.execute(opool, oseqs, toks)
+        gl = gdec.execute(gpool, gseqs, toks)
+        assert helpers.rel_err(gl, ol) <= 2 * LOGIT_TOL, f"advance {advance}"
