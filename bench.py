@@ -388,8 +388,8 @@ def projection_rooflines(rt, et, torch, model, vectors, peaks, peak_kind):
     shapes = [("qkv", qw + 2 * kvw, d, False, et.EPILOGUE_NONE, False), ("o", d, qw, False, et.EPILOGUE_RESIDUAL, True),
               ("gate_up", 2 * ffn, d, True, et.EPILOGUE_SWIGLU, False), ("down", d, ffn, False, et.EPILOGUE_RESIDUAL, True),
               ("head", V, d, False, et.EPILOGUE_NONE, False)]
-    nv = 32 if vectors <= 32 else 64 if vectors <= 64 else 128 if vectors <= 128 else 256
-    kernel = "qlinear_mv_kernel<Q4_0>" if vectors <= 16 else f"qlinear_umma_kernel<Q4_0,{nv}> (+ f16 conversion and split-K sum launches)"
+    nv = 16 if vectors <= 16 else 32 if vectors <= 32 else 64 if vectors <= 64 else 128
+    kernel = "qlinear_gemm_kernel<Q4_0>" if vectors > 128 else f"qlinear_stream_kernel<Q4_0,{nv}>" + (" (+ f16 conversion launch)" if nv > 16 else "")
     out = {}
     for name, rows, cols, interleave, epilogue, residual in shapes:
         us, algorithmic = time_linear(rt, et, torch, Q4_0, rows, cols, vectors, interleave, epilogue, residual)
@@ -784,7 +784,7 @@ def run_gpu_arm(args, rank, world):
             traffic = profile_number("qlinear_umma_q4_0_decode_step.md", "gate_up_dram_bytes_per_launch")
             line["roofline"] = roofline_entry(
                 us, algorithmic, peaks, peak_kind,
-                f"qlinear_umma_kernel<Q4_0,32> fused gate/up [{2 * model['ffn']}x{model['d_model']}], {BATCH} vectors, with its f16 conversion launch",
+                f"qlinear_stream_kernel<Q4_0,32> fused gate/up [{2 * model['ffn']}x{model['d_model']}], {BATCH} vectors, with its f16 conversion launch",
                 traffic, "ncu --set full capture of this launch on the 2-layer case, summary under profiles/" if traffic else None)
             line["roofline_by_projection"] = projection_rooflines(rt, et, torch, model, BATCH, peaks, peak_kind)
             ctx_step = np.full(BATCH, int(mean_ctx))

@@ -49,10 +49,10 @@ def _ptr(t):
     if t is None:
         return None
     if isinstance(t, int):
-        return C.c_void_p(t)
+        return t
     if isinstance(t, np.ndarray):
-        return C.c_void_p(t.ctypes.data)
-    return C.c_void_p(t.data_ptr())
+        return t.ctypes.data
+    return t.data_ptr()
 
 
 # Results of up to this many bytes at a time sit in page-locked memory, which the device writes without a detour through a

@@ -1001,65 +1001,69 @@ __global__ void rope_append_kernel(PoolView pool, const float* qkv, const LaneIn
   __shared__ double2 angle[GROUPS > 1 ? 64 : 1];  // (sine, cosine) per pair
   __shared__ float red[32];
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
-  chain_wait();
   const int lane_id = blockIdx.y, tok = blockIdx.z, tokens = gridDim.z;
-  const LaneInfo info = lanes[lane_id];
   const int D = pool.head_dim, half = D / 2, heads = q_heads + 2 * pool.kv_heads;
   const int width = GROUPS > 1 ? (int)blockDim.x / GROUPS : (int)blockDim.x;  // whole warps
   const int group = GROUPS > 1 ? (int)threadIdx.x / width : 0, pair = (int)threadIdx.x - group * width;
   const bool live = pair < half;  // head dims below 64 leave threads of the warp without a pair
   const int j = live ? pair : 0;
-  const size_t row_width = (size_t)heads * D;
   const size_t row = (size_t)lane_id * tokens + tok;
   const int i0 = layout == 0 ? j : 2 * j, i1 = layout == 0 ? half + j : 2 * j + 1;
   const int head0 = blockIdx.x * HEADS * GROUPS + group;  // this group's heads: head0, head0 + GROUPS, ...
+  const double freq = inv_freq[j];
+  chain_wait();
+  // What the angles and the cells of the cache need, then the heads' inputs, then the angles while those are under way.
+  const LaneInfo info = lanes[lane_id];
   const int pos = info.cursor + tok;
-  float in0[HEADS], in1[HEADS];
-#pragma unroll
-  for (int h = 0; h < HEADS; ++h) {
-    const int head = head0 + h * GROUPS;
-    float r0 = 0.f, r1 = 0.f;
-    if (HEADS * GROUPS == 1 && sum.splits > 0) {  // the projection left its split-K partials unsummed: added up here, in split
-      // order (a narrow shard of a tensor-parallel group has up to 32 splits: eight loads are in flight at a time)
-      const float* p = sum.partials + row * sum.rows_padded + (size_t)head * D;
-      const size_t split_stride = (size_t)sum.vpad * sum.rows_padded;
-      for (int s0 = 0; s0 < sum.splits; s0 += 8) {
-        float first[8], second[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const bool there = s0 + u < sum.splits;
-          first[u] = there ? p[(size_t)(s0 + u) * split_stride + i0] : 0.f;
-          second[u] = there ? p[(size_t)(s0 + u) * split_stride + i1] : 0.f;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          if (s0 + u < sum.splits) {
-            r0 += first[u];
-            r1 += second[u];
-          }
-        }
-      }
-    } else if (head < heads) {
-      const float* src = qkv + row * row_width + (size_t)head * D;
-      r0 = src[i0];
-      r1 = src[i1];
-    }
-    in0[h] = live ? r0 : 0.f;
-    in1[h] = live ? r1 : 0.f;
-  }
   int page = 0, slot = 0;
   if (info.advance > 0 && head0 + (HEADS - 1) * GROUPS >= q_heads) {
     const int block = pos / pool.block_size;
     page = tables[info.table_offset + block];
     slot = pos - block * pool.block_size;
   }
+  // The projection may have left its split-K partials unsummed: they are added up here, in split order (a narrow shard of a
+  // tensor-parallel group has up to 32 splits; eight loads are in flight at a time).
+  constexpr int IN_FLIGHT = 8;
+  const bool summing = HEADS * GROUPS == 1 && sum.splits > 0;
+  const float* partials = sum.partials + row * sum.rows_padded + (size_t)head0 * D;
+  const size_t split_stride = (size_t)sum.vpad * sum.rows_padded;
+  float part0[IN_FLIGHT], part1[IN_FLIGHT], in0[HEADS], in1[HEADS];
+  auto fetch = [&](int s0) {
+#pragma unroll
+    for (int u = 0; u < IN_FLIGHT; ++u)
+      if (s0 + u < sum.splits) {
+        part0[u] = partials[(size_t)(s0 + u) * split_stride + i0];
+        part1[u] = partials[(size_t)(s0 + u) * split_stride + i1];
+      }
+  };
+  if (summing) fetch(0);
+#pragma unroll
+  for (int h = 0; h < HEADS; ++h) {
+    in0[h] = in1[h] = 0.f;
+    if (!summing && live && head0 + h * GROUPS < heads) {
+      const float* src = qkv + (row * heads + head0 + h * GROUPS) * D;
+      in0[h] = src[i0];
+      in1[h] = src[i1];
+    }
+  }
   double s = 0.0, c = 1.0;
-  if (group == 0 && (int)blockIdx.x * HEADS * GROUPS < q_heads + pool.kv_heads) sincos((double)pos * inv_freq[j], &s, &c);
+  if (group == 0 && (int)blockIdx.x * HEADS * GROUPS < q_heads + pool.kv_heads) sincos((double)pos * freq, &s, &c);
   if (GROUPS > 1) {
     if (group == 0 && live) angle[j] = make_double2(s, c);
     __syncthreads();
     s = angle[j].x;
     c = angle[j].y;
+  }
+  if (summing) {
+    for (int s0 = 0; s0 < sum.splits; s0 += IN_FLIGHT) {
+      if (s0 > 0) fetch(s0);
+#pragma unroll
+      for (int u = 0; u < IN_FLIGHT; ++u)
+        if (s0 + u < sum.splits && live) {
+          in0[0] += part0[u];
+          in1[0] += part1[u];
+        }
+    }
   }
 #pragma unroll
   for (int h = 0; h < HEADS; ++h) {

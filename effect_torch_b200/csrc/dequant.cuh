@@ -59,25 +59,46 @@ __device__ __forceinline__ uint32_t fma_h2(uint32_t x, uint32_t y, uint32_t z) {
   return d;
 }
 // One packed word of eight 4-bit codes, logical column j at bit {0,16,8,24,4,20,12,28}[j] -> four half2 in column order,
-// scaled; OFFSET: plus `second`.
-template <bool OFFSET>
+// scaled; OFFSET: plus `second`. RAW: the whole-number codes themselves.
+template <bool OFFSET, bool RAW = false>
 __device__ __forceinline__ void splice_nibbles(uint32_t q, uint32_t scale, uint32_t second, const Splice& k, uint32_t* out) {
   const uint32_t qs = q >> 8;
   const uint32_t lo = OFFSET ? k.bias_lo_k : k.bias_lo, hi = OFFSET ? k.bias_hi_k : k.bias_hi;
   const uint32_t c0 = add_h2(and_or(q, k.mask_lo, k.magic), lo), c1 = add_h2(and_or(qs, k.mask_lo, k.magic), lo);
   const uint32_t c2 = fma_h2(and_or(q, k.mask_hi, k.magic), k.sixteenth, hi), c3 = fma_h2(and_or(qs, k.mask_hi, k.magic), k.sixteenth, hi);
+  if (RAW) { out[0] = c0; out[1] = c1; out[2] = c2; out[3] = c3; return; }
   out[0] = OFFSET ? fma_h2(c0, scale, second) : mul_h2(c0, scale);
   out[1] = OFFSET ? fma_h2(c1, scale, second) : mul_h2(c1, scale);
   out[2] = OFFSET ? fma_h2(c2, scale, second) : mul_h2(c2, scale);
   out[3] = OFFSET ? fma_h2(c3, scale, second) : mul_h2(c3, scale);
 }
 // One word of four int8 codes -> two half2.
-template <bool OFFSET>
+template <bool OFFSET, bool RAW = false>
 __device__ __forceinline__ void splice_bytes(uint32_t w, uint32_t scale, uint32_t second, const Splice& k, uint32_t* out) {
   const uint32_t x = w ^ k.flip;
   const uint32_t c0 = add_h2(__byte_perm(x, k.fill, 0x4140), k.bias_byte), c1 = add_h2(__byte_perm(x, k.fill, 0x4342), k.bias_byte);
+  if (RAW) { out[0] = c0; out[1] = c1; return; }
   out[0] = OFFSET ? fma_h2(c0, scale, second) : mul_h2(c0, scale);
   out[1] = OFFSET ? fma_h2(c1, scale, second) : mul_h2(c1, scale);
+}
+
+// One 32-value block of one row of Q4_0 or Q8_0 in the tiled layout -> 16 half2 of whole-number codes.
+template <int CODEC>
+__device__ __forceinline__ void expand_codes(const unsigned char* q, const Splice& k, uint32_t (&regs)[16]) {
+  static_assert(CODEC == 2 || CODEC == 8, "one scale per block");
+  const uint4 a = *reinterpret_cast<const uint4*>(q);
+  const uint32_t lo[4] = {a.x, a.y, a.z, a.w};
+  if (CODEC == 2) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) splice_nibbles<false, true>(lo[j], 0u, 0u, k, regs + 4 * j);
+  } else {
+    const uint4 b = *reinterpret_cast<const uint4*>(q + 16);
+    const uint32_t hi[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) splice_bytes<false, true>(lo[j], 0u, 0u, k, regs + 2 * j);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) splice_bytes<false, true>(hi[j], 0u, 0u, k, regs + 8 + 2 * j);
+  }
 }
 
 // One 32-value block of one row in the tiled layout: packed words at q, block scale(s) at s -> 16 half2, scaled.

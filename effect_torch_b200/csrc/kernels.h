@@ -35,7 +35,7 @@ cudaError_t launch_qembedding(int codec, const void* indexes, int index_is_i64, 
 // Tiled weights (Q4_0 / Q8_0): 128-row tiles. For row tile t and 32-column block kb the 128 rows' 16 (Q4_0) or 32
 // (Q8_0) payload bytes are contiguous ([tile][block][row][bytes]; Q4_0 nibbles pre-ordered so that masks give f16 pairs
 // in column order), scales are [tile][block][row] f16. Same byte count as the GGUF encoding; rows padded to 128 with
-// zero scales. Both linear kernels (qlinear_mv.cu, qlinear_umma.cu) read this one layout.
+// zero scales. Both linear kernels (qlinear_stream.cu, qlinear_umma.cu) read this one layout.
 // A run of 128-row tiles of one codec inside a tiled weight. A weight fused from parts of different codecs (q and k in
 // Q4_K, v in Q6_K, as GGUF files mix them) holds one segment per run of equal codecs, each repacked in its codec's layout
 // at byte offsets into the weight's arrays; the linear launches one kernel per segment into the same outputs.
@@ -55,9 +55,6 @@ struct TiledWeight {
   uint8_t* quants = nullptr;
   __half* scales = nullptr;
   size_t quant_bytes = 0, scale_bytes = 0;
-  // [rows_padded/128] arrival tickets, zero between launches: taken by the matvec kernel's CTAs that hold part of a row
-  // group's K; the last one to arrive finishes the group
-  int* counters = nullptr;
   int n_segments = 0;       // 0: one segment of `codec` over the whole weight
   TiledSegment segments[kMaxSegments];
 };
@@ -81,7 +78,7 @@ cudaError_t launch_qlinear_reduce(const float* scratch, int splits, int vpad, in
 
 // decode batches up to stream_max_vectors() (qlinear_stream.cu)
 struct StreamPlan {
-  int nv = 32;                  // vectors padded to the MMA N (32, 64 or 128)
+  int nv = 32;                  // vectors padded to the MMA N (16, 32, 64 or 128)
   int tiles = 1, stages = 1;    // 128-row tiles, stages of four 32-value blocks per tile
   int splits = 1, stages_per_split = 1;  // CTAs that share a tile's K: a cluster, or with `deferred` writers of partial sums
   bool deferred = false;
@@ -110,22 +107,6 @@ cudaError_t launch_repack_umma(const TiledWeight& w, const RepackParts& parts, c
 cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, const __half* xh_ready, int64_t vectors, const float* bias,
                                 const float* residual, int epilogue, float* out, __half* out_xh, __half* xh, float* scratch, DeviceStatus* status, int sm_count, cudaStream_t stream,
                                 int* launches);
-
-// small-batch matvec on the 128-row layout (qlinear_mv.cu): up to 32 vectors per pass, mma.sync fed by a bulk-copy ring
-struct MvPlan {
-  int nt = 1;  // groups of 8 vectors per pass (1, 2 or 4)
-  int tiles = 1, groups = 1, spt = 1, units = 1, upc = 1, grid = 1;  // row groups of 1-2 tiles, stages per group, (group, stage) units, units per CTA
-  size_t xh_bytes = 0;       // f16 activations [K/8][nt*8][8] when the caller passes f32 rows (rounded to 256 bytes)
-  size_t partial_bytes = 0;  // [grid][2][nt*8][128] f32 partial tiles of runs that cover part of a tile's K
-};
-MvPlan plan_mv(const TiledWeight& w, int64_t vectors, int sm_count);
-// Largest vector count the front end routes to the matvec kernel (the tcgen05 kernel takes over above it).
-int mv_max_vectors();
-// x f32 [vectors, K] (converted into the head of `scratch` first), or xh_ready in the f16 hand-off layout with row stride
-// xh_nv; scratch holds xh_bytes + partial_bytes of the plan; w.counters holds the tile tickets.
-cudaError_t launch_qlinear_mv(const TiledWeight& w, const float* x, const __half* xh_ready, int64_t vectors, const float* bias,
-                              const float* residual, int epilogue, float* out, __half* out_xh, void* scratch,
-                              DeviceStatus* status, int sm_count, cudaStream_t stream, int* launches, int xh_nv = 32);
 
 // Front end of the tiled linear. `scratch` must hold tiled_scratch_bytes(w, vectors, sm_count).
 size_t tiled_scratch_bytes(const TiledWeight& w, int64_t vectors, int sm_count);

@@ -127,15 +127,8 @@ etc_status build_qweight(etc_runtime* rt, int codec, const void* const* parts, c
     t.scale_bytes = seg.scale_offset + (size_t)seg_rows_padded * kblocks * (tiled_k_quant(pc) ? 4 : 2);
   }
   t.n_segments = n_segments > 1 ? n_segments : 0;
-  // the small-batch matvec kernel (and its arrival tickets) serves single-codec Q4_0 / Q8_0 weights only
-  const size_t counter_bytes = (kquant || mixed) ? 0 : (size_t)(t.rows_padded / 128) * sizeof(int);
   etc_status st = rt->device_alloc(t.quant_bytes, (void**)&t.quants);
   if (st == ETC_OK && t.scale_bytes) st = rt->device_alloc(t.scale_bytes, (void**)&t.scales);
-  if (st == ETC_OK && counter_bytes) {
-    st = rt->device_alloc(counter_bytes, (void**)&t.counters);
-    if (st == ETC_OK && cudaMemsetAsync(t.counters, 0, counter_bytes, rt->stream) != cudaSuccess)
-      st = fail(ETC_EXECUTION, "qweight: clearing the arrival tickets failed");
-  }
   std::vector<void*> staged;
   const uint8_t* device_part[4] = {nullptr, nullptr, nullptr, nullptr};
   for (int p = 0; p < n_parts && st == ETC_OK; ++p) {
@@ -183,7 +176,6 @@ etc_status build_qweight(etc_runtime* rt, int codec, const void* const* parts, c
   if (st != ETC_OK) {
     rt->device_free(t.quants);
     rt->device_free(t.scales);
-    rt->device_free(t.counters);
     delete w;
     return fail(st, message);
   }
@@ -195,7 +187,6 @@ void destroy_qweight(etc_qweight* w) {
   if (!w) return;
   w->rt->device_free(w->tiled.quants);
   w->rt->device_free(w->tiled.scales);
-  w->rt->device_free(w->tiled.counters);
   w->magic = 0;
   delete w;
 }

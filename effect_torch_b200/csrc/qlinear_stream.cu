@@ -54,6 +54,9 @@ constexpr int kWeightWarp = 4 * kDequantGroups, kMmaWarp = kWeightWarp + 1, kAct
 constexpr int kMaxStreamCluster = 8;  // the portable size
 constexpr int kStreamThreads = (kActivationWarp + 1) * 32;
 
+constexpr int kExactVectors = 16;
+constexpr int kDirectVectors = 4;  // at most these many f32 vectors are converted by the linear itself
+
 template <int CODEC, int NV>
 struct StreamCfg {
   static constexpr bool kNibbles = CODEC == 2 || CODEC == 12;
@@ -63,8 +66,12 @@ struct StreamCfg {
   static constexpr uint32_t kStageQ = kStageBlocks * kBlockQ;
   static constexpr uint32_t kStageW = kStageBlocks * (kBlockQ + kBlockS);
   static constexpr uint32_t kStageB = NV * kStageBlocks * 64;
-  static constexpr int kSlots = NV <= 32 ? 3 : 2;  // expanded stages in TMEM
-  static constexpr int kStagesB = NV <= 32 ? (kNibbles ? 6 : 4) : (NV <= 64 && kNibbles ? 3 : 2);
+  // Up to 16 vectors, Q4_0 and Q8_0: the codes go through the MMA unscaled and every block has an accumulator of its own,
+  // whose sums the dequant warps multiply by the block's f32 scale (16 FMA per row in place of 16 products on f16 pairs).
+  static constexpr bool kExact = NV == kExactVectors;
+  static constexpr int kSlots = NV == 32 ? 3 : 2;  // expanded stages in TMEM
+  static constexpr int kAccumulators = kExact ? kSlots * kStageBlocks : 1;
+  static constexpr int kStagesB = NV <= 32 ? (kNibbles || kExact ? 6 : 4) : (NV <= 64 && kNibbles ? 3 : 2);
   // a whole number of stages per dequant group: a ring buffer then belongs to one group, whose own previous round is what
   // tells two phases of the buffer's barrier apart (copies of neighbouring stages may land in either order)
   static constexpr int kStagesW = (int)((104u * 1024 - kStagesB * kStageB) / kStageW) / kDequantGroups * kDequantGroups;
@@ -72,7 +79,7 @@ struct StreamCfg {
   static constexpr int kDone = kStagesB > kSlots ? kStagesB : kSlots;  // barriers on which the MMAs of a stage report
   static constexpr int kBars = 2 * kStagesW + kStagesB + kSlots + kDone + 1;
   static constexpr size_t kSmemBytes = (size_t)kStagesB * kStageB + (size_t)kStagesW * kStageW + kBars * sizeof(uint64_t) + 32;
-  static_assert(NV + kSlots * kStageBlocks * 16 <= (int)kTmemCols, "tensor memory of half an SM");
+  static_assert(NV * kAccumulators + kSlots * kStageBlocks * 16 <= (int)kTmemCols, "tensor memory of half an SM");
   static_assert(kStagesW >= kDequantGroups, "ring");
   static_assert(kSmemBytes <= 112 * 1024, "two CTAs per SM");
   static_assert((size_t)NV * kRows * sizeof(float) <= (size_t)kStagesB * kStageB + (size_t)kStagesW * kStageW, "the accumulator fits the rings");
@@ -81,7 +88,9 @@ struct StreamCfg {
 struct StreamArgs {
   const unsigned char* quants;  // [tile][kblock][128 rows][16 B] or 8-bit codes [tile][kblock][128 rows][32 B]
   const unsigned char* scales;  // [tile][kblock][128] f16 or f16 pairs
-  const __half* xh;             // [K/8][NV][8] f16
+  const __half* xh;             // [K/8][xh_nv][8] f16; xh_nv == NV but for the exact form, where it may be wider
+  const float* x;               // exact form without xh: f32 [vectors, K]
+  int xh_nv;
   const float* bias;
   const float* residual;
   float* out;
@@ -118,6 +127,8 @@ __device__ __forceinline__ void store4(const StreamArgs& a, int v, int c, int n,
   if (a.out_xh) *reinterpret_cast<uint2*>(a.out_xh + ((size_t)(c >> 3) * a.out_xh_nv + v) * 8 + (c & 7)) = pack4(val);
 }
 
+__device__ __forceinline__ void dequant_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(4 * kDequantGroups * 32) : "memory"); }
+
 template <int CODEC, int NV>
 __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(StreamArgs a) {
   using Cfg = StreamCfg<CODEC, NV>;
@@ -151,8 +162,8 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_holder;         // the accumulator at columns [0, NV), then the expanded stages
-  const uint32_t a_tmem = tmem + NV;
+  const uint32_t tmem = *tmem_holder;         // the accumulators from column 0, then the expanded stages
+  const uint32_t a_tmem = tmem + NV * Cfg::kAccumulators;
 
   if (warp < kWeightWarp) {
     // ------------------------------------------------------------------ dequant warps
@@ -168,6 +179,19 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
     const unsigned char* scales = w_ring + Cfg::kStageQ + row * (Cfg::kBlockS / kRows);
     const Splice splice = a.splice;
     bool ok = true;
+    float sums[Cfg::kExact ? NV : 1], scale[kStageBlocks];  // exact form: of this row; the block scales of the stage not yet added
+#pragma unroll
+    for (int v = 0; v < (Cfg::kExact ? NV : 1); ++v) sums[v] = 0.0f;
+    // adds a block's products, which the MMAs of an earlier stage left in its accumulator
+    auto add_block = [&](uint32_t (&products)[16], float block_scale) {
+#pragma unroll
+      for (int v = 0; v < (Cfg::kExact ? 8 : 0); ++v) sums[v] = fmaf(block_scale, __uint_as_float(products[v]), sums[v]);
+      if (a.vectors > 8) {
+#pragma unroll
+        for (int v = 8; v < (Cfg::kExact ? 16 : 0); ++v) sums[v] = fmaf(block_scale, __uint_as_float(products[v]), sums[v]);
+      }
+    };
+    const uint32_t my_products = tmem + lane_base + (uint32_t)(group * kStageBlocks * NV);
     for (int i = group; i < n && ok; i += kDequantGroups) {
       ok = wait_warp(&w_full[w.at], w.parity, abort_flag) && (behind < 0 || wait_warp(&done[freed.at], freed.parity, abort_flag));
       if (!ok) break;
@@ -176,8 +200,22 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
 #pragma unroll
       for (int b = 0; b < kStageBlocks; ++b) {  // blocks beyond the tile's K hold stale bytes that no MMA reads
         uint32_t regs[16];
-        expand_block<CODEC>(payload + stage + b * Cfg::kBlockQ, scales + stage + b * Cfg::kBlockS, splice, regs);
-        tmem_st16(a_tmem + lane_base + (uint32_t)(slot.at * kStageBlocks * 16 + b * 16), regs);
+        if constexpr (Cfg::kExact) {
+          // the stage AS before this one, whose slot and accumulators this group takes over, was a whole one
+          uint32_t products[16];
+          if (behind >= 0) tmem_ld16(my_products + (uint32_t)(b * NV), products);
+          expand_codes<CODEC>(payload + stage + b * Cfg::kBlockQ, splice, regs);
+          const float block_scale = __half2float(*reinterpret_cast<const __half*>(scales + stage + b * Cfg::kBlockS));
+          tmem_st16(a_tmem + lane_base + (uint32_t)(slot.at * kStageBlocks * 16 + b * 16), regs);
+          if (behind >= 0) {
+            tmem_wait_ld16(products);
+            add_block(products, scale[b]);
+          }
+          scale[b] = block_scale;
+        } else {
+          expand_block<CODEC>(payload + stage + b * Cfg::kBlockQ, scales + stage + b * Cfg::kBlockS, splice, regs);
+          tmem_st16(a_tmem + lane_base + (uint32_t)(slot.at * kStageBlocks * 16 + b * 16), regs);
+        }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&w_empty[w.at]);
@@ -191,11 +229,40 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
       else if (behind + kDequantGroups > 0) freed.skip(behind + kDequantGroups);
       behind += kDequantGroups;
     }
-    // ------------------------------------------------------------------ accumulator out of TMEM (half of it per group)
-    chain_wait();  // outputs, residual and scratch may still be in use by the kernel before this one
-    if (wait_warp(d_full, 0, abort_flag)) {
+    const int r = (a.tile0 + tile) * kRows + row;
+    if constexpr (Cfg::kExact) {
+      // ---------------------------------------------------------------- the last stage's products, then both groups' sums
+      static_assert(AS == kDequantGroups, "a group owns a slot");
+      if (ok && behind >= 0 && wait_warp(&done[freed.at], freed.parity, abort_flag)) {
+        tc_fence_after();
+        const int valid = min(kStageBlocks, a.kblocks - (s0 + behind) * kStageBlocks);
+#pragma unroll
+        for (int b = 0; b < kStageBlocks; ++b) {
+          if (b >= valid) break;
+          uint32_t products[16];
+          tmem_ld16(my_products + (uint32_t)(b * NV), products);
+          tmem_wait_ld16(products);
+          add_block(products, scale[b]);
+        }
+      }
+      chain_wait();  // outputs, residual and scratch may still be in use by the kernel before this one
+      float* mine = reinterpret_cast<float*>(smem) + row;
+      dequant_barrier();  // both groups have read their last stage: the rings are free
+      if (group == 1)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) mine[v * kRows] = sums[v];
+      dequant_barrier();
+      if (group == 0)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          const float sum = sums[v] + mine[v * kRows];
+          if (a.deferred) a.scratch[((size_t)split * NV + v) * a.rows_padded + r] = sum;
+          else mine[v * kRows] = sum;
+        }
+    } else if (chain_wait(); wait_warp(d_full, 0, abort_flag)) {
+      // ---------------------------------------------------------------- accumulator out of TMEM (half of it per group)
+      // (outputs, residual and scratch may be in use by the kernel before this one until its end)
       tc_fence_after();
-      const int r = (a.tile0 + tile) * kRows + row;
       // to the consumer's partial sums, or to this CTA's shared memory (the rings are free: every stage has been read)
       float* dst = a.deferred ? a.scratch + (size_t)split * NV * a.rows_padded + r : reinterpret_cast<float*>(smem) + row;
       const size_t stride = a.deferred ? a.rows_padded : kRows;
@@ -230,8 +297,51 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
           for (unsigned spin = 0; spin < (1u << 20) && !mbar_try_wait(&w_full[i % WS], (uint32_t)(i / WS) & 1u); ++spin) __nanosleep(64);
     }
   } else if (warp == kActivationWarp) {
-    // ------------------------------------------------------------------ activation loader (one lane)
-    if (elect_one()) {
+    // ------------------------------------------------------------------ activation loader
+    if (Cfg::kExact && !a.xh) {
+      // Up to kDirectVectors f32 vectors, converted on the way (a launch less): the warp fetches cells of eight columns for as
+      // many stages as four cells per lane cover, then fills their buffers one by one. The rows of absent vectors keep stale
+      // bytes, which reach no other vector's products.
+      chain_wait();  // the activations come from the kernel before this one
+      Ring<BS> b;
+      Ring<DONE> freed;  // the stage BS before this one
+      constexpr int CELLS = 4 * kStageBlocks;  // of a vector in a stage
+      const int per_stage = CELLS * a.vectors, stages = 2 * kDirectVectors / a.vectors, K = a.kblocks * 32;
+      bool ok = true;
+      for (int i0 = 0; i0 < n && ok; i0 += stages) {
+        float4 lo[4], hi[4];
+        int stage[4], cell[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int e = lane + 32 * j, kg = e % CELLS, v = e % per_stage / CELLS;
+          const int column = (s0 + i0 + e / per_stage) * kStageBlocks * 32 + kg * 8;
+          stage[j] = e / per_stage < stages && column < K ? e / per_stage : -1;
+          cell[j] = (kg * NV + v) * 16;
+          if (stage[j] >= 0) {
+            const float4* src = reinterpret_cast<const float4*>(a.x + (size_t)v * K + column);
+            lo[j] = src[0];
+            hi[j] = src[1];
+          }
+        }
+        for (int t = 0; t < stages && i0 + t < n; ++t) {
+          if (i0 + t >= BS) {
+            ok = wait_warp(&done[freed.at], freed.parity, abort_flag);
+            if (!ok) break;
+            freed.next();
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (stage[j] == t) {
+              const uint2 l = pack4(lo[j]), h = pack4(hi[j]);
+              *reinterpret_cast<uint4*>(b_ring + (size_t)b.at * Cfg::kStageB + cell[j]) = make_uint4(l.x, l.y, h.x, h.y);
+            }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads through the async proxy
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&b_full[b.at]);
+          b.next();
+        }
+      }
+    } else if (elect_one()) {
       chain_wait();  // the activations come from the kernel before this one
       Ring<BS> b;
       Ring<DONE> freed;  // the stage BS before this one
@@ -241,10 +351,15 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
           if (!mbar_wait(&done[freed.at], freed.parity, abort_flag)) break;
           freed.next();
         }
-        const int kb = (s0 + i) * kStageBlocks;
-        const uint32_t bytes = (uint32_t)min(kStageBlocks, a.kblocks - kb) * 4u * NV * 16u;
-        mbar_arrive_expect_tx(&b_full[b.at], bytes);
-        bulk_copy_g2s(b_ring + (size_t)b.at * Cfg::kStageB, a.xh + (size_t)kb * 4 * NV * 8, bytes, &b_full[b.at]);
+        const int kb = (s0 + i) * kStageBlocks, groups = min(kStageBlocks, a.kblocks - kb) * 4;  // of eight columns
+        unsigned char* dst = b_ring + (size_t)b.at * Cfg::kStageB;
+        if (Cfg::kExact && a.xh_nv != NV) {  // the first rows of a wider layout
+          mbar_arrive_expect_tx(&b_full[b.at], (uint32_t)groups * NV * 16u);
+          for (int kg = 0; kg < groups; ++kg) bulk_copy_g2s(dst + kg * NV * 16, a.xh + ((size_t)kb * 4 + kg) * a.xh_nv * 8, NV * 16u, &b_full[b.at]);
+        } else {
+          mbar_arrive_expect_tx(&b_full[b.at], (uint32_t)groups * NV * 16u);
+          bulk_copy_g2s(dst, a.xh + (size_t)kb * 4 * NV * 8, (uint32_t)groups * NV * 16u, &b_full[b.at]);
+        }
         issued = i + 1;
         b.next();
       }
@@ -269,6 +384,17 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
         // with constant steps the operands stay in uniform registers (58 cycles per instruction in a loop, 16 unrolled)
         const uint64_t desc = desc0 + (uint64_t)(b.at * (int)(Cfg::kStageB / 16));
         const uint32_t a_cols = a_tmem + (uint32_t)(slot.at * kStageBlocks * 16);
+        if constexpr (Cfg::kExact) {
+          const uint32_t d_cols = tmem + (uint32_t)(slot.at * kStageBlocks * NV);
+#pragma unroll
+          for (int j = 0; j < 2 * kStageBlocks; ++j)
+            if (j < 2 * valid) umma_ts(d_cols + (uint32_t)(j / 2 * NV), a_cols + 8u * j, desc + 2u * NV * j, kIdesc, j & 1);
+          tc_commit(&done[report.at]);
+          b.next();
+          slot.next();
+          report.next();
+          continue;
+        }
         umma_ts(tmem, a_cols, desc, kIdesc, i > 0 ? 1u : 0u);
         if (valid == kStageBlocks) {
 #pragma unroll
@@ -281,7 +407,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
         slot.next();
         report.next();
       }
-      if (ok) tc_commit(d_full);
+      if (ok && !Cfg::kExact) tc_commit(d_full);
     }
   }
   __syncwarp();
@@ -372,7 +498,8 @@ int stream_max_vectors() { return 128; }
 StreamPlan plan_stream(const TiledWeight& w, int64_t vectors, int sm_count, bool deferred) {
   StreamPlan p;
   const int sms = std::max(1, sm_count);
-  p.nv = vectors <= 32 ? 32 : (vectors <= 64 ? 64 : 128);
+  const bool exact = vectors <= kExactVectors && w.n_segments == 0 && (w.codec == 2 || w.codec == 8);
+  p.nv = exact ? kExactVectors : vectors <= 32 ? 32 : (vectors <= 64 ? 64 : 128);
   p.tiles = (int)(w.rows_padded / kRows);
   p.stages = (int)((w.columns / 32 + kStageBlocks - 1) / kStageBlocks);
   p.xh_bytes = ((size_t)(w.columns / 8) * p.nv * 16 + 255) & ~(size_t)255;
@@ -411,17 +538,21 @@ cudaError_t launch_qlinear_stream(const TiledWeight& w, const float* x, const __
   const int K = (int)w.columns;
   __half* xh = reinterpret_cast<__half*>(scratch);
   float* partials = reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + plan.xh_bytes);
-  const bool ready = xh_ready != nullptr && plan.nv == xh_nv;  // the producer stored the f16 layout with this row stride
+  const bool exact = plan.nv == kExactVectors;
+  const bool ready = xh_ready != nullptr && (exact || plan.nv == xh_nv);  // the producer stored the f16 layout with this row stride
   cudaError_t e;
-  if (!ready) {
-    if (!x) return cudaErrorInvalidValue;
-    const int total = (K / 8) * plan.nv, shift = plan.nv == 32 ? 5 : (plan.nv == 64 ? 6 : 7);
+  const bool direct = !ready && exact && vectors <= kDirectVectors;
+  if (!ready && !x) return cudaErrorInvalidValue;
+  if (!ready && !direct) {
+    const int total = (K / 8) * plan.nv, shift = plan.nv == 16 ? 4 : plan.nv == 32 ? 5 : (plan.nv == 64 ? 6 : 7);
     e = launch_chained(convert_hand_off_kernel, dim3((unsigned)std::min((total + 255) / 256, 148 * 4)), dim3(256), 0, stream, x, (int)vectors, K, shift, xh);
     if (e != cudaSuccess) return e;
     if (launches) ++*launches;
   }
   StreamArgs args;
-  args.xh = ready ? xh_ready : xh;
+  args.xh = ready ? xh_ready : direct ? nullptr : xh;
+  args.x = x;
+  args.xh_nv = ready ? xh_nv : plan.nv;
   args.bias = bias;
   args.residual = residual;
   args.out = out;
@@ -453,15 +584,16 @@ cudaError_t launch_qlinear_stream(const TiledWeight& w, const float* x, const __
     }
     auto pass = [&](auto nv_tag) {
       constexpr int NV = decltype(nv_tag)::value;
-      switch (codec) {
-        case 2: return launch_stream_pass<2, NV>(args, tiles, plan.splits, stream);
-        case 8: return launch_stream_pass<8, NV>(args, tiles, plan.splits, stream);
-        case 12: return launch_stream_pass<12, NV>(args, tiles, plan.splits, stream);
-        case 13: return launch_stream_pass<13, NV>(args, tiles, plan.splits, stream);
-        default: return launch_stream_pass<14, NV>(args, tiles, plan.splits, stream);  // 14, and 11 whose re-cut form is the same
+      if (codec == 2) return launch_stream_pass<2, NV>(args, tiles, plan.splits, stream);
+      if (codec == 8) return launch_stream_pass<8, NV>(args, tiles, plan.splits, stream);
+      if constexpr (NV != kExactVectors) {
+        if (codec == 12) return launch_stream_pass<12, NV>(args, tiles, plan.splits, stream);
+        if (codec == 13) return launch_stream_pass<13, NV>(args, tiles, plan.splits, stream);
+        return launch_stream_pass<14, NV>(args, tiles, plan.splits, stream);  // 14, and 11 whose re-cut form is the same
       }
+      return cudaErrorInvalidValue;
     };
-    e = plan.nv == 32 ? pass(std::integral_constant<int, 32>()) : plan.nv == 64 ? pass(std::integral_constant<int, 64>()) : pass(std::integral_constant<int, 128>());
+    e = exact ? pass(std::integral_constant<int, kExactVectors>()) : plan.nv == 32 ? pass(std::integral_constant<int, 32>()) : plan.nv == 64 ? pass(std::integral_constant<int, 64>()) : pass(std::integral_constant<int, 128>());
     if (e != cudaSuccess) return e;
     if (launches) ++*launches;
   }

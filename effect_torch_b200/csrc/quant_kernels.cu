@@ -1,7 +1,7 @@
 // Block-quantized weight kernels for sm_100a: dequantise, quantise, the generic (any codec, raw
 // GGUF layout) linear, the row-gather embedding, the split-K sum of the tcgen05 linear and the
-// front end that routes a tiled linear to the matvec kernel (qlinear_mv.cu, up to 16 vectors) or
-// to the streaming tcgen05 kernel (qlinear_stream.cu, up to 128) or to the large-batch one (qlinear_umma.cu).
+// front end that routes a tiled linear to the streaming kernel (qlinear_stream.cu, up to 128 vectors) or to the
+// large-batch one (qlinear_umma.cu).
 //
 // Replaces crates/runtime-cpu/src/quantized.rs (decode_block :90, linear_into :419,
 // embedding_into :546) of the reference for the CUDA backend.
@@ -454,10 +454,6 @@ cudaError_t launch_qlinear_reduce(const float* scratch, int splits, int vpad, in
 static size_t umma_xh_region(const UmmaPlan& p) { return (p.xh_bytes + 255) & ~(size_t)255; }
 
 size_t tiled_scratch_bytes(const TiledWeight& w, int64_t vectors, int sm_count) {
-  if (w.counters && vectors <= mv_max_vectors()) {
-    const MvPlan p = plan_mv(w, vectors, sm_count);
-    return p.xh_bytes + p.partial_bytes;
-  }
   if (vectors <= stream_max_vectors()) return stream_scratch_bytes(w, vectors, sm_count);
   const UmmaPlan p = plan_umma(w, vectors, sm_count);
   return umma_xh_region(p) + p.scratch_bytes;
@@ -468,9 +464,6 @@ cudaError_t launch_qlinear_tiled(const TiledWeight& w, const float* x, int64_t v
                                  int sm_count, cudaStream_t stream, int* launches, const __half* xh_ready, __half* out_xh, int xh_nv,
                                  DeferredSum* defer) {
   if (defer) *defer = DeferredSum();
-  if (w.counters && vectors <= mv_max_vectors())
-    return launch_qlinear_mv(w, x, xh_ready, vectors, bias, residual, epilogue, out, out_xh, scratch, status, sm_count, stream,
-                             launches, xh_nv);
   if (vectors <= stream_max_vectors())
     return launch_qlinear_stream(w, x, xh_ready, vectors, bias, residual, epilogue, out, out_xh, scratch, status, sm_count, stream, launches, xh_nv, defer);
   const size_t xh_region = umma_xh_region(plan_umma(w, vectors, sm_count));  // f16 activations of every chunk, then the partials

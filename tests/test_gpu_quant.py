@@ -302,3 +302,18 @@ def test_tiled_weight_rejects_unsupported_geometry():
         et.QWeight(rt, gv.Q2_K, [empty((16, 84), dtype=torch.uint8)], [16], 256)
     with pytest.raises(et.BackendError, match="multiple of 256"):
         et.QWeight(rt, gv.Q4_K, [raw], [16], 128)
+
+
+@pytest.mark.parametrize("codec", [gv.Q4_0, gv.Q8_0])
+@pytest.mark.parametrize("rows,columns,vectors", [(70, 64, 1), (130, 192, 16), (200, 704, 8), (4096, 1088, 9), (38100, 320, 3)])
+def test_few_vectors_lose_no_weight_precision(codec, rows, columns, vectors):
+    """Stages that K fills by half, one stage, odd stage counts, one CTA and a whole cluster per row tile: on inputs that f16
+    holds exactly, the sums are those of exact weights."""
+    rng = np.random.default_rng(rows + columns)
+    packed = random_packed(codec, rows, columns, seed=rows)
+    x = rng.normal(size=(vectors, columns)).astype(np.float16).astype(np.float32)
+    qw = et.QWeight(runtime(), codec, [dev(packed)], [rows], columns)
+    out = empty((vectors, rows))
+    qw.linear_into(dev(x), vectors, out)
+    expected = orc.qlinear(codec, x, packed, rows, columns, threads=8)
+    assert helpers.rel_err(host(out), expected) <= 1e-5
