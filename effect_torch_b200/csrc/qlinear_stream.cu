@@ -25,8 +25,10 @@
 // per SM (the HBM rate) the SM issues 2 of its 4 instructions per cycle. Measured alone at 32 vectors with the conversion of
 // f32 activations, before (register-fed dequant warps, MMAs issued at 131 cycles each) and now: [28672 x 4096] 38.8 -> 23.5
 // us, [4096 x 14336] 21.9 -> 17, [4096 x 4096] 12.4 -> 9.4, [128256 x 4096] 118 -> 73.5 (0.61 of the copy bandwidth; Q8_0
-// 123 -> 101, 0.85). In the steady state an SM with two CTAs does a stage in 440 cycles (HBM: 415); what is left is the
-// start of a launch (3 us to the first MMA), the uneven last tiles and the epilogue.
+// 123 -> 101, 0.85). In the form for up to 16 vectors: Q4_0 [28672 x 4096] v8 25.1 -> 20.2 us, [128256 x 4096] v8 74.6 ->
+// 67.4, Q8_0 [28672 x 4096] v16 39.5 -> 26.1 (an mma.sync matvec with tickets between its CTAs before). In the steady state an
+// SM with two CTAs does a stage in 440 cycles (HBM: 415); what is left is the start of a launch (3 us to the first MMA), the
+// uneven last tiles and the epilogue.
 //
 // Every mbarrier wait is bounded: on expiry the abort flag and the status word (3) are raised, all roles run dry, copies
 // in flight are awaited, TMEM is freed.
@@ -129,7 +131,7 @@ __device__ __forceinline__ void store4(const StreamArgs& a, int v, int c, int n,
 
 __device__ __forceinline__ void dequant_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(4 * kDequantGroups * 32) : "memory"); }
 
-template <int CODEC, int NV>
+template <int CODEC, int NV, int USED = NV>
 __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(StreamArgs a) {
   using Cfg = StreamCfg<CODEC, NV>;
   constexpr int WS = Cfg::kStagesW, BS = Cfg::kStagesB, AS = Cfg::kSlots, DONE = Cfg::kDone;
@@ -179,43 +181,53 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
     const unsigned char* scales = w_ring + Cfg::kStageQ + row * (Cfg::kBlockS / kRows);
     const Splice splice = a.splice;
     bool ok = true;
-    float sums[Cfg::kExact ? NV : 1], scale[kStageBlocks];  // exact form: of this row; the block scales of the stage not yet added
+    // exact form: the first USED sums of this row, and the block scales of the stage whose products are not added yet
+    float sums[Cfg::kExact ? USED : 1], scale[kStageBlocks], next_scale[kStageBlocks];
 #pragma unroll
-    for (int v = 0; v < (Cfg::kExact ? NV : 1); ++v) sums[v] = 0.0f;
-    // adds a block's products, which the MMAs of an earlier stage left in its accumulator
-    auto add_block = [&](uint32_t (&products)[16], float block_scale) {
-#pragma unroll
-      for (int v = 0; v < (Cfg::kExact ? 8 : 0); ++v) sums[v] = fmaf(block_scale, __uint_as_float(products[v]), sums[v]);
-      if (a.vectors > 8) {
-#pragma unroll
-        for (int v = 8; v < (Cfg::kExact ? 16 : 0); ++v) sums[v] = fmaf(block_scale, __uint_as_float(products[v]), sums[v]);
-      }
+    for (int v = 0; v < (Cfg::kExact ? USED : 1); ++v) sums[v] = 0.0f;
+    auto load_products = [&](uint32_t taddr, auto& products) {
+      if constexpr (USED == 8) tmem_ld8(taddr, products);
+      else tmem_ld16(taddr, products);
     };
+    auto add_block = [&](auto& products, float block_scale) {
+      pin(products);
+#pragma unroll
+      for (int v = 0; v < (Cfg::kExact ? USED : 0); ++v) sums[v] = fmaf(block_scale, __uint_as_float(products[v]), sums[v]);
+    };
+    constexpr int GROUP = 16 / USED;  // blocks whose products are in registers at a time (all that there is room for)
     const uint32_t my_products = tmem + lane_base + (uint32_t)(group * kStageBlocks * NV);
     for (int i = group; i < n && ok; i += kDequantGroups) {
       ok = wait_warp(&w_full[w.at], w.parity, abort_flag) && (behind < 0 || wait_warp(&done[freed.at], freed.parity, abort_flag));
       if (!ok) break;
       tc_fence_after();
       const uint32_t stage = (uint32_t)w.at * Cfg::kStageW;
+      // exact form: the products of the stage AS before this one (a whole one), whose slot and accumulators this one takes over
+      uint32_t products[Cfg::kExact ? GROUP : 1][Cfg::kExact ? USED : 1];
 #pragma unroll
       for (int b = 0; b < kStageBlocks; ++b) {  // blocks beyond the tile's K hold stale bytes that no MMA reads
         uint32_t regs[16];
         if constexpr (Cfg::kExact) {
-          // the stage AS before this one, whose slot and accumulators this group takes over, was a whole one
-          uint32_t products[16];
-          if (behind >= 0) tmem_ld16(my_products + (uint32_t)(b * NV), products);
+          if (behind >= 0 && b % GROUP == 0) {
+#pragma unroll
+            for (int j = 0; j < GROUP; ++j) load_products(my_products + (uint32_t)((b + j) * NV), products[j]);
+          }
           expand_codes<CODEC>(payload + stage + b * Cfg::kBlockQ, splice, regs);
           const float block_scale = __half2float(*reinterpret_cast<const __half*>(scales + stage + b * Cfg::kBlockS));
           tmem_st16(a_tmem + lane_base + (uint32_t)(slot.at * kStageBlocks * 16 + b * 16), regs);
-          if (behind >= 0) {
-            tmem_wait_ld16(products);
-            add_block(products, scale[b]);
+          if (behind >= 0 && b % GROUP == GROUP - 1) {
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < GROUP; ++j) add_block(products[j], scale[b - GROUP + 1 + j]);
           }
-          scale[b] = block_scale;
+          next_scale[b] = block_scale;
         } else {
           expand_block<CODEC>(payload + stage + b * Cfg::kBlockQ, scales + stage + b * Cfg::kBlockS, splice, regs);
           tmem_st16(a_tmem + lane_base + (uint32_t)(slot.at * kStageBlocks * 16 + b * 16), regs);
         }
+      }
+      if (Cfg::kExact) {
+#pragma unroll
+        for (int b = 0; b < kStageBlocks; ++b) scale[b] = next_scale[b];
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&w_empty[w.at]);
@@ -239,9 +251,9 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
 #pragma unroll
         for (int b = 0; b < kStageBlocks; ++b) {
           if (b >= valid) break;
-          uint32_t products[16];
-          tmem_ld16(my_products + (uint32_t)(b * NV), products);
-          tmem_wait_ld16(products);
+          uint32_t products[USED];
+          load_products(my_products + (uint32_t)(b * NV), products);
+          tmem_wait_ld();
           add_block(products, scale[b]);
         }
       }
@@ -250,11 +262,11 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
       dequant_barrier();  // both groups have read their last stage: the rings are free
       if (group == 1)
 #pragma unroll
-        for (int v = 0; v < NV; ++v) mine[v * kRows] = sums[v];
+        for (int v = 0; v < USED; ++v) mine[v * kRows] = sums[v];
       dequant_barrier();
       if (group == 0)
 #pragma unroll
-        for (int v = 0; v < NV; ++v) {
+        for (int v = 0; v < USED; ++v) {
           const float sum = sums[v] + mine[v * kRows];
           if (a.deferred) a.scratch[((size_t)split * NV + v) * a.rows_padded + r] = sum;
           else mine[v * kRows] = sum;
@@ -482,10 +494,10 @@ __global__ void convert_hand_off_kernel(const float* x, int vectors, int K, int 
   }
 }
 
-template <int CODEC, int NV>
+template <int CODEC, int NV, int USED = NV>
 cudaError_t launch_stream_pass(const StreamArgs& args, int tiles, int splits, cudaStream_t stream) {
   constexpr size_t smem = StreamCfg<CODEC, NV>::kSmemBytes;
-  auto kernel = qlinear_stream_kernel<CODEC, NV>;
+  auto kernel = qlinear_stream_kernel<CODEC, NV, USED>;
   const cudaError_t attr = opt_in_shared_memory(kernel, smem);
   if (attr != cudaSuccess) return attr;
   return launch_chained_cluster(kernel, dim3((unsigned)splits, (unsigned)tiles), dim3(kStreamThreads), smem, stream, args.deferred ? 1u : (unsigned)splits, args);
@@ -541,7 +553,9 @@ cudaError_t launch_qlinear_stream(const TiledWeight& w, const float* x, const __
   const bool exact = plan.nv == kExactVectors;
   const bool ready = xh_ready != nullptr && (exact || plan.nv == xh_nv);  // the producer stored the f16 layout with this row stride
   cudaError_t e;
-  const bool direct = !ready && exact && vectors <= kDirectVectors;
+  // Converting on the way saves a launch (2 us, and 3 us of host time) and slows the stream by some 8 %: even at about 64
+  // stages per SM (18 us of Q4_0).
+  const bool direct = !ready && exact && vectors <= kDirectVectors && (int64_t)plan.tiles * plan.stages <= 64 * (int64_t)sm_count;
   if (!ready && !x) return cudaErrorInvalidValue;
   if (!ready && !direct) {
     const int total = (K / 8) * plan.nv, shift = plan.nv == 16 ? 4 : plan.nv == 32 ? 5 : (plan.nv == 64 ? 6 : 7);
@@ -584,6 +598,8 @@ cudaError_t launch_qlinear_stream(const TiledWeight& w, const float* x, const __
     }
     auto pass = [&](auto nv_tag) {
       constexpr int NV = decltype(nv_tag)::value;
+      if constexpr (NV == kExactVectors)
+        if (args.vectors <= 8) return codec == 2 ? launch_stream_pass<2, NV, 8>(args, tiles, plan.splits, stream) : launch_stream_pass<8, NV, 8>(args, tiles, plan.splits, stream);
       if (codec == 2) return launch_stream_pass<2, NV>(args, tiles, plan.splits, stream);
       if (codec == 8) return launch_stream_pass<8, NV>(args, tiles, plan.splits, stream);
       if constexpr (NV != kExactVectors) {
