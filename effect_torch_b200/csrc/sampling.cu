@@ -321,8 +321,11 @@ struct Row {
       accumulate(m, weighted);
       const int at = min(find_listed(m, before, target, c), m - 1);
       if (threadIdx.x == 0) {
-        sh.decision.picked = sh.key[at];
-        sh.decision.at = before + sh.cumulative[at];
+        // Nothing listed: the bin lies behind the cut at floor_key. The bins of a top-p draw are those of before the cut, and
+        // their sum up to it can be an ulp short of the retained total, which was added up in another order; a draw between
+        // the two has walked past every retained candidate, and the last one of those is the one at the cut.
+        sh.decision.picked = m > 0 ? sh.key[at] : scope.floor_key;
+        sh.decision.at = m > 0 ? before + sh.cumulative[at] : target;
       }
     }
     cluster.sync();

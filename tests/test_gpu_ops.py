@@ -162,6 +162,41 @@ def test_device_sampling_at_the_edges_of_its_slices_and_lists(vocab):
             np.testing.assert_array_equal(host(tokens), want, err_msg=str(mode))
 
 
+def seed_of_the_largest_draw():
+    """The seed whose draw at counter 0 is 1 - 2^-53, the largest there is: the splitmix64 steps run backwards."""
+    bits = (1 << 64) - 1
+    value = bits
+    for shift, factor in ((31, 0x94d049bb133111eb), (27, 0xbf58476d1ce4e5b9), (30, 1)):
+        step = value
+        for _ in range(64 // shift + 1):
+            step = value ^ (step >> shift)
+        value = step * pow(factor, -1, 1 << 64) & bits
+    return (value - 0x9e3779b97f4a7c15) & bits
+
+
+@pytest.mark.parametrize("head", [300, 6000])
+def test_a_draw_just_below_the_retained_total_takes_the_last_retained_candidate(head):
+    """top-p cuts behind the last of `head` candidates that share the maximum's bin of 1/32 in the logit (in the second case
+    more of them than the sorted list holds); the tail starts nine bins further down. The largest draw lies an ulp below
+    the retained total, and the histogram's sum up to the cut, added up in another order, is short of that in about one row
+    of three."""
+    rt = runtime()
+    rng = np.random.default_rng(head)
+    rows, tail = 64, 500
+    top = -(rng.permutation(head).astype(np.float32) + 0.5) / np.float32(32 * head)  # distinct, in (-1/32, 0)
+    values = np.concatenate([[np.float32(0.0)], top, np.float32(-0.3) - rng.random(tail).astype(np.float32)]).astype(np.float32)
+    weights = np.exp(np.sort(values)[::-1].astype(np.float64))
+    top_p = float((weights[:head + 1].sum() - 0.5 * weights[head]) / weights.sum())
+    logits = np.stack([values[rng.permutation(values.size)] for _ in range(rows)])
+    seed = seed_of_the_largest_draw()
+    assert orc.random_unit(seed, 0) == 1.0 - 2.0 ** -53
+    tokens = empty(rows, dtype=torch.int32)
+    rt.sample_rows_into(dev(logits), rows, values.size, tokens, temperature=1.0, top_p=top_p, seed=seed)
+    want = [int(np.flatnonzero(row == top.min())[0]) for row in logits]
+    np.testing.assert_array_equal(host(tokens), want)
+    assert want == [orc.sample_logits(row, temperature=1.0, top_p=top_p, seed=seed) for row in logits]
+
+
 @pytest.mark.parametrize("vocab", [1, 8192, 8195, 40000, 65541])
 def test_argmax_across_the_slices_of_a_row(vocab):
     rng = np.random.default_rng(vocab)
