@@ -639,14 +639,17 @@ etc_status execute_impl(etc_decoder* dec, etc_pool* pool, etc_seq* const* seqs, 
   // the argmax kernel stores its tokens into pinned memory itself; those of a sharded head are settled between the ranks
   if (h_out_tokens && dec->vocab_global > 0 && dec->tp_world > 1)
     e = cudaMemcpyAsync(dec->h_tokens, dec->d_tokens, sizeof(uint32_t) * (size_t)c.batch, cudaMemcpyDeviceToHost, rt->stream);
-  // logits go straight into the caller's buffer when that is page-locked, else through the decoder's own
-  float* const logits_to = h_logits && page_locked(h_logits) ? h_logits : dec->h_logits;
-  if (e == cudaSuccess && h_logits)
-    e = cudaMemcpyAsync(logits_to, dec->logits, sizeof(float) * (size_t)active * c.vocab, cudaMemcpyDeviceToHost, rt->stream);
-  if (e != cudaSuccess) {
-    fail(ETC_TRANSFER, std::string("readback failed: ") + cudaGetErrorString(e));
+  // The caller's buffer is written by steps that commit only. A page-locked one is the target of a copy that follows the status
+  // and the cancellation flag; for any other the logits wait in the decoder's own, copied behind the step.
+  const size_t logits_bytes = sizeof(float) * (size_t)active * c.vocab;
+  const bool direct = h_logits && page_locked(h_logits);
+  if (e == cudaSuccess && h_logits && !direct)
+    e = cudaMemcpyAsync(dec->h_logits, dec->logits, logits_bytes, cudaMemcpyDeviceToHost, rt->stream);
+  auto readback_failed = [&](cudaError_t error) {
+    fail(ETC_TRANSFER, std::string("readback failed: ") + cudaGetErrorString(error));
     return abort_with(ETC_TRANSFER);
-  }
+  };
+  if (e != cudaSuccess) return readback_failed(e);
   // sample-before-commit: the status word carries embedding / non-finite-logit problems
   st = rt->check_status();
   if (st != ETC_OK) {
@@ -659,8 +662,14 @@ etc_status execute_impl(etc_decoder* dec, etc_pool* pool, etc_seq* const* seqs, 
     fail(ETC_CANCELLED, "operation aborted");
     return abort_with(ETC_CANCELLED);
   }
+  if (direct) {
+    e = cudaMemcpyAsync(h_logits, dec->logits, logits_bytes, cudaMemcpyDeviceToHost, rt->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(rt->stream);
+    if (e != cudaSuccess) return readback_failed(e);
+  } else if (h_logits) {
+    std::memcpy(h_logits, dec->h_logits, logits_bytes);
+  }
   if (h_out_tokens) std::memcpy(h_out_tokens, dec->h_tokens, sizeof(uint32_t) * (size_t)active);
-  if (h_logits && logits_to != h_logits) std::memcpy(h_logits, dec->h_logits, sizeof(float) * (size_t)active * c.vocab);
   for (int i = 0; i < active; ++i) {
     etc_seq* s = seqs[i];
     const int start = dec->h_lanes[i].start;
@@ -672,9 +681,7 @@ etc_status execute_impl(etc_decoder* dec, etc_pool* pool, etc_seq* const* seqs, 
   return ETC_OK;
 }
 
-// record of one greedy step, run as the last node of the captured step graph
 }  // namespace
-
 
 extern "C" {
 

@@ -464,7 +464,8 @@ ETC_API etc_status etc_decoder_finalize(etc_decoder* dec);
  * `advance` tokens (h_tokens is [active, advance] u32); h_logits (may be NULL) receives the
  * LastTokenRow logits [active, vocab]. Pads to the compiled batch, runs begin -> commands ->
  * commit; any failure (pool exhausted, capacity, cancellation, device status) rolls back so no
- * cursor or block list changes (napi/mod.rs:4441-4518). `cancelled` may be NULL. */
+ * cursor or block list changes (napi/mod.rs:4441-4518), and h_logits is left alone (of a readback that
+ * itself fails it may hold a part). `cancelled` may be NULL. */
 ETC_API etc_status etc_decoder_execute(etc_decoder* dec, etc_pool* pool, etc_seq* const* seqs, int active,
                                        const uint32_t* h_tokens, int advance, float* h_logits,
                                        const volatile int* cancelled);

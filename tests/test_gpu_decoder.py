@@ -1,8 +1,13 @@
 """GPU parity of the compiled decoder against the CPU oracle: greedy token ids (exact) and teacher-forced
 logits on the tiny f32 model, the quantized tensor-core path within the logits tolerance, and the stateful
 transaction rules (padding, rollback, cancellation, device-resident generation)."""
+import ctypes as C
+import threading
+import time
+
 import numpy as np
 import pytest
+import torch
 
 import effect_torch_b200 as et
 import oracle as orc
@@ -207,6 +212,49 @@ def test_transaction_rollback_padding_and_cancellation(tiny):
     b.release()
     with pytest.raises(et.BackendError, match="kv sequence 1 is released"):
         gdec.execute(pool, [a, b], np.zeros((2, 1), dtype=np.uint32))
+
+
+def execute_into(dec, pool, seqs, tokens, address, flag=None):
+    """etc_decoder_execute with the caller's own logits buffer and cancellation flag."""
+    tokens = np.ascontiguousarray(tokens, dtype=np.uint32)
+    return dec.rt.L.etc_decoder_execute(dec.h, pool.h, dec._seq_array(seqs), tokens.shape[0], tokens.ctypes.data, tokens.shape[1], address,
+                                        None if flag is None else C.cast(C.byref(flag), C.c_void_p))
+
+
+def test_a_step_that_does_not_commit_leaves_a_page_locked_buffer_alone(tiny):
+    cfg = helpers.TINY
+    dec = gpu_decoder(cfg, tiny, batch=2, max_tokens=64, max_advance=16)
+    pool = et.NativeKvPool(runtime(), cfg["layers"], cfg["kv_heads"], cfg["head_dim"], 64, 16, et.KV_F32)
+    tokens = np.arange(32, dtype=np.uint32).reshape(2, 16)
+    want = dec.execute(pool, [pool.makeSequence() for _ in range(2)], tokens)
+    buffer = torch.empty((2, cfg["vocab"]), dtype=torch.float32, pin_memory=True)
+    # the device reports an index that the embedding does not have
+    seqs = [pool.makeSequence() for _ in range(2)]
+    buffer.fill_(-7.0)
+    bad = tokens.copy()
+    bad[1, 3] = cfg["vocab"]
+    assert execute_into(dec, pool, seqs, bad, buffer.data_ptr()) == 5
+    assert bool((buffer == -7.0).all()) and [s.cursor for s in seqs] == [0, 0]
+    # the flag is raised somewhere between the call and its commit: either the step commits or nothing of it is seen
+    for attempt in range(60):
+        seqs = [pool.makeSequence() for _ in range(2)]
+        buffer.fill_(-7.0)
+        flag = C.c_int(0)
+        delay = attempt * 2e-5
+
+        def cancel():
+            until = time.perf_counter() + delay
+            while time.perf_counter() < until:
+                pass
+            flag.value = 1
+
+        thread = threading.Thread(target=cancel)
+        thread.start()
+        status = execute_into(dec, pool, seqs, tokens, buffer.data_ptr(), flag)
+        thread.join()
+        assert status in (0, 7)
+        np.testing.assert_array_equal(buffer.numpy(), want if status == 0 else np.full_like(want, -7.0))
+        assert [s.cursor for s in seqs] == ([16, 16] if status == 0 else [0, 0])
 
 
 def test_sliding_window_decoder_matches_the_oracle():
