@@ -7,6 +7,7 @@
 // before commit, then commit (evict, note tokens, advance cursors) or roll back.
 // The command list is the decode graph of a GQA + RoPE + SwiGLU block wired as
 // packages/core/src/models/MuseGlimmer.ts:284-367 wires its ops.
+#include <cuda.h>
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -557,13 +558,27 @@ etc_status ensure_exact_scratch(etc_decoder* dec, const StepContext& ctx) {
   return ETC_OK;
 }
 
-bool page_locked(const void* p) {
+// All of [p, p + bytes) lies in one page-locked allocation or registration. A buffer that is locked in part, or in pieces, is
+// not: a copy into it would be refused.
+bool page_locked(const void* p, size_t bytes) {
   cudaPointerAttributes attributes;
   if (cudaPointerGetAttributes(&attributes, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return attributes.type == cudaMemoryTypeHost;
+  if (attributes.type != cudaMemoryTypeHost || !attributes.devicePointer) return false;
+  // the extent of the allocation that an address belongs to is known to the driver's interface only
+  static const auto address_range = [] {
+    void* entry = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &entry, 12000, cudaEnableDefault, &found) != cudaSuccess) cudaGetLastError();
+    return reinterpret_cast<CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr)>(entry);
+  }();
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  const CUdeviceptr first = reinterpret_cast<CUdeviceptr>(attributes.devicePointer);
+  if (!address_range || address_range(&start, &size, first) != CUDA_SUCCESS) return false;
+  return first >= start && first - start <= size && bytes <= size - (first - start);
 }
 
 bool uses_exact_attention(const etc_decoder* dec, const etc_pool* pool, int T) {
@@ -642,7 +657,7 @@ etc_status execute_impl(etc_decoder* dec, etc_pool* pool, etc_seq* const* seqs, 
   // The caller's buffer is written by steps that commit only. A page-locked one is the target of a copy that follows the status
   // and the cancellation flag; for any other the logits wait in the decoder's own, copied behind the step.
   const size_t logits_bytes = sizeof(float) * (size_t)active * c.vocab;
-  const bool direct = h_logits && page_locked(h_logits);
+  const bool direct = h_logits && page_locked(h_logits, logits_bytes);
   if (e == cudaSuccess && h_logits && !direct)
     e = cudaMemcpyAsync(dec->h_logits, dec->logits, logits_bytes, cudaMemcpyDeviceToHost, rt->stream);
   auto readback_failed = [&](cudaError_t error) {

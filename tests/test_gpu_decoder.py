@@ -2,6 +2,7 @@
 logits on the tiny f32 model, the quantized tensor-core path within the logits tolerance, and the stateful
 transaction rules (padding, rollback, cancellation, device-resident generation)."""
 import ctypes as C
+import mmap
 import threading
 import time
 
@@ -219,6 +220,37 @@ def execute_into(dec, pool, seqs, tokens, address, flag=None):
     tokens = np.ascontiguousarray(tokens, dtype=np.uint32)
     return dec.rt.L.etc_decoder_execute(dec.h, pool.h, dec._seq_array(seqs), tokens.shape[0], tokens.ctypes.data, tokens.shape[1], address,
                                         None if flag is None else C.cast(C.byref(flag), C.c_void_p))
+
+
+# which of the buffer's eight pages are registered, call by call
+LOCKED_PAGES = {"pageable": [], "whole": [(0, 8)], "with neighbours": [(-1, 10)], "first half": [(0, 4)], "second half": [(4, 4)],
+                "two pieces": [(0, 4), (4, 4)], "both ends": [(0, 2), (6, 2)]}
+
+
+@pytest.mark.parametrize("locked", sorted(LOCKED_PAGES))
+def test_logits_arrive_in_any_buffer(tiny, locked):
+    """Pageable memory, a buffer inside one page-locked registration, and buffers that are locked in part or in pieces, which
+    no single copy may span."""
+    cfg = helpers.TINY
+    dec = gpu_decoder(cfg, tiny, batch=2, max_tokens=64, max_advance=16)
+    pool = et.NativeKvPool(runtime(), cfg["layers"], cfg["kv_heads"], cfg["head_dim"], 64, 16, et.KV_F32)
+    tokens = np.arange(32, dtype=np.uint32).reshape(2, 16)
+    want = dec.execute(pool, [pool.makeSequence() for _ in range(2)], tokens)
+    assert want.nbytes == 8 * mmap.PAGESIZE
+    memory = np.frombuffer(mmap.mmap(-1, 10 * mmap.PAGESIZE), dtype=np.float32)
+    buffer = memory[mmap.PAGESIZE // 4:][:want.size].reshape(want.shape)
+    memory[:] = -7.0
+    cudart, base, registered = torch.cuda.cudart(), buffer.ctypes.data, []
+    try:
+        for first, pages in LOCKED_PAGES[locked]:
+            assert int(cudart.cudaHostRegister(base + first * mmap.PAGESIZE, pages * mmap.PAGESIZE, 0)) == 0
+            registered.append(base + first * mmap.PAGESIZE)
+        assert execute_into(dec, pool, [pool.makeSequence() for _ in range(2)], tokens, base) == 0
+    finally:
+        for address in registered:
+            cudart.cudaHostUnregister(address)
+    np.testing.assert_array_equal(buffer, want)
+    assert (memory[:mmap.PAGESIZE // 4] == -7.0).all() and (memory[-(mmap.PAGESIZE // 4):] == -7.0).all()
 
 
 def test_a_step_that_does_not_commit_leaves_a_page_locked_buffer_alone(tiny):
