@@ -56,8 +56,9 @@ def _ptr(t):
 
 
 # Results of up to this many bytes at a time sit in page-locked memory, which the device writes without a detour through a
-# staging buffer. It comes from torch's caching host allocator, so that it costs neither a registration nor fresh pages once
-# an earlier result has been released; Runtime.close() gives the cache back.
+# staging buffer. It comes from the caching host allocator of a program that has torch loaded, so that it costs neither a
+# registration nor fresh pages once an earlier result has been released; Runtime.close() gives the cache back. A program
+# without torch, or whose memory cannot be locked, gets pageable results.
 _PAGE_LOCKED_MOST = 256 << 20
 _page_locked_lock = threading.RLock()  # a finalizer may run while its thread holds it
 _page_locked_bytes = 0
@@ -74,10 +75,14 @@ def _page_locked_add(nbytes: int) -> bool:
 
 def _result_buffer(shape) -> np.ndarray:
     nbytes = 4 * int(np.prod(shape))
-    if nbytes == 0 or not _page_locked_add(nbytes):
+    torch = sys.modules.get("torch")
+    if nbytes == 0 or torch is None or not _page_locked_add(nbytes):
         return np.empty(shape, dtype=np.float32)
-    import torch
-    array = torch.empty(shape, dtype=torch.float32, pin_memory=True).numpy()
+    try:
+        array = torch.empty(shape, dtype=torch.float32, pin_memory=True).numpy()
+    except Exception:  # no page-locked memory to be had, or a torch that is not wholly loaded or has no CUDA
+        _page_locked_add(-nbytes)
+        return np.empty(shape, dtype=np.float32)
     weakref.finalize(array, _page_locked_add, -nbytes).atexit = False
     return array
 

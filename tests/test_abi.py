@@ -1,14 +1,27 @@
 """The C-ABI library loads and exports every symbol include/et_cuda.h declares (no GPU needed)."""
+import builtins
 import ctypes as C
 import os
 import re
+import sys
+import types
 
+import numpy as np
 import pytest
 
 import effect_torch_b200 as et
 from effect_torch_b200 import _lib
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+_import = builtins.__import__
+
+
+def refuse_torch(name, *args, **kwargs):
+    if name == "torch":
+        raise ImportError("no torch here")
+    return _import(name, *args, **kwargs)
 
 
 def declared_symbols():
@@ -61,6 +74,24 @@ def test_no_cpu_fallback_without_a_device():
         et.Runtime(0)
     assert e.value.reason == "backend-unavailable"
     assert "no CPU fallback" in str(e.value)
+
+
+def test_logits_need_neither_torch_nor_page_locked_memory(monkeypatch):
+    """A result buffer is ordinary memory where torch is not loaded, and where it cannot lock memory, whose bytes are then
+    not counted."""
+    before = et._page_locked_bytes
+    monkeypatch.delitem(sys.modules, "torch", raising=False)
+    monkeypatch.setattr(builtins, "__import__", refuse_torch)
+    assert et._result_buffer((2, 3)).shape == (2, 3) and "torch" not in sys.modules
+
+    def no_memory(*args, **kwargs):
+        raise RuntimeError("CUDA error: out of memory")
+
+    monkeypatch.setitem(sys.modules, "torch", types.SimpleNamespace(empty=no_memory, float32=None))
+    for _ in range(2):
+        buffer = et._result_buffer((4, 5))
+        assert buffer.shape == (4, 5) and buffer.dtype == np.float32 and buffer.flags["C_CONTIGUOUS"]
+    assert et._page_locked_bytes == before
 
 
 def test_every_attention_plan_a_step_can_ask_for_fits_the_decoder_reserve():
