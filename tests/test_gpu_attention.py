@@ -10,7 +10,7 @@ from tests.golden import reference_vectors as gv
 from tests.gpu_util import dev, empty, host, runtime
 
 pytestmark = pytest.mark.gpu
-REL_TOL = 2e-3  # north-star tolerance on attention outputs for the f16 path
+REL_TOL = 2e-3  # tolerance on attention outputs for the f16 path
 
 
 def gpu_attention(pool, layer, seqs, batch, active, advance, q, k, v, scale, op_window=None, pool_window=None):
@@ -154,6 +154,100 @@ def test_prefix_cache_and_prefill_match():
         g2.prefillMatch(tokens)
     g3 = gp.makeSequence()
     assert g3.prefillMatch([1, 2, 3]) == 0
+
+
+def colliding_prompts(slots, block, rng):
+    """Six prompts of two whole blocks and a token whose block hashes all belong into the last two slots of a table of `slots`
+    (second blocks into the first one too), so that its probe sequences wrap; every other prompt has tokens of 2^24 and more,
+    up to 2^32 - 1."""
+    home = lambda h: (h ^ (h >> 32)) % slots
+    prompts = []
+    while len(prompts) < 6:
+        draw = lambda: rng.integers(1 << 24, 1 << 32, size=block) if len(prompts) % 2 else rng.integers(0, 1 << 17, size=block)
+        first = draw()
+        h1 = orc.chain_hash(orc.HASH_SEED, first.astype(np.uint32))
+        if home(h1) < slots - 2:
+            continue
+        while True:
+            second = draw()
+            if home(orc.chain_hash(h1, second.astype(np.uint32))) in (slots - 2, slots - 1, 0):
+                break
+        prompts.append(np.concatenate([first, second, [7]]).astype(np.uint32))
+    return prompts
+
+
+def test_prefix_index_with_colliding_hashes_and_large_tokens():
+    """Pages, matches and counters of a pool whose block hashes collide and wrap in the prefix index, against the oracle, over
+    a long random run of requests. Requests that skip the match list one hash for several blocks; a small pool reclaims
+    cached blocks all the time."""
+    rt, block, capacity = runtime(), 2, 16
+    rng = np.random.default_rng(11)
+    prompts = colliding_prompts(2 * capacity, block, rng)
+    gp = et.NativeKvPool(rt, 1, 1, 2, capacity * block, block, et.KV_F32)
+    op = orc.Pool(1, 1, 2, capacity * block, block, orc.F32)
+    kv = np.zeros((1, 1, 5, 2), np.float32)
+    d_kv = dev(kv)
+    live, matched = [], 0
+    for _ in range(600):
+        if live and (len(live) == 4 or rng.random() < 0.45):
+            g, o = live.pop(int(rng.integers(len(live))))
+            g.release()
+            o.release()
+        else:
+            prompt = prompts[int(rng.integers(len(prompts)))]
+            g, o = gp.makeSequence(), op.make_sequence()
+            done = 0
+            if rng.random() < 0.7:
+                done = g.prefillMatch(prompt)
+                assert done == o.prefill_match(prompt)
+                matched += done
+            rest = 5 - done
+            rt.kv_append_into(gp, 0, [g], 1, 1, rest, d_kv, d_kv, rest)
+            g.commit(prompt[done:])
+            o.set_advance(rest)
+            orc.kv_attention(op, 0, [o], 1, kv[:, :, :rest], kv[:, :, :rest], kv[:, :, :rest], 1.0)
+            o.note_tokens(prompt[done:])
+            o.set_cursor(5)
+            live.append((g, o))
+        for g, o in live:
+            np.testing.assert_array_equal(g.blocks[0], o.blocks)
+        assert (gp.freeBlocks, gp.cachedBlocks) == (op.free_blocks, op.cached_blocks)
+    assert matched > 100
+    # a token that differs in its top byte alone is another token
+    for prompt in prompts[1::2]:
+        g, o = gp.makeSequence(), op.make_sequence()
+        other = prompt.copy()
+        other[0] ^= 1 << 30
+        assert g.prefillMatch(other) == o.prefill_match(other) == 0
+
+
+@pytest.mark.parametrize("tier,otier", [(et.KV_F32, orc.F32), (et.KV_U8, orc.U8)])
+def test_reference_order_attention_beyond_the_contexts_it_keeps_on_chip(tier, otier):
+    """Contexts of 2047 to 2052 positions around the 2048 whose weights stay in shared memory, in one launch (a chunk whose
+    rows lie on both sides) and step by step, and a window that brings a longer context back below it."""
+    rng = np.random.default_rng(12)
+    Hq, Hkv, D, tokens = 2, 1, 64, 2176
+    gp = et.NativeKvPool(runtime(), 1, Hkv, D, tokens, 16, tier)
+    op = orc.Pool(1, Hkv, D, tokens, 16, otier)
+    g, o = gp.makeSequence(), op.make_sequence()
+    normal = lambda heads, t: rng.normal(size=(1, heads, t, D)).astype(np.float32)
+    cursor = 0
+    for advance, window in ((2046, None), (3, None), (1, None), (1, 2048), (1, 2050)):
+        k, v = normal(Hkv, advance), normal(Hkv, advance)
+        ids = np.zeros(advance, dtype=np.uint32)
+        o.set_advance(advance)
+        if advance > 100:  # the cached part
+            runtime().kv_append_into(gp, 0, [g], 1, 1, advance, dev(k), dev(v), advance)
+            orc.kv_attention(op, 0, [o], 1, np.zeros((1, Hq, advance, D), np.float32), k, v, 0.125, mode=1, threads=4)
+        else:
+            q = normal(Hq, advance)
+            out = gpu_attention(gp, 0, [g], 1, 1, advance, q, k, v, 0.125, op_window=window)
+            want = orc.kv_attention(op, 0, [o], 1, q, k, v, 0.125, op_window=window)
+            assert helpers.rel_err(out, want) <= 1e-6, (advance, window)
+        g.commit(ids)
+        o.note_tokens(ids)
+        cursor += advance
+        o.set_cursor(cursor)
 
 
 @pytest.mark.parametrize("tier,otier,tol", [(et.KV_F16, orc.F16, REL_TOL), (et.KV_BF16, orc.BF16, 2e-2), (et.KV_U8, orc.U8, REL_TOL)])

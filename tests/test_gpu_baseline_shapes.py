@@ -13,7 +13,7 @@ from tests import helpers
 from tests.gpu_util import dev, empty, host, runtime
 
 pytestmark = pytest.mark.gpu
-REL_TOL = 2e-3  # north-star tolerance on f16/f32 outputs, as max |err| / max |ref|
+REL_TOL = 2e-3  # tolerance on f16/f32 outputs, as max |err| / max |ref|
 THREADS = max(1, min(16, orc.max_threads()))
 
 

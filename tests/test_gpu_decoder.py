@@ -16,7 +16,7 @@ from tests import helpers
 from tests.gpu_util import runtime
 
 pytestmark = pytest.mark.gpu
-LOGIT_TOL = 2e-3  # north-star tolerance on logits (max |err| / max |ref|)
+LOGIT_TOL = 2e-3  # tolerance on logits (max |err| / max |ref|)
 
 
 def gpu_decoder(cfg, weights, batch, max_tokens, block_size=16, kv_dtype=et.KV_F32, exact=True, max_advance=16, window=None):

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 ALL_CODECS = [gv.Q4_0, gv.Q8_0, gv.Q2_K, gv.Q3_K, gv.Q4_K, gv.Q5_K, gv.Q6_K]
 SCALE_FIELDS = {gv.Q4_0: [0], gv.Q8_0: [0], gv.Q2_K: [80, 82], gv.Q3_K: [108], gv.Q4_K: [0, 2], gv.Q5_K: [0, 2], gv.Q6_K: [208]}
-REL_TOL = 2e-3  # north-star tolerance on f16/f32 linear outputs, as max |err| / max |ref|
+REL_TOL = 2e-3  # tolerance on f16/f32 linear outputs, as max |err| / max |ref|
 
 
 def random_packed(codec, rows, columns, seed):
