@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "activation.cuh"
 #include "chain.cuh"
 #include "kernels.h"
 
@@ -602,7 +603,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs
       if (a.out) a.out[((size_t)lane_id * a.q_heads + head) * D + d] = val;
       if (a.out_xh) {
         const int k = head * D + d;
-        a.out_xh[hand_off_cell(k >> 3, lane_id, a.out_xh_nv, a.q_heads * (D / 8)) + (k & 7)] = __float2half_rn(fminf(fmaxf(val, -65504.f), 65504.f));
+        a.out_xh[hand_off_cell(k >> 3, lane_id, a.out_xh_nv, a.q_heads * (D / 8)) + (k & 7)] = half_sat(val);
       }
     } else {
       float* dst = a.partial + (((size_t)lane_id * a.q_heads + head) * nsplits + split) * (D + 2);
@@ -656,7 +657,7 @@ __global__ void attention_merge_kernel(const float* partial, int q_heads, int sp
     if (out) out[((size_t)lane_id * q_heads + head) * D + d] = val;
     if (out_xh) {
       const int k = head * D + d;
-      out_xh[hand_off_cell(k >> 3, lane_id, xh_nv, q_heads * (D / 8)) + (k & 7)] = __float2half_rn(fminf(fmaxf(val, -65504.f), 65504.f));
+      out_xh[hand_off_cell(k >> 3, lane_id, xh_nv, q_heads * (D / 8)) + (k & 7)] = half_sat(val);
     }
   }
 }
@@ -886,7 +887,7 @@ __global__ void __launch_bounds__(128, U8 ? 2 : 3) attention_chunk_kernel(AttnAr
       const float x = o[i][2 * h] * inv, y = o[i][2 * h + 1] * inv;
       if (a.out) *reinterpret_cast<float2*>(a.out + (row * a.q_heads + head) * D + i * 8 + 2 * t) = make_float2(x, y);
       if (a.out_xh) {
-        const __half2 v = __floats2half2_rn(fminf(fmaxf(x, -65504.f), 65504.f), fminf(fmaxf(y, -65504.f), 65504.f));
+        const __half2 v = half2_sat(x, y);
         *reinterpret_cast<__half2*>(a.out_xh + hand_off_cell(head * (D / 8) + i, row, a.out_xh_nv, a.q_heads * (D / 8)) + 2 * t) = v;
       }
     }

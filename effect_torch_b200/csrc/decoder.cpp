@@ -252,7 +252,7 @@ etc_status project_qkv_raw(StepContext& s, size_t layer, const float* x, int64_t
       ETC_CUDA(launch_dense_linear(a, stream));
       ++s.launches;
     } else {
-      ETC_CUDA(launch_qlinear_generic(w[p]->codec, x, rows, w[p]->columns, (const uint8_t*)w[p]->d_raw, w[p]->rows, nullptr, out[p], stream, &s.launches,
+      ETC_CUDA(launch_qlinear_generic(w[p]->codec, x, rows, w[p]->columns, (const uint8_t*)w[p]->d_raw, w[p]->rows, nullptr, out[p], d->rt->sm_count, stream, &s.launches,
                                       stride));
     }
   }
@@ -281,7 +281,7 @@ etc_status run_linear(StepContext& s, const BoundWeight& raw, etc_qweight* tiled
     return ETC_OK;
   }
   float* target = epilogue == ETC_EPILOGUE_RESIDUAL ? d->proj : out;
-  ETC_CUDA(launch_qlinear_generic(raw.codec, x, vectors, raw.columns, (const uint8_t*)raw.d_raw, raw.rows, nullptr, target, stream, &s.launches));
+  ETC_CUDA(launch_qlinear_generic(raw.codec, x, vectors, raw.columns, (const uint8_t*)raw.d_raw, raw.rows, nullptr, target, d->rt->sm_count, stream, &s.launches));
   if (epilogue == ETC_EPILOGUE_RESIDUAL) {
     ETC_CUDA(launch_add(residual, target, vectors * raw.rows, out, stream));
     ++s.launches;

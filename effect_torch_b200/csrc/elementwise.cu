@@ -12,6 +12,7 @@
 
 #include <algorithm>
 
+#include "activation.cuh"
 #include "chain.cuh"
 #include "kernels.h"
 
@@ -19,10 +20,9 @@ namespace etc {
 
 // silu(gate) * up as the reference's expression interpreter evaluates it, see swiglu_kernel.
 __device__ __forceinline__ float swiglu_value(float g, float up, int exact) {
-  const float half_g = __fdiv_rn(g, 2.0f);
-  const float th = exact ? (float)tanh((double)half_g) : tanhf(half_g);
-  const float sig = __fadd_rn(__fdiv_rn(th, 2.0f), 0.5f);
-  return __fmul_rn(__fmul_rn(g, sig), up);
+  if (!exact) return __fmul_rn(silu_tanh(g), up);
+  const float th = (float)tanh((double)(g * 0.5f));
+  return __fmul_rn(__fmul_rn(g, __fadd_rn(th * 0.5f, 0.5f)), up);
 }
 
 // --------------------------------------------------------------------------------------------
@@ -222,11 +222,6 @@ __device__ __forceinline__ float4 scale4(const float4& v, double scale, const fl
   return make_float4((float)__dmul_rn(__dmul_rn((double)v.x, scale), (double)w.x), (float)__dmul_rn(__dmul_rn((double)v.y, scale), (double)w.y),
                      (float)__dmul_rn(__dmul_rn((double)v.z, scale), (double)w.z), (float)__dmul_rn(__dmul_rn((double)v.w, scale), (double)w.w));
 }
-__device__ __forceinline__ uint2 pack_sat4(const float4& v) {
-  auto sat = [](float f) { return fminf(fmaxf(f, -65504.f), 65504.f); };
-  const __half2 lo = __floats2half2_rn(sat(v.x), sat(v.y)), hi = __floats2half2_rn(sat(v.z), sat(v.w));
-  return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-}
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
@@ -336,7 +331,7 @@ __global__ void __launch_bounds__(kNormThreads) sum_rmsnorm_xh_kernel(float* x, 
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
     const int c = first + kNormCluster * kNormThreads * j;
-    if (c < chunks) *reinterpret_cast<uint2*>(out_xh + hand_off_cell(c >> 1, row, xh_nv, n / 8) + 4 * (c & 1)) = pack_sat4(scale4(v[j], scale, w[j]));
+    if (c < chunks) *reinterpret_cast<uint2*>(out_xh + hand_off_cell(c >> 1, row, xh_nv, n / 8) + 4 * (c & 1)) = pack4(scale4(v[j], scale, w[j]));
   }
 }
 
@@ -385,7 +380,7 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_chunk_xh_kernel(const fl
   for (int j = 0; j < ITEMS; ++j) {
     const int c = threadIdx.x + kNormThreads * j;
     const float4 w = weight && c < chunks ? reinterpret_cast<const float4*>(weight)[c] : make_float4(1.f, 1.f, 1.f, 1.f);
-    const uint2 a = pack_sat4(scale4(v0[j], scale0, w)), b = pack_sat4(scale4(v1[j], scale1, w)), give = odd ? a : b;
+    const uint2 a = pack4(scale4(v0[j], scale0, w)), b = pack4(scale4(v1[j], scale1, w)), give = odd ? a : b;
     const uint2 got = make_uint2(__shfl_xor_sync(0xffffffffu, give.x, 1), __shfl_xor_sync(0xffffffffu, give.y, 1));
     if (c < chunks && (!odd || both))  // n % 8 == 0: both lanes of a pair are inside the row
       *reinterpret_cast<uint4*>(out_xh + hand_off_cell(c >> 1, row0 + odd, 128, n / 8)) =
@@ -614,9 +609,7 @@ cudaError_t launch_embedding_f32(const void* indexes, int index_is_i64, int64_t 
   dim3 grid((unsigned)std::min<int64_t>((columns + 1023) / 1024, 8), (unsigned)count);
   if (index_is_i64)
     return launch_chained(embedding_f32_kernel<long long>, grid, dim3(256), 0, stream, (const long long*)indexes, count, table, rows, columns, out, status);
-  else
-    return launch_chained(embedding_f32_kernel<unsigned int>, grid, dim3(256), 0, stream, (const unsigned int*)indexes, count, table, rows, columns, out, status);
-  return cudaGetLastError();
+  return launch_chained(embedding_f32_kernel<unsigned int>, grid, dim3(256), 0, stream, (const unsigned int*)indexes, count, table, rows, columns, out, status);
 }
 
 // LastTokenRow (crates/runtime-cpu/src/napi/mod.rs:3053-3075) for every lane at once.

@@ -28,7 +28,7 @@ cudaError_t launch_dequantize(int codec, const uint8_t* packed, int64_t rows, in
 cudaError_t launch_quantize(int codec, const float* x, int64_t rows, int64_t columns, uint8_t* packed,
                             cudaStream_t stream);
 cudaError_t launch_qlinear_generic(int codec, const float* x, int64_t vectors, int64_t columns, const uint8_t* weight,
-                                   int64_t rows, const float* bias, float* out, cudaStream_t stream, int* launches, int64_t out_stride = 0);
+                                   int64_t rows, const float* bias, float* out, int sm_count, cudaStream_t stream, int* launches, int64_t out_stride = 0);
 cudaError_t launch_qembedding(int codec, const void* indexes, int index_is_i64, int64_t count, const uint8_t* weight,
                               int64_t rows, int64_t columns, float* out, DeviceStatus* status, cudaStream_t stream);
 
@@ -72,6 +72,9 @@ struct RepackParts {
 };
 cudaError_t launch_repack(const TiledWeight& w, const RepackParts& parts, cudaStream_t stream);
 
+// f32 [vectors, K] to the hand-off layout with row stride nv (16, 32, 64 or 128), absent vectors zero.
+cudaError_t launch_hand_off_convert(const float* x, int64_t vectors, int K, int nv, __half* xh, int sm_count, cudaStream_t stream);
+
 // Sums split-K partials [chunk of vpad vectors][splits][vpad][rows_padded] in split order and runs the epilogue.
 cudaError_t launch_qlinear_reduce(const float* scratch, int splits, int vpad, int vectors, int rows, int rows_padded,
                                   const float* bias, const float* residual, int epilogue, float* out, __half* out_xh, int xh_nv, cudaStream_t stream);
@@ -102,7 +105,6 @@ struct UmmaPlan {
   size_t scratch_bytes = 0;  // split-K partials [chunk][split][nv][rows_padded], all chunks
 };
 UmmaPlan plan_umma(const TiledWeight& w, int64_t vectors, int sm_count);
-cudaError_t launch_repack_umma(const TiledWeight& w, const RepackParts& parts, cudaStream_t stream);
 // x: f32 [vectors, K], converted to f16 in xh first, or xh_ready in the hand-off layout.
 cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, const __half* xh_ready, int64_t vectors, const float* bias,
                                 const float* residual, int epilogue, float* out, __half* out_xh, __half* xh, float* scratch, DeviceStatus* status, int sm_count, cudaStream_t stream,

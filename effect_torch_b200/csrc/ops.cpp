@@ -241,7 +241,7 @@ etc_status etc_qlinear_into(etc_runtime* rt, etc_codec codec, const float* d_x, 
   ETC_TRY(check_codec_geometry("quantized_linear", codec, rows, columns, nullptr));
   if (cancelled && *cancelled) return fail(ETC_CANCELLED, "operation aborted");
   int launches = 0;
-  ETC_CUDA(launch_qlinear_generic(codec, d_x, vectors, columns, (const uint8_t*)d_weight, rows, d_bias, d_out, rt->stream,
+  ETC_CUDA(launch_qlinear_generic(codec, d_x, vectors, columns, (const uint8_t*)d_weight, rows, d_bias, d_out, rt->sm_count, rt->stream,
                                   &launches));
   rt->launches += (uint64_t)launches;
   return ETC_OK;

@@ -38,6 +38,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "activation.cuh"
 #include "chain.cuh"
 #include "dequant.cuh"
 #include "kernels.h"
@@ -108,10 +109,6 @@ struct StreamArgs {
 };
 
 __device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
-__device__ __forceinline__ float sat16(float v) { return fminf(fmaxf(v, -65504.f), 65504.f); }
-__device__ __forceinline__ uint2 pack4(const float4& v) {
-  return make_uint2(h2u(__floats2half2_rn(sat16(v.x), sat16(v.y))), h2u(__floats2half2_rn(sat16(v.z), sat16(v.w))));
-}
 
 // Four consecutive values of an output row: columns c .. c + 3 of vector v, the first `n` of them inside the row.
 __device__ __forceinline__ void store4(const StreamArgs& a, int v, int c, int n, int out_cols, const float4& val) {
@@ -478,22 +475,6 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
   }
 }
 
-// f32 [vectors, K] -> [K/8][NV][8] f16 (rows >= vectors are zero), saturating at the f16 range.
-__global__ void convert_hand_off_kernel(const float* x, int vectors, int K, int nv_shift, __half* xh) {
-  chain_release();
-  chain_wait();
-  const int total = (K / 8) << nv_shift;
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-    const int kg = idx >> nv_shift, n = idx & ((1 << nv_shift) - 1);
-    uint2 lo = make_uint2(0u, 0u), hi = lo;
-    if (n < vectors) {
-      lo = pack4(*reinterpret_cast<const float4*>(x + (size_t)n * K + kg * 8));
-      hi = pack4(*reinterpret_cast<const float4*>(x + (size_t)n * K + kg * 8 + 4));
-    }
-    reinterpret_cast<uint4*>(xh)[idx] = make_uint4(lo.x, lo.y, hi.x, hi.y);
-  }
-}
-
 template <int CODEC, int NV, int USED = NV>
 cudaError_t launch_stream_pass(const StreamArgs& args, int tiles, int splits, cudaStream_t stream) {
   constexpr size_t smem = StreamCfg<CODEC, NV>::kSmemBytes;
@@ -558,8 +539,7 @@ cudaError_t launch_qlinear_stream(const TiledWeight& w, const float* x, const __
   const bool direct = !ready && exact && vectors <= kDirectVectors && (int64_t)plan.tiles * plan.stages <= 64 * (int64_t)sm_count;
   if (!ready && !x) return cudaErrorInvalidValue;
   if (!ready && !direct) {
-    const int total = (K / 8) * plan.nv, shift = plan.nv == 16 ? 4 : plan.nv == 32 ? 5 : (plan.nv == 64 ? 6 : 7);
-    e = launch_chained(convert_hand_off_kernel, dim3((unsigned)std::min((total + 255) / 256, 148 * 4)), dim3(256), 0, stream, x, (int)vectors, K, shift, xh);
+    e = launch_hand_off_convert(x, vectors, K, plan.nv, xh, sm_count, stream);
     if (e != cudaSuccess) return e;
     if (launches) ++*launches;
   }

@@ -24,6 +24,7 @@
 
 #include <algorithm>
 
+#include "activation.cuh"
 #include "chain.cuh"
 #include "codecs.cuh"
 #include "dequant.cuh"
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qlinear_gemm_kernel(GemmArgs 
             const int at = v_base + v0 + v + is_up;
             if (oc >= a.rows / 2 || v + is_up >= left) continue;
             if (a.out) a.out[(size_t)at * (a.rows / 2) + oc] = act;
-            if (a.out_xh) a.out_xh[hand_off_cell(oc >> 3, at, NV, a.rows / 16) + (oc & 7)] = __float2half_rn(fminf(fmaxf(act, -65504.f), 65504.f));
+            if (a.out_xh) a.out_xh[hand_off_cell(oc >> 3, at, NV, a.rows / 16) + (oc & 7)] = half_sat(act);
           }
         } else if (r < a.rows) {
           const size_t at = (size_t)(v_base + v0) * a.rows + r;
@@ -279,31 +280,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qlinear_gemm_kernel(GemmArgs 
   if (warp == kGemmMmaWarp) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
-  }
-}
-
-// f32 [vectors, K] -> xh8 [K/8][NV][8] f16 (rows >= vectors are zero), saturating like the mma.sync path.
-// More than NV vectors: chunk c holds vectors c*NV ... in its own [K/8][NV][8] block.
-__global__ void convert_xh8_kernel(const float* x, int vectors, int K, __half* xh) {
-  constexpr int NV = kGemmVectors;
-  chain_release();
-  chain_wait();
-  const int per_chunk = (K / 8) * NV;
-  const int64_t total = (int64_t)per_chunk * ((vectors + NV - 1) / NV);
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
-    const int chunk = (int)(idx / per_chunk), within = (int)(idx - (int64_t)chunk * per_chunk);
-    const int kg = within / NV, n = chunk * NV + (within - kg * NV);
-    uint4 packed = make_uint4(0u, 0u, 0u, 0u);
-    if (n < vectors) {
-      const float4 lo = *reinterpret_cast<const float4*>(x + (size_t)n * K + kg * 8);
-      const float4 hi = *reinterpret_cast<const float4*>(x + (size_t)n * K + kg * 8 + 4);
-      auto sat = [](float v) { return fminf(fmaxf(v, -65504.f), 65504.f); };
-      packed.x = h2u(__floats2half2_rn(sat(lo.x), sat(lo.y)));
-      packed.y = h2u(__floats2half2_rn(sat(lo.z), sat(lo.w)));
-      packed.z = h2u(__floats2half2_rn(sat(hi.x), sat(hi.y)));
-      packed.w = h2u(__floats2half2_rn(sat(hi.z), sat(hi.w)));
-    }
-    reinterpret_cast<uint4*>(xh)[idx] = packed;
   }
 }
 
@@ -464,7 +440,7 @@ cudaError_t launch_gemm_pass(const GemmArgs& args, int chunks, int splits, cudaS
 
 }  // namespace
 
-cudaError_t launch_repack_umma(const TiledWeight& w, const RepackParts& parts, cudaStream_t stream) {
+cudaError_t launch_repack(const TiledWeight& w, const RepackParts& parts, cudaStream_t stream) {
   const int64_t kblocks = w.columns / 32;
   const int64_t total = w.rows_padded * kblocks;
   if (total == 0) return cudaSuccess;
@@ -497,8 +473,7 @@ cudaError_t launch_qlinear_umma(const TiledWeight& w, const float* x, const __ha
   const int K = (int)w.columns;
   cudaError_t e = cudaSuccess;
   if (!xh_ready) {
-    const int64_t total = (int64_t)(K / 8) * plan.nv * plan.chunks;
-    e = launch_chained(convert_xh8_kernel, dim3((unsigned)std::min<int64_t>((total + 255) / 256, 148 * 8)), dim3(256), 0, stream, x, (int)vectors, K, xh);
+    e = launch_hand_off_convert(x, vectors, K, plan.nv, xh, sm_count, stream);
     if (e != cudaSuccess) return e;
     if (launches) ++*launches;
   }

@@ -9,8 +9,9 @@
 
 #include <algorithm>
 
-#include "codecs.cuh"
+#include "activation.cuh"
 #include "chain.cuh"
+#include "codecs.cuh"
 #include "kernels.h"
 
 namespace etc {
@@ -353,7 +354,7 @@ __global__ void __launch_bounds__(kRawWarps * 32, 2) qlinear_raw_kernel(const fl
 
 template <int CODEC, int VC, int RG>
 cudaError_t launch_qlinear_raw(const float* x, int64_t vectors, int64_t columns, const uint8_t* weight, int64_t rows, const float* bias,
-                               float* out, int64_t out_stride, cudaStream_t stream) {
+                               float* out, int64_t out_stride, int sm_count, cudaStream_t stream) {
   const int windows = (int)((columns + 255) / 256);
   const int chunk = std::min((windows + 3) / 4 * 4, kRawStageBytes / (VC * 4096) * 4);
   const bool wide = kWideBlocks<CODEC> && (reinterpret_cast<uintptr_t>(weight) & 15) == 0;
@@ -361,49 +362,71 @@ cudaError_t launch_qlinear_raw(const float* x, int64_t vectors, int64_t columns,
   const cudaError_t attr = opt_in_shared_memory(kernel, kRawStageBytes);
   if (attr != cudaSuccess) return attr;
   const int64_t groups = (rows + RG - 1) / RG;
-  const unsigned grid = (unsigned)std::min<int64_t>((groups + kRawWarps - 1) / kRawWarps, 148 * 2);
+  const unsigned grid = (unsigned)std::min<int64_t>((groups + kRawWarps - 1) / kRawWarps, 2 * sm_count);
   kernel<<<dim3(grid, (unsigned)((vectors + VC - 1) / VC)), kRawWarps * 32, (size_t)chunk * VC * 1024, stream>>>(x, (int)vectors, columns, weight, rows, bias,
                                                                                                                  out, out_stride, chunk);
   return cudaGetLastError();
 }
-// Rows of a warp: four, unless that leaves warps without any (below 148 SMs x 16 warps x 2).
+// Rows of a warp: four, unless that leaves warps without any (below two rows for each of an SM's 16 warps).
 template <int CODEC, int VC>
 cudaError_t launch_qlinear_raw(const float* x, int64_t vectors, int64_t columns, const uint8_t* weight, int64_t rows, const float* bias,
-                               float* out, int64_t out_stride, cudaStream_t stream) {
-  if (rows > 148 * 32) return launch_qlinear_raw<CODEC, VC, 4>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
-  return launch_qlinear_raw<CODEC, VC, 1>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
+                               float* out, int64_t out_stride, int sm_count, cudaStream_t stream) {
+  if (rows > 32 * (int64_t)sm_count) return launch_qlinear_raw<CODEC, VC, 4>(x, vectors, columns, weight, rows, bias, out, out_stride, sm_count, stream);
+  return launch_qlinear_raw<CODEC, VC, 1>(x, vectors, columns, weight, rows, bias, out, out_stride, sm_count, stream);
 }
 
 struct GenericLaunch {
   const float* x; int64_t vectors, columns; const uint8_t* weight; int64_t rows; const float* bias; float* out; int64_t out_stride;
-  cudaStream_t stream; cudaError_t err; int launches;
+  int sm_count; cudaStream_t stream; cudaError_t err; int launches;
   template <int CODEC> void operator()() {
     err = cudaSuccess;
     if (rows == 0 || vectors == 0) return;
     ++launches;
     // a pass over the weights serves up to 8 vectors; passes of one launch share their rows' bytes in L2
-    if (vectors <= 1) err = launch_qlinear_raw<CODEC, 1>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
-    else if (vectors <= 2) err = launch_qlinear_raw<CODEC, 2>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
-    else if (vectors <= 4) err = launch_qlinear_raw<CODEC, 4>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
-    else if (vectors <= 6) err = launch_qlinear_raw<CODEC, 6>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
-    else err = launch_qlinear_raw<CODEC, 8>(x, vectors, columns, weight, rows, bias, out, out_stride, stream);
+    if (vectors <= 1) err = launch_qlinear_raw<CODEC, 1>(x, vectors, columns, weight, rows, bias, out, out_stride, sm_count, stream);
+    else if (vectors <= 2) err = launch_qlinear_raw<CODEC, 2>(x, vectors, columns, weight, rows, bias, out, out_stride, sm_count, stream);
+    else if (vectors <= 4) err = launch_qlinear_raw<CODEC, 4>(x, vectors, columns, weight, rows, bias, out, out_stride, sm_count, stream);
+    else if (vectors <= 6) err = launch_qlinear_raw<CODEC, 6>(x, vectors, columns, weight, rows, bias, out, out_stride, sm_count, stream);
+    else err = launch_qlinear_raw<CODEC, 8>(x, vectors, columns, weight, rows, bias, out, out_stride, sm_count, stream);
   }
 };
 cudaError_t launch_qlinear_generic(int codec, const float* x, int64_t vectors, int64_t columns, const uint8_t* weight,
-                                   int64_t rows, const float* bias, float* out, cudaStream_t stream, int* launches,
+                                   int64_t rows, const float* bias, float* out, int sm_count, cudaStream_t stream, int* launches,
                                    int64_t out_stride) {
-  GenericLaunch l{x, vectors, columns, weight, rows, bias, out, out_stride ? out_stride : rows, stream, cudaSuccess, 0};
+  GenericLaunch l{x, vectors, columns, weight, rows, bias, out, out_stride ? out_stride : rows, sm_count, stream, cudaSuccess, 0};
   if (!dispatch_codec(codec, l)) return cudaErrorInvalidValue;
   if (launches) *launches += l.launches;
   return l.err;
 }
 
 // ============================================================================================
-// Tiled (128-row) weights: repack front end, split-K sum, dispatch.
+// Tiled (128-row) weights: activations to f16, split-K sum, dispatch.
 // ============================================================================================
-cudaError_t launch_repack(const TiledWeight& w, const RepackParts& parts, cudaStream_t stream) { return launch_repack_umma(w, parts, stream); }
 
-__device__ __forceinline__ float silu_tanh_form(float x) { return x * (tanhf(x * 0.5f) * 0.5f + 0.5f); }
+// f32 [vectors, K] -> the hand-off layout [chunk of nv vectors][K/8][nv][8] f16, absent vectors zero. Cells are counted in 32
+// bits: 2^32 of them would be 137 GB of input.
+__global__ void hand_off_convert_kernel(const float* x, int vectors, int K, int nv_shift, int chunks, __half* xh) {
+  chain_release();
+  chain_wait();
+  const unsigned k8 = K / 8, total = (chunks * k8) << nv_shift;
+  for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    const unsigned column = idx >> nv_shift, chunk = chunks > 1 ? column / k8 : 0u, kg = column - chunk * k8;
+    const int v = (int)((chunk << nv_shift) + (idx & ((1u << nv_shift) - 1)));
+    uint2 lo = make_uint2(0u, 0u), hi = lo;
+    if (v < vectors) {
+      lo = pack4(*reinterpret_cast<const float4*>(x + (size_t)v * K + kg * 8));
+      hi = pack4(*reinterpret_cast<const float4*>(x + (size_t)v * K + kg * 8 + 4));
+    }
+    reinterpret_cast<uint4*>(xh)[idx] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+  }
+}
+cudaError_t launch_hand_off_convert(const float* x, int64_t vectors, int K, int nv, __half* xh, int sm_count, cudaStream_t stream) {
+  int shift = 0;
+  while (1 << shift < nv) ++shift;
+  const int64_t chunks = (vectors + nv - 1) / nv, total = chunks * (K / 8) * nv;
+  return launch_chained(hand_off_convert_kernel, dim3((unsigned)std::min<int64_t>((total + 255) / 256, 8 * sm_count)), dim3(256), 0, stream, x, (int)vectors, K,
+                        shift, (int)chunks, xh);
+}
 
 // Sums the split-K partials [chunk of vpad vectors][split][vpad][rows_padded] in split order and applies bias / epilogue.
 // `residual` and `out` may be the same buffer (the decoder adds projections onto its hidden state in place), so
@@ -426,9 +449,9 @@ __global__ void qlinear_reduce_kernel(const float* scratch, int splits, int vpad
         usum += p[r_up];
       }
       if (bias) { gsum += bias[r_gate]; usum += bias[r_up]; }
-      const float act = silu_tanh_form(gsum) * usum;
+      const float act = silu_tanh(gsum) * usum;
       if (out) out[idx] = act;
-      if (out_xh) out_xh[hand_off_cell(c >> 3, v, xh_nv, out_cols / 8) + (c & 7)] = __float2half_rn(fminf(fmaxf(act, -65504.f), 65504.f));
+      if (out_xh) out_xh[hand_off_cell(c >> 3, v, xh_nv, out_cols / 8) + (c & 7)] = half_sat(act);
     } else {
       float sum = 0.f;
       for (int s = 0; s < splits; ++s) sum += scratch[((size_t)(v / vpad * splits + s) * vpad + v % vpad) * rows_padded + c];

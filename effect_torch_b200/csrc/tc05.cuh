@@ -62,21 +62,6 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0;
 }
 
-// Bounded wait for roles with slack (they run stages ahead, or wait for a whole range): poll, then sleep. A sleeping
-// warp costs the warps that share its scheduler nothing, unlike a spinning or a parked one.
-__device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity, volatile int* abort_flag, unsigned sleep_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long start = clock64();
-  for (unsigned spin = 0; spin < kSpinLimit; ++spin) {
-    __nanosleep(sleep_ns);
-    if (mbar_try_wait(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (clock64() - start > (1ll << 32)) break;
-  }
-  *abort_flag = 1;
-  return false;
-}
-
 __device__ __forceinline__ void bulk_copy_g2s(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(smem_u32(smem_dst)), "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
@@ -159,8 +144,6 @@ __device__ __forceinline__ uint64_t make_b_desc(uint32_t smem_addr, uint32_t lbo
 
 __device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ __half2 u2h(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
-
-__device__ __forceinline__ float silu_tanh(float x) { return x * (tanhf(x * 0.5f) * 0.5f + 0.5f); }
 
 }  // namespace tc05
 }  // namespace etc
