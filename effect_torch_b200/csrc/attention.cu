@@ -916,9 +916,11 @@ AttnPlan plan_attention(int batch, int q_heads, int kv_heads, int head_dim, int 
   const int ctas = std::max(1, batch * kv_heads);
   const int target = std::max(1, sm_count) * 2;
   int splits = std::max(1, target / ctas);
-  // Few sequences of mixed lengths leave the splits beyond the short ones' ends idle: twice as many, where they do not already
-  // follow from filling the SMs once (8 sequences of 512 to 4096 tokens, int8 cache: 30.8 us with 4 splits).
-  if (splits >= 3) splits *= 2;
+  // Two CTAs per SM and no more. Twice as many from three splits on was slower in all of 4 to 8 sequences (8 KV heads of 128,
+  // 512 to 4096 tokens each: f16 4 sequences 12.7 us against 17.1, 8 sequences 21.4 against 26.0, int8 31.9 against 32.7; all
+  // of 2048 tokens: 12.5 against 17.2, 17.3 against 21.5, 20.7 against 23.9). Beyond, lengths decide, which this plan does
+  // not see: 10 and 13 sequences of mixed lengths gain (int8 35.9 against 25.2, 56.0 against 34.8; f16 22.9 against 22.6, 32.9
+  // against 27.8), those of one length lose (24.8 against 28.4, 33.4 against 35.3; 19.8 against 24.2, 23.4 against 28.5).
   // at least 2 pages per warp per split
   splits = std::min(splits, std::max(1, max_pages / (kAttnWarps * 2)));
   p.pages_per_split = std::max(1, (max_pages + splits - 1) / splits);

@@ -117,3 +117,11 @@ def test_every_attention_plan_a_step_can_ask_for_fits_the_decoder_reserve():
     assert et.attention_plan(1, 32, 8, 128, 32)["partial_bytes"] == 66560
     cfg = DecoderConfig(1, 4096, 32, 8, 128, 64, 64, 1e-5, 1e4, 0, -1, 1, 400, 16, et.KV_F16, 0)
     assert et.decoder_attention_reserve(cfg, 1)["partial_bytes"] >= 66560
+
+
+def test_attention_plans_fill_the_device_twice_at_most():
+    for kv_heads in (1, 2, 8):
+        for batch in (1, 2, 4, 8, 12, 13, 18, 19, 64):
+            for pages in (1, 16, 128, 512):
+                plan = et.attention_plan(batch, 4 * kv_heads, kv_heads, 128, pages)
+                assert plan["splits"] == 1 or plan["splits"] * batch * kv_heads <= 2 * 148, (kv_heads, batch, pages)
