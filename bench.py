@@ -320,7 +320,7 @@ def build_decoder(rt, et, torch, model, batch, max_tokens, seed, shared_seed=Non
 def time_linear(rt, et, torch, codec, rows, cols, vectors, interleave=False, epilogue=0, residual=False, target_bytes=300e6, gen=None):
     """One tiled linear shape alone: CUDA events around replays of a graph that walks over more weight copies than L2
     holds. Returns (microseconds per call, algorithmic bytes per call). The call includes the linear's own f16 conversion
-    of the activations and, above 16 vectors, its split-K sum launch."""
+    of the activations (a launch but for up to four rows of the exact form) and, above 128 vectors, its split-K sum launch."""
     # bytes of weights one call streams: the file's encoding for Q4_0 / Q8_0, the re-cut tiled form for the K-quants
     bb = K_TILED_BYTES_PER_32[codec] if codec in K_BLOCK_BYTES else (18 if codec == Q4_0 else 34)
     nparts = 2 if interleave else 1
@@ -750,9 +750,11 @@ def run_gpu_arm(args, rank, world):
         jobs = 1 if tp else world  # replicas each decode their own batch; tensor-parallel ranks share one
         value = jobs * BATCH * K / device_seconds
         e2e_value = jobs * BATCH * K / e2e_seconds
-        max_blocks = max_tokens // BLOCK + 3
-        h2d = BATCH * 4 + BATCH * 16 + BATCH * 8 + BATCH * max_blocks * 4
-        d2h = BATCH * 4 + 32
+        # one copy per step: lane descriptors, ids (room for a chunk per sequence), then the live blocks of every table (mean
+        # over the timed steps); back come the tokens, stored into mapped host memory by the argmax kernel
+        h2d = (BATCH * 16 + BATCH * chunk * 4 + 15) // 16 * 16
+        h2d += BATCH * int(round(np.mean([-(-(PROMPT + W + s) // BLOCK) for s in range(1, K + 1)]) * 4))
+        d2h = BATCH * 4
         line = {
             "metric": METRIC, "value": value, "unit": "tokens/s", "n_gpus": world, "steps": K, "warmup": W,
             "ms_per_step": 1000.0 * device_seconds / K, "higher_is_better": True, "scaling": "strong" if tp else "weak", "vs_baseline": None,
@@ -780,12 +782,12 @@ def run_gpu_arm(args, rank, world):
                                        "for the whole chunk in one launch, tensor-core chunked-prefill attention"}
         if not args.no_kernel_timing:
             us, algorithmic = time_linear(rt, et, torch, Q4_0, 2 * model["ffn"], model["d_model"], BATCH, True, et.EPILOGUE_SWIGLU, False, 264e6)
-            # DRAM bytes per launch of this very kernel and shape, from the committed ncu summary
-            traffic = profile_number("qlinear_umma_q4_0_decode_step.md", "gate_up_dram_bytes_per_launch")
+            # DRAM bytes per launch of this kernel and shape, from the committed ncu summary
+            traffic = profile_number("qlinear_stream_q4_0_decode_step.md", "gate_up_dram_bytes_per_launch")
             line["roofline"] = roofline_entry(
                 us, algorithmic, peaks, peak_kind,
                 f"qlinear_stream_kernel<Q4_0,32> fused gate/up [{2 * model['ffn']}x{model['d_model']}], {BATCH} vectors, with its f16 conversion launch",
-                traffic, "ncu --set full capture of this launch on the 2-layer case, summary under profiles/" if traffic else None)
+                traffic, "ncu capture of the linear in a decode step of the 2-layer case (activations already f16), summary under profiles/" if traffic else None)
             line["roofline_by_projection"] = projection_rooflines(rt, et, torch, model, BATCH, peaks, peak_kind)
             ctx_step = np.full(BATCH, int(mean_ctx))
             pages = int(np.ceil((ctx_step + 1) / BLOCK).sum()) * 6 + 256
