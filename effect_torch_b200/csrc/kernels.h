@@ -32,10 +32,12 @@ cudaError_t launch_qlinear_generic(int codec, const float* x, int64_t vectors, i
 cudaError_t launch_qembedding(int codec, const void* indexes, int index_is_i64, int64_t count, const uint8_t* weight,
                               int64_t rows, int64_t columns, float* out, DeviceStatus* status, cudaStream_t stream);
 
-// Tiled weights (Q4_0 / Q8_0): 128-row tiles. For row tile t and 32-column block kb the 128 rows' 16 (Q4_0) or 32
-// (Q8_0) payload bytes are contiguous ([tile][block][row][bytes]; Q4_0 nibbles pre-ordered so that masks give f16 pairs
-// in column order), scales are [tile][block][row] f16. Same byte count as the GGUF encoding; rows padded to 128 with
-// zero scales. Both linear kernels (qlinear_stream.cu, qlinear_umma.cu) read this one layout.
+// Tiled weights: 128-row tiles, rows padded with zero scales. For row tile t and 32-column block kb the 128 rows' payloads are
+// contiguous ([tile][block][row][bytes]), 16 bytes of 4-bit codes (Q4_0, Q4_K; nibbles pre-ordered so that masks give f16
+// pairs in column order) or 32 bytes of 8-bit ones (Q8_0 and the re-cut Q3_K, Q5_K, Q6_K). Scales are [tile][block][row], one
+// f16 (Q4_0, Q8_0: the byte count of the GGUF encoding) or two (K-quants: scale and minimum, or the scales of the two
+// halves). Both linear kernels (qlinear_stream.cu, qlinear_umma.cu) read this one layout.
+//
 // A run of 128-row tiles of one codec inside a tiled weight. A weight fused from parts of different codecs (q and k in
 // Q4_K, v in Q6_K, as GGUF files mix them) holds one segment per run of equal codecs, each repacked in its codec's layout
 // at byte offsets into the weight's arrays; the linear launches one kernel per segment into the same outputs.

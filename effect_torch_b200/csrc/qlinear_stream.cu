@@ -22,13 +22,14 @@
 // the exchange on [28672 x 4096] and [4096 x 4096]: a fence, an atomic and a chain of L2 round trips.)
 //
 // Roofline: HBM, rows*K/32*{18,34} bytes. Expanding a weight takes about 1.7 instructions, so at 39.5 Q4_0 weights per cycle
-// per SM (the HBM rate) the SM issues 2 of its 4 instructions per cycle. Measured alone at 32 vectors with the conversion of
+// per SM (the HBM rate) the SM would issue 2 of its 4 instructions per cycle for it; with the waits and the epilogue it issues
+// 2.7 at two thirds of that rate ([128256 x 4096], sm__inst_issued). Measured alone at 32 vectors with the conversion of
 // f32 activations, before (register-fed dequant warps, MMAs issued at 131 cycles each) and now: [28672 x 4096] 38.8 -> 23.5
 // us, [4096 x 14336] 21.9 -> 17, [4096 x 4096] 12.4 -> 9.4, [128256 x 4096] 118 -> 73.5 (0.61 of the copy bandwidth; Q8_0
 // 123 -> 101, 0.85). In the form for up to 16 vectors: Q4_0 [28672 x 4096] v8 25.1 -> 20.2 us, [128256 x 4096] v8 74.6 ->
-// 67.4, Q8_0 [28672 x 4096] v16 39.5 -> 26.1 (an mma.sync matvec with tickets between its CTAs before). In the steady state an
-// SM with two CTAs does a stage in 440 cycles (HBM: 415); what is left is the start of a launch (3 us to the first MMA), the
-// uneven last tiles and the epilogue.
+// 67.4, Q8_0 [28672 x 4096] v16 39.5 -> 26.1 (an mma.sync matvec with tickets between its CTAs before). By the slope
+// over K an SM with two CTAs does a stage in 580 cycles at 32 vectors and 473 at 8 (HBM: 410); the rest is the start of a launch
+// (3 us to the first MMA), the uneven last tiles and the epilogue.
 //
 // Every mbarrier wait is bounded: on expiry the abort flag and the status word (3) are raised, all roles run dry, copies
 // in flight are awaited, TMEM is freed.
