@@ -179,9 +179,9 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_kernel(const float* __
 #pragma unroll
   for (int p = 0; p < kQuantPasses; ++p) {
     const int block = p * (kQuantThreads / 4) + (threadIdx.x >> 2);
-    float extreme = v[p][0];
+    float extreme = 0.0f;  // a NaN never takes its place: the block's other values decide
 #pragma unroll
-    for (int i = 1; i < 8; ++i)
+    for (int i = 0; i < 8; ++i)
       if (fabsf(v[p][i]) > fabsf(extreme)) extreme = v[p][i];
 #pragma unroll
     for (int off = 1; off < 4; off <<= 1) {
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_kernel(const float* __
       if (fabsf(o) > fabsf(extreme) || (fabsf(o) == fabsf(extreme) && (part & off))) extreme = o;
     }
     uint32_t code[8], word[2];
-    const float d = CODEC == kQ4_0 ? __fmul_rn(fabsf(extreme) > 0.0f ? extreme : 0.0f, -0.125f)  // exact
+    const float d = CODEC == kQ4_0 ? __fmul_rn(extreme, -0.125f)  // exact
                                    : __fdiv_rn(fabsf(extreme), 127.0f);
     const float inv = d != 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
 #pragma unroll

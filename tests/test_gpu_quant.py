@@ -112,6 +112,25 @@ def test_quantizer_tails(codec, rows, columns):
     np.testing.assert_array_equal(host(packed), orc.quantize(codec, w))
 
 
+@pytest.mark.parametrize("codec", [orc.Q4_0, orc.Q8_0])
+def test_quantizer_of_blocks_with_values_that_are_not_finite(codec):
+    """A NaN takes no part in its block's scale, wherever it stands; an infinity makes the scale infinite."""
+    rng = np.random.default_rng(29)
+    x = rng.normal(size=(40, 32)).astype(np.float32)
+    x[np.arange(32), np.arange(32)] = np.nan
+    x[32, ::8] = np.nan
+    x[33, :31] = np.nan
+    x[34] = np.nan
+    x[35, 5] = np.inf
+    x[36, 30] = -np.inf
+    x[37, 0], x[37, 17] = np.nan, np.inf
+    x[38] = 0.0
+    x[39] = -0.0
+    packed = empty((40, et.encoded_row_bytes(codec, 32)), dtype=torch.uint8)
+    runtime().quantize_into(codec, dev(x), 40, 32, packed)
+    np.testing.assert_array_equal(host(packed), orc.quantize(codec, x).reshape(40, -1))
+
+
 def test_linear_rejects_bad_geometry_and_observes_cancellation():
     rt = runtime()
     x, w, out = empty((1, 256)), empty((1, 144), dtype=torch.uint8), empty((1, 1))
