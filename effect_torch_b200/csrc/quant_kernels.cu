@@ -179,19 +179,27 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_kernel(const float* __
 #pragma unroll
   for (int p = 0; p < kQuantPasses; ++p) {
     const int block = p * (kQuantThreads / 4) + (threadIdx.x >> 2);
-    float extreme = 0.0f;  // a NaN never takes its place: the block's other values decide
+    // the block's value of largest magnitude, for Q8_0 its magnitude; a NaN is never taken
+    float extreme = 0.0f;
+    if (CODEC == kQ8_0) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (fabsf(v[p][i]) > fabsf(extreme)) extreme = v[p][i];
+      for (int i = 0; i < 8; ++i) extreme = fmaxf(extreme, fabsf(v[p][i]));
 #pragma unroll
-    for (int off = 1; off < 4; off <<= 1) {
-      const float o = __shfl_xor_sync(0xffffffffu, extreme, off);
-      // the earlier element wins ties: it sits in the lower lane
-      if (fabsf(o) > fabsf(extreme) || (fabsf(o) == fabsf(extreme) && (part & off))) extreme = o;
+      for (int off = 1; off < 4; off <<= 1) extreme = fmaxf(extreme, __shfl_xor_sync(0xffffffffu, extreme, off));
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (fabsf(v[p][i]) > fabsf(extreme)) extreme = v[p][i];
+#pragma unroll
+      for (int off = 1; off < 4; off <<= 1) {
+        const float o = __shfl_xor_sync(0xffffffffu, extreme, off);
+        // the earlier element wins ties: it sits in the lower lane
+        if (fabsf(o) > fabsf(extreme) || (fabsf(o) == fabsf(extreme) && (part & off))) extreme = o;
+      }
     }
     uint32_t code[8], word[2];
     const float d = CODEC == kQ4_0 ? __fmul_rn(extreme, -0.125f)  // exact
-                                   : __fdiv_rn(fabsf(extreme), 127.0f);
+                                   : __fdiv_rn(extreme, 127.0f);
     const float inv = d != 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
