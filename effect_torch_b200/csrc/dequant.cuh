@@ -26,28 +26,13 @@ struct Ring {
   }
 };
 
-// Splice constants as launch arguments, so that the compiler keeps them in registers: a three-input logic operation or an
-// f16x2 FMA has room for one immediate, and every second one costs an instruction (the ALU pipe, which does the splicing at
-// half rate, was 59 % busy with them, 436 instructions per warp and stage of 128 x 128 weights).
-struct Splice {
-  uint32_t magic = 0x64006400u;      // half2(1024, 1024): a code spliced into the mantissa reads 1024 + code
-  uint32_t mask_lo = 0x000F000Fu, mask_hi = 0x00F000F0u;
-  uint32_t sixteenth = 0x2C002C00u;  // half2(1/16, 1/16)
-  uint32_t bias_lo = 0xE408E408u, bias_hi = 0xD480D480u;      // half2(-1032), half2(-72): Q4_0 codes minus 8
-  uint32_t bias_lo_k = 0xE400E400u, bias_hi_k = 0xD400D400u;  // half2(-1024), half2(-64): unsigned codes
-  uint32_t bias_byte = 0xE480E480u;  // half2(-1152): bytes plus 128
-  uint32_t fill = 0x64646464u, flip = 0x80808080u;
-};
-__device__ __forceinline__ uint32_t and_or(uint32_t x, uint32_t mask, uint32_t fill) {
-  uint32_t d;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(x), "r"(mask), "r"(fill));  // (x & mask) | fill
-  return d;
-}
-__device__ __forceinline__ uint32_t add_h2(uint32_t x, uint32_t y) {
-  uint32_t d;
-  asm("add.f16x2 %0, %1, %2;" : "=r"(d) : "r"(x), "r"(y));
-  return d;
-}
+// Codes in the tiled layout stand where a masked word reads as f16: bits 0 to 10 of a half count in units of 2^-24 whether the
+// half is subnormal or in the first normal binade, so a code at bit p is the f16 number code * 2^(p - 24). One FMA then scales
+// it and subtracts the offset, with the one rounding that scaling the whole-number code has:
+//     weight = code * 2^(p - 24) * (scale * 2^(24 - p)) - offset * scale,
+// in which all products are exact while scale * 2^21 is a finite f16. Larger scales (2^-5 and more) take a second form with
+// the same results. (Splicing codes into the mantissa of 1024, taking 1024 off again and scaling cost 8 FMAs for eight 4-bit
+// codes where this costs 4; a dequant warp had 366 instructions per stage of 128 x 128 weights, now under 300.)
 __device__ __forceinline__ uint32_t mul_h2(uint32_t x, uint32_t y) {
   uint32_t d;
   asm("mul.f16x2 %0, %1, %2;" : "=r"(d) : "r"(x), "r"(y));
@@ -58,69 +43,129 @@ __device__ __forceinline__ uint32_t fma_h2(uint32_t x, uint32_t y, uint32_t z) {
   asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(x), "r"(y), "r"(z));
   return d;
 }
-// One packed word of eight 4-bit codes, logical column j at bit {0,16,8,24,4,20,12,28}[j] -> four half2 in column order,
-// scaled; OFFSET: plus `second`. RAW: the whole-number codes themselves.
-template <bool OFFSET, bool RAW = false>
-__device__ __forceinline__ void splice_nibbles(uint32_t q, uint32_t scale, uint32_t second, const Splice& k, uint32_t* out) {
-  const uint32_t qs = q >> 8;
-  const uint32_t lo = OFFSET ? k.bias_lo_k : k.bias_lo, hi = OFFSET ? k.bias_hi_k : k.bias_hi;
-  const uint32_t c0 = add_h2(and_or(q, k.mask_lo, k.magic), lo), c1 = add_h2(and_or(qs, k.mask_lo, k.magic), lo);
-  const uint32_t c2 = fma_h2(and_or(q, k.mask_hi, k.magic), k.sixteenth, hi), c3 = fma_h2(and_or(qs, k.mask_hi, k.magic), k.sixteenth, hi);
-  if (RAW) { out[0] = c0; out[1] = c1; out[2] = c2; out[3] = c3; return; }
-  out[0] = OFFSET ? fma_h2(c0, scale, second) : mul_h2(c0, scale);
-  out[1] = OFFSET ? fma_h2(c1, scale, second) : mul_h2(c1, scale);
-  out[2] = OFFSET ? fma_h2(c2, scale, second) : mul_h2(c2, scale);
-  out[3] = OFFSET ? fma_h2(c3, scale, second) : mul_h2(c3, scale);
-}
-// One word of four int8 codes -> two half2.
-template <bool OFFSET, bool RAW = false>
-__device__ __forceinline__ void splice_bytes(uint32_t w, uint32_t scale, uint32_t second, const Splice& k, uint32_t* out) {
-  const uint32_t x = w ^ k.flip;
-  const uint32_t c0 = add_h2(__byte_perm(x, k.fill, 0x4140), k.bias_byte), c1 = add_h2(__byte_perm(x, k.fill, 0x4342), k.bias_byte);
-  if (RAW) { out[0] = c0; out[1] = c1; return; }
-  out[0] = OFFSET ? fma_h2(c0, scale, second) : mul_h2(c0, scale);
-  out[1] = OFFSET ? fma_h2(c1, scale, second) : mul_h2(c1, scale);
+
+// Masks of the code pairs in a word and in the word rotated right by 8: 4-bit codes at bits 3 and 7 of a half, bytes at bit 3.
+constexpr uint32_t kCodesLow = 0x00780078u, kCodesHigh = 0x07800780u, kBytes = 0x07F807F8u;
+__device__ __forceinline__ uint32_t rotate8(uint32_t q) { return __funnelshift_r(q, q, 8); }
+
+// Of a codec in the tiled layout: 4-bit codes or bytes, one f16 or two per block, the second a minimum or the second half's
+// scale, and what is taken off a code.
+template <int CODEC>
+struct Coding {
+  static constexpr bool kNibbles = CODEC == 2 || CODEC == 12, kPair = CODEC >= 12, kMinimum = CODEC == 12 || CODEC == 13;
+  static constexpr int kOffset = kMinimum ? 0 : (kNibbles ? 8 : 128);
+};
+
+// The scales of a block at s, each twice in a register.
+template <int CODEC>
+__device__ __forceinline__ void load_scales(const unsigned char* s, uint32_t& scale, uint32_t& second) {
+  const uint32_t raw = Coding<CODEC>::kPair ? *reinterpret_cast<const uint32_t*>(s) : (uint32_t)*reinterpret_cast<const unsigned short*>(s);
+  scale = __byte_perm(raw, raw, 0x1010);
+  second = Coding<CODEC>::kPair ? __byte_perm(raw, raw, 0x3232) : 0u;
 }
 
-// One 32-value block of one row of Q4_0 or Q8_0 in the tiled layout -> 16 half2 of whole-number codes.
+// The magnitude of x or y, whichever is larger (the sign means nothing); a NaN gives way to the other.
+__device__ __forceinline__ uint32_t larger_h2(uint32_t x, uint32_t y) {
+  uint32_t d;
+  asm("max.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(d) : "r"(x), "r"(y));
+  return d;
+}
+// Whether every lane's scales of N blocks are below 2^-5 (or NaN, which both forms carry through).
+template <int CODEC, int N>
+__device__ __forceinline__ bool small_scales(const uint32_t (&scale)[N], const uint32_t (&second)[N]) {
+  uint32_t most = scale[0];
+#pragma unroll
+  for (int b = 1; b < N; ++b) most = larger_h2(most, scale[b]);
+  if (CODEC == 14)
+#pragma unroll
+    for (int b = 0; b < N; ++b) most = larger_h2(most, second[b]);
+  return __all_sync(0xffffffffu, (most & 0x7fffu) < 0x2800u || (most & 0x7fffu) > 0x7c00u);
+}
+
+// What one word's codes need of their scale.
+template <int CODEC, bool LARGE>
+struct Factors {
+  uint32_t scale, low, high, bias;
+  __device__ __forceinline__ Factors(uint32_t s, uint32_t minimum) : scale(s) {
+    if (LARGE) {
+      bias = minimum ^ 0x80008000u;
+    } else {
+      const uint32_t part = mul_h2(s, 0x68006800u);                       // * 2^11
+      low = mul_h2(part, 0x64006400u);                                    // * 2^21
+      high = Coding<CODEC>::kNibbles ? mul_h2(part, 0x54005400u) : 0u;    // * 2^17
+      bias = Coding<CODEC>::kMinimum ? minimum ^ 0x80008000u : mul_h2(s, Coding<CODEC>::kOffset == 8 ? 0xC800C800u : 0xD800D800u);
+    }
+  }
+  // masked codes at bit 3 (HIGH: 7) of each half -> weights
+  template <bool HIGH>
+  __device__ __forceinline__ uint32_t weights(uint32_t codes) const {
+    if (!LARGE) return fma_h2(codes, HIGH ? high : low, bias);
+    // * 2^15 and * 2^6 (2^2): the whole-number code, less its offset
+    constexpr int kOffset = Coding<CODEC>::kOffset;
+    const uint32_t off = kOffset == 0 ? 0u : kOffset == 8 ? (HIGH ? 0xC000C000u : 0xB000B000u) : 0xC000C000u;  // -2, -1/8; -2
+    const uint32_t whole = mul_h2(fma_h2(codes, 0x78007800u, off), HIGH ? 0x44004400u : 0x54005400u);
+    return Coding<CODEC>::kMinimum ? fma_h2(whole, scale, bias) : mul_h2(whole, scale);
+  }
+};
+
+// One 32-value block of one row in the tiled layout (packed words at q) -> 16 half2 in column order.
+template <int CODEC, bool LARGE>
+__device__ __forceinline__ void expand_block(const unsigned char* q, uint32_t scale, uint32_t second, uint32_t (&regs)[16]) {
+  const uint4 a = *reinterpret_cast<const uint4*>(q);
+  const uint32_t lo[4] = {a.x, a.y, a.z, a.w};
+  const Factors<CODEC, LARGE> f(scale, second);
+  if constexpr (Coding<CODEC>::kNibbles) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t r = rotate8(lo[j]);
+      regs[4 * j] = f.template weights<false>(lo[j] & kCodesLow);
+      regs[4 * j + 1] = f.template weights<false>(r & kCodesLow);
+      regs[4 * j + 2] = f.template weights<true>(lo[j] & kCodesHigh);
+      regs[4 * j + 3] = f.template weights<true>(r & kCodesHigh);
+    }
+  } else {
+    const uint4 b = *reinterpret_cast<const uint4*>(q + 16);
+    const uint32_t hi[4] = {b.x, b.y, b.z, b.w};
+    const Factors<CODEC, LARGE> g(CODEC == 14 ? second : scale, second);  // the same as f but for two scales per block
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      regs[2 * j] = f.template weights<false>(lo[j] & kBytes);
+      regs[2 * j + 1] = f.template weights<false>(rotate8(lo[j]) & kBytes);
+      regs[8 + 2 * j] = g.template weights<false>(hi[j] & kBytes);
+      regs[8 + 2 * j + 1] = g.template weights<false>(rotate8(hi[j]) & kBytes);
+    }
+  }
+}
+
+// One block of Q4_0 or Q8_0 -> 16 half2 of whole-number codes / 64, which the block's f32 scale makes up for. (Left at 2^-17
+// the codes would be subnormal, and the tensor core aligns the products of subnormals by their exponent field: three bits of
+// the sum lost.)
+constexpr float kCodeUnits = 64.0f;
 template <int CODEC>
-__device__ __forceinline__ void expand_codes(const unsigned char* q, const Splice& k, uint32_t (&regs)[16]) {
+__device__ __forceinline__ void expand_codes(const unsigned char* q, uint32_t (&regs)[16]) {
   static_assert(CODEC == 2 || CODEC == 8, "one scale per block");
+  constexpr uint32_t kOff = CODEC == 2 ? 0xB000B000u : 0xC000C000u;  // -8 / 64, -128 / 64
   const uint4 a = *reinterpret_cast<const uint4*>(q);
   const uint32_t lo[4] = {a.x, a.y, a.z, a.w};
   if (CODEC == 2) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) splice_nibbles<false, true>(lo[j], 0u, 0u, k, regs + 4 * j);
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t r = rotate8(lo[j]);
+      regs[4 * j] = fma_h2(lo[j] & kCodesLow, 0x78007800u, kOff);  // * 2^15
+      regs[4 * j + 1] = fma_h2(r & kCodesLow, 0x78007800u, kOff);
+      regs[4 * j + 2] = fma_h2(lo[j] & kCodesHigh, 0x68006800u, kOff);  // * 2^11
+      regs[4 * j + 3] = fma_h2(r & kCodesHigh, 0x68006800u, kOff);
+    }
   } else {
     const uint4 b = *reinterpret_cast<const uint4*>(q + 16);
     const uint32_t hi[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) splice_bytes<false, true>(lo[j], 0u, 0u, k, regs + 2 * j);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) splice_bytes<false, true>(hi[j], 0u, 0u, k, regs + 8 + 2 * j);
-  }
-}
-
-// One 32-value block of one row in the tiled layout: packed words at q, block scale(s) at s -> 16 half2, scaled.
-template <int CODEC>
-__device__ __forceinline__ void expand_block(const unsigned char* q, const unsigned char* s, const Splice& k, uint32_t (&regs)[16]) {
-  constexpr bool kPair = CODEC >= 12, kOffset = CODEC == 12 || CODEC == 13;
-  const uint32_t sraw = kPair ? *reinterpret_cast<const uint32_t*>(s) : (uint32_t)*reinterpret_cast<const unsigned short*>(s);
-  const uint32_t scale = __byte_perm(sraw, sraw, 0x1010);
-  // the block's minimum, negated, or the scale of its second half
-  const uint32_t second = kPair ? __byte_perm(sraw, sraw, 0x3232) ^ (kOffset ? 0x80008000u : 0u) : 0u;
-  const uint4 a = *reinterpret_cast<const uint4*>(q);
-  const uint32_t lo[4] = {a.x, a.y, a.z, a.w};
-  if (CODEC == 2 || CODEC == 12) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) splice_nibbles<kOffset>(lo[j], scale, second, k, regs + 4 * j);
-  } else {
-    const uint4 b = *reinterpret_cast<const uint4*>(q + 16);
-    const uint32_t hi[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) splice_bytes<kOffset>(lo[j], scale, second, k, regs + 2 * j);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) splice_bytes<kOffset>(hi[j], CODEC == 14 ? second : scale, second, k, regs + 8 + 2 * j);
+    for (int j = 0; j < 4; ++j) {
+      regs[2 * j] = fma_h2(lo[j] & kBytes, 0x78007800u, kOff);
+      regs[2 * j + 1] = fma_h2(rotate8(lo[j]) & kBytes, 0x78007800u, kOff);
+      regs[8 + 2 * j] = fma_h2(hi[j] & kBytes, 0x78007800u, kOff);
+      regs[8 + 2 * j + 1] = fma_h2(rotate8(hi[j]) & kBytes, 0x78007800u, kOff);
+    }
   }
 }
 

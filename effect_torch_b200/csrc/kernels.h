@@ -33,8 +33,8 @@ cudaError_t launch_qembedding(int codec, const void* indexes, int index_is_i64, 
                               int64_t rows, int64_t columns, float* out, DeviceStatus* status, cudaStream_t stream);
 
 // Tiled weights: 128-row tiles, rows padded with zero scales. For row tile t and 32-column block kb the 128 rows' payloads are
-// contiguous ([tile][block][row][bytes]), 16 bytes of 4-bit codes (Q4_0, Q4_K; nibbles pre-ordered so that masks give f16
-// pairs in column order) or 32 bytes of 8-bit ones (Q8_0 and the re-cut Q3_K, Q5_K, Q6_K). Scales are [tile][block][row], one
+// contiguous ([tile][block][row][bytes]), 16 bytes of 4-bit codes (Q4_0, Q4_K; nibbles placed so that masks give f16
+// pairs in column order, see dequant.cuh) or 32 bytes of 8-bit ones (Q8_0 and the re-cut Q3_K, Q5_K, Q6_K). Scales are [tile][block][row], one
 // f16 (Q4_0, Q8_0: the byte count of the GGUF encoding) or two (K-quants: scale and minimum, or the scales of the two
 // halves). Both linear kernels (qlinear_stream.cu, qlinear_umma.cu) read this one layout.
 //

@@ -21,15 +21,12 @@
 // of (tile, stage) units with the pieces of cut tiles exchanged through memory and a ticket per tile took 10 to 17 us for
 // the exchange on [28672 x 4096] and [4096 x 4096]: a fence, an atomic and a chain of L2 round trips.)
 //
-// Roofline: HBM, rows*K/32*{18,34} bytes. Expanding a weight takes about 1.7 instructions, so at 39.5 Q4_0 weights per cycle
-// per SM (the HBM rate) the SM would issue 2 of its 4 instructions per cycle for it; with the waits and the epilogue it issues
-// 2.7 at two thirds of that rate ([128256 x 4096], sm__inst_issued). Measured alone at 32 vectors with the conversion of
-// f32 activations, before (register-fed dequant warps, MMAs issued at 131 cycles each) and now: [28672 x 4096] 38.8 -> 23.5
-// us, [4096 x 14336] 21.9 -> 17, [4096 x 4096] 12.4 -> 9.4, [128256 x 4096] 118 -> 73.5 (0.61 of the copy bandwidth; Q8_0
-// 123 -> 101, 0.85). In the form for up to 16 vectors: Q4_0 [28672 x 4096] v8 25.1 -> 20.2 us, [128256 x 4096] v8 74.6 ->
-// 67.4, Q8_0 [28672 x 4096] v16 39.5 -> 26.1 (an mma.sync matvec with tickets between its CTAs before). By the slope
-// over K an SM with two CTAs does a stage in 580 cycles at 32 vectors and 473 at 8 (HBM: 410); the rest is the start of a launch
-// (3 us to the first MMA), the uneven last tiles and the epilogue.
+// Roofline: HBM, rows*K/32*{18,34} bytes. A dequant warp has some 240 instructions per stage of 128 x 128 Q4_0 weights (an FMA
+// and a mask per pair, see dequant.cuh); with the loaders and the MMA warp an SM issues 1306 per stage, at 65 % of its slots.
+// [128256 x 4096] x 32, activations ready, with the codes spliced and scaled in two steps and as it is: 547 and 506 cycles per
+// stage (HBM delivers one in 410), 79.1 and 73.3 us; x 64: 90.4 and 85.8; [28672 x 4096] x 32: 26.5 and 24.1. In the form for
+// up to 16 vectors: Q4_0 [128256 x 4096] v8 70.5 us, Q8_0 100.4 (0.88 of the copy bandwidth). The rest is the start of a
+// launch (3 us to the first MMA), the uneven last tiles and the epilogue.
 //
 // Every mbarrier wait is bounded: on expiry the abort flag and the status word (3) are raised, all roles run dry, copies
 // in flight are awaited, TMEM is freed.
@@ -106,7 +103,6 @@ struct StreamArgs {
   int tile0;                    // first tile of this launch in the output (a segment of a weight fused from several codecs)
   int stages, stages_per_split; // of a tile; of a CTA
   int deferred;                 // partial sums only
-  Splice splice;
 };
 
 __device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
@@ -177,7 +173,6 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
     int behind = group - AS;
     const unsigned char* payload = w_ring + row * (Cfg::kBlockQ / kRows);
     const unsigned char* scales = w_ring + Cfg::kStageQ + row * (Cfg::kBlockS / kRows);
-    const Splice splice = a.splice;
     bool ok = true;
     // exact form: the first USED sums of this row, and the block scales of the stage whose products are not added yet
     float sums[Cfg::kExact ? USED : 1], scale[kStageBlocks], next_scale[kStageBlocks];
@@ -195,33 +190,52 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
     constexpr int GROUP = 16 / USED;  // blocks whose products are in registers at a time (all that there is room for)
     const uint32_t my_products = tmem + lane_base + (uint32_t)(group * kStageBlocks * NV);
     for (int i = group; i < n && ok; i += kDequantGroups) {
-      ok = wait_warp(&w_full[w.at], w.parity, abort_flag) && (behind < 0 || wait_warp(&done[freed.at], freed.parity, abort_flag));
+      ok = wait_warp(&w_full[w.at], w.parity, abort_flag);
       if (!ok) break;
-      tc_fence_after();
       const uint32_t stage = (uint32_t)w.at * Cfg::kStageW;
-      // exact form: the products of the stage AS before this one (a whole one), whose slot and accumulators this one takes over
-      uint32_t products[Cfg::kExact ? GROUP : 1][Cfg::kExact ? USED : 1];
+      auto slot_is_free = [&] {
+        ok = behind < 0 || wait_warp(&done[freed.at], freed.parity, abort_flag);
+        if (ok) tc_fence_after();
+        return ok;
+      };
+      const uint32_t slot_cols = a_tmem + lane_base + (uint32_t)(slot.at * kStageBlocks * 16);
+      if constexpr (Cfg::kExact) {
+        if (!slot_is_free()) break;
+        // the products of the stage AS before this one (a whole one), whose slot and accumulators this one takes over
+        uint32_t products[GROUP][USED];
 #pragma unroll
-      for (int b = 0; b < kStageBlocks; ++b) {  // blocks beyond the tile's K hold stale bytes that no MMA reads
-        uint32_t regs[16];
-        if constexpr (Cfg::kExact) {
+        for (int b = 0; b < kStageBlocks; ++b) {  // blocks beyond the tile's K hold stale bytes that no MMA reads
+          uint32_t regs[16];
           if (behind >= 0 && b % GROUP == 0) {
 #pragma unroll
             for (int j = 0; j < GROUP; ++j) load_products(my_products + (uint32_t)((b + j) * NV), products[j]);
           }
-          expand_codes<CODEC>(payload + stage + b * Cfg::kBlockQ, splice, regs);
-          const float block_scale = __half2float(*reinterpret_cast<const __half*>(scales + stage + b * Cfg::kBlockS));
-          tmem_st16(a_tmem + lane_base + (uint32_t)(slot.at * kStageBlocks * 16 + b * 16), regs);
+          expand_codes<CODEC>(payload + stage + b * Cfg::kBlockQ, regs);
+          const float block_scale = __half2float(*reinterpret_cast<const __half*>(scales + stage + b * Cfg::kBlockS)) * kCodeUnits;
+          tmem_st16(slot_cols + b * 16, regs);
           if (behind >= 0 && b % GROUP == GROUP - 1) {
             tmem_wait_ld();
 #pragma unroll
             for (int j = 0; j < GROUP; ++j) add_block(products[j], scale[b - GROUP + 1 + j]);
           }
           next_scale[b] = block_scale;
-        } else {
-          expand_block<CODEC>(payload + stage + b * Cfg::kBlockQ, scales + stage + b * Cfg::kBlockS, splice, regs);
-          tmem_st16(a_tmem + lane_base + (uint32_t)(slot.at * kStageBlocks * 16 + b * 16), regs);
         }
+      } else {
+        uint32_t first[kStageBlocks], second[kStageBlocks];
+#pragma unroll
+        for (int b = 0; b < kStageBlocks; ++b) load_scales<CODEC>(scales + stage + b * Cfg::kBlockS, first[b], second[b]);
+        auto expand = [&](auto large) {
+#pragma unroll
+          for (int b = 0; b < kStageBlocks; ++b) {
+            uint32_t regs[16];
+            expand_block<CODEC, decltype(large)::value>(payload + stage + b * Cfg::kBlockQ, first[b], second[b], regs);
+            if (b == 0 && !slot_is_free()) return;
+            tmem_st16(slot_cols + b * 16, regs);
+          }
+        };
+        if (small_scales<CODEC>(first, second)) expand(std::false_type());
+        else expand(std::true_type());
+        if (!ok) break;
       }
       if (Cfg::kExact) {
 #pragma unroll

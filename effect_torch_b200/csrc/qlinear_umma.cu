@@ -23,6 +23,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "activation.cuh"
 #include "chain.cuh"
@@ -75,7 +76,6 @@ struct GemmArgs {
   int vectors, rows, rows_padded, kblocks, epilogue;
   int tiles, tile0;             // of this launch (a segment of a weight fused from several codecs), and its first in the output
   int stages, stages_per_split;
-  Splice splice;
 };
 
 template <int CODEC>
@@ -118,7 +118,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qlinear_gemm_kernel(GemmArgs 
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const unsigned char* payload = w_ring + mine * Cfg::kTileW + row * (Cfg::kBlockQ / kUmmaRows);
     const unsigned char* scales = w_ring + mine * Cfg::kTileW + Cfg::kTileQ + row * (Cfg::kBlockS / kUmmaRows);
-    const Splice splice = a.splice;
     {
       Ring<WS> w;
       Ring<AS> slot;
@@ -131,13 +130,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1) qlinear_gemm_kernel(GemmArgs 
         tc_fence_after();
         if (mine < live_tiles) {
           const uint32_t stage = (uint32_t)w.at * Cfg::kStageW;
+          constexpr int kMine = kStageBlocks / 2;  // blocks beyond the weight's K hold stale bytes that no MMA reads
+          const unsigned char* q = payload + stage + half * kMine * Cfg::kBlockQ;
+          const uint32_t cols = a_tmem + lane_base + (uint32_t)((slot.at * kGemmTiles + mine) * kStageBlocks * 16 + half * kMine * 16);
+          uint32_t first[kMine], second[kMine];
 #pragma unroll
-          for (int j = 0; j < kStageBlocks / 2; ++j) {  // blocks beyond the weight's K hold stale bytes that no MMA reads
-            const int b = half * (kStageBlocks / 2) + j;
-            uint32_t regs[16];
-            expand_block<CODEC>(payload + stage + b * Cfg::kBlockQ, scales + stage + b * Cfg::kBlockS, splice, regs);
-            tmem_st16(a_tmem + lane_base + (uint32_t)((slot.at * kGemmTiles + mine) * kStageBlocks * 16 + b * 16), regs);
-          }
+          for (int b = 0; b < kMine; ++b) load_scales<CODEC>(scales + stage + (half * kMine + b) * Cfg::kBlockS, first[b], second[b]);
+          auto expand = [&](auto large) {
+#pragma unroll
+            for (int b = 0; b < kMine; ++b) {
+              uint32_t regs[16];
+              expand_block<CODEC, decltype(large)::value>(q + b * Cfg::kBlockQ, first[b], second[b], regs);
+              tmem_st16(cols + b * 16, regs);
+            }
+          };
+          if (small_scales<CODEC>(first, second)) expand(std::false_type());
+          else expand(std::true_type());
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&w_empty[w.at]);
@@ -311,8 +319,11 @@ __global__ void repack_umma_kernel(RepackParts parts, int codec, int64_t rows, i
     const int64_t tile = r / kUmmaRows, row = r % kUmmaRows;
     uint32_t* dst = quants + ((tile * kblocks + kb) * kUmmaRows + row) * words;
     __half scale = __float2half_rn(0.0f), second = __float2half_rn(0.0f);
+    const int pos[8] = {0, 16, 8, 24, 4, 20, 12, 28}, byte_pos[4] = {0, 16, 8, 24};
+    // the positions that dequant.cuh reads: every word three bits up, signed bytes plus 128
+    auto place = [](uint32_t word) { return __funnelshift_l(word, word, 3); };
     if (!src_row) {
-      for (int w = 0; w < words; ++w) dst[w] = codec == 2 ? 0x88888888u : 0u;
+      for (int w = 0; w < words; ++w) dst[w] = 0u;  // the scales are 0
     } else if (codec == 12) {
       // Q4_K (crates/runtime-cpu/src/quantized.rs:180-199): sub-block `sub` of the 256-value block, value = d*sc*code - dmin*m
       const uint8_t* blk = src_row + (kb >> 3) * bb;
@@ -321,14 +332,13 @@ __global__ void repack_umma_kernel(RepackParts parts, int codec, int64_t rows, i
       scale_min_k4(sub, blk + 4, sc, mn);
       scale = __float2half_rn(__fmul_rn(fp16_at(blk, 0), (float)sc));
       second = __float2half_rn(__fmul_rn(fp16_at(blk, 2), (float)mn));
-      const int pos[8] = {0, 16, 8, 24, 4, 20, 12, 28};
       for (int w = 0; w < 4; ++w) {
         uint32_t word = 0;
         for (int j = 0; j < 8; ++j) {
           const int raw = blk[16 + (sub >> 1) * 32 + 8 * w + j];
           word |= (uint32_t)((sub & 1) ? (raw >> 4) : (raw & 0x0f)) << pos[j];
         }
-        dst[w] = word;
+        dst[w] = place(word);
       }
     } else if (codec == 11) {
       // Q3_K (quantized.rs:142-176): block `sub` of the 256-value block is groups 2*sub and 2*sub+1 of 16 values,
@@ -351,9 +361,9 @@ __global__ void repack_umma_kernel(RepackParts parts, int codec, int64_t rows, i
         for (int j = 0; j < 4; ++j) {
           const int v = 4 * w + j;
           const int code = ((blk[32 + half * 32 + v] >> (2 * lane)) & 3) - ((blk[v] & mask) == 0 ? 4 : 0);
-          word |= (uint32_t)(code & 0xff) << (8 * j);
+          word |= (uint32_t)(code + 128) << byte_pos[j];
         }
-        dst[w] = word;
+        dst[w] = place(word);
       }
     } else if (codec == 13) {
       // Q5_K (quantized.rs:203-234): sub-block `sub`, value = d*sc*code - dmin*m with a 5-bit code (low nibble + one high
@@ -371,9 +381,9 @@ __global__ void repack_umma_kernel(RepackParts parts, int codec, int64_t rows, i
         for (int j = 0; j < 4; ++j) {
           const int v = 4 * w + j;
           const int code = ((sub & 1) ? (ql[v] >> 4) : (ql[v] & 0x0f)) + ((blk[16 + v] & mask) == 0 ? 0 : 16);
-          word |= (uint32_t)code << (8 * j);
+          word |= (uint32_t)code << byte_pos[j];
         }
-        dst[w] = word;
+        dst[w] = place(word);
       }
     } else if (codec == 14) {
       // Q6_K (quantized.rs:238-261): values 32*sub .. 32*sub+31 of the 256-value block, value = d*scale*(code - 32) with one
@@ -393,29 +403,28 @@ __global__ void repack_umma_kernel(RepackParts parts, int codec, int64_t rows, i
           const int low = (quarter & 1) ? ql[index + 32] : ql[index];
           const int low4 = (quarter & 2) ? (low >> 4) : (low & 0x0f);
           const int code = (low4 | (((qh[index] >> (2 * quarter)) & 3) << 4)) - 32;
-          word |= (uint32_t)(code & 0xff) << (8 * j);
+          word |= (uint32_t)(code + 128) << byte_pos[j];
         }
-        dst[w] = word;
+        dst[w] = place(word);
       }
     } else {
       const uint8_t* blk = src_row + kb * bb;
       scale = __ushort_as_half((unsigned short)(blk[0] | (blk[1] << 8)));
       if (codec == 2) {
-        const int pos[8] = {0, 16, 8, 24, 4, 20, 12, 28};
-        for (int w = 0; w < 4; ++w) {
+          for (int w = 0; w < 4; ++w) {
           uint32_t word = 0;
           for (int j = 0; j < 8; ++j) {
             const int i = 8 * w + j;
             const uint32_t code = i < 16 ? (blk[2 + i] & 0x0fu) : (uint32_t)(blk[2 + i - 16] >> 4);
             word |= code << pos[j];
           }
-          dst[w] = word;
+          dst[w] = place(word);
         }
       } else {
         for (int w = 0; w < 8; ++w) {
           uint32_t word = 0;
-          for (int j = 0; j < 4; ++j) word |= (uint32_t)blk[2 + 4 * w + j] << (8 * j);
-          dst[w] = word;
+          for (int j = 0; j < 4; ++j) word |= (uint32_t)(blk[2 + 4 * w + j] ^ 0x80u) << byte_pos[j];
+          dst[w] = place(word);
         }
       }
     }

@@ -183,6 +183,33 @@ def test_tiling_preserves_every_weight(codec):
 
 
 @pytest.mark.parametrize("codec", [gv.Q4_0, gv.Q8_0])
+@pytest.mark.parametrize("vectors", [32, 128, 200])
+def test_expansion_is_exact_for_every_code_and_scale(codec, vectors):
+    """Both forms of the expansion to f16 (block scales below and from 2^-5 on) give each weight scale * code rounded once to
+    f16: all codes under scales at the line between the forms, subnormal, tiny, large and of either sign. x picks out single
+    weights, whose f32 sums with zeros are exact."""
+    columns, bb = 128, orc.block_bytes(codec)
+    line = 2.0 ** -5
+    scales = np.array([line, np.nextafter(np.float16(line), np.float16(0)), line * 1.5, 0.006, 6e-8, 6.1e-5, 0.0, 1.0, 200.0], np.float16)
+    scales = np.concatenate([scales, -scales])
+    rng = np.random.default_rng(5)
+    rows = 8 * len(scales)
+    raw = rng.integers(0, 256, size=(rows, columns // 32, bb), dtype=np.uint8)
+    # most rows hold one scale (whole warps take one form), the last ones a mix
+    raw[:, :, 0:2] = np.repeat(scales, 8)[:, None, None].view(np.uint8).reshape(rows, 1, 2)
+    raw[-40:, :, 0:2] = rng.choice(scales, size=(40, columns // 32, 1)).view(np.uint8)
+    packed = raw.reshape(rows, -1)
+    expected = orc.dequantize(codec, packed, rows, columns).astype(np.float16).astype(np.float32)
+    qw = et.QWeight(runtime(), codec, [dev(packed)], [rows], columns)
+    x = np.zeros((vectors, columns), np.float32)
+    x[np.arange(min(vectors, columns)), np.arange(min(vectors, columns))] = 1.0
+    out = empty((vectors, rows))
+    qw.linear_into(dev(x), vectors, out)
+    n = min(vectors, columns)
+    np.testing.assert_array_equal(host(out)[:n].T, expected[:, :n])
+
+
+@pytest.mark.parametrize("codec", [gv.Q4_0, gv.Q8_0])
 @pytest.mark.parametrize("rows,columns", [(256, 512), (200, 1024), (1024, 4096)])
 @pytest.mark.parametrize("vectors", [1, 5, 8, 9, 16, 32, 40, 64, 100, 300])
 def test_tiled_linear_matches_the_oracle(codec, rows, columns, vectors):
