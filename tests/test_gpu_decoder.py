@@ -499,6 +499,59 @@ def test_chunks_at_the_edges_of_the_attention_tiles(q_heads, kv_heads, head_dim,
         assert helpers.rel_err(gl, ol) <= 2 * tol, f"advance {advance}"
 
 
+def test_steps_of_wide_q8_0_layers_repeat_bit_for_bit():
+    """A stage's block scales are used a round after its buffer is handed back to the loader: a load that came back late
+    took the next round's scales (a wrong step in some fifty of this shape). 120 runs of three steps, all alike; the first
+    run, whose split plan is another, does not count."""
+    d, ffn, vocab, B, context = 4096, 14336, 16000, 8, 48
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(3)
+    max_tokens = B * (context + 32)
+    dec = et.Executable(runtime(), layers=2, d_model=d, q_heads=32, kv_heads=8, head_dim=128, ffn=ffn, vocab=vocab, rms_eps=1e-5, rope_theta=500000.0,
+                        batch=B, max_tokens=max_tokens, block_size=16, kv_dtype=et.KV_F16, exact=False, max_advance=context)
+    dec.set_weight(et.W_TOK_EMBD, 0, torch.randn((vocab, d), generator=gen, device="cuda").mul_(0.02))
+    ones = torch.ones(d, device="cuda")
+    dec.set_weight(et.W_OUT_NORM, 0, ones)
+
+    def put(slot, layer, rows, columns):
+        packed = torch.randint(0, 256, (rows, columns // 32, 34), generator=gen, device="cuda", dtype=torch.uint8)
+        packed[:, :, :2] = torch.rand((rows, columns // 32, 1), generator=gen, device="cuda").mul_(3e-4).half().view(torch.uint8)
+        torch.cuda.synchronize()
+        dec.set_weight(slot, layer, packed.view(rows, -1), codec=et.Q8_0, rows=rows, columns=columns)
+
+    for layer in range(2):
+        dec.set_weight(et.W_ATTN_NORM, layer, ones)
+        dec.set_weight(et.W_FFN_NORM, layer, ones)
+        for slot, rows, columns in ((et.W_Q, 4096, d), (et.W_K, 1024, d), (et.W_V, 1024, d), (et.W_O, d, 4096), (et.W_GATE, ffn, d), (et.W_UP, ffn, d),
+                                    (et.W_DOWN, d, ffn)):
+            put(slot, layer, rows, columns)
+    put(et.W_HEAD, 0, vocab, d)
+    dec.finalize()
+    pool = et.NativeKvPool(runtime(), 2, 8, 128, max_tokens, 16, et.KV_F16)
+    rng = np.random.default_rng(4)
+    prompts = rng.integers(0, vocab, size=(B, context + 1)).astype(np.uint32)
+    feed = rng.integers(0, vocab, size=(3, B, 1)).astype(np.uint32)
+    seqs = [pool.makeSequence() for _ in range(B)]
+    dec.execute(pool, seqs, prompts[:, :context])
+    for seq in seqs:
+        seq.release()
+
+    def run():
+        seqs = [pool.makeSequence() for _ in range(B)]
+        for seq, prompt in zip(seqs, prompts):
+            seq.prefillMatch(prompt)
+        out = [np.array(dec.execute(pool, seqs, tokens)) for tokens in feed]
+        for seq in seqs:
+            seq.release()
+        return out
+
+    run()
+    expected = run()
+    for i in range(120):
+        for step, (got, want) in enumerate(zip(run(), expected)):
+            assert np.array_equal(got, want), f"run {i}, step {step}: {(got != want).sum()} logits differ"
+
+
 @pytest.mark.parametrize("d_model", [1088, 4160, 8192])
 def test_norms_at_the_edges_of_their_row_widths(d_model):
     """Residual widths that end inside a cluster's share, just above the width of the narrower form and at the limit, for
