@@ -268,6 +268,12 @@ cudaError_t launch_attention_exact(const PoolView& pool, const float* q, const L
 // the 4 warps merge their (m, l, O) through shared memory. With splits > 1 the CTA writes an
 // unnormalised partial (m, l, O) per query head and attention_merge_kernel combines the splits.
 //
+// FUSED (the decoder's one-token steps): the CTA also does what rope_append_kernel does for its heads. It adds up the fused
+// q/k/v projection's split-K partials of its G query heads (every split of a lane does, they are a few KB from L2), rotates
+// them, and the CTA whose range holds the new token's page rotates and stores the new K and V rows. Cached rows, lanes and
+// tables were written before this step, so all pages but the new token's, and the angles, are on their way before the wait for
+// the projection. One launch and its chain of L2 round trips less per layer (RoPE alone took 3.6 us of a 65 us layer).
+//
 // Roofline: HBM-bound: bytes = sum_lanes ctx * 2 * kv_heads * D * sizeof(kv) (+ q, out, tables).
 // --------------------------------------------------------------------------------------------
 constexpr int kAttnWarps = 4;
@@ -333,6 +339,15 @@ struct AttnArgs {
   float scale_log2;        // scale * log2(e)
   long long op_window;
 };
+// fused RoPE and append: the projection's rows [B, q heads | k heads | v heads, D] (or their split-K partials)
+struct FusedAttnArgs : AttnArgs {
+  const float* qkv;
+  DeferredSum sum;
+  const double* inv_freq;
+  int rope_layout;
+  void *slab[2];           // K and V again, to store the new rows
+  float *slab_scale[2];
+};
 
 // smem per warp per stage: K page then V page, each 16 rows x D*2 bytes, 16-byte chunk c of row r
 // stored at chunk (c ^ (r & 7)) within its 128-byte group.
@@ -341,33 +356,42 @@ __device__ __forceinline__ int swizzled_offset(int row, int chunk) {  // in byte
   return row * (D * 2) + ((chunk & ~7) | ((chunk ^ row) & 7)) * 16;
 }
 
+// The same for a page of code bytes: rows of D bytes, conflict free for ldmatrix over eight rows.
+template <int D>
+__device__ __forceinline__ int swizzled_bytes(int row, int chunk) {
+  return row * D + (chunk ^ (D == 128 ? row & 7 : (row >> 1) & 3)) * 16;
+}
+
 // Four bytes b0..b3 -> halves 1024 + b, minus 1152 = b - 128 (exact).
+template <unsigned LO = 0x4140, unsigned HI = 0x4342>  // which two bytes go into lo, and into hi
 __device__ __forceinline__ void bytes_to_half2(uint32_t w, uint32_t& lo, uint32_t& hi) {
   const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);
-  uint32_t lo_bits = __byte_perm(w, 0x64646464u, 0x4140), hi_bits = __byte_perm(w, 0x64646464u, 0x4342);
+  uint32_t lo_bits = __byte_perm(w, 0x64646464u, LO), hi_bits = __byte_perm(w, 0x64646464u, HI);
   const __half2 l = __hsub2(*reinterpret_cast<__half2*>(&lo_bits), bias), h = __hsub2(*reinterpret_cast<__half2*>(&hi_bits), bias);
   lo = *reinterpret_cast<const uint32_t*>(&l);
   hi = *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// U8: the int8 tier (code - 128) * scale with one scale per cached row (napi/mod.rs:3474-3476): pages travel as bytes, a warp
-// widens the page it is about to use to f16 integers in a staging page of its own, and the row scales multiply the score
-// columns (K) and the probabilities before P V (V), so the tensor core only ever sees exact small integers.
-template <int D, bool BF16, bool U8>
-__global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs a) {
+// U8: the int8 tier (code - 128) * scale with one scale per cached row (napi/mod.rs:3474-3476): pages travel as bytes, and the
+// row scales multiply the score columns (K) and the probabilities before P V (V), so the tensor core only ever sees exact small
+// integers. ldmatrix hands a thread four code bytes at a time, which it widens to two f16 pairs in registers: of K the columns
+// 4 t .. 4 t + 3 of a row, which become the operand's columns 2 t, 2 t + 1, 2 t + 8 and 2 t + 9 (the query fragments are
+// permuted alike, inside each sum of 16); of V, transposed, two columns of two rows, which go to two neighbouring output tiles
+// (columns 2 n and 2 n + 1 of every 16).
+template <int D, bool BF16, bool U8, bool FUSED>
+__global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(std::conditional_t<FUSED, FusedAttnArgs, AttnArgs> a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  constexpr int PAGE_BYTES = kPageTokens * D * 2;               // one page as MMA operands (f16 / bf16)
-  constexpr int RAW_PAGE = U8 ? kPageTokens * D : PAGE_BYTES;   // one page as cached
+  constexpr int RAW_PAGE = kPageTokens * D * (U8 ? 1 : 2);      // one page as cached
   constexpr int SCALE_BYTES = U8 ? kPageTokens * 4 : 0;         // its row scales
   constexpr int STAGE_BYTES = 2 * (RAW_PAGE + SCALE_BYTES);
-  constexpr int WARP_BYTES = kAttnStages * STAGE_BYTES + (U8 ? 2 * PAGE_BYTES : 0);  // ring (+ the widened K and V page)
+  constexpr int WARP_BYTES = kAttnStages * STAGE_BYTES;         // a warp's ring
   constexpr int CHUNKS = D / 8;    // 16-byte chunks per row
   constexpr int KSTEPS = D / 16;   // k16 steps of the QK^T product
   constexpr int DTILES = D / 8;    // n-tiles of the PV product
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
-  chain_wait();
+  if (!FUSED) chain_wait();
   const int split = blockIdx.x, kv_head = blockIdx.y, lane_id = blockIdx.z;
   const LaneInfo info = a.lanes[lane_id];
   const int G = a.q_heads / a.kv_heads;
@@ -381,26 +405,26 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs
   const int last_page = idle_lane ? first_page : (end - 1) / kPageTokens + 1;  // exclusive
   const int p0 = first_page + split * a.pages_per_split;
   const int p1 = min(last_page, p0 + a.pages_per_split);
+  const int new_page = last_page - 1;  // FUSED: of the token that this step appends, the last page of the warp that has it
 
   unsigned char* my_smem = smem + (size_t)warp * WARP_BYTES;
-  unsigned char* wide = my_smem + kAttnStages * STAGE_BYTES;  // U8: this warp's widened K page, then V page
   const int* table = a.tables + info.table_offset;
   const size_t page_stride = (size_t)a.kv_heads * RAW_PAGE;  // bytes between consecutive pages
   const unsigned char* kbase = reinterpret_cast<const unsigned char*>(a.k) + (size_t)kv_head * RAW_PAGE;
   const unsigned char* vbase = reinterpret_cast<const unsigned char*>(a.v) + (size_t)kv_head * RAW_PAGE;
 
-  auto issue = [&](int page_index, int stage) {
-    if (page_index < p1) {
+  auto issue = [&](int page_index, int stage, bool but_new = false) {
+    if (page_index < p1 && !(FUSED && but_new && page_index == new_page)) {
       const size_t off = (size_t)table[page_index] * page_stride;
       unsigned char* ks = my_smem + stage * STAGE_BYTES;
       unsigned char* vs = ks + RAW_PAGE;
       if (U8) {
-        // bytes as they are (row-major), then the 16 row scales of K and of V
+        // the bytes, then the 16 row scales of K and of V
 #pragma unroll
         for (int i = 0; i < RAW_PAGE / 16 / 32; ++i) {
-          const int c = lane + 32 * i;
-          cp_async16(ks + c * 16, kbase + off + (size_t)c * 16);
-          cp_async16(vs + c * 16, vbase + off + (size_t)c * 16);
+          const int c = lane + 32 * i, so = swizzled_bytes<D>(c / (D / 16), c % (D / 16));
+          cp_async16(ks + so, kbase + off + (size_t)c * 16);
+          cp_async16(vs + so, vbase + off + (size_t)c * 16);
         }
         if (lane < 8) {
           const size_t si = ((size_t)table[page_index] * a.kv_heads + kv_head) * kPageTokens;  // 16 floats = 4 chunks each
@@ -420,48 +444,127 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs
     }
     cp_async_commit();  // always commit so group counting stays uniform
   };
-  // U8: bytes of one cached page -> f16 integers (code - 128) in the swizzled operand layout
-  auto widen = [&](const unsigned char* raw, unsigned char* dst) {
-#pragma unroll
-    for (int i = 0; i < RAW_PAGE / 16 / 32; ++i) {
-      const int c = lane + 32 * i;  // 16 codes: row c / (D/16), columns 16 * (c % (D/16)) ...
-      const int row = c / (D / 16), chunk = 2 * (c % (D / 16));
-      const uint4 codes = *reinterpret_cast<const uint4*>(raw + c * 16);
-      const uint32_t w[4] = {codes.x, codes.y, codes.z, codes.w};
-      uint32_t h[8];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bytes_to_half2(w[j], h[2 * j], h[2 * j + 1]);
-      *reinterpret_cast<uint4*>(dst + swizzled_offset<D>(row, chunk)) = make_uint4(h[0], h[1], h[2], h[3]);
-      *reinterpret_cast<uint4*>(dst + swizzled_offset<D>(row, chunk + 1)) = make_uint4(h[4], h[5], h[6], h[7]);
-    }
-  };
-
   // this warp's pages: p0 + warp, p0 + warp + 4, ...; the first copies are in flight while the query rows are fetched
   int next_issue = p0 + warp;
 #pragma unroll
   for (int s = 0; s < kAttnStages - 1; ++s) {
-    issue(next_issue, s);
+    issue(next_issue, s, true);
     next_issue += kAttnWarps;
+  }
+
+  // fused: query rows 0..G-1 of this KV head, [G][D] f32, in a ring stage that the loop fills last
+  // (U8: behind the rings)
+  float* q_rows = reinterpret_cast<float*>(smem + (U8 ? kAttnWarps * WARP_BYTES : (kAttnStages - 1) * STAGE_BYTES));
+  if constexpr (FUSED) {
+    constexpr int HALF = D / 2, STEP = kAttnWarps * 32 / HALF, ITEMS = 3, IN_FLIGHT = 8;
+    __shared__ double2 angle[HALF];  // (sine, cosine) per pair
+    __shared__ float fresh[2][D];    // the new K row, the new V row
+    const int j = threadIdx.x % HALF, h0 = threadIdx.x / HALF;
+    const bool works = p0 < p1, appends = works && new_page < p1;
+    if (works && h0 == 0) {
+      double sine, cosine;
+      sincos((double)info.cursor * a.inv_freq[j], &sine, &cosine);
+      angle[j] = make_double2(sine, cosine);
+    }
+    chain_wait();
+    if (works) {  // the same for the whole CTA
+      const int i0 = a.rope_layout == 0 ? j : 2 * j, i1 = a.rope_layout == 0 ? HALF + j : 2 * j + 1;
+      const int heads = a.q_heads + 2 * a.kv_heads, mine = appends ? G + 2 : G;
+      auto head_of = [&](int h) { return h < G ? kv_head * G + h : a.q_heads + (h - G) * a.kv_heads + kv_head; };
+      const size_t split_stride = (size_t)a.sum.vpad * a.sum.rows_padded;
+      const int splits = max(a.sum.splits, 1);  // one "split": the finished rows
+      const float* rows = a.sum.splits > 0 ? a.sum.partials + (size_t)lane_id * a.sum.rows_padded : a.qkv + (size_t)lane_id * heads * D;
+      __syncthreads();  // the angles
+      const double sine = angle[j].x, cosine = angle[j].y;
+      for (int hb = h0; hb < mine; hb += STEP * ITEMS) {
+        float x0[ITEMS], x1[ITEMS];
+#pragma unroll
+        for (int u = 0; u < ITEMS; ++u) x0[u] = x1[u] = 0.0f;
+        for (int s0 = 0; s0 < splits; s0 += IN_FLIGHT) {
+          float part0[ITEMS][IN_FLIGHT], part1[ITEMS][IN_FLIGHT];
+#pragma unroll
+          for (int u = 0; u < ITEMS; ++u)
+#pragma unroll
+            for (int t = 0; t < IN_FLIGHT; ++t)
+              if (hb + u * STEP < mine && s0 + t < splits) {
+                const float* src = rows + (size_t)(s0 + t) * split_stride + (size_t)head_of(hb + u * STEP) * D;
+                part0[u][t] = src[i0];
+                part1[u][t] = src[i1];
+              }
+#pragma unroll
+          for (int u = 0; u < ITEMS; ++u)
+#pragma unroll
+            for (int t = 0; t < IN_FLIGHT; ++t)
+              if (hb + u * STEP < mine && s0 + t < splits) {
+                x0[u] += part0[u][t];
+                x1[u] += part1[u][t];
+              }
+        }
+#pragma unroll
+        for (int u = 0; u < ITEMS; ++u) {
+          const int h = hb + u * STEP;
+          if (h >= mine) break;
+          float r0 = x0[u], r1 = x1[u];
+          if (h <= G) {  // not the value row
+            const double first = (double)r0, second = (double)r1;
+            r0 = (float)__dsub_rn(__dmul_rn(first, cosine), __dmul_rn(second, sine));
+            r1 = (float)__dadd_rn(__dmul_rn(second, cosine), __dmul_rn(first, sine));
+          }
+          float* dst = h < G ? q_rows + h * D : fresh[h - G];
+          dst[i0] = r0;
+          dst[i1] = r1;
+        }
+      }
+      __syncthreads();  // the rows
+      if (appends && warp < 2) {  // warp 0 stores K, warp 1 V
+        const int slot = info.cursor % kPageTokens;
+        const size_t row = ((size_t)table[new_page] * a.kv_heads + kv_head) * kPageTokens + slot;
+        void* slab = warp == 0 ? a.slab[0] : a.slab[1];
+        const float* src = fresh[warp];
+        if (U8) {  // one scale per cached row, as kv_append_kernel (pool.rs:224-240)
+          float amax = 0.0f;
+#pragma unroll
+          for (int d = lane; d < D; d += 32) amax = fmaxf(amax, fabsf(src[d]));
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+          const float scale = __fadd_rn(__fdiv_rn(amax, 127.0f), 1e-12f);
+          if (lane == 0) (warp == 0 ? a.slab_scale[0] : a.slab_scale[1])[row] = scale;
+#pragma unroll
+          for (int d = lane; d < D; d += 32)
+            reinterpret_cast<uint8_t*>(slab)[row * D + d] = (uint8_t)(fminf(fmaxf(roundf(__fdiv_rn(src[d], scale)), -127.0f), 127.0f) + 128.0f);
+        } else {
+#pragma unroll
+          for (int d = 2 * lane; d < D; d += 64) reinterpret_cast<uint32_t*>(slab)[(row * D + d) / 2] = pack2<BF16>(src[d], src[d + 1]);
+        }
+      }
+    }
   }
 
   // Q fragments: rows 0..G-1 = query heads of this KV head, scaled into the exp2 domain
   uint32_t qf[KSTEPS][4];
   {
     const bool lo_ok = g < G, hi_ok = g + 8 < G;
-    const float* qrow_lo = a.q + ((size_t)lane_id * a.q_heads + kv_head * G + (lo_ok ? g : 0)) * D;
-    const float* qrow_hi = a.q + ((size_t)lane_id * a.q_heads + kv_head * G + (hi_ok ? g + 8 : 0)) * D;
+    const float* qrow_lo = FUSED ? q_rows + (lo_ok ? g : 0) * D : a.q + ((size_t)lane_id * a.q_heads + kv_head * G + (lo_ok ? g : 0)) * D;
+    const float* qrow_hi = FUSED ? q_rows + (hi_ok ? g + 8 : 0) * D : a.q + ((size_t)lane_id * a.q_heads + kv_head * G + (hi_ok ? g + 8 : 0)) * D;
 #pragma unroll
     for (int ks = 0; ks < KSTEPS; ++ks) {
-      const int c0 = ks * 16 + 2 * t;
+      const int c0 = ks * 16 + (U8 ? 4 : 2) * t, c1 = c0 + (U8 ? 2 : 8);
       float2 x0 = lo_ok ? *reinterpret_cast<const float2*>(qrow_lo + c0) : make_float2(0.f, 0.f);
       float2 x1 = hi_ok ? *reinterpret_cast<const float2*>(qrow_hi + c0) : make_float2(0.f, 0.f);
-      float2 x2 = lo_ok ? *reinterpret_cast<const float2*>(qrow_lo + c0 + 8) : make_float2(0.f, 0.f);
-      float2 x3 = hi_ok ? *reinterpret_cast<const float2*>(qrow_hi + c0 + 8) : make_float2(0.f, 0.f);
+      float2 x2 = lo_ok ? *reinterpret_cast<const float2*>(qrow_lo + c1) : make_float2(0.f, 0.f);
+      float2 x3 = hi_ok ? *reinterpret_cast<const float2*>(qrow_hi + c1) : make_float2(0.f, 0.f);
       qf[ks][0] = pack2<BF16>(x0.x * a.scale_log2, x0.y * a.scale_log2);
       qf[ks][1] = pack2<BF16>(x1.x * a.scale_log2, x1.y * a.scale_log2);
       qf[ks][2] = pack2<BF16>(x2.x * a.scale_log2, x2.y * a.scale_log2);
       qf[ks][3] = pack2<BF16>(x3.x * a.scale_log2, x3.y * a.scale_log2);
     }
+  }
+  if constexpr (FUSED) {
+    __syncthreads();  // the query rows have been read, the new rows are stored
+    // the new token's page where it is among the first ones of its warp
+#pragma unroll
+    for (int s = 0; s < kAttnStages - 1; ++s)
+      if (p0 + warp + s * kAttnWarps == new_page) issue(new_page, s);
   }
 
   float o[DTILES][4];
@@ -475,29 +578,38 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs
   for (int page_index = p0 + warp; page_index < p1; page_index += kAttnWarps) {
     issue(next_issue, (stage + kAttnStages - 1) % kAttnStages);
     next_issue += kAttnWarps;
-    cp_async_wait<kAttnStages - 1>();
+    if (FUSED && page_index == new_page) cp_async_wait<0>();  // it may have been requested out of turn
+    else cp_async_wait<kAttnStages - 1>();
     __syncwarp();
     const unsigned char* ks_page = my_smem + stage * STAGE_BYTES;
     const unsigned char* vs_page = ks_page + RAW_PAGE;
     const float* page_scales = reinterpret_cast<const float*>(my_smem + stage * STAGE_BYTES + 2 * RAW_PAGE);  // U8: K rows, then V rows
-    if (U8) {
-      widen(ks_page, wide);
-      widen(vs_page, wide + PAGE_BYTES);
-      __syncwarp();
-      ks_page = wide;
-      vs_page = wide + PAGE_BYTES;
-    }
 
     // S = Q K^T : two n-tiles of 8 tokens
     float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+    if constexpr (U8) {
 #pragma unroll
-    for (int ks = 0; ks < KSTEPS; ++ks) {
-      uint32_t kf[4];
-      const int row = (lane & 7) + ((lane >> 4) << 3);
-      const int chunk = 2 * ks + ((lane >> 3) & 1);
-      ldmatrix_x4(kf, ks_page + swizzled_offset<D>(row, chunk));
-      mma_16816<BF16>(s0, qf[ks], kf[0], kf[1]);
-      mma_16816<BF16>(s1, qf[ks], kf[2], kf[3]);
+      for (int ks = 0; ks < KSTEPS; ks += 2) {
+        uint32_t codes[4], b0, b1;  // step ks: rows 0-7, rows 8-15; step ks + 1
+        ldmatrix_x4(codes, ks_page + swizzled_bytes<D>((lane & 7) + (((lane >> 3) & 1) << 3), ks + (lane >> 4)));
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          bytes_to_half2(codes[2 * u], b0, b1);
+          mma_16816<BF16>(s0, qf[ks + u], b0, b1);
+          bytes_to_half2(codes[2 * u + 1], b0, b1);
+          mma_16816<BF16>(s1, qf[ks + u], b0, b1);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int ks = 0; ks < KSTEPS; ++ks) {
+        uint32_t kf[4];
+        const int row = (lane & 7) + ((lane >> 4) << 3);
+        const int chunk = 2 * ks + ((lane >> 3) & 1);
+        ldmatrix_x4(kf, ks_page + swizzled_offset<D>(row, chunk));
+        mma_16816<BF16>(s0, qf[ks], kf[0], kf[1]);
+        mma_16816<BF16>(s1, qf[ks], kf[2], kf[3]);
+      }
     }
     if (U8) {  // score of token column c carries that cached row's K scale
       const float ka0 = page_scales[2 * t], ka1 = page_scales[2 * t + 1], kb0 = page_scales[2 * t + 8], kb1 = page_scales[2 * t + 9];
@@ -544,17 +656,29 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs
     pf[2] = pack2<BF16>(p1v[0], p1v[1]);  // row g,   tokens 2t+8, 2t+9
     pf[3] = pack2<BF16>(p1v[2], p1v[3]);
     // O = O * alpha + P V
+    auto accumulate = [&](float (&acc)[4], uint32_t b0, uint32_t b1) {
+      acc[0] *= alpha_lo; acc[1] *= alpha_lo; acc[2] *= alpha_hi; acc[3] *= alpha_hi;
+      mma_16816<BF16>(acc, pf, b0, b1);
+    };
 #pragma unroll
-    for (int dp = 0; dp < DTILES / 2; ++dp) {
+    for (int dp = 0; dp < DTILES / 2; dp += U8 ? 2 : 1) {
       uint32_t vf[4];
       const int row = (lane & 7) + (((lane >> 3) & 1) << 3);
-      const int chunk = 2 * dp + (lane >> 4);
-      ldmatrix_x4_trans(vf, vs_page + swizzled_offset<D>(row, chunk));
+      if constexpr (U8) {  // columns 16 dp .. 16 dp + 31: rows 0-7 and 8-15 of the first 16, then of the others
+        ldmatrix_x4_trans(vf, vs_page + swizzled_bytes<D>(row, dp + (lane >> 4)));
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        float (&acc)[4] = o[2 * dp + j];
-        acc[0] *= alpha_lo; acc[1] *= alpha_lo; acc[2] *= alpha_hi; acc[3] *= alpha_hi;
-        mma_16816<BF16>(acc, pf, vf[2 * j], vf[2 * j + 1]);
+        for (int u = 0; u < 2; ++u) {
+          uint32_t even0, odd0, even1, odd1;
+          bytes_to_half2<0x4240, 0x4341>(vf[2 * u], even0, odd0);
+          bytes_to_half2<0x4240, 0x4341>(vf[2 * u + 1], even1, odd1);
+          accumulate(o[2 * (dp + u)], even0, even1);
+          accumulate(o[2 * (dp + u) + 1], odd0, odd1);
+        }
+      } else {
+        const int chunk = 2 * dp + (lane >> 4);
+        ldmatrix_x4_trans(vf, vs_page + swizzled_offset<D>(row, chunk));
+        accumulate(o[2 * dp], vf[0], vf[1]);
+        accumulate(o[2 * dp + 1], vf[2], vf[3]);
       }
     }
     __syncwarp();
@@ -574,10 +698,12 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(AttnArgs
   float* ml = mm + kAttnWarps * 16;                    // [warp][16]
 #pragma unroll
   for (int i = 0; i < DTILES; ++i) {
-    float* lo = mo + ((size_t)warp * 16 + g) * D + i * 8 + 2 * t;
+    // U8: tiles 2 n and 2 n + 1 hold the even and the odd columns of 16
+    const int c0 = U8 ? i / 2 * 16 + 4 * t + (i & 1) : i * 8 + 2 * t, c1 = c0 + (U8 ? 2 : 1);
+    float* lo = mo + ((size_t)warp * 16 + g) * D;
     float* hi = lo + 8 * D;
-    lo[0] = o[i][0]; lo[1] = o[i][1];
-    hi[0] = o[i][2]; hi[1] = o[i][3];
+    lo[c0] = o[i][0]; lo[c1] = o[i][1];
+    hi[c0] = o[i][2]; hi[c1] = o[i][3];
   }
   if (t == 0) {
     mm[warp * 16 + g] = m_lo; mm[warp * 16 + g + 8] = m_hi;
@@ -936,15 +1062,15 @@ size_t plan_attention_max_scratch(int batch, int q_heads, int kv_heads, int head
   return need;
 }
 
-template <int D, bool BF16, bool U8>
-static cudaError_t launch_attention_mma_t(const PoolView& pool, const AttnArgs& args, int batch, int grid_x,
+template <int D, bool BF16, bool U8, bool FUSED>
+static cudaError_t launch_attention_mma_t(const PoolView& pool, const std::conditional_t<FUSED, FusedAttnArgs, AttnArgs>& args, int batch, int grid_x,
                                           cudaStream_t stream) {
   constexpr size_t page = (size_t)kPageTokens * D * 2;
-  constexpr size_t ring = U8 ? (size_t)kAttnWarps * (kAttnStages * 2 * (kPageTokens * D + kPageTokens * 4) + 2 * page)
+  constexpr size_t ring = U8 ? (size_t)kAttnWarps * kAttnStages * 2 * (kPageTokens * D + kPageTokens * 4) + (FUSED ? 16 * D * sizeof(float) : 0)
                              : (size_t)kAttnWarps * kAttnStages * 2 * page;
   constexpr size_t merge = (size_t)kAttnWarps * 16 * (D + 2) * sizeof(float);
   constexpr size_t smem = ring > merge ? ring : merge;
-  auto kernel = attention_mma_kernel<D, BF16, U8>;
+  auto kernel = attention_mma_kernel<D, BF16, U8, FUSED>;
   const cudaError_t attr = opt_in_shared_memory(kernel, smem);
   if (attr != cudaSuccess) return attr;
   dim3 grid((unsigned)grid_x, (unsigned)pool.kv_heads, (unsigned)batch);
@@ -954,9 +1080,20 @@ static cudaError_t launch_attention_mma_t(const PoolView& pool, const AttnArgs& 
 cudaError_t launch_attention_mma(const PoolView& pool, const float* q, const LaneInfo* lanes, const int* tables,
                                  int batch, int q_heads, double scale, long long op_window, float* out,
                                  const AttnPlan& plan, float* scratch, cudaStream_t stream, int* launches, __half* out_xh, int xh_nv,
-                                 int tokens) {
+                                 int tokens, const FusedRope* rope) {
   if (batch == 0) return cudaSuccess;
-  AttnArgs args;
+  if (rope && tokens != 1) return cudaErrorInvalidValue;
+  FusedAttnArgs args;
+  if (rope) {
+    args.qkv = rope->qkv;
+    args.sum = rope->sum;
+    args.inv_freq = rope->inv_freq;
+    args.rope_layout = rope->layout;
+    args.slab[0] = pool.k;
+    args.slab[1] = pool.v;
+    args.slab_scale[0] = pool.k_scale;
+    args.slab_scale[1] = pool.v_scale;
+  }
   args.out_xh = out_xh;
   args.out_xh_nv = xh_nv;
   args.k = pool.k; args.v = pool.v; args.q = q; args.lanes = lanes; args.tables = tables; args.out = out;
@@ -972,7 +1109,9 @@ cudaError_t launch_attention_mma(const PoolView& pool, const float* q, const Lan
   auto launch = [&](auto wide, auto bf16, auto u8) {
     constexpr int D = decltype(wide)::value ? 128 : 64;
     constexpr bool BF16 = decltype(bf16)::value, U8 = decltype(u8)::value;
-    return tokens > 1 ? launch_attention_chunk_t<D, BF16, U8>(args, batch, stream) : launch_attention_mma_t<D, BF16, U8>(pool, args, batch, plan.splits, stream);
+    if (tokens > 1) return launch_attention_chunk_t<D, BF16, U8>(args, batch, stream);
+    return rope ? launch_attention_mma_t<D, BF16, U8, true>(pool, args, batch, plan.splits, stream)
+                : launch_attention_mma_t<D, BF16, U8, false>(pool, args, batch, plan.splits, stream);
   };
   auto dispatch = [&](auto wide) {
     if (pool.dtype == kKvU8) return launch(wide, std::false_type(), std::true_type());

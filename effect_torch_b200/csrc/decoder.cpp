@@ -359,20 +359,25 @@ etc_status enqueue_step(StepContext& s) {
   for (int l = 0; l < c.layers; ++l) {
     const size_t li = (size_t)l;
     const PoolView view = s.pool->view(l);
+    const bool fast_attention = d->tiled && !c.exact && attention_mma_supported(view, Hq, T);
     if (xh) {
       ETC_TRY(norm_hand_off(s, d->hidden, d->attn_norm[li], rows, pending));
     } else {
       ETC_CUDA(launch_rmsnorm(d->hidden, (const float*)d->attn_norm[li].d_raw, c.rms_eps, rows, c.d_model, d->normed, stream));
       ++s.launches;
     }
-    const bool fast_attention = d->tiled && !c.exact && attention_mma_supported(view, Hq, T);
     DeferredSum qkv_sum;  // the RoPE / append kernel can sum the fused projection's partials itself
     if (d->tiled)
       ETC_TRY(run_linear(s, d->wq[li], d->t_qkv[li], d->normed, rows, d->qkv, ETC_EPILOGUE_NONE, nullptr, xh ? d->xh_norm : nullptr, nullptr, &qkv_sum));
     else
       ETC_TRY(project_qkv_raw(s, li, d->normed, rows, qkvw));
-    ETC_CUDA(launch_rope_append(view, d->qkv, d->d_lanes, d->d_tables, d->d_inv_freq, c.rope_layout, B, Hq, d->qr, stream, &qkv_sum, T));
-    ++s.launches;
+    // one token per lane: the attention kernel rotates and appends on its way in
+    const bool fused_rope = fast_attention && T == 1;
+    const FusedRope rope = {d->qkv, qkv_sum, d->d_inv_freq, c.rope_layout};
+    if (!fused_rope) {
+      ETC_CUDA(launch_rope_append(view, d->qkv, d->d_lanes, d->d_tables, d->d_inv_freq, c.rope_layout, B, Hq, d->qr, stream, &qkv_sum, T));
+      ++s.launches;
+    }
     if (fast_attention) {
       const AttnPlan plan = plan_attention(B, Hq, Hkv, D, std::max(1, s.max_pages), d->rt->sm_count);
       if (plan.scratch_bytes > d->attn_scratch_bytes)
@@ -380,7 +385,7 @@ etc_status enqueue_step(StepContext& s) {
                                        std::to_string(plan.scratch_bytes) + " bytes of partials, the decoder holds " +
                                        std::to_string(d->attn_scratch_bytes));
       ETC_CUDA(launch_attention_mma(view, d->qr, d->d_lanes, d->d_tables, B, Hq, scale, c.window, xh ? nullptr : d->attl, plan,
-                                    d->attn_scratch, stream, &s.launches, xh ? d->xh_att : nullptr, hand_off_stride(rows), T));
+                                    d->attn_scratch, stream, &s.launches, xh ? d->xh_att : nullptr, hand_off_stride(rows), T, fused_rope ? &rope : nullptr));
     } else {
       ETC_CUDA(launch_attention_exact(view, d->qr, d->d_lanes, d->d_tables, B, Hq, T, scale, c.window, d->attl, d->exact_scratch, s.max_ctx, stream, true));
       ++s.launches;

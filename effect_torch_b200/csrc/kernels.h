@@ -239,10 +239,19 @@ AttnPlan plan_attention(int batch, int q_heads, int kv_heads, int head_dim, int 
 // Largest scratch plan_attention can ask for with tables of at most max_pages pages.
 size_t plan_attention_max_scratch(int batch, int q_heads, int kv_heads, int head_dim, int max_pages, int sm_count);
 bool attention_mma_supported(const PoolView& pool, int q_heads, int tokens);
+// For a decode step: q is not given but comes from the fused projection's rows (or their partials), RoPE and the append of the
+// new token's K and V happen in the attention kernel. Everything else that the kernel reads (cached rows, lanes, tables) must
+// have been written before the launches of this step.
+struct FusedRope {
+  const float* qkv;
+  DeferredSum sum;
+  const double* inv_freq;
+  int layout;
+};
 cudaError_t launch_attention_mma(const PoolView& pool, const float* q, const LaneInfo* lanes, const int* tables,
                                  int batch, int q_heads, double scale, long long op_window, float* out,
                                  const AttnPlan& plan, float* scratch, cudaStream_t stream, int* launches,
-                                 __half* out_xh = nullptr, int xh_nv = 32, int tokens = 1);
+                                 __half* out_xh = nullptr, int xh_nv = 32, int tokens = 1, const FusedRope* rope = nullptr);
 // Fused RoPE(q), RoPE(k) and KV append: qkv [B * tokens, (Hq+2*Hkv)*D] f32 (the fused projection output) ->
 // q_out [B, tokens, Hq, D] f32 rotated, K/V rows written to the pool at positions cursor .. cursor + tokens - 1.
 cudaError_t launch_rope_append(const PoolView& pool, const float* qkv, const LaneInfo* lanes, const int* tables,

@@ -499,6 +499,41 @@ def test_chunks_at_the_edges_of_the_attention_tiles(q_heads, kv_heads, head_dim,
         assert helpers.rel_err(gl, ol) <= 2 * tol, f"advance {advance}"
 
 
+@pytest.mark.parametrize("q_heads,kv_heads,head_dim,kv_dtype,okv,tol,layout,window", [
+    (4, 2, 64, et.KV_F16, orc.F16, LOGIT_TOL, 0, None), (8, 1, 128, et.KV_F16, orc.F16, LOGIT_TOL, 1, 40), (16, 1, 64, et.KV_BF16, orc.BF16, 2e-2, 1, None),
+    (2, 2, 128, et.KV_U8, orc.U8, 1e-2, 0, 40), (16, 1, 64, et.KV_U8, orc.U8, 1e-2, 1, None)])
+def test_decode_steps_that_rotate_and_append_inside_attention(q_heads, kv_heads, head_dim, kv_dtype, okv, tol, layout, window):
+    """One-token steps across page boundaries, with the new token's page first, second and later among its warp's pages and
+    lanes of different lengths (up to 33 pages: several splits of the context); the last lane is padded. Tolerances as for
+    chunks at the edges of the attention tiles, whose model and tiers these are."""
+    cfg = dict(helpers.TINY_Q, layers=2, q_heads=q_heads, kv_heads=kv_heads, head_dim=head_dim, vocab=512)
+    w = helpers.make_weights(cfg, seed=6, codec=orc.Q4_0)
+    rng = np.random.default_rng(9)
+    B, max_tokens = 5, 2048
+    odec = orc.Decoder(cfg["layers"], cfg["d_model"], q_heads, kv_heads, head_dim, cfg["ffn"], cfg["vocab"], eps=cfg["rms_eps"], theta=cfg["rope_theta"],
+                       window=window, batch=B, rope_layout=layout)
+    helpers.load_into(odec, w)
+    odec.set_mode(faithful=False, threads=max(1, min(8, orc.max_threads())))
+    gdec = et.Executable(runtime(), layers=cfg["layers"], d_model=cfg["d_model"], q_heads=q_heads, kv_heads=kv_heads, head_dim=head_dim, ffn=cfg["ffn"],
+                         vocab=cfg["vocab"], rms_eps=cfg["rms_eps"], rope_theta=cfg["rope_theta"], batch=B, max_tokens=max_tokens, block_size=16,
+                         kv_dtype=kv_dtype, exact=False, max_advance=128, window=window, rope_layout=layout)
+    helpers.load_into(gdec, w)
+    gdec.finalize()
+    opool = orc.Pool(cfg["layers"], kv_heads, head_dim, max_tokens, 16, okv)
+    gpool = et.NativeKvPool(runtime(), cfg["layers"], kv_heads, head_dim, max_tokens, 16, kv_dtype)
+    oseqs, gseqs = [opool.make_sequence() for _ in range(B - 1)], [gpool.makeSequence() for _ in range(B - 1)]
+    for lane, tokens in enumerate((1, 15, 63, 527 if window is None else 100)):
+        for first in range(0, tokens, 128):
+            toks = rng.integers(0, cfg["vocab"], size=(1, min(128, tokens - first))).astype(np.uint32)
+            odec.execute(opool, oseqs[lane:lane + 1], toks)
+            gdec.execute(gpool, gseqs[lane:lane + 1], toks)
+    for step in range(5):
+        toks = rng.integers(0, cfg["vocab"], size=(B - 1, 1)).astype(np.uint32)
+        ol, _ = odec.execute(opool, oseqs, toks)
+        gl = gdec.execute(gpool, gseqs, toks)
+        assert helpers.rel_err(gl, ol) <= 2 * tol, f"step {step}"
+
+
 def test_steps_of_wide_q8_0_layers_repeat_bit_for_bit():
     """A stage's block scales are used a round after its buffer is handed back to the loader: a load that came back late
     took the next round's scales (a wrong step in some fifty of this shape). 120 runs of three steps, all alike; the first
