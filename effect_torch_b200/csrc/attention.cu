@@ -255,6 +255,140 @@ cudaError_t launch_attention_exact(const PoolView& pool, const float* q, const L
   }
 }
 
+// The same for one-token steps of the decoder with an f32 cache whose contexts fit in shared memory, RoPE and append included. A
+// CTA per (query head, lane) fetches the cached rows, which were written before this step, and the angles before it waits for
+// the projection; then it rotates its query and the new K row, which all query heads of a KV head do and the first of them
+// stores. K rows are padded so that a warp's 16-byte reads of 32 positions do not conflict. Two launches (9.2 us with its
+// 4-byte loads of K from memory at one line per thread, 1.8 us for RoPE) in one of 4 at contexts of 32 to 95.
+constexpr size_t kExactStepSmem = 200 * 1024;
+static int exact_step_slots(int max_ctx) { return (max_ctx + 3) & ~3; }  // keeps what follows them 16-byte aligned
+static size_t exact_step_smem(int head_dim, int max_ctx) {
+  return (size_t)exact_step_slots(max_ctx) * ((2 * head_dim + 4) * sizeof(float) + sizeof(double)) + 2 * head_dim * sizeof(double);
+}
+
+__global__ void __launch_bounds__(128) attention_exact_step_kernel(PoolView pool, const float* qkv, const LaneInfo* lanes, const int* tables,
+                                                                   const double* inv_freq, int layout, int q_heads, double scale,
+                                                                   long long op_window, float* out, int slots) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ double red[4];
+  const int D = pool.head_dim, half = D / 2, pitch = D + 4;
+  double* q_s = reinterpret_cast<double*>(smem);                     // [D]
+  double2* angle = reinterpret_cast<double2*>(q_s + D);              // [D / 2] (sine, cosine)
+  double* weight_s = reinterpret_cast<double*>(angle + half);        // [slots], a multiple of 4
+  float* k_s = reinterpret_cast<float*>(weight_s + slots);           // [slots][pitch]
+  float* v_s = k_s + (size_t)slots * pitch;                          // [slots][D]
+  chain_release();
+  const int head = blockIdx.x, lane_id = blockIdx.y, group = q_heads / pool.kv_heads, kv_head = head / group;
+  const LaneInfo info = lanes[lane_id];
+  float* orow = out + ((size_t)lane_id * q_heads + head) * D;
+  if (info.advance == 0) {  // padded lane: output stays zero (napi/mod.rs:3371-3372)
+    chain_wait();
+    for (int d = threadIdx.x; d < D; d += blockDim.x) orow[d] = 0.0f;
+    return;
+  }
+  const int end = info.cursor + 1;
+  const int begin = op_window >= 0 ? max((int)max((long long)end - op_window, 0ll), info.start) : info.start;
+  const int cached = min(max(end - begin, 0), slots) - 1;  // positions before the new one
+  const int* table = tables + info.table_offset;
+  auto row_of = [&](int pos) {
+    const int block = pos / pool.block_size;
+    return ((size_t)table[block] * pool.kv_heads + kv_head) * pool.block_size + (pos - block * pool.block_size);
+  };
+  const int quads = D / 4;
+  for (int i = threadIdx.x; i < cached * quads; i += blockDim.x) {
+    const int at = i / quads, c = 4 * (i - at * quads);
+    const size_t src = row_of(begin + at) * D + c;
+    const unsigned kd = (unsigned)__cvta_generic_to_shared(k_s + at * pitch + c), vd = (unsigned)__cvta_generic_to_shared(v_s + at * D + c);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(kd), "l"(reinterpret_cast<const float*>(pool.k) + src) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(vd), "l"(reinterpret_cast<const float*>(pool.v) + src) : "memory");
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int j = threadIdx.x; j < half; j += blockDim.x) {
+    double s, c;
+    sincos((double)info.cursor * inv_freq[j], &s, &c);
+    angle[j] = make_double2(s, c);
+  }
+  __syncthreads();  // the angles
+  chain_wait();
+  const size_t fresh = row_of(info.cursor) * D;
+  const bool stores = head == kv_head * group;
+  const float* row = qkv + (size_t)lane_id * (q_heads + 2 * pool.kv_heads) * D;
+  for (int i = threadIdx.x; i < 3 * half; i += blockDim.x) {
+    const int what = i / half, j = i - what * half;  // 0: query, 1: key, 2: value
+    const int i0 = layout == 0 ? j : 2 * j, i1 = layout == 0 ? half + j : 2 * j + 1;
+    const float* src = row + (size_t)(what == 0 ? head : q_heads + (what - 1) * pool.kv_heads + kv_head) * D;
+    float r0 = src[i0], r1 = src[i1];
+    if (what < 2) {
+      const double first = (double)r0, second = (double)r1, s = angle[j].x, c = angle[j].y;
+      r0 = (float)__dsub_rn(__dmul_rn(first, c), __dmul_rn(second, s));
+      r1 = (float)__dadd_rn(__dmul_rn(second, c), __dmul_rn(first, s));
+    }
+    if (what == 0) {
+      q_s[i0] = (double)r0;
+      q_s[i1] = (double)r1;
+      continue;
+    }
+    float* dst = what == 1 ? k_s + (size_t)cached * pitch : v_s + (size_t)cached * D;
+    dst[i0] = r0;
+    dst[i1] = r1;
+    if (stores) {
+      float* slab = reinterpret_cast<float*>(what == 1 ? pool.k : pool.v) + fresh;
+      slab[i0] = r0;
+      slab[i1] = r1;
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  const int span = cached + 1;
+  double local_max = -INFINITY;
+  for (int i = threadIdx.x; i < span; i += blockDim.x) {
+    const float4* k4 = reinterpret_cast<const float4*>(k_s + (size_t)i * pitch);
+    double score = 0.0;
+#pragma unroll 4
+    for (int c = 0; c < quads; ++c) {
+      const float4 k = k4[c];
+      score += q_s[4 * c] * (double)k.x;  // exact products: contracted or not, one rounding per term
+      score += q_s[4 * c + 1] * (double)k.y;
+      score += q_s[4 * c + 2] * (double)k.z;
+      score += q_s[4 * c + 3] * (double)k.w;
+    }
+    const double scaled = __dmul_rn(score, scale);
+    weight_s[i] = scaled;
+    local_max = fmax(local_max, scaled);
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) local_max = fmax(local_max, __shfl_xor_sync(0xffffffffu, local_max, off));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = local_max;
+  __syncthreads();
+  const double maximum = fmax(fmax(red[0], red[1]), fmax(red[2], red[3]));
+  for (int i = threadIdx.x; i < span; i += blockDim.x) weight_s[i] = exp(__dsub_rn(weight_s[i], maximum));
+  __syncthreads();
+  for (int c = threadIdx.x; c < D; c += blockDim.x) {
+    double result = 0.0, denominator = 0.0;
+#pragma unroll 8
+    for (int i = 0; i < span; ++i) {
+      const double w = weight_s[i];
+      result = __dadd_rn(result, __dmul_rn(w, (double)v_s[(size_t)i * D + c]));
+      denominator = __dadd_rn(denominator, w);
+    }
+    orow[c] = (float)__ddiv_rn(result, denominator);
+  }
+}
+
+bool attention_exact_step_supported(const PoolView& pool, int q_heads, int max_ctx) {
+  return pool.dtype == kKvF32 && pool.kv_heads > 0 && q_heads % pool.kv_heads == 0 && pool.head_dim % 4 == 0 &&
+         exact_step_smem(pool.head_dim, max_ctx) <= kExactStepSmem;
+}
+
+cudaError_t launch_attention_exact_step(const PoolView& pool, const float* qkv, const LaneInfo* lanes, const int* tables, const double* inv_freq, int layout,
+                                        int batch, int q_heads, double scale, long long op_window, float* out, int max_ctx, cudaStream_t stream) {
+  if (batch == 0) return cudaSuccess;
+  const cudaError_t attr = opt_in_shared_memory(attention_exact_step_kernel, kExactStepSmem);
+  if (attr != cudaSuccess) return attr;
+  return launch_chained(attention_exact_step_kernel, dim3((unsigned)q_heads, (unsigned)batch), dim3(128), exact_step_smem(pool.head_dim, max_ctx), stream, pool,
+                        qkv, lanes, tables, inv_freq, layout, q_heads, scale, op_window, out, exact_step_slots(max_ctx));
+}
+
 // --------------------------------------------------------------------------------------------
 // Tensor-core flash-decoding (one query token per lane, f16 or bf16 pages of 16 tokens).
 //

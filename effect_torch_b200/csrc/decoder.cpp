@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <vector>
 
 #include "common.h"
@@ -225,14 +226,33 @@ DenseArgs dense_args(const float* x, int64_t rows, const BoundWeight& w) {
   return a;
 }
 
+void add_norm(DenseArgs& a, const BoundWeight* norm, double eps) {
+  if (!norm) return;
+  a.norm_weight = (const float*)norm->d_raw;
+  a.norm_eps = eps;
+}
+
+// The norm ahead of a dense projection is computed inside it where few rows meet a narrow weight: x is the residual stream then.
+bool norm_rides(const StepContext& s, int64_t rows, const BoundWeight& norm, std::initializer_list<const BoundWeight*> weights) {
+  etc_decoder* d = s.dec;
+  if (d->tiled) return false;
+  for (const BoundWeight* w : weights) {
+    DenseArgs a = dense_args(d->hidden, rows, *w);
+    a.norm_weight = (const float*)norm.d_raw;
+    if (w->codec != ETC_CODEC_F32 || !dense_narrow_supported(a)) return false;
+  }
+  return true;
+}
+
 // q, k and v of raw weights side by side in d->qkv, the layout of the fused projection.
-etc_status project_qkv_raw(StepContext& s, size_t layer, const float* x, int64_t rows, int64_t stride) {
+etc_status project_qkv_raw(StepContext& s, size_t layer, const float* x, int64_t rows, int64_t stride, const BoundWeight* norm) {
   etc_decoder* d = s.dec;
   cudaStream_t stream = d->rt->stream;
   const BoundWeight* w[3] = {&d->wq[layer], &d->wk[layer], &d->wv[layer]};
   float* out[3] = {d->qkv, d->qkv + w[0]->rows, d->qkv + w[0]->rows + w[1]->rows};
   if (w[0]->codec == ETC_CODEC_F32 && w[1]->codec == ETC_CODEC_F32 && w[2]->codec == ETC_CODEC_F32) {
     DenseArgs a = dense_args(x, rows, *w[0]);
+    add_norm(a, norm, d->cfg.rms_eps);
     a.parts = 3;
     a.out_stride = stride;
     for (int p = 0; p < 3; ++p) {
@@ -262,7 +282,7 @@ etc_status project_qkv_raw(StepContext& s, size_t layer, const float* x, int64_t
 // out = x W^T (+ epilogue) for one projection, choosing the tensor-core tiling when it exists.
 etc_status run_linear(StepContext& s, const BoundWeight& raw, etc_qweight* tiled_w, const float* x, int64_t vectors, float* out,
                       int epilogue, const float* residual, const __half* xh_ready = nullptr, __half* out_xh = nullptr,
-                      DeferredSum* defer = nullptr) {
+                      DeferredSum* defer = nullptr, const BoundWeight* norm = nullptr) {
   etc_decoder* d = s.dec;
   cudaStream_t stream = d->rt->stream;
   if (defer) *defer = DeferredSum();
@@ -275,6 +295,7 @@ etc_status run_linear(StepContext& s, const BoundWeight& raw, etc_qweight* tiled
     DenseArgs dense = dense_args(x, vectors, raw);
     dense.out[0] = out;
     dense.out_stride = raw.rows;
+    add_norm(dense, norm, d->cfg.rms_eps);
     dense.residual = epilogue == ETC_EPILOGUE_RESIDUAL ? residual : nullptr;
     ETC_CUDA(launch_dense_linear(dense, stream));
     ++s.launches;
@@ -360,9 +381,10 @@ etc_status enqueue_step(StepContext& s) {
     const size_t li = (size_t)l;
     const PoolView view = s.pool->view(l);
     const bool fast_attention = d->tiled && !c.exact && attention_mma_supported(view, Hq, T);
+    const bool rides_attn = norm_rides(s, rows, d->attn_norm[li], {&d->wq[li], &d->wk[li], &d->wv[li]});
     if (xh) {
       ETC_TRY(norm_hand_off(s, d->hidden, d->attn_norm[li], rows, pending));
-    } else {
+    } else if (!rides_attn) {
       ETC_CUDA(launch_rmsnorm(d->hidden, (const float*)d->attn_norm[li].d_raw, c.rms_eps, rows, c.d_model, d->normed, stream));
       ++s.launches;
     }
@@ -370,11 +392,12 @@ etc_status enqueue_step(StepContext& s) {
     if (d->tiled)
       ETC_TRY(run_linear(s, d->wq[li], d->t_qkv[li], d->normed, rows, d->qkv, ETC_EPILOGUE_NONE, nullptr, xh ? d->xh_norm : nullptr, nullptr, &qkv_sum));
     else
-      ETC_TRY(project_qkv_raw(s, li, d->normed, rows, qkvw));
+      ETC_TRY(project_qkv_raw(s, li, rides_attn ? d->hidden : d->normed, rows, qkvw, rides_attn ? &d->attn_norm[li] : nullptr));
     // one token per lane: the attention kernel rotates and appends on its way in
     const bool fused_rope = fast_attention && T == 1;
+    const bool exact_step = !fast_attention && T == 1 && qkv_sum.splits == 0 && attention_exact_step_supported(view, Hq, s.max_ctx);
     const FusedRope rope = {d->qkv, qkv_sum, d->d_inv_freq, c.rope_layout};
-    if (!fused_rope) {
+    if (!fused_rope && !exact_step) {
       ETC_CUDA(launch_rope_append(view, d->qkv, d->d_lanes, d->d_tables, d->d_inv_freq, c.rope_layout, B, Hq, d->qr, stream, &qkv_sum, T));
       ++s.launches;
     }
@@ -386,6 +409,9 @@ etc_status enqueue_step(StepContext& s) {
                                        std::to_string(d->attn_scratch_bytes));
       ETC_CUDA(launch_attention_mma(view, d->qr, d->d_lanes, d->d_tables, B, Hq, scale, c.window, xh ? nullptr : d->attl, plan,
                                     d->attn_scratch, stream, &s.launches, xh ? d->xh_att : nullptr, hand_off_stride(rows), T, fused_rope ? &rope : nullptr));
+    } else if (exact_step) {
+      ETC_CUDA(launch_attention_exact_step(view, d->qkv, d->d_lanes, d->d_tables, d->d_inv_freq, c.rope_layout, B, Hq, scale, c.window, d->attl, s.max_ctx, stream));
+      ++s.launches;
     } else {
       ETC_CUDA(launch_attention_exact(view, d->qr, d->d_lanes, d->d_tables, B, Hq, T, scale, c.window, d->attl, d->exact_scratch, s.max_ctx, stream, true));
       ++s.launches;
@@ -393,22 +419,24 @@ etc_status enqueue_step(StepContext& s) {
     const bool xh_o = xh && fast_attention;
     ETC_TRY(project_into_hidden(s, d->wo[li], d->tiled ? d->t_o[li] : nullptr, d->attl, rows, xh_o ? d->xh_att : nullptr, 0,
                                 xh ? &pending : nullptr));
+    const bool rides_ffn = norm_rides(s, rows, d->ffn_norm[li], {&d->gate[li], &d->up[li]});
     if (xh) {
       ETC_TRY(norm_hand_off(s, d->hidden, d->ffn_norm[li], rows, pending));
-    } else {
+    } else if (!rides_ffn) {
       ETC_CUDA(launch_rmsnorm(d->hidden, (const float*)d->ffn_norm[li].d_raw, c.rms_eps, rows, c.d_model, d->normed, stream));
       ++s.launches;
     }
     if (d->tiled) {
       ETC_TRY(run_linear(s, d->gate[li], d->t_gu[li], d->normed, rows, xh ? nullptr : d->act, ETC_EPILOGUE_SWIGLU, nullptr,
                          xh ? d->xh_norm : nullptr, xh ? d->xh_act : nullptr));
-    } else if (DenseArgs ffn = dense_args(d->normed, rows, d->gate[li]);
+    } else if (DenseArgs ffn = dense_args(rides_ffn ? d->hidden : d->normed, rows, d->gate[li]);
                d->gate[li].codec == ETC_CODEC_F32 && d->up[li].codec == ETC_CODEC_F32 && dense_linear_supported(ffn)) {
       ffn.w[1] = (const float*)d->up[li].d_raw;
       ffn.out[0] = d->act;
       ffn.out_stride = c.ffn;
       ffn.swiglu = 1;
       ffn.exact = c.exact;
+      add_norm(ffn, rides_ffn ? &d->ffn_norm[li] : nullptr, c.rms_eps);
       ETC_CUDA(launch_dense_linear(ffn, stream));
       ++s.launches;
     } else {
@@ -430,13 +458,15 @@ etc_status enqueue_step(StepContext& s) {
     ++s.launches;
     head_in = d->last;
   }
+  const bool rides_head = norm_rides(s, B, d->out_norm, {&d->head});
   if (xh) {
     ETC_TRY(norm_hand_off(s, head_in, d->out_norm, B, pending));
-  } else {
+  } else if (!rides_head) {
     ETC_CUDA(launch_rmsnorm(head_in, (const float*)d->out_norm.d_raw, c.rms_eps, B, c.d_model, d->normed, stream));
     ++s.launches;
   }
-  ETC_TRY(run_linear(s, d->head, d->tiled ? d->t_head : nullptr, d->normed, B, d->logits, ETC_EPILOGUE_NONE, nullptr, xh ? d->xh_norm : nullptr));
+  ETC_TRY(run_linear(s, d->head, d->tiled ? d->t_head : nullptr, rides_head ? head_in : d->normed, B, d->logits, ETC_EPILOGUE_NONE, nullptr,
+                     xh ? d->xh_norm : nullptr, nullptr, nullptr, rides_head ? &d->out_norm : nullptr));
   if (d->vocab_global > 0 && d->tp_world > 1) {
     // vocabulary-parallel head: every rank picks its best row, the ranks exchange (logit, token) pairs over peer memory
     if (!d->tp_peer) return fail(ETC_EXECUTION, "tensor parallel: a vocabulary-parallel head needs the peer exchange regions (etc_decoder_tp_peer_import)");

@@ -25,6 +25,21 @@ __device__ __forceinline__ float swiglu_value(float g, float up, int exact) {
   return __fmul_rn(__fmul_rn(g, __fadd_rn(th * 0.5f, 0.5f)), up);
 }
 
+__device__ __forceinline__ double square4(const float4& v) {
+  return (double)v.x * (double)v.x + (double)v.y * (double)v.y + (double)v.z * (double)v.z + (double)v.w * (double)v.w;
+}
+__device__ __forceinline__ float4 scale4(const float4& v, double scale, const float4& w) {
+  return make_float4((float)__dmul_rn(__dmul_rn((double)v.x, scale), (double)w.x), (float)__dmul_rn(__dmul_rn((double)v.y, scale), (double)w.y),
+                     (float)__dmul_rn(__dmul_rn((double)v.z, scale), (double)w.z), (float)__dmul_rn(__dmul_rn((double)v.w, scale), (double)w.w));
+}
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+
+constexpr int kNormThreads = 256, kNormItems = 8192 / 4 / kNormThreads;
+
 // --------------------------------------------------------------------------------------------
 // Dense linear, bit-exact with the reference: every output element is one sequential fmaf chain over k
 // (out = fma(x[m,k], W[n,k], out)), four cycles per k whatever is done, so for the small models that run in f32 what counts is
@@ -112,6 +127,123 @@ __global__ void __launch_bounds__(256) dense_linear_kernel(DenseArgs a) {
   }
 }
 
+// The same chain where a decode step's few rows meet a narrow weight (the small f32 models): a CTA holds the whole of 32 weight
+// rows in shared memory, fetched before the wait for the kernel ahead, so that only the input rows, the chain itself and the
+// store are left behind it. A warp carries ROWS input rows. (In the ring above eight warps read the same tile, 10 cycles of
+// shared-memory path per k where the chain needs four, with a barrier per 64 columns: 4 rows in a step's chain took 9 us for
+// k = 688 and 4.1 for 256, now 3.8 and 2.2.) The norm ahead of the projection may come along: every CTA computes
+// it for its own copy of the rows, with the sums of rmsnorm_rows_kernel, instead of a launch of 2 us.
+// With SWIGLU lanes 0 to 15 hold gate rows and lanes 16 to 31 their up rows.
+constexpr int kNarrowThreads = 128, kNarrowRows = 16;
+constexpr size_t kNarrowSmem = 220 * 1024;
+static size_t narrow_smem(const DenseArgs& a) { return sizeof(float) * (32 * (size_t)(a.k + 4) + (size_t)a.m * a.k); }
+
+template <int ROWS, bool SWIGLU>
+__global__ void __launch_bounds__(kNarrowThreads) dense_narrow_kernel(DenseArgs a) {
+  chain_release();
+  extern __shared__ __align__(16) float tile_s[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int OUTS = SWIGLU ? 16 : 32;
+  int tile = blockIdx.x, part = 0;
+  if (!SWIGLU)
+    while (part + 1 < a.parts && tile >= (int)((a.n[part] + 31) / 32)) tile -= (int)((a.n[part++] + 31) / 32);
+  const int64_t n = a.n[part], n0 = (int64_t)tile * OUTS;
+  const int k = (int)a.k, quads = k / 4, pitch = k + 4, m = (int)a.m;
+  float* x_s = tile_s + 32 * pitch;
+  auto copy16 = [](float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+  };
+  auto fill_weights = [&] {  // rows beyond the matrix repeat its last one: their results are not stored
+    for (int r = warp; r < 32; r += kNarrowThreads / 32) {
+      const float* src = (SWIGLU ? a.w[r / OUTS] : a.w[part]) + min(n0 + r % OUTS, n - 1) * k;
+      for (int q = lane; q < quads; q += 32) copy16(tile_s + r * pitch + 4 * q, src + 4 * q);
+    }
+  };
+  if (a.constant_weights) fill_weights();
+  chain_wait();
+  if (!a.constant_weights) fill_weights();
+  if (a.norm_weight) {
+    for (int r = warp; r < m; r += kNarrowThreads / 32) {
+      const float4* src = reinterpret_cast<const float4*>(a.x + (int64_t)r * k);
+      float4* dst = reinterpret_cast<float4*>(x_s + r * k);
+      double total = 0.0;
+      for (int p = 0; p < kNormThreads / 32 && 32 * p < quads; ++p) {  // the partial sum of warp p of rmsnorm_rows_kernel
+        double sum = 0.0;
+        for (int q = 32 * p + lane; q < quads; q += kNormThreads) {
+          const float4 v = src[q];
+          dst[q] = v;
+          sum += square4(v);
+        }
+        total += warp_sum(sum);
+      }
+      const double scale = 1.0 / sqrt(total / (double)k + a.norm_eps);
+      for (int q = lane; q < quads; q += 32) dst[q] = scale4(dst[q], scale, reinterpret_cast<const float4*>(a.norm_weight)[q]);
+    }
+  } else {
+    for (int i = threadIdx.x; i < m * quads; i += kNarrowThreads) copy16(x_s + 4 * i, a.x + 4 * (int64_t)i);
+  }
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  const int row0 = warp * ROWS;
+  if (row0 >= m) return;
+  const float4* w4 = reinterpret_cast<const float4*>(tile_s + lane * pitch);
+  const float4* x4[ROWS];
+  float acc[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    x4[r] = reinterpret_cast<const float4*>(x_s + min(row0 + r, m - 1) * k);
+    acc[r] = 0.0f;
+  }
+  // a few quads at a time, the next ones on their way while these are added
+  constexpr int AHEAD = ROWS == 4 ? 2 : 4;
+  float4 w[2][AHEAD], x[2][AHEAD][ROWS];
+  auto fetch = [&](int buffer, int q0) {
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int q = min(q0 + u, quads - 1);
+      w[buffer][u] = w4[q];
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) x[buffer][u][r] = x4[r][q];
+    }
+  };
+  auto add = [&](int buffer, int n_quads) {
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      if (u >= n_quads) break;
+      const float4 wv = w[buffer][u];
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const float4 xv = x[buffer][u][r];
+        acc[r] = fmaf(xv.w, wv.w, fmaf(xv.z, wv.z, fmaf(xv.y, wv.y, fmaf(xv.x, wv.x, acc[r]))));
+      }
+    }
+  };
+  fetch(0, 0);
+  int q = 0;
+  for (; q + 2 * AHEAD <= quads; q += 2 * AHEAD) {
+    fetch(1, q + AHEAD);
+    add(0, AHEAD);
+    fetch(0, q + 2 * AHEAD);
+    add(1, AHEAD);
+  }
+  if (q < quads) {
+    fetch(1, q + AHEAD);
+    add(0, min(AHEAD, quads - q));
+    add(1, quads - q - AHEAD);
+  }
+  const int64_t col = n0 + lane % OUTS;
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    float value = acc[r];
+    if (SWIGLU) value = swiglu_value(value, __shfl_down_sync(0xffffffffu, value, 16), a.exact);
+    if (row0 + r >= m || col >= n || lane >= OUTS) continue;
+    const int64_t at = (row0 + r) * a.out_stride + col;
+    if (!SWIGLU && a.bias) value += a.bias[col];
+    if (!SWIGLU && a.residual) value = __fadd_rn(a.residual[at], value);
+    a.out[part][at] = value;
+  }
+}
+
 // The same chain for operands that 16-byte copies cannot fetch (k not a multiple of 4, unaligned pointers).
 __global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict__ x, int64_t m, int64_t k,
                                                          const float* __restrict__ w, int64_t n,
@@ -161,8 +293,26 @@ static cudaError_t launch_dense_t(const DenseArgs& a, cudaStream_t stream) {
   return launch_chained(kernel, dim3(tiles, (unsigned)((a.m + 8 * MT - 1) / (8 * MT))), dim3(256), smem, stream, a);
 }
 
+bool dense_narrow_supported(const DenseArgs& a) {
+  return dense_linear_supported(a) && a.m <= kNarrowRows && narrow_smem(a) <= kNarrowSmem && ((uintptr_t)a.norm_weight % 16) == 0;
+}
+
+template <bool SWIGLU>
+static cudaError_t launch_narrow(const DenseArgs& a, cudaStream_t stream) {
+  // Four warps, one per scheduler: a 16-byte load takes eight cycles of a scheduler's register path, be it a broadcast input or
+  // a weight, so that a row per warp (two loads to 16 cycles of chained FMAs) does better than two rows in each of two warps.
+  auto kernel = a.m <= 4 ? dense_narrow_kernel<1, SWIGLU> : a.m <= 8 ? dense_narrow_kernel<2, SWIGLU> : dense_narrow_kernel<4, SWIGLU>;
+  const cudaError_t attr = opt_in_shared_memory(kernel, kNarrowSmem);
+  if (attr != cudaSuccess) return attr;
+  unsigned tiles = 0;
+  for (int p = 0; p < (SWIGLU ? 1 : a.parts); ++p) tiles += (unsigned)((a.n[p] + (SWIGLU ? 15 : 31)) / (SWIGLU ? 16 : 32));
+  return launch_chained(kernel, dim3(tiles), dim3(kNarrowThreads), narrow_smem(a), stream, a);
+}
+
 cudaError_t launch_dense_linear(const DenseArgs& a, cudaStream_t stream) {
   if (a.m == 0 || a.n[0] == 0) return cudaSuccess;
+  if (dense_narrow_supported(a)) return a.swiglu ? launch_narrow<true>(a, stream) : launch_narrow<false>(a, stream);
+  if (a.norm_weight) return cudaErrorInvalidValue;
   if (!dense_linear_supported(a)) {
     if (a.swiglu) return cudaErrorInvalidValue;
     for (int p = 0; p < a.parts; ++p) {
@@ -215,22 +365,8 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
   }
 }
 
-__device__ __forceinline__ double square4(const float4& v) {
-  return (double)v.x * (double)v.x + (double)v.y * (double)v.y + (double)v.z * (double)v.z + (double)v.w * (double)v.w;
-}
-__device__ __forceinline__ float4 scale4(const float4& v, double scale, const float4& w) {
-  return make_float4((float)__dmul_rn(__dmul_rn((double)v.x, scale), (double)w.x), (float)__dmul_rn(__dmul_rn((double)v.y, scale), (double)w.y),
-                     (float)__dmul_rn(__dmul_rn((double)v.z, scale), (double)w.z), (float)__dmul_rn(__dmul_rn((double)v.w, scale), (double)w.w));
-}
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  return v;
-}
-
 // Single-pass variants for n <= 8192, n % 4 == 0: the row stays in registers between the reduction and the scaling (same
 // f64 arithmetic). f32 row-major:
-constexpr int kNormThreads = 256, kNormItems = 8192 / 4 / kNormThreads;
 __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const float* x, const float* weight, double eps, int n,
                                                                    float* out) {
   __shared__ double partial[kNormThreads / 32];

@@ -178,7 +178,10 @@ struct DenseArgs {
   const float* residual = nullptr;  // parts == 1 only
   int swiglu = 0, exact = 0;
   int constant_weights = 0;         // no earlier kernel of the stream writes the weights: they are fetched ahead of it
+  const float* norm_weight = nullptr;  // x goes through RMSNorm on the way; only where dense_narrow_supported
+  double norm_eps = 0.0;
 };
+bool dense_narrow_supported(const DenseArgs& a);  // few rows, 32 weight rows and all inputs in shared memory
 bool dense_linear_supported(const DenseArgs& a);  // k a multiple of 4, 16-byte aligned operands
 cudaError_t launch_dense_linear(const DenseArgs& a, cudaStream_t stream);
 cudaError_t launch_linear_f32(const float* x, int64_t m, int64_t k, const float* w, int64_t n, const float* bias,
@@ -252,6 +255,11 @@ cudaError_t launch_attention_mma(const PoolView& pool, const float* q, const Lan
                                  int batch, int q_heads, double scale, long long op_window, float* out,
                                  const AttnPlan& plan, float* scratch, cudaStream_t stream, int* launches,
                                  __half* out_xh = nullptr, int xh_nv = 32, int tokens = 1, const FusedRope* rope = nullptr);
+// RoPE, append and reference-order attention of a decode step (f32 cache, contexts of at most max_ctx in shared memory). As with
+// FusedRope, all it reads but qkv must have been written before the launches of this step.
+bool attention_exact_step_supported(const PoolView& pool, int q_heads, int max_ctx);
+cudaError_t launch_attention_exact_step(const PoolView& pool, const float* qkv, const LaneInfo* lanes, const int* tables, const double* inv_freq, int layout,
+                                        int batch, int q_heads, double scale, long long op_window, float* out, int max_ctx, cudaStream_t stream);
 // Fused RoPE(q), RoPE(k) and KV append: qkv [B * tokens, (Hq+2*Hkv)*D] f32 (the fused projection output) ->
 // q_out [B, tokens, Hq, D] f32 rotated, K/V rows written to the pool at positions cursor .. cursor + tokens - 1.
 cudaError_t launch_rope_append(const PoolView& pool, const float* qkv, const LaneInfo* lanes, const int* tables,

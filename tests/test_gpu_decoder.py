@@ -587,6 +587,30 @@ def test_steps_of_wide_q8_0_layers_repeat_bit_for_bit():
             assert np.array_equal(got, want), f"run {i}, step {step}: {(got != want).sum()} logits differ"
 
 
+@pytest.mark.parametrize("geometry,batch,window", [
+    (dict(d_model=160, q_heads=6, kv_heads=3, head_dim=32, ffn=200, vocab=777), 7, None), (dict(d_model=68, q_heads=3, kv_heads=1, head_dim=20, ffn=36, vocab=33), 1, 7),
+    (dict(d_model=256, q_heads=2, kv_heads=2, head_dim=128, ffn=1320, vocab=100), 12, None)])
+def test_f32_steps_with_norm_and_rope_inside_their_neighbours(geometry, batch, window):
+    """Reference-order steps whose norms ride along with the projections and whose attention rotates and appends: widths that
+    do not fill tiles, one row, more than eight, a padded lane, an f32 context that grows across pages and one beyond shared
+    memory (the third model: 128 x 2 columns, 290 tokens). Logits as on the tiny model."""
+    cfg = dict(geometry, layers=2, rms_eps=1e-5, rope_theta=10000.0)
+    w = helpers.make_weights(cfg, seed=8)
+    rng = np.random.default_rng(batch)
+    active = max(1, batch - 1)
+    max_tokens = batch * 320
+    odec = helpers.oracle_decoder(cfg, w, batch=batch, window=window)
+    gdec = gpu_decoder(cfg, w, batch=batch, max_tokens=max_tokens, max_advance=64, window=window)
+    opool = orc.Pool(2, cfg["kv_heads"], cfg["head_dim"], max_tokens, 16, orc.F32)
+    gpool = et.NativeKvPool(runtime(), 2, cfg["kv_heads"], cfg["head_dim"], max_tokens, 16, et.KV_F32)
+    oseqs, gseqs = [opool.make_sequence() for _ in range(active)], [gpool.makeSequence() for _ in range(active)]
+    for advance in (1, 13, 1, 1, 1, 1) + ((60,) * 4 + (30, 1, 1) if cfg["head_dim"] == 128 else (5, 1, 1)):
+        toks = rng.integers(0, cfg["vocab"], size=(active, advance)).astype(np.uint32)
+        ol, _ = odec.execute(opool, oseqs, toks)
+        gl = gdec.execute(gpool, gseqs, toks)
+        assert helpers.rel_err(gl, ol) <= 1e-5, f"advance {advance}"
+
+
 @pytest.mark.parametrize("d_model", [1088, 4160, 8192])
 def test_norms_at_the_edges_of_their_row_widths(d_model):
     """Residual widths that end inside a cluster's share, just above the width of the narrower form and at the limit, for

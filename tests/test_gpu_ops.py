@@ -87,7 +87,8 @@ def test_argmax_large_rows_and_non_finite_logits():
         rt.synchronize()
 
 
-@pytest.mark.parametrize("m,k,n", [(1, 4, 1), (16, 64, 33), (17, 68, 31), (33, 260, 65), (5, 192, 640), (3, 66, 40)])
+@pytest.mark.parametrize("m,k,n", [(1, 4, 1), (16, 64, 33), (17, 68, 31), (33, 260, 65), (5, 192, 640), (3, 66, 40),
+                                   (2, 1500, 33), (4, 1024, 32), (8, 1536, 48), (9, 28, 40), (16, 688, 70), (4, 1700, 33)])
 def test_dense_linear_at_the_edges_of_its_tiles(m, k, n):
     """Stages that are not full, rows and columns that do not fill a tile, both row counts per CTA, and a k that 16-byte copies
     cannot fetch: every element one fused multiply-add chain over k, bit for bit."""
