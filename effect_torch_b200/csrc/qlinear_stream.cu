@@ -524,13 +524,19 @@ StreamPlan plan_stream(const TiledWeight& w, int64_t vectors, int sm_count, bool
     const int splits = std::min(std::max(1, sms * (p.nv <= 64 ? 2 : 1) / p.tiles), std::max(1, p.stages / 2));
     p.stages_per_split = (p.stages + splits - 1) / splits;
   } else {
-    // The stages of the fullest SM, a third more when it has one CTA (nothing overlaps its waits), plus two per CTA of a
-    // cluster for its exchange (measured on 32 to 112 tiles). Clusters are powers of two (three or six CTAs pack a GPC badly)
-    // and are used while all of them are resident at once: [128256 x 4096] takes 73 us with one CTA per tile, 96 with two.
+    // In stages: those of the fullest SM less what its CTAs expand ahead of the activations (one and a half each), more for a
+    // CTA that has an SM for itself (nothing overlaps its waits; the exact form's are longer), and a cluster's exchange, which
+    // grows with the vectors. Clusters are powers of two (three or six CTAs pack a GPC badly) and are used while all of them are
+    // resident at once, or nearly ([128256 x 4096] takes 73 us with one CTA per tile, 96 with two); from four CTAs on seven
+    // eighths of the places can be filled, beyond that a second wave follows. Measured back to back over 4 to 144 tiles, 8 to
+    // 112 stages, 1 to 100 vectors; against a rule that did not count the work done ahead: [4096 x 4096] x 1 7.9 -> 6.8 us,
+    // [2048 x 4096] x 8 8.6 -> 7.3, [9216 x 14336] x 24 30.6 -> 23.2, [4096 x 4096] x 100 13.8 both.
+    const double single = exact ? 1.5 : 1.1, exchange = p.nv <= 32 ? 1.0 : p.nv == 64 ? 2.25 : 2.5;
     double best = 1e30;
-    for (int s = 1; s <= std::min(kMaxStreamCluster, std::max(1, p.stages / 2)) && (s == 1 || p.tiles * s <= 2 * sms); s *= 2) {
+    for (int s = 1, log = 0; s <= std::min(kMaxStreamCluster, std::max(1, p.stages / 2)) && (s == 1 || p.tiles * s <= 2 * sms); s *= 2, ++log) {
       const int per = (p.stages + s - 1) / s, ctas = (p.tiles * s + sms - 1) / sms;
-      const double cost = ctas * per * (ctas > 1 ? 1.0 : 1.33) + 2.0 * s;
+      const int waves = s >= 4 && p.tiles * s > 2 * sms * 7 / 8 ? ctas + 1 : ctas;
+      const double cost = waves * std::max(per - 1.5, 0.5) * (waves > 1 ? 1.0 : single) + log * exchange;
       if (cost < best) { best = cost; p.stages_per_split = per; }
     }
   }
