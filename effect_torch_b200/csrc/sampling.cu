@@ -13,12 +13,15 @@
 // are in candidate order, finds the bin in which a running sum crosses its target; that bin's few hundred candidates are
 // gathered into the first CTA, sorted by key and summed in order. A bin that holds more than the list (rows with few
 // distinct values, or everything far below the maximum) is narrowed by 10 bits of the key at a time first. When top_k
-// leaves few enough candidates the list holds all of them and decides everything, and only they are exponentiated.
+// leaves few enough candidates the list holds all of them and decides everything, and only they are exponentiated; the bins
+// they are in follow from the threads' largest candidates alone, and only threads whose largest is in them look again.
 // The token-order walk is a prefix sum over the warps' slices and a second look at the one that holds the draw.
 //
 // What bounds it: at 32 rows x 128256 the logits are 16 MB (2.5 us of HBM); the rest is latency, half a dozen passes over
 // shared memory with a cluster barrier (about a microsecond) between them. A single CTA per row that re-read the row for
-// each of 7 radix digits per select, with f64 atomics on 256 bins, took 2192 us with top-k 40 and top-p 0.95; this takes 24.6.
+// each of 7 radix digits per select, with f64 atomics on 256 bins, took 2192 us with top-k 40 and top-p 0.95; a histogram of all
+// candidates, four-byte loads and a sorting network for any list 24.6; this takes 18.4 (one row 18.8 -> 14.3; 8 rows with top-p
+// alone 45.1 -> 37.7). 64 registers: two CTAs per SM (at 128 and one CTA 32.6 us).
 //
 // Sums are f64 like the reference's but associated differently (histogram bins, scans), so a comparison of a running sum
 // against the draw or the top-p threshold can come out differently only when the two are within about vocab x 2^-52 of
@@ -40,6 +43,7 @@ constexpr int kSampleThreads = 512;
 constexpr int kSampleWarps = kSampleThreads / 32;
 constexpr int kBins = 1024;           // also the digits of a narrowing step (10 bits of the key)
 constexpr int kList = 1024;           // candidates that can be sorted
+constexpr int kRankSorted = 256;      // up to this many by counting (two barriers) instead of a network of them (36 for 256)
 constexpr int kMaxSlice = 16384;      // logits a CTA keeps in shared memory (64 KB: two CTAs per SM)
 constexpr int kMaxSampleCluster = 8;  // the portable cluster size
 constexpr int kSliceTarget = 4096;    // a row is spread over more CTAs until a slice is this short
@@ -79,7 +83,7 @@ __device__ __forceinline__ float key_value(uint64_t key) {
   return __uint_as_float((ordered & 0x80000000u) ? (ordered ^ 0x80000000u) : ~ordered);
 }
 
-struct Shared {
+struct alignas(16) Shared {
   double weight[kBins];       // this CTA's bins; in the first CTA afterwards: inclusive sums over the row's bins
   double sum[kBins];
   uint32_t count[kBins];
@@ -114,6 +118,7 @@ struct Scope {
   int shift = 0;
   uint64_t prefix = 0, mask = 0, floor_key = 0;
   __device__ __forceinline__ int first_level(float v) const { return (int)fminf((best - v) * per_unit, (float)(kBins - 1)); }
+  __device__ __forceinline__ bool whole() const { return bin < 0 && floor_key == 0; }  // every candidate, by first-level bins
   // -1: not in scope
   __device__ __forceinline__ int digit(float v, uint64_t key) const {
     if (key < floor_key) return -1;
@@ -132,22 +137,42 @@ struct Row {
   int n;
   uint32_t token0;
   double mx, temperature;
+  bool quads;        // x + n start on 16 bytes: a thread's candidates are groups of four
+  float mine;        // the largest of this thread's candidates
   __device__ double weight_of(float v) const { return exp(((double)v - mx) / temperature); }
 
-  // Inclusive sums of the cluster's bins, in the first CTA. WEIGHTED: of weights too.
-  template <bool WEIGHTED>
+  // f(index, value) for each of this thread's candidates.
+  template <typename F>
+  __device__ __forceinline__ void each(F&& f) const {
+    const int n4 = quads ? n / 4 : 0;
+    for (int q = threadIdx.x; q < n4; q += kSampleThreads) {
+      const float4 v = reinterpret_cast<const float4*>(x)[q];
+      f(4 * q, v.x);
+      f(4 * q + 1, v.y);
+      f(4 * q + 2, v.z);
+      f(4 * q + 3, v.w);
+    }
+    for (int i = 4 * n4 + threadIdx.x; i < n; i += kSampleThreads) f(i, x[i]);
+  }
+
+  // Inclusive sums of the cluster's bins, in the first CTA. WEIGHTED: of weights too. LARGEST: of each thread's largest
+  // candidate only.
+  template <bool WEIGHTED, bool LARGEST = false>
   __device__ void histogram(const Scope& scope) {
     for (int b = threadIdx.x; b < kBins; b += kSampleThreads) {
       sh.count[b] = 0u;
       if (WEIGHTED) sh.weight[b] = 0.0;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += kSampleThreads) {
-      const float v = x[i];
-      const int b = scope.digit(v, sort_key(v, token0 + (uint32_t)i));
-      if (b < 0) continue;
-      atomicAdd(&sh.count[b], 1u);
-      if (WEIGHTED) atomicAdd(&sh.weight[b], weight_of(v));
+    if (LARGEST) {
+      if (mine > -INFINITY) atomicAdd(&sh.count[scope.first_level(mine)], 1u);
+    } else {
+      each([&](int i, float v) {
+        const int b = scope.whole() ? scope.first_level(v) : scope.digit(v, sort_key(v, token0 + (uint32_t)i));
+        if (b < 0) return;
+        atomicAdd(&sh.count[b], 1u);
+        if (WEIGHTED) atomicAdd(&sh.weight[b], weight_of(v));
+      });
     }
     cluster.sync();
     if (cluster.block_rank() == 0) {
@@ -155,13 +180,24 @@ struct Row {
       const int b0 = threadIdx.x * PER, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
       uint32_t c[PER] = {};
       double w[PER] = {};
-      for (unsigned r = 0; r < cluster.num_blocks(); ++r) {
-        const Shared* peer = cluster.map_shared_rank(&sh, r);
+      static_assert(PER == 2 && kMaxSampleCluster % 4 == 0, "a pair of bins per thread");
+      for (unsigned r0 = 0; r0 < cluster.num_blocks(); r0 += 4) {  // four peers' bins are requested before the first is added
+        uint2 counts[4];
+        double2 weights[4];
 #pragma unroll
-        for (int j = 0; j < PER; ++j) {
-          c[j] += peer->count[b0 + j];
-          if (WEIGHTED) w[j] += peer->weight[b0 + j];
-        }
+        for (unsigned u = 0; u < 4; ++u)
+          if (r0 + u < cluster.num_blocks()) {
+            const Shared* peer = cluster.map_shared_rank(&sh, r0 + u);
+            counts[u] = *reinterpret_cast<const uint2*>(peer->count + b0);
+            if (WEIGHTED) weights[u] = *reinterpret_cast<const double2*>(peer->weight + b0);
+          }
+#pragma unroll
+        for (unsigned u = 0; u < 4; ++u)
+          if (r0 + u < cluster.num_blocks()) {
+            c[0] += counts[u].x;
+            c[1] += counts[u].y;
+            if (WEIGHTED) { w[0] += weights[u].x; w[1] += weights[u].y; }
+          }
       }
       // counts are exact in f64 too, so one scan over (count, weight) pairs
       uint32_t cs = 0;
@@ -216,19 +252,43 @@ struct Row {
     cluster.sync();
   }
 
-  // Candidates of the bins [lo, hi] of the scope, sorted by descending key, in the first CTA's list (at most kList).
-  __device__ void gather(const Scope& scope, int lo, int hi) {
-    for (int i = threadIdx.x; i < n; i += kSampleThreads) {
-      const float v = x[i];
-      const uint64_t key = sort_key(v, token0 + (uint32_t)i);
-      const int b = scope.digit(v, key);
-      if (b < lo || b > hi) continue;
+  // Candidates of the bins [lo, hi] of the scope into the first CTA's list (the first kList of them; `listed` counts all).
+  __device__ void collect(const Scope& scope, int lo, int hi) {
+    const auto list = [&](uint64_t key) {
       const uint32_t at = atomicAdd(&first.listed, 1u);
       if (at < (uint32_t)kList) first.key[at] = key;
+    };
+    if (scope.whole() && lo == 0) {
+      if (scope.first_level(mine) <= hi)  // (-infinity, of a thread without candidates, is in the last bin)
+        each([&](int i, float v) {
+          if (scope.first_level(v) <= hi) list(sort_key(v, token0 + (uint32_t)i));
+        });
+    } else {
+      each([&](int i, float v) {
+        const uint64_t key = sort_key(v, token0 + (uint32_t)i);
+        const int b = scope.digit(v, key);
+        if (b >= lo && b <= hi) list(key);
+      });
     }
     cluster.sync();
+  }
+
+  // The first CTA sorts its list by descending key.
+  __device__ void sort_list() {
     if (cluster.block_rank() != 0) return;
     const int m = min((int)sh.listed, kList);
+    if (m <= kRankSorted) {  // no two keys are alike: a key's place is the number of larger ones
+      const uint64_t mine_key = threadIdx.x < m ? sh.key[threadIdx.x] : 0ull;
+      int place = 0;
+      if (threadIdx.x < m) {
+#pragma unroll 8
+        for (int j = 0; j < m; ++j) place += sh.key[j] > mine_key;
+      }
+      __syncthreads();
+      if (threadIdx.x < m) sh.key[place] = mine_key;
+      __syncthreads();
+      return;
+    }
     int padded = 32;
     while (padded < m) padded <<= 1;
     for (int i = m + threadIdx.x; i < padded; i += kSampleThreads) sh.key[i] = 0ull;
@@ -315,7 +375,8 @@ struct Row {
       }
       cluster.sync();  // the decision is read before the next one is written
     }
-    gather(scope, lo, hi);
+    collect(scope, lo, hi);
+    sort_list();
     if (cluster.block_rank() == 0) {
       const int m = min((int)sh.listed, kList);
       accumulate(m, weighted);
@@ -332,7 +393,7 @@ struct Row {
   }
 };
 
-__global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(SampleArgs a) {
+__global__ void __launch_bounds__(kSampleThreads, 2) sample_rows_kernel(SampleArgs a) {
   extern __shared__ __align__(16) float cache[];
   __shared__ Shared sh;
   cg::cluster_group cluster = cg::this_cluster();
@@ -348,19 +409,45 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(SampleArgs 
     if (!isfinite(v)) bad = min(bad, (long long)(begin + i));
     best = fmaxf(best, v);
   };
-  if (a.cached) {
-    int i = threadIdx.x;
+  // in groups of four where the slice starts on 16 bytes, four of them in flight per thread
+  const bool quads = (reinterpret_cast<uintptr_t>(source) & 15) == 0;
+  const int n4 = quads ? n / 4 : 0;
+  constexpr int IN_FLIGHT = 4;
+  for (int q0 = threadIdx.x; q0 < n4; q0 += IN_FLIGHT * kSampleThreads) {
+    float4 v[IN_FLIGHT];
+#pragma unroll
+    for (int u = 0; u < IN_FLIGHT; ++u)
+      if (q0 + u * kSampleThreads < n4) v[u] = reinterpret_cast<const float4*>(source)[q0 + u * kSampleThreads];
+#pragma unroll
+    for (int u = 0; u < IN_FLIGHT; ++u) {
+      const int q = q0 + u * kSampleThreads;
+      if (q >= n4) break;
+      if (a.cached) reinterpret_cast<float4*>(cache)[q] = v[u];
+      see(4 * q, v[u].x);
+      see(4 * q + 1, v[u].y);
+      see(4 * q + 2, v[u].z);
+      see(4 * q + 3, v[u].w);
+    }
+  }
+  {
+    int i = 4 * n4 + threadIdx.x;
     for (; i + 3 * kSampleThreads < n; i += 4 * kSampleThreads) {  // four loads in flight
       float v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) v[u] = source[i + u * kSampleThreads];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) { cache[i + u * kSampleThreads] = v[u]; see(i + u * kSampleThreads, v[u]); }
+      for (int u = 0; u < 4; ++u) {
+        if (a.cached) cache[i + u * kSampleThreads] = v[u];
+        see(i + u * kSampleThreads, v[u]);
+      }
     }
-    for (; i < n; i += kSampleThreads) { const float v = source[i]; cache[i] = v; see(i, v); }
-  } else {
-    for (int i = threadIdx.x; i < n; i += kSampleThreads) see(i, source[i]);
+    for (; i < n; i += kSampleThreads) {
+      const float v = source[i];
+      if (a.cached) cache[i] = v;
+      see(i, v);
+    }
   }
+  const float mine = best;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, off));
@@ -377,11 +464,13 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(SampleArgs 
   cluster.sync();
   best = -INFINITY;
   bad = 0x7fffffffffffffffll;
-  for (int r = 0; r < ranks; ++r) {
-    const Shared* peer = cluster.map_shared_rank(&sh, r);
-    best = fmaxf(best, peer->best);
-    bad = min(bad, peer->bad);
-  }
+#pragma unroll
+  for (int r = 0; r < kMaxSampleCluster; ++r)
+    if (r < ranks) {
+      const Shared* peer = cluster.map_shared_rank(&sh, r);
+      best = fmaxf(best, peer->best);
+      bad = min(bad, peer->bad);
+    }
   if (bad != 0x7fffffffffffffffll) {  // the same answer in every CTA of the row
     if (rank == 0 && threadIdx.x == 0) {
       a.tokens[row] = 0u;
@@ -393,7 +482,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(SampleArgs 
     cluster.sync();
     return;
   }
-  Row r{cluster, sh, *cluster.map_shared_rank(&sh, 0), a.cached ? cache : source, n, (uint32_t)begin, (double)best, a.temperature};
+  Row r{cluster, sh, *cluster.map_shared_rank(&sh, 0), a.cached ? cache : source, n, (uint32_t)begin, (double)best, a.temperature, quads, mine};
   const double unit = random_unit(a.seeds ? a.seeds[row] : a.seed, a.counters ? a.counters[row] : a.counter);
   const bool has_top_k = a.top_k > 0 && a.top_k < a.vocab;
 
@@ -439,13 +528,11 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(SampleArgs 
   scope.best = best;
   scope.per_unit = fminf((float)(32.0 / a.temperature), 1e30f);  // bins of 1/32 in the logarithm of the weight, the last one open
   if (has_top_k) {
-    r.histogram<false>(scope);
-    r.find_bin(0.0, (double)a.top_k, kReaches);
-    if (r.first.decision.up_to <= (uint32_t)kList) {
-      // ---- few enough: the list decides everything
-      r.gather(scope, 0, r.first.decision.bin);
-      if (rank != 0) return;
+    // The list decides everything where it holds the first top_k candidates. They are in the bins up to the one at which a count
+    // of the threads' largest candidates alone reaches top_k, and only the threads whose largest is there have any.
+    const auto from_list = [&] {
       const int k = (int)a.top_k;
+      r.sort_list();
       r.accumulate(k, true);
       int kept = k;
       double total = sh.cumulative[k - 1];
@@ -455,6 +542,25 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(SampleArgs 
       }
       const int at = min(r.find_listed(kept, 0.0, unit * total, kExceeds), kept - 1);
       if (threadIdx.x == 0) a.tokens[row] = key_token(sh.key[at]);
+    };
+    if (a.top_k <= kList) {
+      r.histogram<false, true>(scope);
+      r.find_bin(0.0, (double)a.top_k, kReaches);
+      const int bin = r.first.decision.bin;
+      if (bin >= 0) {
+        r.collect(scope, 0, bin);
+        const bool fits = r.first.listed <= (uint32_t)kList;
+        cluster.barrier_arrive();  // the first CTA stays until the others have read that
+        if (fits && rank == 0) from_list();
+        cluster.barrier_wait();
+        if (fits) return;
+      }
+    }
+    r.histogram<false>(scope);
+    r.find_bin(0.0, (double)a.top_k, kReaches);
+    if (r.first.decision.up_to <= (uint32_t)kList) {
+      r.collect(scope, 0, r.first.decision.bin);
+      if (rank == 0) from_list();
       return;
     }
     r.resolve(scope, false, (double)a.top_k, kReaches);

@@ -163,6 +163,27 @@ def test_device_sampling_at_the_edges_of_its_slices_and_lists(vocab):
             np.testing.assert_array_equal(host(tokens), want, err_msg=str(mode))
 
 
+@pytest.mark.parametrize("vocab", [1025, 8200, 100003])
+@pytest.mark.parametrize("top_k", [1, 31, 255, 256, 257, 1023, 1024])
+def test_top_k_lists_at_the_edges_of_their_sorts(vocab, top_k):
+    """List lengths around what is sorted by counting and what the list holds; a row of ties, one whose largest candidates all
+    sit with one thread (so that its neighbours' largest reach far down), one with fewer candidates above the floor than
+    top_k; slices that do not start on 16 bytes."""
+    rt = runtime()
+    rng = np.random.default_rng(vocab + top_k)
+    rows = 5
+    logits = (rng.normal(size=(rows, vocab)) * 2.0).astype(np.float32)
+    logits[1] = np.round(logits[1] * 8.0) / 8.0
+    logits[2, np.arange(0, min(vocab, 64 * 512), 512)] += 40.0
+    logits[3] = np.where(rng.random(vocab) < 20.0 / vocab, logits[3], np.float32(-200.0))
+    d = dev(logits)
+    tokens = empty(rows, dtype=torch.int32)
+    for seed, top_p in ((1, 1.0), (2, 0.9), (3, 0.999)):
+        rt.sample_rows_into(d, rows, vocab, tokens, temperature=0.9, top_k=top_k, top_p=top_p, seed=seed)
+        want = [orc.sample_logits(row, temperature=0.9, top_k=top_k, top_p=top_p, seed=seed) for row in logits]
+        np.testing.assert_array_equal(host(tokens), want)
+
+
 def seed_of_the_largest_draw():
     """The seed whose draw at counter 0 is 1 - 2^-53, the largest there is: the splitmix64 steps run backwards."""
     bits = (1 << 64) - 1
