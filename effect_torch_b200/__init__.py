@@ -10,6 +10,7 @@ without the built library, or calling them without a CUDA device, raises.
 from __future__ import annotations
 
 import ctypes as C
+import importlib
 import sys
 import threading
 import weakref
@@ -87,6 +88,41 @@ def _result_buffer(shape) -> np.ndarray:
     return array
 
 
+class _ThroughCtypes:
+    """The functions of the extension module (calls.cpp) where it could not be built."""
+
+    def __getattr__(self, name):
+        if name.startswith("_"):
+            raise AttributeError(name)
+        entry = getattr(_lib.load(), "etc_" + name)
+        extra = (None,) * (len(entry.argtypes) - {"qlinear_into": 9}.get(name, len(entry.argtypes)))  # no cancellation flag
+
+        def call(*args):
+            return entry(*(a if a is None or isinstance(a, (int, float)) else _ptr(a) for a in args), *extra)
+
+        setattr(self, name, call)
+        return call
+
+
+class _LoadedOnUse:
+    """Stands in for the extension module until an operator is called: it links to the library, which has to be there first."""
+
+    def __getattr__(self, name):
+        global _calls
+        if name.startswith("_"):
+            raise AttributeError(name)
+        _lib.load()
+        try:
+            module = importlib.import_module(__name__ + "._calls")
+        except ImportError:
+            module = _ThroughCtypes()
+        _calls = module
+        return getattr(module, name)
+
+
+_calls = _LoadedOnUse()
+
+
 def device_count() -> int:
     n = C.c_int(0)
     _check(_lib.load().etc_device_count(C.byref(n)))
@@ -135,7 +171,7 @@ class Runtime:
         self.L = _lib.load()
         h = C.c_void_p()
         _check(self.L.etc_runtime_create(device, C.byref(h)))
-        self.h = h
+        self.h = h.value
         self.device = device
 
     def close(self):
@@ -186,13 +222,16 @@ class Runtime:
 
     # ---- ops on device tensors (torch tensors or raw device addresses) -------------------
     def dequantize_into(self, codec, packed, rows, columns, out):
-        _check(self.L.etc_dequantize_into(self.h, codec, _ptr(packed), rows, columns, _ptr(out)))
+        _check(_calls.dequantize_into(self.h, codec, packed, rows, columns, out))
 
     def quantize_into(self, codec, x, rows, columns, packed):
-        _check(self.L.etc_quantize_into(self.h, codec, _ptr(x), rows, columns, _ptr(packed)))
+        _check(_calls.quantize_into(self.h, codec, x, rows, columns, packed))
 
     def qlinear_into(self, codec, x, vectors, columns, weight, rows, bias, out, cancelled=None):
-        flag = None if cancelled is None else C.cast(C.pointer(C.c_int(int(cancelled))), C.c_void_p)
+        if cancelled is None:
+            _check(_calls.qlinear_into(self.h, codec, x, vectors, columns, weight, rows, bias, out))
+            return
+        flag = C.cast(C.pointer(C.c_int(int(cancelled))), C.c_void_p)
         _check(self.L.etc_qlinear_into(self.h, codec, _ptr(x), vectors, columns, _ptr(weight), rows, _ptr(bias), _ptr(out), flag))
 
     def qembedding_into(self, codec, indexes, index_is_i64, count, weight, rows, columns, out):
@@ -226,8 +265,8 @@ class Runtime:
     def sample_rows_into(self, logits, rows, vocab, tokens, temperature=1.0, top_k=None, top_p=1.0, seed=0, counter=0, seeds=None,
                          counters=None):
         """One token per row into the device tensor `tokens` (uint32); per-row (seed, counter) as device u64 tensors, or the scalars."""
-        _check(self.L.etc_sample_rows_into(self.h, _ptr(logits), rows, vocab, temperature, 0 if top_k is None else top_k, top_p, seed,
-                                           counter, _ptr(seeds), _ptr(counters), _ptr(tokens)))
+        _check(_calls.sample_rows_into(self.h, logits, rows, vocab, temperature, 0 if top_k is None else top_k, top_p, seed, counter, seeds,
+                                       counters, tokens))
 
     def kv_attention_into(self, pool, layer, seqs, batch, active, advance, q, k, v, q_heads, tokens, scale, op_window=None,
                           pool_window=None, out=None):
@@ -259,9 +298,8 @@ class Runtime:
     def paged_attention_into(self, pool, layer, lanes, tables, batch, max_pages, q, q_heads, scale, out, scratch, scratch_bytes,
                              op_window=None):
         """Flash-decoding over device-resident lane descriptors [batch, 4] i32 and block tables (asynchronous, capturable)."""
-        _check(self.L.etc_paged_attention_into(self.h, pool.h, layer, _ptr(lanes), _ptr(tables), batch, max_pages, _ptr(q), q_heads,
-                                               scale, NO_WINDOW if op_window is None else op_window, _ptr(out), _ptr(scratch),
-                                               scratch_bytes))
+        _check(_calls.paged_attention_into(self.h, pool.h, layer, lanes, tables, batch, max_pages, q, q_heads, scale,
+                                           NO_WINDOW if op_window is None else op_window, out, scratch, scratch_bytes))
 
 
 def peer_region_bytes(capacity: int, world: int) -> int:
@@ -279,7 +317,7 @@ class QWeight:
         rows = (C.c_int64 * n)(*part_rows)
         h = C.c_void_p()
         _check(rt.L.etc_qweight_create(rt.h, codec, ptrs, rows, n, columns, int(interleave8), int(on_device), C.byref(h)))
-        self.h = h
+        self.h = h.value
         self.rows = sum(part_rows)
         self.columns = columns
         self.interleave8 = interleave8
@@ -307,8 +345,7 @@ class QWeight:
         return b.value
 
     def linear_into(self, x, vectors, out, bias=None, residual=None, epilogue=EPILOGUE_NONE, scratch=None, scratch_bytes=0):
-        _check(self.rt.L.etc_qlinear_tiled_into(self.rt.h, self.h, _ptr(x), vectors, _ptr(bias), _ptr(residual), epilogue,
-                                                _ptr(out), _ptr(scratch), scratch_bytes))
+        _check(_calls.qlinear_tiled_into(self.rt.h, self.h, x, vectors, bias, residual, epilogue, out, scratch, scratch_bytes))
 
     def linear_static_into(self, x, vectors, out, bias=None, residual=None, epilogue=EPILOGUE_NONE):
         """The same linear with its scratch in the library's fixed device array: the call allocates nothing."""
@@ -335,7 +372,7 @@ class NativeKvPool:
         self.rt = rt
         h = C.c_void_p()
         _check(rt.L.etc_pool_create(rt.h, layers, kv_heads, head_dim, max_tokens, block_size, dtype, C.byref(h)))
-        self.h = h
+        self.h = h.value
         self.layers, self.kv_heads, self.head_dim = layers, kv_heads, head_dim
         self.max_tokens, self.block_size, self.dtype = max_tokens, block_size, dtype
 

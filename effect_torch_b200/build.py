@@ -12,10 +12,12 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libetcuda.so")
+CALLS = os.path.join(HERE, "_calls.so")  # the extension module of calls.cpp
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -39,9 +41,27 @@ def _stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_calls(force: bool = False) -> None:
+    """The CPython module that calls the library without ctypes; without the interpreter's headers there is none."""
+    src, header = os.path.join(HERE, "calls.cpp"), os.path.join(os.path.dirname(HERE), "include", "et_cuda.h")
+    include = sysconfig.get_paths()["include"]
+    if not os.path.exists(os.path.join(include, "Python.h")):
+        return
+    if not force and os.path.exists(CALLS) and os.path.getmtime(CALLS) > max(map(os.path.getmtime, (src, header))):
+        return
+    host_cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
+    subprocess.run([host_cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-I", include, src, "-o", CALLS, LIB, "-Wl,-rpath,$ORIGIN"],
+                   check=True)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not _stale():
-        return LIB
+    if force or _stale():
+        _build_library(verbose)
+    build_calls(force)
+    return LIB
+
+
+def _build_library(verbose: bool) -> None:
     objs = []
     build_dir = os.path.join(HERE, "build")
     os.makedirs(build_dir, exist_ok=True)
@@ -67,7 +87,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
         raise RuntimeError("nvcc failed (see output above)")
     link = [_nvcc(), "-ccbin", host_cxx, "-shared", "-o", LIB] + objs + ["-lcudart"] + ARCH_FLAGS
     subprocess.run(link, check=True)
-    return LIB
 
 
 if __name__ == "__main__":

@@ -393,6 +393,8 @@ struct Row {
   }
 };
 
+// FILTERED: top-k or top-p (a kernel of its own, so that the walk in token order is not held to the other's registers).
+template <bool FILTERED>
 __global__ void __launch_bounds__(kSampleThreads, 2) sample_rows_kernel(SampleArgs a) {
   extern __shared__ __align__(16) float cache[];
   __shared__ Shared sh;
@@ -484,9 +486,9 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_rows_kernel(SampleAr
   }
   Row r{cluster, sh, *cluster.map_shared_rank(&sh, 0), a.cached ? cache : source, n, (uint32_t)begin, (double)best, a.temperature, quads, mine};
   const double unit = random_unit(a.seeds ? a.seeds[row] : a.seed, a.counters ? a.counters[row] : a.counter);
-  const bool has_top_k = a.top_k > 0 && a.top_k < a.vocab;
+  const bool has_top_k = FILTERED && a.top_k > 0 && a.top_k < a.vocab;
 
-  if (!has_top_k && a.top_p >= 1.0) {
+  if constexpr (!FILTERED) {
     // ---- walk in token order: every warp sums its part of the slice, then the one that holds the draw walks it
     const int part = (a.slice + kSampleWarps - 1) / kSampleWarps;
     const int lo = min(n, warp * part), hi = min(n, lo + part);
@@ -521,7 +523,7 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_rows_kernel(SampleAr
     }
     cluster.sync();
     return;
-  }
+  } else {
 
   // ---- filtered: candidates in (value descending, token ascending) order
   Scope scope;
@@ -595,6 +597,7 @@ __global__ void __launch_bounds__(kSampleThreads, 2) sample_rows_kernel(SampleAr
   }
   r.resolve(scope, true, unit * total, kExceeds);
   if (rank == 0 && threadIdx.x == 0) a.tokens[row] = key_token(sh.decision.picked);
+  }
 }
 
 }  // namespace
@@ -607,7 +610,9 @@ cudaError_t launch_sample_rows(const float* logits, int64_t rows, int64_t vocab,
   while (ranks < kMaxSampleCluster && (vocab + ranks - 1) / ranks > kSliceTarget) ranks *= 2;
   const int slice = (int)((vocab + ranks - 1) / ranks);
   SampleArgs a{logits, vocab, temperature, top_p, top_k, seed, counter, seeds, counters, tokens, status, slice, slice <= kMaxSlice};
-  const cudaError_t attr = opt_in_shared_memory(sample_rows_kernel, kMaxSlice * sizeof(float));
+  const bool filtered = (top_k > 0 && top_k < vocab) || top_p < 1.0;
+  auto kernel = filtered ? sample_rows_kernel<true> : sample_rows_kernel<false>;
+  const cudaError_t attr = opt_in_shared_memory(kernel, kMaxSlice * sizeof(float));
   if (attr != cudaSuccess) return attr;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3((unsigned)(rows * ranks));
@@ -620,7 +625,7 @@ cudaError_t launch_sample_rows(const float* logits, int64_t rows, int64_t vocab,
   attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
   config.attrs = attribute;
   config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, sample_rows_kernel, a);
+  return cudaLaunchKernelEx(&config, kernel, a);
 }
 
 }  // namespace etc
