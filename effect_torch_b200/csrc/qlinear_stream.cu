@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
     const unsigned char* scales = w_ring + Cfg::kStageQ + row * (Cfg::kBlockS / kRows);
     bool ok = true;
     // exact form: the first USED sums of this row, and the block scales of the stage whose products are not added yet
-    float sums[Cfg::kExact ? USED : 1], scale[kStageBlocks];
+    float sums[Cfg::kExact ? USED : 1], scale[kStageBlocks], next_scale[kStageBlocks];
 #pragma unroll
     for (int v = 0; v < (Cfg::kExact ? USED : 1); ++v) sums[v] = 0.0f;
     auto load_products = [&](uint32_t taddr, auto& products) {
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
       ok = wait_warp(&w_full[w.at], w.parity, abort_flag);
       if (!ok) break;
       const uint32_t stage = (uint32_t)w.at * Cfg::kStageW;
-      int held_back = 0;
+      uint32_t seen = 0;
       auto slot_is_free = [&] {
         ok = behind < 0 || wait_warp(&done[freed.at], freed.parity, abort_flag);
         if (ok) tc_fence_after();
@@ -203,9 +203,8 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
       if constexpr (Cfg::kExact) {
         if (!slot_is_free()) break;
         // the products of the stage AS before this one (a whole one), whose slot and accumulators this one takes over
-        uint32_t products[GROUP][USED], bits[kStageBlocks], seen = 0;
-#pragma unroll
-        for (int b = 0; b < kStageBlocks; ++b) bits[b] = *reinterpret_cast<const unsigned short*>(scales + stage + b * Cfg::kBlockS);
+        uint32_t products[GROUP][USED];
+        seen = 0;
 #pragma unroll
         for (int b = 0; b < kStageBlocks; ++b) {  // blocks beyond the tile's K hold stale bytes that no MMA reads
           uint32_t regs[16];
@@ -214,6 +213,9 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
             for (int j = 0; j < GROUP; ++j) load_products(my_products + (uint32_t)((b + j) * NV), products[j]);
           }
           expand_codes<CODEC>(payload + stage + b * Cfg::kBlockQ, regs);
+          const uint32_t bits = *reinterpret_cast<const unsigned short*>(scales + stage + b * Cfg::kBlockS);
+          seen |= bits;
+          next_scale[b] = __half2float(__ushort_as_half((unsigned short)bits)) * kCodeUnits;
           tmem_st16(slot_cols + b * 16, regs);
           if (behind >= 0 && b % GROUP == GROUP - 1) {
             tmem_wait_ld();
@@ -222,15 +224,12 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
           }
         }
 #pragma unroll
-        for (int b = 0; b < kStageBlocks; ++b) {
-          seen |= bits[b];
-          scale[b] = __half2float(__ushort_as_half((unsigned short)bits[b])) * kCodeUnits;
-        }
+        for (int b = 0; b < kStageBlocks; ++b) scale[b] = next_scale[b];
         // The scales are used a round later. An arrival on w_empty does not wait for loads whose results nothing has used yet
         // (nor does a fence): the next round's bytes came back as scales, in one step of some fifty where launches overlap
-        // just so. The arrival's address takes every lane's scales in: bits 16 and up of them, which are zero.
+        // just so. The arrival's address takes the scales in, of which bits 16 and up are zero; a load's results are there
+        // for all lanes of the converged warp or for none.
         asm volatile("mov.b32 %0, %0;" : "+r"(seen));
-        held_back = __any_sync(0xffffffffu, seen >> 16);
       } else {
         uint32_t first[kStageBlocks], second[kStageBlocks];
 #pragma unroll
@@ -249,7 +248,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
         if (!ok) break;
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&w_empty[w.at + held_back]);
+      if (lane == 0) mbar_arrive(&w_empty[w.at + (seen >> 16)]);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
