@@ -506,13 +506,38 @@ __device__ __forceinline__ void bytes_to_half2(uint32_t w, uint32_t& lo, uint32_
   hi = *reinterpret_cast<const uint32_t*>(&h);
 }
 
+// SORTED: the lane with `rank` longer ones before it (of equals, the first first), by a CTA that has a thread per lane. CTAs
+// start in the order of their index, so that the longest lanes do not start last and run on alone. 64 lanes of 128 to 4096
+// tokens x 8 heads 98.8 -> 90 us (1.00 of the copy bandwidth).
+constexpr int kMaxSortedLanes = kAttnWarps * 32;
+__device__ __forceinline__ int lane_by_length(const LaneInfo* lanes, int n, int rank) {
+  extern __shared__ __align__(128) unsigned char smem[];  // not in use yet
+  int* lengths = reinterpret_cast<int*>(smem);
+  const int t = threadIdx.x;
+  if (t < n) {
+    const LaneInfo info = lanes[t];
+    lengths[t] = info.advance > 0 ? info.cursor - info.start : -1;
+  }
+  __syncthreads();
+  if (t < n) {
+    const int mine = lengths[t];
+    int before = 0;
+    for (int j = 0; j < n; ++j) before += lengths[j] > mine || (lengths[j] == mine && j < t);
+    if (before == rank) lengths[kMaxSortedLanes] = t;
+  }
+  __syncthreads();
+  const int found = lengths[kMaxSortedLanes];
+  __syncthreads();  // before the first copies overwrite it
+  return __shfl_sync(0xffffffffu, found, 0);
+}
+
 // U8: the int8 tier (code - 128) * scale with one scale per cached row (napi/mod.rs:3474-3476): pages travel as bytes, and the
 // row scales multiply the score columns (K) and the probabilities before P V (V), so the tensor core only ever sees exact small
 // integers. ldmatrix hands a thread four code bytes at a time, which it widens to two f16 pairs in registers: of K the columns
 // 4 t .. 4 t + 3 of a row, which become the operand's columns 2 t, 2 t + 1, 2 t + 8 and 2 t + 9 (the query fragments are
 // permuted alike, inside each sum of 16); of V, transposed, two columns of two rows, which go to two neighbouring output tiles
 // (columns 2 n and 2 n + 1 of every 16).
-template <int D, bool BF16, bool U8, bool FUSED>
+template <int D, bool BF16, bool U8, bool FUSED, bool SORTED>
 __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(std::conditional_t<FUSED, FusedAttnArgs, AttnArgs> a) {
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int RAW_PAGE = kPageTokens * D * (U8 ? 1 : 2);      // one page as cached
@@ -526,7 +551,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(std::con
   const int g = lane >> 2, t = lane & 3;
   chain_release();  // the next kernel of the step may be scheduled; it waits for this one before touching memory
   if (!FUSED) chain_wait();
-  const int split = blockIdx.x, kv_head = blockIdx.y, lane_id = blockIdx.z;
+  const int split = blockIdx.x, kv_head = blockIdx.y;
+  const int lane_id = SORTED ? lane_by_length(a.lanes, gridDim.z, blockIdx.z) : blockIdx.z;
   const LaneInfo info = a.lanes[lane_id];
   const int G = a.q_heads / a.kv_heads;
   const int nsplits = gridDim.x;
@@ -547,9 +573,27 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(std::con
   const unsigned char* kbase = reinterpret_cast<const unsigned char*>(a.k) + (size_t)kv_head * RAW_PAGE;
   const unsigned char* vbase = reinterpret_cast<const unsigned char*>(a.v) + (size_t)kv_head * RAW_PAGE;
 
+  // SORTED: the warp's page numbers, 32 at a time, one per lane: the copies then wait for a shuffle instead of a table look-up
+  // each (of an address that is not known to be uniform: 30 % of a page's time).
+  int held_from = p0 + warp;
+  auto look_up = [&] {
+    const int at = held_from + lane * kAttnWarps;
+    return at < p1 ? table[at] : 0;
+  };
+  int held = SORTED ? look_up() : 0;
+  auto page_of = [&](int page_index) {
+    if (!SORTED) return table[page_index];
+    if (page_index >= held_from + 32 * kAttnWarps) {
+      held_from += 32 * kAttnWarps;
+      held = look_up();
+    }
+    return __shfl_sync(0xffffffffu, held, (page_index - held_from) / kAttnWarps);
+  };
+
   auto issue = [&](int page_index, int stage, bool but_new = false) {
     if (page_index < p1 && !(FUSED && but_new && page_index == new_page)) {
-      const size_t off = (size_t)table[page_index] * page_stride;
+      const int page = page_of(page_index);
+      const size_t off = (size_t)page * page_stride;
       unsigned char* ks = my_smem + stage * STAGE_BYTES;
       unsigned char* vs = ks + RAW_PAGE;
       if (U8) {
@@ -561,7 +605,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_mma_kernel(std::con
           cp_async16(vs + so, vbase + off + (size_t)c * 16);
         }
         if (lane < 8) {
-          const size_t si = ((size_t)table[page_index] * a.kv_heads + kv_head) * kPageTokens;  // 16 floats = 4 chunks each
+          const size_t si = ((size_t)page * a.kv_heads + kv_head) * kPageTokens;  // 16 floats = 4 chunks each
           const float* src = (lane < 4 ? a.k_scale : a.v_scale) + si + (lane & 3) * 4;
           cp_async16(my_smem + stage * STAGE_BYTES + 2 * RAW_PAGE + lane * 16, src);
         }
@@ -1186,6 +1230,7 @@ AttnPlan plan_attention(int batch, int q_heads, int kv_heads, int head_dim, int 
   p.pages_per_split = std::max(1, (max_pages + splits - 1) / splits);
   p.splits = std::max(1, (max_pages + p.pages_per_split - 1) / p.pages_per_split);
   p.scratch_bytes = p.splits > 1 ? (size_t)batch * q_heads * p.splits * (head_dim + 2) * sizeof(float) : 0;
+  p.sm_count = std::max(1, sm_count);
   return p;
 }
 
@@ -1196,7 +1241,7 @@ size_t plan_attention_max_scratch(int batch, int q_heads, int kv_heads, int head
   return need;
 }
 
-template <int D, bool BF16, bool U8, bool FUSED>
+template <int D, bool BF16, bool U8, bool FUSED, bool SORTED>
 static cudaError_t launch_attention_mma_t(const PoolView& pool, const std::conditional_t<FUSED, FusedAttnArgs, AttnArgs>& args, int batch, int grid_x,
                                           cudaStream_t stream) {
   constexpr size_t page = (size_t)kPageTokens * D * 2;
@@ -1204,7 +1249,7 @@ static cudaError_t launch_attention_mma_t(const PoolView& pool, const std::condi
                              : (size_t)kAttnWarps * kAttnStages * 2 * page;
   constexpr size_t merge = (size_t)kAttnWarps * 16 * (D + 2) * sizeof(float);
   constexpr size_t smem = ring > merge ? ring : merge;
-  auto kernel = attention_mma_kernel<D, BF16, U8, FUSED>;
+  auto kernel = attention_mma_kernel<D, BF16, U8, FUSED, SORTED>;
   const cudaError_t attr = opt_in_shared_memory(kernel, smem);
   if (attr != cudaSuccess) return attr;
   dim3 grid((unsigned)grid_x, (unsigned)pool.kv_heads, (unsigned)batch);
@@ -1244,8 +1289,16 @@ cudaError_t launch_attention_mma(const PoolView& pool, const float* q, const Lan
     constexpr int D = decltype(wide)::value ? 128 : 64;
     constexpr bool BF16 = decltype(bf16)::value, U8 = decltype(u8)::value;
     if (tokens > 1) return launch_attention_chunk_t<D, BF16, U8>(args, batch, stream);
-    return rope ? launch_attention_mma_t<D, BF16, U8, true>(pool, args, batch, plan.splits, stream)
-                : launch_attention_mma_t<D, BF16, U8, false>(pool, args, batch, plan.splits, stream);
+    // Longest lanes first from half as many CTAs again as an SM holds at once (by shared memory and registers: two of f16 pages of
+    // 128 columns, three of bytes, four of 64 columns); finding a CTA's lane costs a microsecond, more than it gives below
+    // (320 CTAs of 500 to 600 tokens 25.8 -> 27.6 us).
+    constexpr int kAtOnce = D == 64 ? 4 : U8 ? 3 : 2;
+    const bool sorted = batch <= kMaxSortedLanes && 2ll * batch * pool.kv_heads * plan.splits >= 3ll * kAtOnce * plan.sm_count;
+    auto decode = [&](auto fused, auto longest_first) {
+      return launch_attention_mma_t<D, BF16, U8, decltype(fused)::value, decltype(longest_first)::value>(pool, args, batch, plan.splits, stream);
+    };
+    if (rope) return sorted ? decode(std::true_type(), std::true_type()) : decode(std::true_type(), std::false_type());
+    return sorted ? decode(std::false_type(), std::true_type()) : decode(std::false_type(), std::false_type());
   };
   auto dispatch = [&](auto wide) {
     if (pool.dtype == kKvU8) return launch(wide, std::false_type(), std::true_type());

@@ -237,6 +237,7 @@ struct AttnPlan {
   int splits = 1;
   int pages_per_split = 0;
   size_t scratch_bytes = 0;
+  int sm_count = 1;
 };
 AttnPlan plan_attention(int batch, int q_heads, int kv_heads, int head_dim, int max_pages, int sm_count);
 // Largest scratch plan_attention can ask for with tables of at most max_pages pages.

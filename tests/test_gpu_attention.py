@@ -322,3 +322,46 @@ def test_tensor_core_decode_attention_with_a_window():
     rt.kv_attention_decode_into(gp, 0, [gs], 1, 1, dev(q.reshape(1, Hq, D)), dev(k1.reshape(1, Hkv, D)), dev(v1.reshape(1, Hkv, D)),
                                 Hq, 0.1, op_window=100, out=out)
     assert helpers.rel_err(host(out).reshape(1, Hq, 1, D), expected) <= REL_TOL
+
+
+@pytest.mark.parametrize("tier,D,batch", [(et.KV_F16, 128, 56), (et.KV_BF16, 128, 128), (et.KV_U8, 128, 90), (et.KV_F16, 64, 120)])
+def test_longest_lanes_first_changes_no_result(tier, D, batch):
+    """Many lanes are served by falling length: every lane's result equals, bit for bit, what it is in a batch of 28 to 32,
+    whose lanes go in their own order. Lengths of one token to 70 pages (more than a warp holds page numbers for would need
+    128; 2200 tokens of one lane), equal lengths, lanes without a query and a window."""
+    rt = runtime()
+    rng = np.random.default_rng(batch)
+    Hq, Hkv = 16, 8
+    lengths = rng.integers(1, 90, size=batch)
+    lengths[3], lengths[batch - 1], lengths[5:9] = 2200, 1100, 33
+    pages = int(sum(-(-int(n) // 16) for n in lengths)) + 1
+    pool = et.NativeKvPool(rt, 1, Hkv, D, pages * 16, 16, tier)
+    lanes, table, kept = np.zeros((batch, 4), np.int32), [], []
+    for i, n in enumerate(int(x) for x in lengths):
+        seq = pool.makeSequence()
+        k, v = (dev(rng.normal(size=(1, Hkv, n, D)).astype(np.float32)) for _ in range(2))
+        rt.kv_append_into(pool, 0, [seq], 1, 1, n, k, v, n)
+        seq.commit(np.zeros(n, np.uint32))
+        rt.synchronize()
+        blocks, head = seq.blocks
+        lanes[i] = (n - 1, 0 if i % 17 == 4 else 1, 0, len(table) - head)
+        table.extend(int(b) for b in blocks)
+        kept.append(seq)
+    tables = dev(np.asarray(table, np.int32))
+    q = rng.normal(size=(batch, Hq, D)).astype(np.float32)
+
+    def attend(first, last, window):
+        part = np.ascontiguousarray(lanes[first:last])
+        out = empty((last - first, Hq, D))
+        most = int(-(-lengths.max() // 16))
+        plan = et.attention_plan(last - first, Hq, Hkv, D, most, sm_count=rt.capabilities()["sm_count"])
+        assert plan["splits"] == 1
+        rt.paged_attention_into(pool, 0, dev(part), tables, last - first, most, dev(q[first:last]), Hq, 0.1, out, None, 0, op_window=window)
+        return host(out)
+
+    parts = batch // 28
+    bounds = [batch * i // parts for i in range(parts + 1)]
+    for window in (None, 40):
+        whole = attend(0, batch, window)
+        for first, last in zip(bounds, bounds[1:]):
+            np.testing.assert_array_equal(whole[first:last].view(np.uint32), attend(first, last, window).view(np.uint32))
