@@ -50,8 +50,8 @@ def build_calls(force: bool = False) -> None:
     if not force and os.path.exists(CALLS) and os.path.getmtime(CALLS) > max(map(os.path.getmtime, (src, header))):
         return
     host_cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
-    subprocess.run([host_cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-I", include, src, "-o", CALLS, LIB, "-Wl,-rpath,$ORIGIN"],
-                   check=True)
+    subprocess.run([host_cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-I", include, src, "-o", CALLS, "-L", HERE, "-l:" + os.path.basename(LIB),
+                    "-Wl,-rpath,$ORIGIN"], check=True)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

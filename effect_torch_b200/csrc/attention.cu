@@ -1,6 +1,6 @@
 // Paged KV kernels for sm_100a: page-pool append (all four tiers), reference-order attention in
-// f64, tensor-core flash-decoding over the block table with split-KV merge, and the fused
-// RoPE + append used by one-token decode steps.
+// f64, tensor-core flash-decoding over the block table with split-KV merge, RoPE and append inside
+// both for a decoder's one-token steps, and as a kernel of their own for chunks.
 //
 // Replaces kv_attention_into of the reference (crates/runtime-cpu/src/napi/mod.rs:3320-3565):
 // the scatter (:3397-3459) and the attend loop (:3461-3542), and the slab tiers of
