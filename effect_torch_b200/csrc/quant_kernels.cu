@@ -141,9 +141,11 @@ cudaError_t launch_qembedding(int codec, const void* indexes, int index_is_i64, 
 //         unrounded f32 d; ties between equal magnitudes keep the first element.
 //   Q8_0: d = absmax / 127 stored as f16; code = clamp(round-half-away(x * (1/d)), -127, 127).
 // HBM-bound on the f32 input once the integer conversions are gone: a code is the low byte of value + 2^23 added with
-// rounding down. A CTA takes 128 blocks, four 16-byte loads per thread in flight; the packed blocks are put together in
+// rounding down. A CTA takes 128 blocks, two 32-byte loads per thread in flight; the packed blocks are put together in
 // shared memory (18 and 34 bytes fit no vector store) and leave as one contiguous 16-byte-wide copy. A warp per block with
-// byte stores took 247 us (Q4_0) and 167 us (Q8_0) on [14336 x 4096] (235 MB in); this takes 51 and 56 us.
+// byte stores took 247 us (Q4_0) and 167 us (Q8_0) on [14336 x 4096] (235 MB in); this takes 49 and 51 us, 394 and 424 us on
+// [128256 x 4096]. With two 16-byte loads per thread, which ask for every sector twice: 51 and 53, 435 and 451 us; they stay
+// for inputs on a 16-byte boundary only.
 // ============================================================================================
 constexpr int kQuantThreads = 256;
 constexpr int kQuantPasses = 2;
@@ -156,6 +158,12 @@ __device__ __forceinline__ uint32_t low_bytes(uint32_t a, uint32_t b, uint32_t c
   return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
 }
 
+// Eight consecutive values from a 32-byte boundary in one request, read once.
+__device__ __forceinline__ void load_eight(const float* src, float (&v)[8]) {
+  asm volatile("ld.global.cs.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(src));
+}
+
 template <int CODEC>
 __global__ void __launch_bounds__(kQuantThreads) quantize_kernel(const float* __restrict__ x, int64_t total_blocks, uint8_t* __restrict__ out) {
   constexpr int BB = CodecTraits<CODEC>::kBytes;
@@ -163,12 +171,16 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_kernel(const float* __
   const int64_t first = blockIdx.x * (int64_t)kQuantBlocks;
   const int blocks = (int)min((int64_t)kQuantBlocks, total_blocks - first);
   const int part = threadIdx.x & 3;
-  const bool wide_in = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const bool wide_in = (reinterpret_cast<uintptr_t>(x) & 15) == 0, widest_in = (reinterpret_cast<uintptr_t>(x) & 31) == 0;
   float v[kQuantPasses][8];
 #pragma unroll
   for (int p = 0; p < kQuantPasses; ++p) {
     const int block = p * (kQuantThreads / 4) + (threadIdx.x >> 2);
     const float* src = x + (first + block) * 32 + part * 8;
+    if (widest_in && block < blocks) {
+      load_eight(src, v[p]);
+      continue;
+    }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       float4 q = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -113,6 +113,18 @@ def test_quantizer_tails(codec, rows, columns):
 
 
 @pytest.mark.parametrize("codec", [orc.Q4_0, orc.Q8_0])
+@pytest.mark.parametrize("shift", [0, 1, 2, 4, 8])
+def test_quantizer_of_inputs_on_any_boundary(codec, shift):
+    """Loads of 32 bytes, of 16 and of single values; the last CTA has three blocks."""
+    w = np.random.default_rng(shift).normal(0, 0.02, size=(43, 288)).astype(np.float32)
+    held = empty((w.size + shift,))
+    held[shift:] = dev(w).reshape(-1)
+    packed = empty((43, orc.encoded_row_bytes(codec, 288)), dtype=torch.uint8)
+    runtime().quantize_into(codec, held[shift:], 43, 288, packed)
+    np.testing.assert_array_equal(host(packed), orc.quantize(codec, w))
+
+
+@pytest.mark.parametrize("codec", [orc.Q4_0, orc.Q8_0])
 def test_quantizer_of_blocks_with_values_that_are_not_finite(codec):
     """A NaN takes no part in its block's scale, wherever it stands; an infinity makes the scale infinite."""
     rng = np.random.default_rng(29)
