@@ -20,10 +20,20 @@ namespace etc {
 // Dequantise: bit-exact with the reference decoders. HBM-bound on the f32 output (4 B written per 0.5-1 B read).
 // Eight threads share a 256-value window (see Runs in codecs.cuh), so headers and 16-byte payload loads are paid once per
 // 32 values; a warp's four windows pass through shared memory because a thread's runs are 64 bytes each and stores that
-// far apart would use half of every sector. One thread per value with byte loads took 170 us on [14336 x 4096] Q4_0 (235 MB
-// out); this takes 44 us, 6.0 TB/s.
+// far apart would use half of every sector. They leave as 32 bytes per thread (outputs on a 16-byte boundary only: 16). Up to 64
+// CTAs per SM, of which some 12 to 16 are resident: a warp waits for its loads before it stores, so what keeps HBM busy is a new
+// CTA beside it, not a long loop. [14336 x 4096] (235 MB out) Q4_0 44 us, Q8_0 48; [128256 x 4096] 378 and 414 us, 0.97 of
+// the copy bandwidth. 16-byte stores and 12 CTAs per SM: 44, 63, 458 and 551 us; 32-byte stores and 12: 47, 53, 393 and 443.
+// One thread per value with byte loads took 170 us on [14336 x 4096] Q4_0.
 // ============================================================================================
 constexpr int kDequantWarps = 4;
+
+// Eight consecutive values to a 32-byte boundary in one request.
+__device__ __forceinline__ void store_eight(float* dst, float4 a, float4 b) {
+  asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x),
+               "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
 
 template <int CODEC, bool WIDE>
 __global__ void __launch_bounds__(kDequantWarps * 32) dequantize_kernel(const uint8_t* __restrict__ packed, int64_t total,
@@ -33,6 +43,7 @@ __global__ void __launch_bounds__(kDequantWarps * 32) dequantize_kernel(const ui
   constexpr int64_t kWindowBytes = 256 / CodecTraits<CODEC>::kValues * CodecTraits<CODEC>::kBytes;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = lane & 7, w = lane >> 3;
   const int64_t groups = (total + 1023) / 1024;  // of four windows: consecutive values, whatever row they belong to
+  const bool widest_out = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
   float4* mine = stage[warp];
   auto place = [](int quad) { return quad ^ ((quad >> 3) & 7); };
   for (int64_t g = blockIdx.x * (int64_t)kDequantWarps + warp; g < groups; g += (int64_t)gridDim.x * kDequantWarps) {
@@ -50,11 +61,20 @@ __global__ void __launch_bounds__(kDequantWarps * 32) dequantize_kernel(const ui
       }
     }
     __syncwarp();
+    if (widest_out) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int q = lane + 32 * j;
-      const int64_t at = g * 1024 + 4 * q;
-      if (at < total) __stcs(reinterpret_cast<float4*>(out + at), mine[place(q)]);
+      for (int j = 0; j < 4; ++j) {
+        const int q = 2 * lane + 64 * j;
+        const int64_t at = g * 1024 + 4 * q;
+        if (at < total) store_eight(out + at, mine[place(q)], mine[place(q + 1)]);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int q = lane + 32 * j;
+        const int64_t at = g * 1024 + 4 * q;
+        if (at < total) __stcs(reinterpret_cast<float4*>(out + at), mine[place(q)]);
+      }
     }
     __syncwarp();
   }
@@ -74,7 +94,7 @@ struct DequantLaunch {
     const int64_t total = rows * columns;
     if (total == 0) { err = cudaSuccess; return; }
     if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) {
-      const int64_t blocks = std::min<int64_t>((total + 1024 * kDequantWarps - 1) / (1024 * kDequantWarps), 148 * 12);
+      const int64_t blocks = std::min<int64_t>((total + 1024 * kDequantWarps - 1) / (1024 * kDequantWarps), 148 * 64);
       if (kWideBlocks<CODEC> && (reinterpret_cast<uintptr_t>(packed) & 15) == 0)
         dequantize_kernel<CODEC, kWideBlocks<CODEC>><<<(unsigned)blocks, kDequantWarps * 32, 0, stream>>>(packed, total, out);
       else

@@ -124,6 +124,20 @@ def test_quantizer_of_inputs_on_any_boundary(codec, shift):
     np.testing.assert_array_equal(host(packed), orc.quantize(codec, w))
 
 
+@pytest.mark.parametrize("codec", [orc.Q4_0, orc.Q8_0, orc.Q4_K, orc.Q6_K])
+@pytest.mark.parametrize("shift", [0, 1, 4, 8])
+@pytest.mark.parametrize("rows", [1, 13])
+def test_dequantize_to_any_boundary(codec, shift, rows):
+    """Stores of 32 bytes, of 16 and of single values; the last warp has one or two of its four windows; nothing beyond the end is written."""
+    columns = 1280 if codec not in (orc.Q4_0, orc.Q8_0) else 1312
+    packed = random_packed(codec, rows, columns, seed=shift)
+    out = empty((rows * columns + shift + 8,))
+    runtime().dequantize_into(codec, dev(packed), rows, columns, out[shift:])
+    got, expected = host(out), orc.dequantize(codec, packed, rows, columns).reshape(-1)
+    np.testing.assert_array_equal(got[shift:shift + expected.size].view(np.uint32), expected.view(np.uint32))
+    assert not got[:shift].any() and not got[shift + expected.size:].any()
+
+
 @pytest.mark.parametrize("codec", [orc.Q4_0, orc.Q8_0])
 def test_quantizer_of_blocks_with_values_that_are_not_finite(codec):
     """A NaN takes no part in its block's scale, wherever it stands; an infinity makes the scale infinite."""
