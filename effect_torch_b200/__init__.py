@@ -11,6 +11,8 @@ from __future__ import annotations
 
 import ctypes as C
 import importlib
+import math
+import operator
 import sys
 import threading
 import weakref
@@ -89,16 +91,24 @@ def _result_buffer(shape) -> np.ndarray:
 
 
 class _ThroughCtypes:
-    """The functions of the extension module (calls.cpp) where it could not be built."""
+    """The functions of the extension module (calls.cpp) where it could not be built. Each parameter takes what it takes there:
+    an address whatever _ptr knows, a whole number anything with __index__ (numpy integers, one-element tensors), a real number
+    anything with __float__."""
+
+    _CONVERT = {_lib.P: _ptr, _lib.D: lambda value: math.ldexp(value, 0)}  # ldexp: as PyFloat_AsDouble, which refuses text
 
     def __getattr__(self, name):
         if name.startswith("_"):
             raise AttributeError(name)
         entry = getattr(_lib.load(), "etc_" + name)
-        extra = (None,) * (len(entry.argtypes) - {"qlinear_into": 9}.get(name, len(entry.argtypes)))  # no cancellation flag
+        convert = [self._CONVERT.get(kind, operator.index) for kind in entry.argtypes]
+        expected = {"qlinear_into": 9}.get(name, len(convert))
+        extra = (None,) * (len(convert) - expected)  # no cancellation flag
 
         def call(*args):
-            return entry(*(a if a is None or isinstance(a, (int, float)) else _ptr(a) for a in args), *extra)
+            if len(args) != expected:
+                raise TypeError(f"expected {expected} arguments, got {len(args)}")
+            return entry(*(to(value) for to, value in zip(convert, args)), *extra)
 
         setattr(self, name, call)
         return call
