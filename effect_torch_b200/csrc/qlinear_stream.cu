@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
       ok = wait_warp(&w_full[w.at], w.parity, abort_flag);
       if (!ok) break;
       const uint32_t stage = (uint32_t)w.at * Cfg::kStageW;
-      uint32_t seen = 0;
+      int hands_back = 0;  // the lane that arrives on w_empty
       auto slot_is_free = [&] {
         ok = behind < 0 || wait_warp(&done[freed.at], freed.parity, abort_flag);
         if (ok) tc_fence_after();
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
         if (!slot_is_free()) break;
         // the products of the stage AS before this one (a whole one), whose slot and accumulators this one takes over
         uint32_t products[GROUP][USED];
-        seen = 0;
+        uint32_t seen = 0;
 #pragma unroll
         for (int b = 0; b < kStageBlocks; ++b) {  // blocks beyond the tile's K hold stale bytes that no MMA reads
           uint32_t regs[16];
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
           }
           expand_codes<CODEC>(payload + stage + b * Cfg::kBlockQ, regs);
           const uint32_t bits = *reinterpret_cast<const unsigned short*>(scales + stage + b * Cfg::kBlockS);
-          seen |= bits;
+          seen ^= bits;
           next_scale[b] = __half2float(__ushort_as_half((unsigned short)bits)) * kCodeUnits;
           tmem_st16(slot_cols + b * 16, regs);
           if (behind >= 0 && b % GROUP == GROUP - 1) {
@@ -227,9 +227,9 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
         for (int b = 0; b < kStageBlocks; ++b) scale[b] = next_scale[b];
         // The scales are used a round later. An arrival on w_empty does not wait for loads whose results nothing has used yet
         // (nor does a fence): the next round's bytes came back as scales, in one step of some fifty where launches overlap
-        // just so. The arrival's address takes the scales in, of which bits 16 and up are zero; a load's results are there
-        // for all lanes of the converged warp or for none.
-        asm volatile("mov.b32 %0, %0;" : "+r"(seen));
+        // just so. Which of two lanes arrives therefore hangs on a bit of every scale that the warp has loaded: the vote has
+        // no result before all of them are in registers, whatever order the instructions are put in.
+        hands_back = __popc(__ballot_sync(0xffffffffu, seen & 1u)) & 1;
       } else {
         uint32_t first[kStageBlocks], second[kStageBlocks];
 #pragma unroll
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) qlinear_stream_kernel(Strea
         if (!ok) break;
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&w_empty[w.at + (seen >> 16)]);
+      if (lane == hands_back) mbar_arrive(&w_empty[w.at]);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();

@@ -534,11 +534,14 @@ def test_decode_steps_that_rotate_and_append_inside_attention(q_heads, kv_heads,
         assert helpers.rel_err(gl, ol) <= 2 * tol, f"step {step}"
 
 
-def test_steps_of_wide_q8_0_layers_repeat_bit_for_bit():
+@pytest.mark.parametrize("codec,B", [(et.Q8_0, 8), (et.Q8_0, 16), (et.Q4_0, 8), (et.Q4_0, 16)])
+def test_steps_of_wide_layers_repeat_bit_for_bit(codec, B):
     """A stage's block scales are used a round after its buffer is handed back to the loader: a load that came back late
-    took the next round's scales (a wrong step in some fifty of this shape). 120 runs of three steps, all alike; the first
-    run, whose split plan is another, does not count."""
-    d, ffn, vocab, B, context = 4096, 14336, 16000, 8, 48
+    took the next round's scales (a wrong step in some fifty of Q8_0 at 8 sequences). Both codecs whose codes go through the
+    tensor cores unscaled, at the forms for up to 8 and up to 16 vectors. 120 runs of three steps, all alike; the first run,
+    whose split plan is another, does not count."""
+    d, ffn, vocab, context = 4096, 14336, 16000, 48
+    block_bytes, scale = (34, 3e-4) if codec == et.Q8_0 else (18, 5e-3)
     gen = torch.Generator(device="cuda")
     gen.manual_seed(3)
     max_tokens = B * (context + 32)
@@ -549,10 +552,10 @@ def test_steps_of_wide_q8_0_layers_repeat_bit_for_bit():
     dec.set_weight(et.W_OUT_NORM, 0, ones)
 
     def put(slot, layer, rows, columns):
-        packed = torch.randint(0, 256, (rows, columns // 32, 34), generator=gen, device="cuda", dtype=torch.uint8)
-        packed[:, :, :2] = torch.rand((rows, columns // 32, 1), generator=gen, device="cuda").mul_(3e-4).half().view(torch.uint8)
+        packed = torch.randint(0, 256, (rows, columns // 32, block_bytes), generator=gen, device="cuda", dtype=torch.uint8)
+        packed[:, :, :2] = torch.rand((rows, columns // 32, 1), generator=gen, device="cuda").mul_(scale).half().view(torch.uint8)
         torch.cuda.synchronize()
-        dec.set_weight(slot, layer, packed.view(rows, -1), codec=et.Q8_0, rows=rows, columns=columns)
+        dec.set_weight(slot, layer, packed.view(rows, -1), codec=codec, rows=rows, columns=columns)
 
     for layer in range(2):
         dec.set_weight(et.W_ATTN_NORM, layer, ones)
