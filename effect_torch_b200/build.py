@@ -17,7 +17,7 @@ import sysconfig
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libetcuda.so")
-CALLS = os.path.join(HERE, "_calls.so")  # the extension module of calls.cpp
+CALLS = os.path.join(HERE, "_calls" + sysconfig.get_config_var("EXT_SUFFIX"))  # the extension module of calls.cpp, for this interpreter
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -42,16 +42,23 @@ def _stale() -> bool:
 
 
 def build_calls(force: bool = False) -> None:
-    """The CPython module that calls the library without ctypes; without the interpreter's headers there is none."""
+    """The CPython module that calls the library without ctypes. Without the interpreter's headers, or where it does not
+    compile, there is none (_ThroughCtypes stands in): no module of an older header stays, and none that any interpreter loads."""
     src, header = os.path.join(HERE, "calls.cpp"), os.path.join(os.path.dirname(HERE), "include", "et_cuda.h")
+    newest = max(map(os.path.getmtime, (src, header)))
+    for module in glob.glob(os.path.join(HERE, "_calls*.so")):
+        if os.path.basename(module) == "_calls.so" or os.path.getmtime(module) <= newest or (force and module == CALLS):
+            os.remove(module)
     include = sysconfig.get_paths()["include"]
-    if not os.path.exists(os.path.join(include, "Python.h")):
-        return
-    if not force and os.path.exists(CALLS) and os.path.getmtime(CALLS) > max(map(os.path.getmtime, (src, header))):
+    if os.path.exists(CALLS) or not os.path.exists(os.path.join(include, "Python.h")):
         return
     host_cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
-    subprocess.run([host_cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-I", include, src, "-o", CALLS, "-L", HERE, "-l:" + os.path.basename(LIB),
-                    "-Wl,-rpath,$ORIGIN"], check=True)
+    command = [host_cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-I", include, src, "-o", CALLS, "-L", HERE,
+               "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN"]
+    try:
+        subprocess.run(command, check=True, stderr=subprocess.PIPE, text=True)
+    except (OSError, subprocess.CalledProcessError) as error:
+        sys.stderr.write(f"--- calls.cpp: no extension module, its operators go through ctypes\n{getattr(error, 'stderr', None) or error}\n")
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

@@ -1,6 +1,8 @@
 """The extension module of the operators called once per layer and its stand-in through ctypes: both convert the same arguments
 and refuse the same ones (no GPU needed: the calls end at the handle check, or in a library that records them)."""
 import importlib
+import os
+import sysconfig
 import types
 
 import numpy as np
@@ -8,7 +10,7 @@ import pytest
 import torch
 
 import effect_torch_b200 as et
-from effect_torch_b200 import _lib
+from effect_torch_b200 import _lib, build
 
 # parameters by operator: p an address, w a whole number, r a real number
 PARAMETERS = {"dequantize_into": "pwpwwp", "quantize_into": "pwpwwp", "qlinear_into": "pwpwwpwpp", "qlinear_tiled_into": "pppwppwppw",
@@ -63,3 +65,47 @@ def test_the_stand_in_hands_over_what_the_arguments_stand_for(name, monkeypatch)
         assert args[:len(kinds)] == tuple(meant[kind] for kind in kinds)
         assert args[len(kinds):] == (None,) * (len(entry.argtypes) - len(kinds))
         assert all(type(a) in (int, float, type(None)) for a in args)
+
+
+def test_the_module_belongs_to_this_interpreter():
+    assert os.path.basename(module().__file__) == "_calls" + sysconfig.get_config_var("EXT_SUFFIX") != "_calls.so"
+
+
+@pytest.fixture
+def tree(tmp_path, monkeypatch):
+    """A source tree with a calls.cpp that needs neither the header nor the library, and an older module of every kind."""
+    here = tmp_path / "package"
+    here.mkdir()
+    (tmp_path / "include").mkdir()
+    lib = here / "libetcuda.so"
+    lib.symlink_to(_lib.LIB_PATH)
+    for path in ("_calls.so", os.path.basename(build.CALLS), "_calls.cpython-311-other.so"):
+        (here / path).write_bytes(b"")
+        os.utime(here / path, (1, 1))
+    (tmp_path / "include" / "et_cuda.h").write_text("")
+    (here / "calls.cpp").write_text("int answer() { return 42; }")
+    for name, value in (("HERE", str(here)), ("LIB", str(lib)), ("CALLS", str(here / os.path.basename(build.CALLS)))):
+        monkeypatch.setattr(build, name, value)
+    return here
+
+
+def modules(tree):
+    return sorted(path.name for path in tree.glob("_calls*.so"))
+
+
+def test_building_the_module_leaves_no_other_one(tree):
+    build.build_calls()
+    assert modules(tree) == [os.path.basename(build.CALLS)]
+    built = os.path.getmtime(build.CALLS)
+    (tree / "_calls.so").write_bytes(b"")
+    build.build_calls()
+    assert modules(tree) == [os.path.basename(build.CALLS)] and os.path.getmtime(build.CALLS) == built
+    os.utime(build.CALLS, (1, 1))  # older than the header
+    build.build_calls()
+    assert os.path.getmtime(build.CALLS) > 1
+
+
+def test_a_module_that_does_not_compile_leaves_the_stand_in(tree, capsys):
+    (tree / "calls.cpp").write_text("int answer( { return 42; }")
+    build.build_calls()
+    assert modules(tree) == [] and "through ctypes" in capsys.readouterr().err
