@@ -92,9 +92,9 @@ def load_into(target, weights):
     put(11, 0, weights["head"])
 
 
-def oracle_decoder(cfg, weights, batch, window=None):
+def oracle_decoder(cfg, weights, batch, window=None, rope_layout=0):
     dec = orc.Decoder(cfg["layers"], cfg["d_model"], cfg["q_heads"], cfg["kv_heads"], cfg["head_dim"], cfg["ffn"], cfg["vocab"],
-                      eps=cfg["rms_eps"], theta=cfg["rope_theta"], window=window, batch=batch)
+                      eps=cfg["rms_eps"], theta=cfg["rope_theta"], window=window, batch=batch, rope_layout=rope_layout)
     load_into(dec, weights)
     dec.set_mode(faithful=False, threads=max(1, min(8, orc.max_threads())))
     return dec

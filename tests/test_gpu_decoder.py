@@ -19,11 +19,11 @@ pytestmark = pytest.mark.gpu
 LOGIT_TOL = 2e-3  # tolerance on logits (max |err| / max |ref|)
 
 
-def gpu_decoder(cfg, weights, batch, max_tokens, block_size=16, kv_dtype=et.KV_F32, exact=True, max_advance=16, window=None):
+def gpu_decoder(cfg, weights, batch, max_tokens, block_size=16, kv_dtype=et.KV_F32, exact=True, max_advance=16, window=None, rope_layout=0):
     dec = et.Executable(runtime(), layers=cfg["layers"], d_model=cfg["d_model"], q_heads=cfg["q_heads"], kv_heads=cfg["kv_heads"],
                         head_dim=cfg["head_dim"], ffn=cfg["ffn"], vocab=cfg["vocab"], rms_eps=cfg["rms_eps"],
                         rope_theta=cfg["rope_theta"], batch=batch, max_tokens=max_tokens, block_size=block_size, kv_dtype=kv_dtype,
-                        exact=exact, max_advance=max_advance, window=window)
+                        exact=exact, max_advance=max_advance, window=window, rope_layout=rope_layout)
     helpers.load_into(dec, weights)
     dec.finalize()
     return dec
@@ -534,6 +534,55 @@ def test_decode_steps_that_rotate_and_append_inside_attention(q_heads, kv_heads,
         assert helpers.rel_err(gl, ol) <= 2 * tol, f"step {step}"
 
 
+@pytest.mark.parametrize("batch,head_dim,kv_dtype,okv,tol,layout,window,longest", [
+    (56, 128, et.KV_F16, orc.F16, LOGIT_TOL, 0, None, 2160), (112, 64, et.KV_BF16, orc.BF16, 2e-2, 1, None, 200),
+    (84, 128, et.KV_U8, orc.U8, 1e-2, 1, None, 200), (64, 128, et.KV_F16, orc.F16, LOGIT_TOL, 1, 40, 200)])
+def test_decode_steps_of_many_lanes_served_by_length(batch, head_dim, kv_dtype, okv, tol, layout, window, longest):
+    """Batches whose lanes go by falling length in the attention that also rotates and appends: ragged and equal lengths, the
+    new token first, last and alone in its page, a lane of more than 128 pages (a warp's second set of page numbers), padded
+    lanes and a window. Tolerances as for the steps above."""
+    kv_heads = 8
+    cfg = dict(helpers.TINY_Q, layers=2, q_heads=kv_heads, kv_heads=kv_heads, head_dim=head_dim, ffn=256, vocab=512)
+    rng = np.random.default_rng(batch)
+    active = batch - 2
+    lengths = rng.integers(1, 40, size=active)
+    lengths[:6], lengths[active // 2], lengths[-1] = (15, 16, 17, 31, 32, 32), longest, 100
+    rows_per_sm = 4 if head_dim == 64 else 3 if kv_dtype == et.KV_U8 else 2
+    sms = runtime().capabilities()["sm_count"]
+    plan = et.attention_plan(batch, kv_heads, kv_heads, head_dim, -(-int(lengths.max() + 4) // 16), sm_count=sms)
+    assert 2 * batch * kv_heads * plan["splits"] >= 3 * rows_per_sm * sms, "lanes go in their own order"
+    w = helpers.make_weights(cfg, seed=6, codec=orc.Q4_0)
+    max_tokens = 16 * int(sum(-(-(n + 4) // 16) for n in lengths) + 2 * batch)
+    odec = orc.Decoder(cfg["layers"], cfg["d_model"], kv_heads, kv_heads, head_dim, cfg["ffn"], cfg["vocab"], eps=cfg["rms_eps"], theta=cfg["rope_theta"],
+                       window=window, batch=batch, rope_layout=layout)
+    helpers.load_into(odec, w)
+    odec.set_mode(faithful=False, threads=max(1, min(8, orc.max_threads())))
+    gdec = et.Executable(runtime(), layers=cfg["layers"], d_model=cfg["d_model"], q_heads=kv_heads, kv_heads=kv_heads, head_dim=head_dim, ffn=cfg["ffn"],
+                         vocab=cfg["vocab"], rms_eps=cfg["rms_eps"], rope_theta=cfg["rope_theta"], batch=batch, max_tokens=max_tokens, block_size=16,
+                         kv_dtype=kv_dtype, exact=False, max_advance=16, window=window, rope_layout=layout)
+    helpers.load_into(gdec, w)
+    gdec.finalize()
+    opool = orc.Pool(cfg["layers"], kv_heads, head_dim, max_tokens, 16, okv)
+    gpool = et.NativeKvPool(runtime(), cfg["layers"], kv_heads, head_dim, max_tokens, 16, kv_dtype)
+    oseqs, gseqs = [opool.make_sequence() for _ in range(active)], [gpool.makeSequence() for _ in range(active)]
+    one = orc.Decoder(cfg["layers"], cfg["d_model"], kv_heads, kv_heads, head_dim, cfg["ffn"], cfg["vocab"], eps=cfg["rms_eps"], theta=cfg["rope_theta"],
+                      window=window, batch=1, rope_layout=layout)  # the oracle computes padded lanes too
+    helpers.load_into(one, w)
+    one.set_mode(faithful=False, threads=max(1, min(8, orc.max_threads())))
+    for first in range(0, longest, 16):  # sixteen tokens of every lane in turn: the lanes' pages mix
+        for lane in range(active):
+            advance = min(16, int(lengths[lane]) - first)
+            if advance > 0:
+                toks = rng.integers(0, cfg["vocab"], size=(1, advance)).astype(np.uint32)
+                one.execute(opool, oseqs[lane:lane + 1], toks, want_logits=False, want_sampled=False)
+                gdec.execute(gpool, gseqs[lane:lane + 1], toks)
+    for step in range(3):
+        toks = rng.integers(0, cfg["vocab"], size=(active, 1)).astype(np.uint32)
+        ol, _ = odec.execute(opool, oseqs, toks)
+        gl = gdec.execute(gpool, gseqs, toks)
+        assert helpers.rel_err(gl, ol) <= 2 * tol, f"step {step}"
+
+
 @pytest.mark.parametrize("codec,B", [(et.Q8_0, 8), (et.Q8_0, 16), (et.Q4_0, 8), (et.Q4_0, 16)])
 def test_steps_of_wide_layers_repeat_bit_for_bit(codec, B):
     """A stage's block scales are used a round after its buffer is handed back to the loader: a load that came back late
@@ -593,17 +642,18 @@ def test_steps_of_wide_layers_repeat_bit_for_bit(codec, B):
 @pytest.mark.parametrize("geometry,batch,window", [
     (dict(d_model=160, q_heads=6, kv_heads=3, head_dim=32, ffn=200, vocab=777), 7, None), (dict(d_model=68, q_heads=3, kv_heads=1, head_dim=20, ffn=36, vocab=33), 1, 7),
     (dict(d_model=256, q_heads=2, kv_heads=2, head_dim=128, ffn=1320, vocab=100), 12, None)])
-def test_f32_steps_with_norm_and_rope_inside_their_neighbours(geometry, batch, window):
+@pytest.mark.parametrize("layout", [et.HALF_SPLIT, et.INTERLEAVED_PAIRS])
+def test_f32_steps_with_norm_and_rope_inside_their_neighbours(geometry, batch, window, layout):
     """Reference-order steps whose norms ride along with the projections and whose attention rotates and appends: widths that
     do not fill tiles, one row, more than eight, a padded lane, an f32 context that grows across pages and one beyond shared
-    memory (the third model: 128 x 2 columns, 290 tokens). Logits as on the tiny model."""
+    memory (the third model: 128 x 2 columns, 290 tokens), in both RoPE layouts. Logits as on the tiny model."""
     cfg = dict(geometry, layers=2, rms_eps=1e-5, rope_theta=10000.0)
     w = helpers.make_weights(cfg, seed=8)
     rng = np.random.default_rng(batch)
     active = max(1, batch - 1)
     max_tokens = batch * 320
-    odec = helpers.oracle_decoder(cfg, w, batch=batch, window=window)
-    gdec = gpu_decoder(cfg, w, batch=batch, max_tokens=max_tokens, max_advance=64, window=window)
+    odec = helpers.oracle_decoder(cfg, w, batch=batch, window=window, rope_layout=layout)
+    gdec = gpu_decoder(cfg, w, batch=batch, max_tokens=max_tokens, max_advance=64, window=window, rope_layout=layout)
     opool = orc.Pool(2, cfg["kv_heads"], cfg["head_dim"], max_tokens, 16, orc.F32)
     gpool = et.NativeKvPool(runtime(), 2, cfg["kv_heads"], cfg["head_dim"], max_tokens, 16, et.KV_F32)
     oseqs, gseqs = [opool.make_sequence() for _ in range(active)], [gpool.makeSequence() for _ in range(active)]
