@@ -1,6 +1,6 @@
 // Programmatic dependent launch for the kernels of a decode step. A kernel launched with launch_chained may be
 // scheduled while its predecessor in the stream is still running (as soon as every CTA of the predecessor has called
-// chain_release or exited), which hides launch latency and CTA ramp-up between the ~260 short kernels of a step. Such a
+// chain_release or exited), which hides launch latency and CTA ramp-up between the some 230 short kernels of a step. Such a
 // kernel calls chain_wait() before its first access to global memory that an earlier kernel writes or still reads:
 // the wait returns once the predecessor has completed and its writes are visible, so the stream's semantics stay
 // those of plain serialisation. Both calls do nothing in a kernel that was launched the ordinary way.

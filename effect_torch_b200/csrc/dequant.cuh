@@ -32,7 +32,7 @@ struct Ring {
 //     weight = code * 2^(p - 24) * (scale * 2^(24 - p)) - offset * scale,
 // in which all products are exact while scale * 2^21 is a finite f16. Larger scales (2^-5 and more) take a second form with
 // the same results. (Splicing codes into the mantissa of 1024, taking 1024 off again and scaling cost 8 FMAs for eight 4-bit
-// codes where this costs 4; a dequant warp had 366 instructions per stage of 128 x 128 weights, now under 300.)
+// codes where this costs 4; a dequant warp had 366 instructions per stage of 128 x 128 weights, now 255.)
 __device__ __forceinline__ uint32_t mul_h2(uint32_t x, uint32_t y) {
   uint32_t d;
   asm("mul.f16x2 %0, %1, %2;" : "=r"(d) : "r"(x), "r"(y));

@@ -21,7 +21,7 @@
 // of (tile, stage) units with the pieces of cut tiles exchanged through memory and a ticket per tile took 10 to 17 us for
 // the exchange on [28672 x 4096] and [4096 x 4096]: a fence, an atomic and a chain of L2 round trips.)
 //
-// Roofline: HBM, rows*K/32*{18,34} bytes. A dequant warp has some 240 instructions per stage of 128 x 128 Q4_0 weights (an FMA
+// Roofline: HBM, rows*K/32*{18,34} bytes. A dequant warp has 255 instructions per stage of 128 x 128 Q4_0 weights (an FMA
 // and a mask per pair, see dequant.cuh); with the loaders and the MMA warp an SM issues 1306 per stage, at 65 % of its slots.
 // [128256 x 4096] x 32, activations ready, with the codes spliced and scaled in two steps and as it is: 547 and 506 cycles per
 // stage (HBM delivers one in 410), 79.1 and 73.3 us; x 64: 90.4 and 85.8; [28672 x 4096] x 32: 26.5 and 24.1. In the form for

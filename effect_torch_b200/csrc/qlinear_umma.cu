@@ -342,8 +342,8 @@ __global__ void repack_umma_kernel(RepackParts parts, int codec, int64_t rows, i
       }
     } else if (codec == 11) {
       // Q3_K (quantized.rs:142-176): block `sub` of the 256-value block is groups 2*sub and 2*sub+1 of 16 values,
-      // value = d*(scale6 - 32)*(low2 - (high bit clear ? 4 : 0)); stored as int8 codes with one f16 scale per group, the
-      // layout of the re-cut Q6_K
+      // value = d*(scale6 - 32)*(low2 - (high bit clear ? 4 : 0)); stored as byte codes (plus 128) with one f16 scale per
+      // group, the layout of the re-cut Q6_K
       const uint8_t* blk = src_row + (kb >> 3) * bb;
       const int sub = (int)(kb & 7), half = sub >> 2, lane = sub & 3;
       const uint8_t* packed = blk + 96;
@@ -411,7 +411,7 @@ __global__ void repack_umma_kernel(RepackParts parts, int codec, int64_t rows, i
       const uint8_t* blk = src_row + kb * bb;
       scale = __ushort_as_half((unsigned short)(blk[0] | (blk[1] << 8)));
       if (codec == 2) {
-          for (int w = 0; w < 4; ++w) {
+        for (int w = 0; w < 4; ++w) {
           uint32_t word = 0;
           for (int j = 0; j < 8; ++j) {
             const int i = 8 * w + j;
