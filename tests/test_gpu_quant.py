@@ -17,16 +17,33 @@ SCALE_FIELDS = {gv.Q4_0: [0], gv.Q8_0: [0], gv.Q2_K: [80, 82], gv.Q3_K: [108], g
 REL_TOL = 2e-3  # tolerance on f16/f32 linear outputs, as max |err| / max |ref|
 
 
-def random_packed(codec, rows, columns, seed):
+def random_packed(codec, rows, columns, seed, spread=0.01):
     """Random packed bytes with finite f16 scale fields (every bit pattern of the code bytes is legal)."""
     rng = np.random.default_rng(seed)
     bb, bv = orc.block_bytes(codec), orc.block_values(codec)
     blocks = rows * columns // bv
     raw = rng.integers(0, 256, size=(blocks, bb), dtype=np.uint8)
     for off in SCALE_FIELDS[codec]:
-        scale = rng.normal(0, 0.01, size=blocks).astype(np.float16)
+        scale = rng.normal(0, spread, size=blocks).astype(np.float16)
         raw[:, off:off + 2] = scale.view(np.uint8).reshape(blocks, 2)
     return raw.reshape(rows, columns // bv * bb)
+
+
+# Block scales of K-quants as files have them (weights near 0.01), and as random_packed draws them: effective scales below and
+# from 2^-5 on, the line between the two forms of the expansion to f16.
+K_SPREADS = ["model", "wide"]
+
+
+def k_packed(codec, rows, columns, seed, spread):
+    return random_packed(codec, rows, columns, seed, helpers.K_SCALE_SIGMA[codec] / 2 if spread == "model" else 0.01)
+
+
+def whole_warps_below_the_line(scales, blocks):
+    """scales [rows, 32-value blocks (, scales per block)] -> for each dequant warp (32 rows) and run of `blocks` blocks that it
+    expands together, whether all of its scales are below 2^-5."""
+    rows, total = scales.shape[:2]
+    runs = np.abs(scales.astype(np.float64)).reshape(rows // 32, 32, total // blocks, -1)
+    return runs.max(axis=(1, 3)) < 2.0 ** -5
 
 
 @pytest.mark.parametrize("codec", [gv.Q2_K, gv.Q3_K, gv.Q4_K, gv.Q5_K, gv.Q6_K])
@@ -219,11 +236,18 @@ def test_expansion_is_exact_for_every_code_and_scale(codec, vectors):
     scales = np.array([line, np.nextafter(np.float16(line), np.float16(0)), line * 1.5, 0.006, 6e-8, 6.1e-5, 0.0, 1.0, 200.0], np.float16)
     scales = np.concatenate([scales, -scales])
     rng = np.random.default_rng(5)
-    rows = 8 * len(scales)
+    # a warp (32 rows) of each scale, then three with scales below the line mixed and three with all of them mixed
+    mixed = 3 * 32
+    rows = 32 * len(scales) + 2 * mixed
     raw = rng.integers(0, 256, size=(rows, columns // 32, bb), dtype=np.uint8)
-    # most rows hold one scale (whole warps take one form), the last ones a mix
-    raw[:, :, 0:2] = np.repeat(scales, 8)[:, None, None].view(np.uint8).reshape(rows, 1, 2)
-    raw[-40:, :, 0:2] = rng.choice(scales, size=(40, columns // 32, 1)).view(np.uint8)
+    held = np.empty((rows, columns // 32), np.float16)
+    held[:-2 * mixed] = np.repeat(scales, 32)[:, None]
+    held[-2 * mixed:-mixed] = rng.choice(scales[np.abs(scales) < line], size=(mixed, columns // 32))
+    held[-mixed:] = rng.choice(scales, size=(mixed, columns // 32))
+    raw[:, :, 0:2] = held[:, :, None].view(np.uint8).reshape(rows, columns // 32, 2)
+    for blocks in (2, 4):  # that a warp of the two linears expands together
+        small = whole_warps_below_the_line(held, blocks).all(axis=1)
+        assert [int(small[:9].sum()), int(small[9:18].sum())] == [5, 5] and small[1] and small[18:21].all() and not small[21:].any()
     packed = raw.reshape(rows, -1)
     expected = orc.dequantize(codec, packed, rows, columns).astype(np.float16).astype(np.float32)
     qw = et.QWeight(runtime(), codec, [dev(packed)], [rows], columns)
@@ -316,12 +340,69 @@ def test_single_split_launch_with_more_tiles_than_sms(codec, ffn, d, vectors):
     np.testing.assert_array_equal(runs[0], runs[1])
 
 
+def recut(codec, packed, rows, columns):
+    """The re-cut form of K-quant rows, from what the oracle decodes of them with their fields replaced: f16 scales
+    [rows, 32-value blocks, 1 or 2] (two where each half of a block has its own), f16 minima or None, and f64 codes [rows, columns]."""
+    blocks = packed.reshape(-1, orc.block_bytes(codec))
+
+    def decode(d, dmin, code_bytes=()):
+        changed = blocks.copy()
+        for off, value in zip(SCALE_FIELDS[codec], (d, dmin)):
+            changed[:, off:off + 2] = np.array([value], np.float16).view(np.uint8)
+        for first, last, value in code_bytes:
+            changed[:, first:last] = value
+        return orc.dequantize(codec, changed.reshape(rows, -1), rows, columns)
+
+    def field(off):  # of each 256-value block, as f32, repeated over its 32-value blocks
+        return np.repeat(np.ascontiguousarray(blocks[:, off:off + 2]).view(np.float16).astype(np.float32).reshape(rows, -1), 8, axis=1)
+
+    ones = {gv.Q3_K: [(0, 32, 0xff), (32, 96, 0x55)], gv.Q4_K: [(16, 144, 0x11)], gv.Q5_K: [(16, 48, 0), (48, 176, 0x11)],
+            gv.Q6_K: [(0, 128, 0x11), (128, 192, 0xaa)]}[codec]  # every code 1
+    per_value = decode(1.0, 0.0, ones)  # the whole-number sub-scales
+    minimum = codec in (gv.Q4_K, gv.Q5_K)
+    sub = per_value.reshape(rows, columns // 32, 32)[:, :, ::32 if minimum else 16]
+    scales = (field(SCALE_FIELDS[codec][0])[:, :, None] * sub).astype(np.float16)
+    minima = None
+    if minimum:
+        zeros = [(16, 144, 0)] if codec == gv.Q4_K else [(16, 176, 0)]
+        minima = (field(2) * -decode(0.0, 1.0, zeros).reshape(rows, columns // 32, 32)[:, :, 0]).astype(np.float16)
+    codes = np.divide(decode(1.0, 0.0), per_value, out=np.zeros((rows, columns)), where=per_value != 0, dtype=np.float64)
+    return scales, minima, codes
+
+
 @pytest.mark.parametrize("codec", [gv.Q3_K, gv.Q4_K, gv.Q5_K, gv.Q6_K])
-def test_k_quant_tiling_preserves_every_weight(codec):
+@pytest.mark.parametrize("spread", K_SPREADS)
+@pytest.mark.parametrize("vectors", [32, 128, 512])
+def test_k_quant_expansion_rounds_once(codec, spread, vectors):
+    """Both forms of the expansion give a re-cut weight as scale * code (- minimum) of its f16 scales, rounded once to f16: at
+    the scales of model files (whole warps below the line between the forms) and beyond it. x picks out single weights."""
+    rows, columns = 128, 512
+    packed = k_packed(codec, rows, columns, 17, spread)
+    scales, minima, codes = recut(codec, packed, rows, columns)
+    assert np.array_equal(codes, np.rint(codes)) and np.ptp(codes) == {gv.Q3_K: 7, gv.Q4_K: 15, gv.Q5_K: 31, gv.Q6_K: 63}[codec]
+    for blocks in (2, 4):
+        small = whole_warps_below_the_line(scales, blocks)
+        assert small.all() if spread == "model" else not small.all()
+    weights = np.repeat(scales.astype(np.float64), 32 // scales.shape[2], axis=2).reshape(rows, columns) * codes
+    if minima is not None:
+        weights -= np.repeat(minima.astype(np.float64), 32, axis=1)
+    expected = weights.astype(np.float16).astype(np.float32)
+    qw = et.QWeight(runtime(), codec, [dev(packed)], [rows], columns)
+    x = np.zeros((vectors, columns), np.float32)
+    picked = np.sort(np.random.default_rng(1).permutation(columns)[:vectors])
+    x[np.arange(vectors), picked] = 1.0
+    out = empty((vectors, rows))
+    qw.linear_into(dev(x), vectors, out)
+    np.testing.assert_array_equal(host(out).T, expected[:, picked])
+
+
+@pytest.mark.parametrize("codec", [gv.Q3_K, gv.Q4_K, gv.Q5_K, gv.Q6_K])
+@pytest.mark.parametrize("spread", K_SPREADS)
+def test_k_quant_tiling_preserves_every_weight(codec, spread):
     """The 256-value K-quant blocks are re-cut into 32-value blocks at load (effective scales rounded to f16): x = identity
     picks out single weights, which must equal the reference decode to the f16 precision of the MMA operands."""
     rows, columns = 40, 512
-    packed = random_packed(codec, rows, columns, seed=11)
+    packed = k_packed(codec, rows, columns, 11, spread)
     deq = orc.dequantize(codec, packed, rows, columns)
     qw = et.QWeight(runtime(), codec, [dev(packed)], [rows], columns)
     out = empty((columns, rows))
@@ -333,9 +414,10 @@ def test_k_quant_tiling_preserves_every_weight(codec):
 @pytest.mark.parametrize("codec", [gv.Q3_K, gv.Q4_K, gv.Q5_K, gv.Q6_K])
 @pytest.mark.parametrize("rows,columns", [(256, 512), (200, 1024), (1024, 4096)])
 @pytest.mark.parametrize("vectors", [1, 8, 17, 32, 64, 300])
-def test_k_quant_tiled_linear_matches_the_oracle(codec, rows, columns, vectors):
+@pytest.mark.parametrize("spread", K_SPREADS)
+def test_k_quant_tiled_linear_matches_the_oracle(codec, rows, columns, vectors, spread):
     rng = np.random.default_rng(rows + columns + vectors)
-    packed = random_packed(codec, rows, columns, seed=rows + vectors)
+    packed = k_packed(codec, rows, columns, rows + vectors, spread)
     x = rng.normal(size=(vectors, columns)).astype(np.float32)
     qw = et.QWeight(runtime(), codec, [dev(packed)], [rows], columns)
     out = empty((vectors, rows))
@@ -345,10 +427,11 @@ def test_k_quant_tiled_linear_matches_the_oracle(codec, rows, columns, vectors):
 
 
 @pytest.mark.parametrize("codec", [gv.Q3_K, gv.Q4_K, gv.Q5_K, gv.Q6_K])
-def test_k_quant_fused_gate_up_and_residual_epilogues(codec):
+@pytest.mark.parametrize("spread", K_SPREADS)
+def test_k_quant_fused_gate_up_and_residual_epilogues(codec, spread):
     rng = np.random.default_rng(21)
     d, ffn, vectors = 512, 256, 20
-    pg, pu, pd = random_packed(codec, ffn, d, 1), random_packed(codec, ffn, d, 2), random_packed(codec, d, ffn, 3)
+    pg, pu, pd = k_packed(codec, ffn, d, 1, spread), k_packed(codec, ffn, d, 2, spread), k_packed(codec, d, ffn, 3, spread)
     x = rng.normal(size=(vectors, d)).astype(np.float32)
     residual = rng.normal(size=(vectors, d)).astype(np.float32)
     rt = runtime()
