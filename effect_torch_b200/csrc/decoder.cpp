@@ -232,14 +232,16 @@ void add_norm(DenseArgs& a, const BoundWeight* norm, double eps) {
   a.norm_eps = eps;
 }
 
-// The norm ahead of a dense projection is computed inside it where few rows meet a narrow weight: x is the residual stream then.
+// The norm ahead of a dense launch of these weights is computed inside it: x is the residual stream then.
 bool norm_rides(const StepContext& s, int64_t rows, const BoundWeight& norm, std::initializer_list<const BoundWeight*> weights) {
   etc_decoder* d = s.dec;
   if (d->tiled) return false;
+  int64_t tiles = 0;
+  for (const BoundWeight* w : weights) tiles += (w->rows + 31) / 32;
   for (const BoundWeight* w : weights) {
     DenseArgs a = dense_args(d->hidden, rows, *w);
     a.norm_weight = (const float*)norm.d_raw;
-    if (w->codec != ETC_CODEC_F32 || !dense_narrow_supported(a)) return false;
+    if (w->codec != ETC_CODEC_F32 || !dense_norm_rides(a, tiles, d->rt->sm_count)) return false;
   }
   return true;
 }

@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(256) dense_linear_kernel(DenseArgs a) {
 // rows in shared memory, fetched before the wait for the kernel ahead, so that only the input rows, the chain itself and the
 // store are left behind it. A warp carries ROWS input rows. (In the ring above eight warps read the same tile, 10 cycles of
 // shared-memory path per k where the chain needs four, with a barrier per 64 columns: 4 rows in a step's chain took 9 us for
-// k = 688 and 4.1 for 256, now 3.8 and 2.2.) The norm ahead of the projection may come along: every CTA computes
-// it for its own copy of the rows, with the sums of rmsnorm_rows_kernel, instead of a launch of 2 us.
+// k = 688 and 4.1 for 256, now 3.8 and 2.2.) The norm ahead of the projection may come along where that pays (dense_norm_rides): every
+// CTA computes it for its own copy of the rows, with the sums of rmsnorm_rows_kernel, instead of a launch.
 // With SWIGLU lanes 0 to 15 hold gate rows and lanes 16 to 31 their up rows.
 constexpr int kNarrowThreads = 128, kNarrowRows = 16;
 constexpr size_t kNarrowSmem = 220 * 1024;
@@ -295,6 +295,14 @@ static cudaError_t launch_dense_t(const DenseArgs& a, cudaStream_t stream) {
 
 bool dense_narrow_supported(const DenseArgs& a) {
   return dense_linear_supported(a) && a.m <= kNarrowRows && narrow_smem(a) <= kNarrowSmem && ((uintptr_t)a.norm_weight % 16) == 0;
+}
+
+// The norm inside saves a launch, of which the chain hides all but a few tenths of a microsecond, and costs every CTA its rows' sums
+// one after the other. It pays with a row per warp, two 16-byte loads per lane and row, and one CTA per SM. Steps of four layers, inside
+// and as launches: 256 columns x 1 row 74.2 and 75.8 us, x 4 82.4 and 82.9; beyond the line 256 x 5 102 and 97, x 16 158 and
+// 127, 512 x 1 115.5 and 114.3, 512 x 8 197 and 170, 1280 x 8 (128256 outputs) 1143 and 638.
+bool dense_norm_rides(const DenseArgs& a, int64_t tiles, int sm_count) {
+  return dense_narrow_supported(a) && a.m <= 4 && a.k <= 256 && tiles <= sm_count;
 }
 
 template <bool SWIGLU>

@@ -178,10 +178,11 @@ struct DenseArgs {
   const float* residual = nullptr;  // parts == 1 only
   int swiglu = 0, exact = 0;
   int constant_weights = 0;         // no earlier kernel of the stream writes the weights: they are fetched ahead of it
-  const float* norm_weight = nullptr;  // x goes through RMSNorm on the way; only where dense_narrow_supported
+  const float* norm_weight = nullptr;  // x goes through RMSNorm on the way; only where dense_norm_rides
   double norm_eps = 0.0;
 };
 bool dense_narrow_supported(const DenseArgs& a);  // few rows, 32 weight rows and all inputs in shared memory
+bool dense_norm_rides(const DenseArgs& a, int64_t tiles, int sm_count);  // of a launch with that many tiles of 32 weight rows
 bool dense_linear_supported(const DenseArgs& a);  // k a multiple of 4, 16-byte aligned operands
 cudaError_t launch_dense_linear(const DenseArgs& a, cudaStream_t stream);
 cudaError_t launch_linear_f32(const float* x, int64_t m, int64_t k, const float* w, int64_t n, const float* bias,

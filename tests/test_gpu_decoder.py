@@ -640,12 +640,13 @@ def test_steps_of_wide_layers_repeat_bit_for_bit(codec, B):
 
 
 @pytest.mark.parametrize("geometry,batch,window", [
-    (dict(d_model=160, q_heads=6, kv_heads=3, head_dim=32, ffn=200, vocab=777), 7, None), (dict(d_model=68, q_heads=3, kv_heads=1, head_dim=20, ffn=36, vocab=33), 1, 7),
+    (dict(d_model=160, q_heads=6, kv_heads=3, head_dim=32, ffn=200, vocab=777), 7, None), (dict(d_model=160, q_heads=6, kv_heads=3, head_dim=32, ffn=200, vocab=777), 4, None),
+    (dict(d_model=68, q_heads=3, kv_heads=1, head_dim=20, ffn=36, vocab=33), 1, 7),
     (dict(d_model=256, q_heads=2, kv_heads=2, head_dim=128, ffn=1320, vocab=100), 12, None)])
 @pytest.mark.parametrize("layout", [et.HALF_SPLIT, et.INTERLEAVED_PAIRS])
 def test_f32_steps_with_norm_and_rope_inside_their_neighbours(geometry, batch, window, layout):
     """Reference-order steps whose norms ride along with the projections and whose attention rotates and appends: widths that
-    do not fill tiles, one row, more than eight, a padded lane, an f32 context that grows across pages and one beyond shared
+    do not fill tiles, one row, four, more than eight (with the norms as launches), a padded lane, an f32 context that grows across pages and one beyond shared
     memory (the third model: 128 x 2 columns, 290 tokens), in both RoPE layouts. Logits as on the tiny model."""
     cfg = dict(geometry, layers=2, rms_eps=1e-5, rope_theta=10000.0)
     w = helpers.make_weights(cfg, seed=8)
@@ -662,6 +663,27 @@ def test_f32_steps_with_norm_and_rope_inside_their_neighbours(geometry, batch, w
         ol, _ = odec.execute(opool, oseqs, toks)
         gl = gdec.execute(gpool, gseqs, toks)
         assert helpers.rel_err(gl, ol) <= 1e-5, f"advance {advance}"
+
+
+def launches_of_a_step(cfg, batch, context=1):
+    """Launches of one f32 step of `batch` sequences of `context` tokens."""
+    dec = gpu_decoder(cfg, helpers.make_weights(cfg, seed=2), batch=batch, max_tokens=batch * 16 * (context // 16 + 2), max_advance=64)
+    pool = et.NativeKvPool(runtime(), cfg["layers"], cfg["kv_heads"], cfg["head_dim"], batch * 16 * (context // 16 + 2), 16, et.KV_F32)
+    seqs = [pool.makeSequence() for _ in range(batch)]
+    for first in range(0, context - 1, 64):
+        dec.executeSampled(pool, seqs, np.zeros((batch, min(64, context - 1 - first)), np.uint32))
+    dec.executeSampled(pool, seqs, np.zeros((batch, 1), np.uint32))
+    return dec.diagnostics()["launches_per_step"]
+
+
+@pytest.mark.parametrize("change,batch,apart", [
+    ({}, 4, 0), ({}, 5, 5), (dict(d_model=260), 1, 5), (dict(vocab=32 * 149), 1, 1), (dict(ffn=16 * 149), 4, 2)])
+def test_norms_ride_where_they_cost_less_than_a_launch(change, batch, apart):
+    """A norm inside its projection is repeated by every CTA: up to four rows of up to 256 columns and a CTA per SM at most."""
+    if runtime().capabilities()["sm_count"] != 148:
+        pytest.skip("sizes for 148 SMs")
+    small = {**helpers.TINY, "layers": 2, "vocab": 2048}
+    assert launches_of_a_step({**small, **change}, batch) == launches_of_a_step(small, 1) + apart
 
 
 @pytest.mark.parametrize("d_model", [1088, 4160, 8192])
