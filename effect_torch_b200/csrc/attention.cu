@@ -375,9 +375,17 @@ __global__ void __launch_bounds__(128) attention_exact_step_kernel(PoolView pool
   }
 }
 
-bool attention_exact_step_supported(const PoolView& pool, int q_heads, int max_ctx) {
-  return pool.dtype == kKvF32 && pool.kv_heads > 0 && q_heads % pool.kv_heads == 0 && pool.head_dim % 4 == 0 &&
-         exact_step_smem(pool.head_dim, max_ctx) <= kExactStepSmem;
+// Many lanes of long contexts leave one or two CTAs to an SM, which wait for their rows wave after wave; from some number of CTAs
+// per SM on the two launches, which read the rows where they are, are as fast or faster. Whole steps of four layers, one launch and
+// two, by CTAs per SM: 64 columns, one CTA at a time 7 610 and 673 us, 14 969 and 990, 21 1292 and 1243, 28 1602 and 1549 (two
+// at a time: 28 1159 and 1456); 32 columns 14 1431 and 1417, 21 1997 and 1871; 128 columns, one at a time 10 1178 and
+// 1301, 14 1398 and 1316, 28 2441 and 2180; two at a time 10 815 and 987, 14 1157 and 1013, 28 1497 and 1471.
+bool attention_exact_step_supported(const PoolView& pool, int batch, int q_heads, int max_ctx, int sm_count) {
+  const size_t smem = exact_step_smem(pool.head_dim, max_ctx);
+  if (pool.dtype != kKvF32 || pool.kv_heads <= 0 || q_heads % pool.kv_heads != 0 || pool.head_dim % 4 != 0 || smem > kExactStepSmem) return false;
+  const int at_once = (int)(kSmSharedBytes / (smem + kCtaSharedReserve));
+  const int64_t ctas = (int64_t)batch * q_heads;
+  return pool.head_dim >= 128 ? at_once > 2 || ctas <= 12ll * sm_count : at_once > 1 || ctas <= 16ll * sm_count;
 }
 
 cudaError_t launch_attention_exact_step(const PoolView& pool, const float* qkv, const LaneInfo* lanes, const int* tables, const double* inv_freq, int layout,

@@ -44,6 +44,9 @@ inline cudaError_t launch_chained(void (*kernel)(KernelArgs...), dim3 grid, dim3
   return launch_chained_cluster(kernel, grid, block, smem, stream, 1, std::forward<Args>(args)...);
 }
 
+// Shared memory of an SM, and what every resident CTA takes of it besides its own.
+constexpr size_t kSmSharedBytes = 228 * 1024, kCtaSharedReserve = 1024;
+
 // Opts a kernel in to `bytes` of dynamic shared memory once per (kernel, device): the attribute belongs to the function
 // on a device, so a process that drives several GPUs has to set it on each. Thread-safe.
 template <typename Kernel>

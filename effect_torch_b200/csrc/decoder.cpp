@@ -397,7 +397,7 @@ etc_status enqueue_step(StepContext& s) {
       ETC_TRY(project_qkv_raw(s, li, rides_attn ? d->hidden : d->normed, rows, qkvw, rides_attn ? &d->attn_norm[li] : nullptr));
     // one token per lane: the attention kernel rotates and appends on its way in
     const bool fused_rope = fast_attention && T == 1;
-    const bool exact_step = !fast_attention && T == 1 && qkv_sum.splits == 0 && attention_exact_step_supported(view, Hq, s.max_ctx);
+    const bool exact_step = !fast_attention && T == 1 && qkv_sum.splits == 0 && attention_exact_step_supported(view, B, Hq, s.max_ctx, d->rt->sm_count);
     const FusedRope rope = {d->qkv, qkv_sum, d->d_inv_freq, c.rope_layout};
     if (!fused_rope && !exact_step) {
       ETC_CUDA(launch_rope_append(view, d->qkv, d->d_lanes, d->d_tables, d->d_inv_freq, c.rope_layout, B, Hq, d->qr, stream, &qkv_sum, T));

@@ -259,7 +259,7 @@ cudaError_t launch_attention_mma(const PoolView& pool, const float* q, const Lan
                                  __half* out_xh = nullptr, int xh_nv = 32, int tokens = 1, const FusedRope* rope = nullptr);
 // RoPE, append and reference-order attention of a decode step (f32 cache, contexts of at most max_ctx in shared memory). As with
 // FusedRope, all it reads but qkv must have been written before the launches of this step.
-bool attention_exact_step_supported(const PoolView& pool, int q_heads, int max_ctx);
+bool attention_exact_step_supported(const PoolView& pool, int batch, int q_heads, int max_ctx, int sm_count);
 cudaError_t launch_attention_exact_step(const PoolView& pool, const float* qkv, const LaneInfo* lanes, const int* tables, const double* inv_freq, int layout,
                                         int batch, int q_heads, double scale, long long op_window, float* out, int max_ctx, cudaStream_t stream);
 // Fused RoPE(q), RoPE(k) and KV append: qkv [B * tokens, (Hq+2*Hkv)*D] f32 (the fused projection output) ->

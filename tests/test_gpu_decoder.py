@@ -686,6 +686,16 @@ def test_norms_ride_where_they_cost_less_than_a_launch(change, batch, apart):
     assert launches_of_a_step({**small, **change}, batch) == launches_of_a_step(small, 1) + apart
 
 
+@pytest.mark.parametrize("head_dim,q_heads,context,batch", [(64, 32, 224, 74), (128, 16, 100, 111)])
+def test_attention_of_many_f32_lanes_takes_two_launches(head_dim, q_heads, context, batch):
+    """Where an SM holds one or two CTAs of the attention step that also rotates and appends, and has more than sixteen (128
+    columns: twelve) to run, RoPE and attention are launches of their own; the last batch below the line and the first beyond."""
+    if runtime().capabilities()["sm_count"] != 148:
+        pytest.skip("sizes for 148 SMs")
+    cfg = dict(helpers.TINY, layers=2, d_model=64, q_heads=q_heads, kv_heads=4, head_dim=head_dim, ffn=64, vocab=64)
+    assert launches_of_a_step(cfg, batch + 1, context) == launches_of_a_step(cfg, batch, context) + 2
+
+
 @pytest.mark.parametrize("d_model", [1088, 4160, 8192])
 def test_norms_at_the_edges_of_their_row_widths(d_model):
     """Residual widths that end inside a cluster's share, just above the width of the narrower form and at the limit, for
