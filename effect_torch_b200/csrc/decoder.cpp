@@ -215,8 +215,9 @@ struct StepContext {
 };
 
 // A dense weight of the decoder as (the first) weight of a dense launch.
-DenseArgs dense_args(const float* x, int64_t rows, const BoundWeight& w) {
+DenseArgs dense_args(const etc_decoder* d, const float* x, int64_t rows, const BoundWeight& w) {
   DenseArgs a;
+  a.sm_count = d->rt->sm_count;
   a.x = x;
   a.m = rows;
   a.k = w.columns;
@@ -239,9 +240,9 @@ bool norm_rides(const StepContext& s, int64_t rows, const BoundWeight& norm, std
   int64_t tiles = 0;
   for (const BoundWeight* w : weights) tiles += (w->rows + 31) / 32;
   for (const BoundWeight* w : weights) {
-    DenseArgs a = dense_args(d->hidden, rows, *w);
+    DenseArgs a = dense_args(d, d->hidden, rows, *w);
     a.norm_weight = (const float*)norm.d_raw;
-    if (w->codec != ETC_CODEC_F32 || !dense_norm_rides(a, tiles, d->rt->sm_count)) return false;
+    if (w->codec != ETC_CODEC_F32 || !dense_norm_rides(a, tiles)) return false;
   }
   return true;
 }
@@ -253,7 +254,7 @@ etc_status project_qkv_raw(StepContext& s, size_t layer, const float* x, int64_t
   const BoundWeight* w[3] = {&d->wq[layer], &d->wk[layer], &d->wv[layer]};
   float* out[3] = {d->qkv, d->qkv + w[0]->rows, d->qkv + w[0]->rows + w[1]->rows};
   if (w[0]->codec == ETC_CODEC_F32 && w[1]->codec == ETC_CODEC_F32 && w[2]->codec == ETC_CODEC_F32) {
-    DenseArgs a = dense_args(x, rows, *w[0]);
+    DenseArgs a = dense_args(d, x, rows, *w[0]);
     add_norm(a, norm, d->cfg.rms_eps);
     a.parts = 3;
     a.out_stride = stride;
@@ -268,7 +269,7 @@ etc_status project_qkv_raw(StepContext& s, size_t layer, const float* x, int64_t
   }
   for (int p = 0; p < 3; ++p) {
     if (w[p]->codec == ETC_CODEC_F32) {
-      DenseArgs a = dense_args(x, rows, *w[p]);
+      DenseArgs a = dense_args(d, x, rows, *w[p]);
       a.out[0] = out[p];
       a.out_stride = stride;
       ETC_CUDA(launch_dense_linear(a, stream));
@@ -294,7 +295,7 @@ etc_status run_linear(StepContext& s, const BoundWeight& raw, etc_qweight* tiled
     return ETC_OK;
   }
   if (raw.codec == ETC_CODEC_F32) {
-    DenseArgs dense = dense_args(x, vectors, raw);
+    DenseArgs dense = dense_args(d, x, vectors, raw);
     dense.out[0] = out;
     dense.out_stride = raw.rows;
     add_norm(dense, norm, d->cfg.rms_eps);
@@ -431,7 +432,7 @@ etc_status enqueue_step(StepContext& s) {
     if (d->tiled) {
       ETC_TRY(run_linear(s, d->gate[li], d->t_gu[li], d->normed, rows, xh ? nullptr : d->act, ETC_EPILOGUE_SWIGLU, nullptr,
                          xh ? d->xh_norm : nullptr, xh ? d->xh_act : nullptr));
-    } else if (DenseArgs ffn = dense_args(rides_ffn ? d->hidden : d->normed, rows, d->gate[li]);
+    } else if (DenseArgs ffn = dense_args(d, rides_ffn ? d->hidden : d->normed, rows, d->gate[li]);
                d->gate[li].codec == ETC_CODEC_F32 && d->up[li].codec == ETC_CODEC_F32 && dense_linear_supported(ffn)) {
       ffn.w[1] = (const float*)d->up[li].d_raw;
       ffn.out[0] = d->act;

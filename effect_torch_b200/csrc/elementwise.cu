@@ -293,16 +293,29 @@ static cudaError_t launch_dense_t(const DenseArgs& a, cudaStream_t stream) {
   return launch_chained(kernel, dim3(tiles, (unsigned)((a.m + 8 * MT - 1) / (8 * MT))), dim3(256), smem, stream, a);
 }
 
+static unsigned narrow_tiles(const DenseArgs& a) {
+  unsigned tiles = 0;
+  for (int p = 0; p < (a.swiglu ? 1 : a.parts); ++p) tiles += (unsigned)((a.n[p] + (a.swiglu ? 15 : 31)) / (a.swiglu ? 16 : 32));
+  return tiles;
+}
+// Five to eight rows fill the ring's CTAs, whose copies overlap its chains; here one CTA to an SM loads and then computes, and after
+// some waves of that the ring is ahead. [n x k] x rows, this kernel and the ring: [40000 x 728] x 8 57.9 and 50.7 us, [65536 x 800] x 7
+// 92.7 and 84.4, [128256 x 1024] x 8 220 and 207; x 5 [65536 x 1024] 110 and 114, [128256 x 800] 177 and 165. Up to four rows
+// and from nine on, where the ring's rows are not full or are read twice, this kernel is 1.15 to 5 times as fast at every width.
+static bool ring_is_faster(const DenseArgs& a) {
+  const bool alone = 2 * (narrow_smem(a) + kCtaSharedReserve) > kSmSharedBytes;
+  return !a.swiglu && alone && a.m > 4 && a.m <= 8 && narrow_tiles(a) > (a.m <= 6 ? 16u : 8u) * (unsigned)a.sm_count;
+}
 bool dense_narrow_supported(const DenseArgs& a) {
-  return dense_linear_supported(a) && a.m <= kNarrowRows && narrow_smem(a) <= kNarrowSmem && ((uintptr_t)a.norm_weight % 16) == 0;
+  return dense_linear_supported(a) && a.m <= kNarrowRows && narrow_smem(a) <= kNarrowSmem && ((uintptr_t)a.norm_weight % 16) == 0 && !ring_is_faster(a);
 }
 
 // The norm inside saves a launch, of which the chain hides all but a few tenths of a microsecond, and costs every CTA its rows' sums
 // one after the other. It pays with a row per warp, two 16-byte loads per lane and row, and one CTA per SM. Steps of four layers, inside
 // and as launches: 256 columns x 1 row 74.2 and 75.8 us, x 4 82.4 and 82.9; beyond the line 256 x 5 102 and 97, x 16 158 and
 // 127, 512 x 1 115.5 and 114.3, 512 x 8 197 and 170, 1280 x 8 (128256 outputs) 1143 and 638.
-bool dense_norm_rides(const DenseArgs& a, int64_t tiles, int sm_count) {
-  return dense_narrow_supported(a) && a.m <= 4 && a.k <= 256 && tiles <= sm_count;
+bool dense_norm_rides(const DenseArgs& a, int64_t tiles) {
+  return dense_narrow_supported(a) && a.m <= 4 && a.k <= 256 && tiles <= a.sm_count;
 }
 
 template <bool SWIGLU>
@@ -312,9 +325,7 @@ static cudaError_t launch_narrow(const DenseArgs& a, cudaStream_t stream) {
   auto kernel = a.m <= 4 ? dense_narrow_kernel<1, SWIGLU> : a.m <= 8 ? dense_narrow_kernel<2, SWIGLU> : dense_narrow_kernel<4, SWIGLU>;
   const cudaError_t attr = opt_in_shared_memory(kernel, kNarrowSmem);
   if (attr != cudaSuccess) return attr;
-  unsigned tiles = 0;
-  for (int p = 0; p < (SWIGLU ? 1 : a.parts); ++p) tiles += (unsigned)((a.n[p] + (SWIGLU ? 15 : 31)) / (SWIGLU ? 16 : 32));
-  return launch_chained(kernel, dim3(tiles), dim3(kNarrowThreads), narrow_smem(a), stream, a);
+  return launch_chained(kernel, dim3(narrow_tiles(a)), dim3(kNarrowThreads), narrow_smem(a), stream, a);
 }
 
 cudaError_t launch_dense_linear(const DenseArgs& a, cudaStream_t stream) {
@@ -334,8 +345,9 @@ cudaError_t launch_dense_linear(const DenseArgs& a, cudaStream_t stream) {
 }
 
 cudaError_t launch_linear_f32(const float* x, int64_t m, int64_t k, const float* w, int64_t n, const float* bias,
-                              float* out, cudaStream_t stream) {
+                              float* out, int sm_count, cudaStream_t stream) {
   DenseArgs a;
+  a.sm_count = sm_count;
   a.x = x; a.m = m; a.k = k; a.w[0] = w; a.n[0] = n; a.out[0] = out; a.out_stride = n; a.bias = bias;
   return launch_dense_linear(a, stream);
 }

@@ -180,13 +180,14 @@ struct DenseArgs {
   int constant_weights = 0;         // no earlier kernel of the stream writes the weights: they are fetched ahead of it
   const float* norm_weight = nullptr;  // x goes through RMSNorm on the way; only where dense_norm_rides
   double norm_eps = 0.0;
+  int sm_count = 1;
 };
-bool dense_narrow_supported(const DenseArgs& a);  // few rows, 32 weight rows and all inputs in shared memory
-bool dense_norm_rides(const DenseArgs& a, int64_t tiles, int sm_count);  // of a launch with that many tiles of 32 weight rows
+bool dense_narrow_supported(const DenseArgs& a);  // few rows, 32 weight rows and all inputs in shared memory, and faster than the ring
+bool dense_norm_rides(const DenseArgs& a, int64_t tiles);  // of a launch with that many tiles of 32 weight rows
 bool dense_linear_supported(const DenseArgs& a);  // k a multiple of 4, 16-byte aligned operands
 cudaError_t launch_dense_linear(const DenseArgs& a, cudaStream_t stream);
 cudaError_t launch_linear_f32(const float* x, int64_t m, int64_t k, const float* w, int64_t n, const float* bias,
-                              float* out, cudaStream_t stream);
+                              float* out, int sm_count, cudaStream_t stream);
 cudaError_t launch_rmsnorm(const float* x, const float* weight, double eps, int64_t rows, int64_t n, float* out,
                            cudaStream_t stream);
 cudaError_t launch_rope(const float* x, const int64_t* offsets, int64_t n_offsets, const double* inv_freq, int layout,

@@ -327,7 +327,7 @@ etc_status etc_qembedding_into(etc_runtime* rt, etc_codec codec, const void* d_i
 etc_status etc_linear_f32_into(etc_runtime* rt, const float* d_x, int64_t m, int64_t k, const float* d_w, int64_t n,
                                const float* d_bias, float* d_out) {
   ETC_TRY(activate(rt));
-  ETC_CUDA(launch_linear_f32(d_x, m, k, d_w, n, d_bias, d_out, rt->stream));
+  ETC_CUDA(launch_linear_f32(d_x, m, k, d_w, n, d_bias, d_out, rt->sm_count, rt->stream));
   rt->launches++;
   return ETC_OK;
 }

@@ -88,10 +88,12 @@ def test_argmax_large_rows_and_non_finite_logits():
 
 
 @pytest.mark.parametrize("m,k,n", [(1, 4, 1), (16, 64, 33), (17, 68, 31), (33, 260, 65), (5, 192, 640), (3, 66, 40),
-                                   (2, 1500, 33), (4, 1024, 32), (8, 1536, 48), (9, 28, 40), (16, 688, 70), (4, 1700, 33)])
+                                   (2, 1500, 33), (4, 1024, 32), (8, 1536, 48), (9, 28, 40), (16, 688, 70), (4, 1700, 33),
+                                   (8, 728, 32 * 8 * 148), (8, 728, 32 * 8 * 148 + 1), (7, 764, 37901), (6, 800, 32 * 16 * 148 + 5), (5, 1024, 32 * 16 * 148)])
 def test_dense_linear_at_the_edges_of_its_tiles(m, k, n):
     """Stages that are not full, rows and columns that do not fill a tile, both row counts per CTA, and a k that 16-byte copies
-    cannot fetch: every element one fused multiply-add chain over k, bit for bit."""
+    cannot fetch; five to eight rows on weights up to and beyond the width from which on the ring serves them: every element
+    one fused multiply-add chain over k, bit for bit."""
     rng = np.random.default_rng(m + k + n)
     x, w = rng.normal(size=(m, k)).astype(np.float32), rng.normal(size=(n, k)).astype(np.float32)
     out = empty((m, n))
