@@ -285,9 +285,12 @@ cudaError_t launch_quantize(int codec, const float* x, int64_t rows, int64_t col
 // The activations are staged in the order the threads ask for them (the run layout is the codec's), once per CTA when
 // they fit in kRawStageBytes, else in chunks of columns.
 //
-// What bounds it: instruction issue; a decoded weight costs about 2.3 instructions (byte splice, bias, FMA), each vector half
-// an FMA and 1 / (4 RG) of a shared-memory load (which takes four cycles of the SM's one load path: RG = 4 keeps that below the
-// FMAs). Two CTAs per SM share the rows evenly. One warp per row that decoded value by value took 204 us on Q4_K
+// What bounds it: latency. On Q4_K [14336 x 4096] with 5 vectors (the form for 6) 18.8 million warp instructions are issued, 10 per
+// weight of a warp, which is 36 % of the schedulers' slots: 128 registers and the staged activations leave four warps to a scheduler, of
+// which 3.2 are there on average (3584 row groups are 12.1 per CTA for eight warps, so that half of them idle in the second
+// round), and the wait for a window's payload, requested when it is used, is the largest of their stalls (31 %). Of the issued
+// ones each vector takes half an FMA per weight and 1 / (4 RG) of a shared-memory load (four cycles of the SM's one load path: RG = 4
+// keeps that below the FMAs). Two CTAs per SM share the rows evenly. One warp per row that decoded value by value took 204 us on Q4_K
 // [14336 x 4096] with 5 vectors (5 us of HBM); this takes 42 us, 20 with one vector.
 // ============================================================================================
 constexpr int kRawWarps = 8;
