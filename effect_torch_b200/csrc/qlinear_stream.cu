@@ -523,19 +523,19 @@ StreamPlan plan_stream(const TiledWeight& w, int64_t vectors, int sm_count, bool
     const int splits = std::min(std::max(1, sms * (p.nv <= 64 ? 2 : 1) / p.tiles), std::max(1, p.stages / 2));
     p.stages_per_split = (p.stages + splits - 1) / splits;
   } else {
-    // In stages: those of the fullest SM less what its CTAs expand ahead of the activations (one and a half each), more for a
-    // CTA that has an SM for itself (nothing overlaps its waits; the exact form's are longer), and a cluster's exchange, which
-    // grows with the vectors. Clusters are powers of two (three or six CTAs pack a GPC badly) and are used while all of them are
-    // resident at once, or nearly ([128256 x 4096] takes 73 us with one CTA per tile, 96 with two); from four CTAs on seven
-    // eighths of the places can be filled, beyond that a second wave follows. Measured back to back over 4 to 144 tiles, 8 to
-    // 112 stages, 1 to 100 vectors; against a rule that did not count the work done ahead: [4096 x 4096] x 1 7.9 -> 6.8 us,
-    // [2048 x 4096] x 8 8.6 -> 7.3, [9216 x 14336] x 24 30.6 -> 23.2, [4096 x 4096] x 100 13.8 both.
-    const double single = exact ? 1.5 : 1.1, exchange = p.nv <= 32 ? 1.0 : p.nv == 64 ? 2.25 : 2.5;
+    // In stages: those of the fullest SM less what its CTAs expand ahead of the activations (one and a half each), a third more
+    // for a CTA that has an SM for itself (nothing overlaps its waits), and a cluster's exchange, which grows with the vectors.
+    // Clusters are powers of two (three or six CTAs pack a GPC badly) and are used while all of them are resident at once
+    // ([128256 x 4096] takes 73 us with one CTA per tile, 96 with two); those of four and more fill seven eighths of the places at
+    // most, and a second wave costs more than they give ([9216 x 1024] x 1 to 32 in fours 8.9 to 11.4 us, in pairs 5.3 to 7.3).
+    // Every choice was measured back to back over 2 to 224 tiles, 4 to 224 stages, 1 to 100 vectors and four codecs: this rule's
+    // is 0.9 % from the best on average (with a floor of half a stage and a wave more instead 1.8, without the work done ahead 5.5).
+    const double exchange = p.nv <= 16 ? 0.75 : p.nv == 32 ? 2.0 : p.nv == 64 ? 2.25 : 3.5;
     double best = 1e30;
     for (int s = 1, log = 0; s <= std::min(kMaxStreamCluster, std::max(1, p.stages / 2)) && (s == 1 || p.tiles * s <= 2 * sms); s *= 2, ++log) {
+      if (s >= 4 && p.tiles * s > 2 * sms * 7 / 8) break;
       const int per = (p.stages + s - 1) / s, ctas = (p.tiles * s + sms - 1) / sms;
-      const int waves = s >= 4 && p.tiles * s > 2 * sms * 7 / 8 ? ctas + 1 : ctas;
-      const double cost = waves * std::max(per - 1.5, 0.5) * (waves > 1 ? 1.0 : single) + log * exchange;
+      const double cost = ctas * std::max(per - 1.5, 1.0) * (ctas > 1 ? 1.0 : 1.33) + log * exchange + (s > 1 && ctas > 1 ? 0.5 : 0.0);
       if (cost < best) { best = cost; p.stages_per_split = per; }
     }
   }
