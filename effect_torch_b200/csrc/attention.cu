@@ -1298,10 +1298,14 @@ cudaError_t launch_attention_mma(const PoolView& pool, const float* q, const Lan
     constexpr bool BF16 = decltype(bf16)::value, U8 = decltype(u8)::value;
     if (tokens > 1) return launch_attention_chunk_t<D, BF16, U8>(args, batch, stream);
     // Longest lanes first from half as many CTAs again as an SM holds at once (by shared memory and registers: two of f16 pages of
-    // 128 columns, three of bytes, four of 64 columns); finding a CTA's lane costs a microsecond, more than it gives below
-    // (320 CTAs of 500 to 600 tokens 25.8 -> 27.6 us).
+    // 128 columns, three of bytes, four of 64 columns), where a CTA has up to 32 pages and more for each such round: finding its
+    // lane costs every CTA some two microseconds. Without and with it, lanes of equal length and of 3 to 100 % of the longest (8 heads
+    // of 128 columns, f16): 64 lanes (1.7 rounds) of 500 tokens 29.7 and 32.2 us, 18.8 and 19.0, of 1000 47.8 and 50.0, 32.5
+    // and 31.4, of 4096 159 and 162, 96 and 86; 128 lanes (3.5) of 500 54.7 and 61.3, 34.3 and 42.9, of 2000 161 and
+    // 168, 97.6 and 101, with one lane in ten long 61.6 and 53.0, of 4096 312 and 320, 187 and 181, 98.5 and 75.6.
     constexpr int kAtOnce = D == 64 ? 4 : U8 ? 3 : 2;
-    const bool sorted = batch <= kMaxSortedLanes && 2ll * batch * pool.kv_heads * plan.splits >= 3ll * kAtOnce * plan.sm_count;
+    const int64_t ctas = (int64_t)batch * pool.kv_heads * plan.splits, places = (int64_t)kAtOnce * plan.sm_count;
+    const bool sorted = batch <= kMaxSortedLanes && 2 * ctas >= 3 * places && plan.pages_per_split * places >= 32 * ctas;
     auto decode = [&](auto fused, auto longest_first) {
       return launch_attention_mma_t<D, BF16, U8, decltype(fused)::value, decltype(longest_first)::value>(pool, args, batch, plan.splits, stream);
     };
