@@ -166,9 +166,10 @@ def test_device_sampling_at_the_edges_of_its_slices_and_lists(vocab):
 
 
 @pytest.mark.parametrize("vocab", [1025, 8200, 100003])
-@pytest.mark.parametrize("top_k", [1, 31, 255, 256, 257, 1023, 1024])
+@pytest.mark.parametrize("top_k", [1, 31, 85, 86, 200, 201, 255, 256, 257, 1023, 1024])
 def test_top_k_lists_at_the_edges_of_their_sorts(vocab, top_k):
-    """List lengths around what is sorted by counting and what the list holds; a row of ties, one whose largest candidates all
+    """List lengths around what is sorted by counting, what the threads' largest candidates are counted for (200, or a
+    third of the smallest row's 256 threads) and what the list holds; a row of ties, one whose largest candidates all
     sit with one thread (so that its neighbours' largest reach far down), one with fewer candidates above the floor than
     top_k; slices that do not start on 16 bytes."""
     rt = runtime()
